@@ -211,6 +211,10 @@ __device__ __forceinline__ void tc_wait(uint64_t * bar, unsigned parity, volatil
         }
     }
 }
+// Whether the CTA has given up, the same answer for all the lanes of mask. Another warp may set the flag between two lanes' reads: a
+// warp that leaves a loop with warp-wide operations in it leaves it by this vote (lanes that disagreed would wait for each other, some
+// at such an operation, the others at the kernel's last barrier, and neither wait is bounded).
+__device__ __forceinline__ bool gave_up(unsigned mask, const volatile WaitCtl * wc) { return __any_sync(mask, wc->dead != 0) != 0; }
 
 // ---- tcgen05 ----
 // Shared-memory matrix descriptors (no swizzle, version 1), as their 32-bit halves: the low half holds the start address and the
@@ -427,7 +431,8 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
     unsigned rseq = lane;        // this lane's tile in the sequence of all tiles of all side-groups
     unsigned issued = 0xffffffu; // the lane's last three copies as bytes (slot << 1 | phase parity), 0xff: none
     int G = 0x7fffffff;
-    for (int nk = 0, nv = 0; nv < G && !sm.wc.dead;) {
+    bool dead = false;
+    for (int nk = 0, nv = 0; nv < G;) {
         const bool isK = nk < G && nk < nv + NSB;
         TileSrc t;
         int nt;
@@ -470,17 +475,17 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
             nt = sm.tasks[nv % NTASK].nt;
             if (lane < nt) t = sm.vsrc[nv % NTASK][lane];
         }
+        const int rs = rseq % NRAW;
+        const unsigned round = rseq / NRAW;
+        if (lane < GT && round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
+        dead = gave_up(FULL_MASK, &sm.wc);
+        if (dead) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
         if (lane < GT) {
-            const int rs = rseq % NRAW;
-            const unsigned round = rseq / NRAW;
-            if (round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
-            if (!sm.wc.dead) { // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
-                if (lane < nt) {
-                    issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[rs], &sm.raw_full[rs]);
-                    issued = (issued << 8) | ((unsigned) rs << 1) | (round & 1u);
-                } else {
-                    mbar_arrive(&sm.raw_full[rs]);
-                }
+            if (lane < nt) {
+                issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[rs], &sm.raw_full[rs]);
+                issued = (issued << 8) | ((unsigned) rs << 1) | (round & 1u);
+            } else {
+                mbar_arrive(&sm.raw_full[rs]);
             }
             rseq += GT;
         }
@@ -490,7 +495,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
     }
     // a CTA whose waits gave up reaches this point with copies possibly in flight: they must land before the CTA's shared memory is
     // released (bounded; in a normal run every copy was waited for by its consumer long ago)
-    if (sm.wc.dead && lane < GT)
+    if (dead && lane < GT)
         for (int j = 0; j < 3; j++) {
             const unsigned e = (issued >> (8 * j)) & 0xffu;
             if (e == 0xffu) continue;
@@ -583,7 +588,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             const SideSrc ksrc = make_src(kv, 0, g, ws), vsrc = make_src(kv, 1, g, ws);
             unsigned rseq = lane; // this lane's tile in the sequence of all tiles of all side-groups
             unsigned issued = 0xffffffu; // the lane's last three copies as bytes (slot << 1 | phase parity), 0xff: none
-            for (int nk = 0, nv = 0; nv < G && !sm.wc.dead;) {
+            bool dead = false;
+            for (int nk = 0, nv = 0; nv < G;) {
                 const bool isK = nk < G && nk < nv + NSB;
                 Task k;
                 if (isK) { // a group's K comes first: its task is computed here, once, and left for the other roles (the waits on
@@ -598,7 +604,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 const int rs = rseq % NRAW;
                 const unsigned round = rseq / NRAW;
                 if (round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
-                if (sm.wc.dead) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
+                dead = gave_up(0xfu, &sm.wc);
+                if (dead) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
                 if (lane < k.nt) {
                     issue_tile(S, k.pos0 + lane * ATP, k.c1, sm.raw[rs], &sm.raw_full[rs]);
                     issued = (issued << 8) | ((unsigned) rs << 1) | (round & 1u);
@@ -611,9 +618,9 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             }
             // a CTA whose waits gave up reaches this point with copies possibly in flight: they must land before the CTA's shared
             // memory is released (bounded; in a normal run every copy was waited for by its consumer long ago)
-            if (sm.wc.dead && lane == 0) // (the query block too)
+            if (dead && lane == 0) // (the query block too)
                 for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.q_ready, 0u, 1000u); it++) {}
-            if (sm.wc.dead)
+            if (dead)
                 for (int j = 0; j < 3; j++) {
                     const unsigned e = (issued >> (8 * j)) & 0xffu;
                     if (e == 0xffu) continue;
@@ -717,12 +724,13 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         const bool st = w == 0;
         int rs = q, rph = 0, os = 0, oph = 0; // raw slot / phase of this warp's tile, operand slot / phase
         bool owrap = false;
-        for (int nk = 0, nv = 0; nv < G && !sm.wc.dead;) {
+        for (int nk = 0, nv = 0; nv < G;) {
             const bool isK = nk < G && nk < nv + NSB;
             const int side = isK ? 0 : 1, grp = isK ? nk - NSB : nv;
             (void) grp; // (the stamps' group index)
             if (st) TC_STAMP(grp, side ? 8 : 11);
             tc_wait(&sm.raw_full[rs], rph, &sm.wc, a.status);
+            if (gave_up(FULL_MASK, &sm.wc)) break;
             if (st) TC_STAMP(grp, side ? 9 : 12);
             const GroupRec & kr = sm.tasks[(isK ? nk : nv) % NTASK];
             if (batch && isK && (kr.flags & REC_END)) G = nk + 1;
