@@ -216,6 +216,19 @@ __device__ __forceinline__ void tc_wait(uint64_t * bar, unsigned parity, volatil
 // at such an operation, the others at the kernel's last barrier, and neither wait is bounded).
 __device__ __forceinline__ bool gave_up(unsigned mask, const volatile WaitCtl * wc) { return __any_sync(mask, wc->dead != 0) != 0; }
 
+// The last copies of a producer lane, newest first, as bytes (slot << 1 | phase parity; 0xff: nothing was copied for that slot's turn):
+// they must land before the CTA's shared memory is released, also when a consumer gives up after the producer has fetched everything
+// and left its loop. Only the last turn of each of the lane's slots can be in flight (the one before it was waited for before the slot
+// was filled again). Bounded; in a normal run the producer has nothing else to do and every copy lands.
+constexpr unsigned NO_COPY = 0xffu;
+__device__ __forceinline__ void drain_copies(uint64_t * raw_full, unsigned issued, int slots) {
+    for (int j = 0; j < slots; j++) {
+        const unsigned e = (issued >> (8 * j)) & 0xffu;
+        if (e == NO_COPY) continue;
+        for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&raw_full[e >> 1], e & 1u, 1000u); it++) {}
+    }
+}
+
 // ---- tcgen05 ----
 // Shared-memory matrix descriptors (no swizzle, version 1), as their 32-bit halves: the low half holds the start address and the
 // byte distance between the two 8-element groups along K of one instruction ("leading"), the high half the distance between 8-row
@@ -429,9 +442,8 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         return t;
     };
     unsigned rseq = lane;        // this lane's tile in the sequence of all tiles of all side-groups
-    unsigned issued = 0xffffffu; // the lane's last three copies as bytes (slot << 1 | phase parity), 0xff: none
+    unsigned issued = ~0u;       // the lane's last copies (drain_copies)
     int G = 0x7fffffff;
-    bool dead = false;
     for (int nk = 0, nv = 0; nv < G;) {
         const bool isK = nk < G && nk < nv + NSB;
         TileSrc t;
@@ -478,29 +490,18 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         const int rs = rseq % NRAW;
         const unsigned round = rseq / NRAW;
         if (lane < GT && round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
-        dead = gave_up(FULL_MASK, &sm.wc);
-        if (dead) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
+        if (gave_up(FULL_MASK, &sm.wc)) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
         if (lane < GT) {
-            if (lane < nt) {
-                issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[rs], &sm.raw_full[rs]);
-                issued = (issued << 8) | ((unsigned) rs << 1) | (round & 1u);
-            } else {
-                mbar_arrive(&sm.raw_full[rs]);
-            }
+            if (lane < nt) issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[rs], &sm.raw_full[rs]);
+            else mbar_arrive(&sm.raw_full[rs]);
+            issued = (issued << 8) | (lane < nt ? ((unsigned) rs << 1) | (round & 1u) : NO_COPY);
             rseq += GT;
         }
         __syncwarp();
         if (isK) nk++;
         else nv++;
     }
-    // a CTA whose waits gave up reaches this point with copies possibly in flight: they must land before the CTA's shared memory is
-    // released (bounded; in a normal run every copy was waited for by its consumer long ago)
-    if (dead && lane < GT)
-        for (int j = 0; j < 3; j++) {
-            const unsigned e = (issued >> (8 * j)) & 0xffu;
-            if (e == 0xffu) continue;
-            for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.raw_full[e >> 1], e & 1u, 1000u); it++) {}
-        }
+    if (lane < GT) drain_copies(sm.raw_full, issued, NRAW / GT);
 }
 
 // KB / VB: the bits of the K / V main rows the instance is compiled for (0: any, decided per tile at run time). A compiled-in
@@ -587,8 +588,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         if (lane < GT) {
             const SideSrc ksrc = make_src(kv, 0, g, ws), vsrc = make_src(kv, 1, g, ws);
             unsigned rseq = lane; // this lane's tile in the sequence of all tiles of all side-groups
-            unsigned issued = 0xffffffu; // the lane's last three copies as bytes (slot << 1 | phase parity), 0xff: none
-            bool dead = false;
+            unsigned issued = ~0u; // the lane's last copies (drain_copies)
             for (int nk = 0, nv = 0; nv < G;) {
                 const bool isK = nk < G && nk < nv + NSB;
                 Task k;
@@ -604,28 +604,17 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 const int rs = rseq % NRAW;
                 const unsigned round = rseq / NRAW;
                 if (round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
-                dead = gave_up(0xfu, &sm.wc);
-                if (dead) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
-                if (lane < k.nt) {
-                    issue_tile(S, k.pos0 + lane * ATP, k.c1, sm.raw[rs], &sm.raw_full[rs]);
-                    issued = (issued << 8) | ((unsigned) rs << 1) | (round & 1u);
-                } else {
-                    mbar_arrive(&sm.raw_full[rs]);
-                }
+                if (gave_up(0xfu, &sm.wc)) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
+                if (lane < k.nt) issue_tile(S, k.pos0 + lane * ATP, k.c1, sm.raw[rs], &sm.raw_full[rs]);
+                else mbar_arrive(&sm.raw_full[rs]);
+                issued = (issued << 8) | (lane < k.nt ? ((unsigned) rs << 1) | (round & 1u) : NO_COPY);
                 rseq += GT;
                 if (isK) nk++;
                 else nv++;
             }
-            // a CTA whose waits gave up reaches this point with copies possibly in flight: they must land before the CTA's shared
-            // memory is released (bounded; in a normal run every copy was waited for by its consumer long ago)
-            if (dead && lane == 0) // (the query block too)
+            if (lane == 0) // (the query block too: the issuer may give up on it)
                 for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.q_ready, 0u, 1000u); it++) {}
-            if (dead)
-                for (int j = 0; j < 3; j++) {
-                    const unsigned e = (issued >> (8 * j)) & 0xffu;
-                    if (e == 0xffu) continue;
-                    for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.raw_full[e >> 1], e & 1u, 1000u); it++) {}
-                }
+            drain_copies(sm.raw_full, issued, NRAW / GT);
         }
         }
     } else if (warp == W_ISSUE) {

@@ -41,6 +41,74 @@ def test_expired_wait_returns_error_and_engine_stays_usable(mk, torch_cuda, monk
     eng.close()
 
 
+# (layers, positions, entry): the kernel's batch instance with more items than CTAs, with one or two groups per CTA (the producer has
+# fetched everything before anyone waits) and behind every entry that takes it; last, the spread instance with one group per CTA
+@pytest.mark.parametrize("entry,layers,n,T", [("step_layers", 16, 3000, 3), ("step_layers", 3, 70, 1), ("step_layers_partial", 16, 3000, 3), ("step_batch", 1, 3000, 4),
+                                              ("attend", 1, 70, 8), ("attend", 1, 2000, 8), ("attend_static", 1, 30, 1), ("attend_static", 1, 3000, 8), ("attend", 1, 2590, 8)])
+def test_expired_wait_in_every_mode(mk, torch_cuda, monkeypatch, entry, layers, n, T):
+    torch = torch_cuda
+    monkeypatch.setenv("MK_KV_ATTN", "tc")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    rows = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    seqs = [0, 1, 2] if entry == "step_batch" else [mk.engine.SEQ_MAIN]
+    ns = [300, 1500, n] if entry == "step_batch" else [n]
+    eng = mk.Engine(layers, n + 64, "K*=5r,V*=6", 2048)
+    if entry == "step_batch":
+        eng.slots_open(3, n + 64)
+        eng.reserve_batch(3)
+    K, V = rows(layers, n, 4, 256), rows(layers, n, 4, 256)
+    Kt, Vt, Q = (rows(layers, len(ns) * T, h, 256) for h in (4, 4, 24))
+
+    def fill():
+        for s, m in zip(seqs, ns):
+            for l in range(layers):
+                eng.append(l, 0, K[l, :m], V[l, :m], seq=s)
+                if entry in ("attend", "attend_static"):
+                    eng.append(l, m, Kt[l], Vt[l], seq=s)
+        eng.sync()
+
+    def call():
+        O = torch.zeros((layers, len(ns) * T, 24, 256), dtype=torch.float32, device="cuda")
+        if entry == "step_layers":
+            eng.step_layers(n, Kt, Vt, Q, O)
+        elif entry == "step_layers_partial":
+            ml = torch.zeros((layers, 4, 48, 2), dtype=torch.float32, device="cuda")
+            O = torch.zeros((layers, 4, 48, 256), dtype=torch.float32, device="cuda")
+            eng.step_layers_partial(n, Kt, Vt, Q, 0, n + T, 0, n + T, O, ml)
+        elif entry == "step_batch":
+            eng.step_batch(seqs, 0, ns, [T] * 3, Kt[0], Vt[0], Q[0], O[0])
+        elif entry == "attend":
+            eng.attend(0, n, Q[0], O[0])
+        else:
+            eng.attend_static(0, n, Q[0], O[0])
+        return O
+
+    fill()
+    good = call()
+    eng.sync()
+    # first every wait that does not succeed at once gives up; then short limits, with which a launch gives up somewhere or not at all
+    for limits in (None, (20, 2, 2), (20, 20, 20), (20, 100, 100)):
+        try:
+            eng.wait_limits(*limits) if limits else eng.wait_limits_expire_now()
+            O = call()
+            try:
+                eng.sync()
+                gave_up = False
+            except mk.EngineError as e:
+                assert "gave up waiting" in str(e)
+                gave_up = True
+        finally:
+            eng.wait_limits()
+        assert gave_up or limits
+        if gave_up:  # (mk_kv_sync reset the engine)
+            fill()
+            O = call()
+            eng.sync()
+        assert torch.equal(O, good), (entry, limits, gave_up)
+    eng.close()
+
+
 def test_split_sequence_refuses_whole_sequence_calls(mk, torch_cuda):
     torch = torch_cuda
     eng = mk.Engine(1, 4096, "K*=5r,V*=6", 2048)
