@@ -89,9 +89,12 @@ constexpr int Q_BYTES = AR * HD * 2, P_BYTES = AR * GP * 2;
 constexpr unsigned S_COL = 0, S_STRIDE = 64, O_COL0 = NSB * 64, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512; // an O^T half: 48 columns for P's high part, 48 for its low part
 static_assert(O_COL1 + 2 * AR <= TMEM_COLS, "tensor-memory columns");
 static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
-// The accumulator's reference max of a row is set REF_MARGIN above the running max it is taken from and moves when the running max
-// passes it by more than REF_SLACK: exp(running - reference) stays within [e^-3 for the row's largest terms, e^10.5 < fp16 max].
-constexpr float REF_SLACK = 10.5f, REF_MARGIN = 3.f;
+// The accumulator's reference max of a row is set REF_BELOW below the running max it is taken from and moves when the running max
+// passes it by more than REF_SLACK: beta = exp(running - reference) of the row's largest terms stays within [e^2, e^11 < fp16 max].
+// P beta is held as two fp16 parts, whose step is 2^-24 for small products: e^-2 2^-24 of the row's largest term, below P's own
+// rounding. (With the reference 3 above the running max the parts of weights under e^-7 were subnormal: rows with one position 14 above
+// the others came out 2e-6 .. 7e-6 off 64 bits, relative 2-norm, where P's rounding gives 3e-7; now 2e-7 .. 6e-7.)
+constexpr float REF_SLACK = 11.f, REF_BELOW = 2.f;
 constexpr float LOG2E = 1.4426950408889634f;
 
 struct WaitCtl { // the launch's wait limits and the CTA's give-up flag
@@ -930,10 +933,10 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 if (alive && !batch && q == 0 && k.nb > 1 && k.b + 3 < k.nb) __stcg(a.xb + xb0 + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(M));
                 carry = M;
                 if (M != -CUDART_INF_F) {
-                    if (m_acc == -CUDART_INF_F) m_acc = M + REF_MARGIN;
+                    if (m_acc == -CUDART_INF_F) m_acc = M - REF_BELOW;
                     else if (M > m_acc + REF_SLACK) {
-                        f = exp_any(m_acc - (M + REF_MARGIN));
-                        m_acc = M + REF_MARGIN;
+                        f = exp_any(m_acc - (M - REF_BELOW));
+                        m_acc = M - REF_BELOW;
                     }
                 }
                 beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);

@@ -1,0 +1,53 @@
+"""Rows whose softmax puts nearly all weight on one position (14 above the others): the many weights of e^-14 must come out as the
+reference's fp16 P leaves them, not coarser. Oracle and kernel round the same P, so what is left between them is the order of fp32
+sums: a partial here is at most two 128-position groups = 16 tensor-core steps, each of which may drop one unit in the last place
+(2^-23) of the accumulator that holds the large term; the sums of the weights add less than that. Bound: 2-norm of the difference
+at most 16 x 2^-23 = 1.9e-6 of the result's (products kept against a reference 3 above the maximum were 4e-6 .. 7e-6 off)."""
+import numpy as np
+import pytest
+
+import kv_oracle as ko
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("spec,win", [("", 0), ("K*=6,V*=5", 2048)])
+@pytest.mark.parametrize("n,T", [(1016, 8), (2000, 3), (5003, 4)])
+def test_small_weights_keep_their_precision(mk, torch_cuda, spec, win, n, T):
+    torch = torch_cuda
+    layers = 2
+    rng = np.random.default_rng([n, T])
+    u = np.sign(rng.standard_normal((4, 256)))
+    K = (0.25 * rng.standard_normal((layers, n + T, 4, 256))).astype(np.float16)
+    V = rng.standard_normal((layers, n + T, 4, 256)).astype(np.float16)
+    K[:, 2 * n // 5] = (u * (14 / 16)).astype(np.float16)  # q . k / 16 = 14 there, N(0, 0.25) elsewhere
+    Q = (np.repeat(u, 6, axis=0) + 0.05 * rng.standard_normal((layers, T, 24, 256))).astype(np.float16)
+    Kd, Vd, Qd = (torch.from_numpy(x).cuda() for x in (K, V, Q))
+    Kt, Vt = Kd[:, n:].contiguous(), Vd[:, n:].contiguous()
+    eng = mk.Engine(layers, n + 64, spec, win)
+    one = mk.Engine(1, 64, spec, win)  # the two layers' rows again, as two sequences of one layer
+    one.slots_open(layers, n + 64)
+    one.reserve_batch(layers)
+    ref = []
+    for l in range(layers):
+        orc = ko.Cache(1, n + 64, spec, win)
+        orc.append(0, 0, K[l], V[l])
+        ref.append(orc.attend(0, n, Q[l]).astype(np.float64))
+        orc.close()
+        eng.append(l, 0, Kd[l, :n], Vd[l, :n])
+        one.append(0, 0, Kd[l, :n], Vd[l, :n], seq=l)
+    eng.sync()
+    out = {k: torch.zeros((layers, T, 24, 256), dtype=torch.float32, device="cuda") for k in ("layers", "attend", "static", "batch")}
+    eng.step_layers(n, Kt, Vt, Qd, out["layers"])
+    for l in range(layers):
+        eng.attend(l, n, Qd[l], out["attend"][l])
+        eng.attend_static(l, n, Qd[l], out["static"][l])
+    one.step_batch([0, 1], 0, [n, n], [T, T], Kt.view(-1, 4, 256), Vt.view(-1, 4, 256), Qd.view(-1, 24, 256), out["batch"].view(-1, 24, 256))
+    eng.sync()
+    one.sync()
+    for k, O in out.items():
+        for l in range(layers):
+            d = np.linalg.norm(O[l].cpu().numpy() - ref[l]) / np.linalg.norm(ref[l])
+            assert d <= 16 * 2.0 ** -23, (k, l, d)
+    eng.close()
+    one.close()
