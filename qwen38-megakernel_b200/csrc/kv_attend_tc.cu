@@ -800,13 +800,16 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
         // which of the warp's rows this thread's position must not see in group k: row token t sees positions <= n + t, positions past
         // the chunk end see nothing (0 for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their
-        // queries are zero, so are their scores, and no one reads what becomes of them.
+        // queries are zero, so are their scores, and no one reads what becomes of them. A group that ends its chunk but lies before the
+        // new tokens is one test for all rows: chunks shorter than a group (contexts up to 1,920 positions) have no other groups, and
+        // with the row loop for each of them 16 layers of 1,187 positions took 60.3 us instead of 53.5, one call 2 us more.
         const int tok0 = batch ? 0 : row0 % T; // token of the warp's first row (row = (head % 6) T + t)
         auto row_mask = [&](const GroupRec & k) -> unsigned {
             const int Tk = batch ? k.T : T, nn = batch ? k.n : n;
             unsigned m = 0u;
-            if (k.pos0 + GP - 1 > min(k.c1 - 1, nn)) { // (the group reaches the chunk's end or the new tokens: the last groups only)
+            if (k.pos0 + GP - 1 > min(k.c1 - 1, nn)) { // (the group reaches the chunk's end or the new tokens)
                 const int p_abs = k.pos0 + prow;
+                if (k.c1 - 1 <= nn) return p_abs >= k.c1 ? (1u << RS) - 1u : 0u;
                 int t = batch ? row0 % Tk : tok0;
 #pragma unroll 1
                 for (int i = 0; i < RS; i++) {

@@ -73,3 +73,28 @@ def test_ranges_in_one_launch_match_oracle(mk, torch_cuda):
             assert np.abs(O[l].cpu().numpy() - orc.attend(l, n, Q[l])).max() <= 2e-3
     for eng in engs:
         eng.close()
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 638, 1022, 1023, 1024, 1025, 1727, 1728, 1729, 2175, 2176])
+def test_chunks_that_end_beside_the_new_tokens(mk, torch_cuda, n):
+    """chunks of 32, 64, 96 and 128 positions whose last position is the first new token, the one before it or a later one: what a row
+    must not see there differs by token in the first and last case only. Every entry that runs such chunks."""
+    torch = torch_cuda
+    spec, win, T = "K*=5r,V*=6", 2048, min(8, ko.att_cap_T(n, 8))
+    eng, orc = mk.Engine(2, n + 64, spec, win), ko.Cache(2, n + 64, spec, win)
+    for l in range(2):
+        fill_both(torch, eng, orc, l, 0, n, seed=70 + l)
+    K, V, Q = rows(2, 7, n, T)
+    Qd = torch.from_numpy(Q).cuda()
+    O = torch.full((3, 2, T, 24, 256), float("nan"), dtype=torch.float32, device="cuda")
+    eng.step_layers(n, torch.from_numpy(K).cuda(), torch.from_numpy(V).cuda(), Qd, O[0])
+    for l in range(2):
+        eng.attend(l, n, Qd[l], O[1, l])
+        eng.attend_static(l, n, Qd[l], O[2, l])
+    eng.sync()
+    for l in range(2):
+        orc.append(l, n, K[l], V[l])
+        Oref = orc.attend(l, n, Q[l])
+        for e in range(3):
+            check_flips(O[e, l].cpu().numpy(), Oref, orc, l, n, Q[l], (n, T, l, e))
+    eng.close()
