@@ -398,13 +398,14 @@ cudaError_t launch_attend_static(const AttnJob & job, int num_sms, int * status,
     j.cpi = 1;
     j.titem0 = 0;
     if (num_sms > 0) {
-        // One CTA per (kv head, chunk) either way, but the unpack and the MMAs of this kernel take 3.8 us per 128 positions against about
-        // 6 of the mma.sync one: 20,011 positions, 2 tokens: 47.1 us against 69.6.
+        // One CTA per (kv head, chunk) either way, but the unpack and the MMAs of this kernel take 3.6 us per 128 positions against about
+        // 6 of the mma.sync one: 20,011 positions, 2 tokens: 43.5 us against 69.8. Short chunks are not paired here (chunks_per_item): the
+        // call has the SMs to itself, one group per CTA instead of two takes 1,000 positions, 1 token from 20.5 us to 18.5 (mma.sync: 21.7)
+        // and 2,551, 8 tokens from 21.9 to 20.5 (32.9), and a partial's sum stays as short as the mma.sync kernel's.
         j.Qp = qp;
-        j.cpi = chunks_per_item(j.cs);
         e = launch_qprep(nullptr, &j, 1, stream);
         if (e != cudaSuccess) return e;
-        const int items = NKV * ((j.nch + j.cpi - 1) / j.cpi);
+        const int items = NKV * j.nch;
         return launch_attend_tc_batch(nullptr, j, 1, true, true, std::max(num_sms, items), items, j.T, nullptr, part, ml, status, stream);
     }
     // every partial row the merge reads is written by the split kernel of the same call: nothing has to start at zero.

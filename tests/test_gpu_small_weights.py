@@ -48,6 +48,7 @@ def test_small_weights_keep_their_precision(mk, torch_cuda, spec, win, n, T):
     for k, O in out.items():
         for l in range(layers):
             d = np.linalg.norm(O[l].cpu().numpy() - ref[l]) / np.linalg.norm(ref[l])
-            assert d <= 16 * 2.0 ** -23, (k, l, d)
+            # (the no-allocation entry does not pair the chunks of 64 and 128 positions: 4 and 8 steps, half the others' bound)
+            assert d <= (8 if k == "static" and n < 5000 else 16) * 2.0 ** -23, (k, l, d)
     eng.close()
     one.close()
