@@ -39,7 +39,10 @@ const char * mk_build_info(void);
 
 /* Replaces mk_new / mk_new2 (capi.cpp:266-312) for the KV path: instead of a model file, the shapes and the reference's
  * MK_KV / MK_KV_WIN settings (loader.cu:1329-1366, 1478-1503). layers: attention layers (1 .. 17); ctx: positions per
- * sequence; kv_spec: e.g. "K*=5r,V*=6" (NULL / "": q8_0); kv_win: e.g. 2048 (0: no window). NULL on error. */
+ * sequence; kv_spec: e.g. "K*=5r,V*=6" (NULL / "": q8_0); kv_win: e.g. 2048 (0: no window). NULL on error.
+ * Device memory besides the rows: split-K partials, 3.96 MB per layer (one launch serves all layers of mk_kv_step_layers; 63.4 MB at 16
+ * layers) and at least 7.3 MB; 7.3 MB whatever the layers with MK_KV_ATTN=fast. mk_kv_reserve_batch(njobs) raises that to 3.96 MB per
+ * job where it is more. */
 void * mk_kv_new(int layers, int ctx, const char * kv_spec, int kv_win, int flags);
 /* capi.cpp:418-424 */
 void mk_free(void * h);

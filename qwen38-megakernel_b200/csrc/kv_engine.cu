@@ -156,7 +156,9 @@ void KvEngine::init_device_state() {
             MKKV_CK(cudaMemset(prof_, 0, attend_fast_prof_words(num_sms_) * sizeof(unsigned long long)));
         }
     alloc_seq(main_, cfg.ctx);
-    ensure_work(std::max(NKV * ATT_NCH * cfg.layers, num_sms_), cfg.layers); // (a decode step's layers may go out as one launch)
+    // partials: a spread launch writes one per SM; the tensor-core kernel's one launch for a step's layers one per (layer, kv head, run of
+    // chunks): 3.96 MB a layer
+    ensure_work(std::max(NKV * ATT_NCH * (use_tc_ ? cfg.layers : 1), num_sms_), cfg.layers);
     ensure_qprep(cfg.layers);
 }
 

@@ -98,3 +98,18 @@ def test_chunks_that_end_beside_the_new_tokens(mk, torch_cuda, n):
         for e in range(3):
             check_flips(O[e, l].cpu().numpy(), Oref, orc, l, n, Q[l], (n, T, l, e))
     eng.close()
+
+
+def test_scratch_of_the_one_launch_step_is_taken_where_it_can_run(mk, torch_cuda, monkeypatch):
+    """partials for all layers at once (80 slots of 48 x 258 floats a layer) only in an engine whose steps can be one launch"""
+    torch = torch_cuda
+    held = {}
+    for kernel, layers in (("fast", 16), ("tc", 1), ("tc", 16)):
+        monkeypatch.setenv("MK_KV_ATTN", kernel)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        eng = mk.Engine(layers, 64)
+        held[kernel, layers] = before - torch.cuda.mem_get_info()[0]
+        eng.close()
+    partials, rows = 16 * 80 * 48 * 258 * 4, 32 << 20
+    assert held["tc", 16] >= partials - (4 << 20) and held["fast", 16] < rows and held["tc", 1] < rows, held
