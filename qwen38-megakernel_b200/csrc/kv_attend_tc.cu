@@ -1404,7 +1404,8 @@ cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, flo
 // one CTA), every CTA running its share of the (job, kv head, run of the job's cpi chunks) items, then the merge kernel over the
 // jobs' partials (a head's partials: its first slots).
 cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & first, int njobs, bool uniform, bool one_format, int num_sms, int nitems, int max_T,
-                                   unsigned * next, float * part, float2 * ml, int * status, cudaStream_t stream, float * raw_part, float2 * raw_ml) {
+                                   unsigned * next, float * part, float2 * ml, int * status, cudaStream_t stream, float * raw_part, float2 * raw_ml,
+                                   unsigned long long * prof) {
     if (njobs < 1 || nitems < 1 || (njobs > 1 && !jobs_dev) || (nitems > num_sms && !next) || !first.Qp) return cudaErrorNotSupported;
     tc::Args a;
     a.one = first;
@@ -1426,7 +1427,7 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     a.done_target = 0;
     a.raw_part = nullptr;
     a.raw_ml = nullptr;
-    a.prof = nullptr;
+    a.prof = prof;
     a.wait_hint_ns = g_wait_hint_ns;
     a.wait_rounds = g_wait_rounds;
     a.poll_rounds = g_poll_rounds;

@@ -182,7 +182,8 @@ void KvEngine::ensure_xch(int nb) {
 void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items, int max_T) {
     if (use_tc_ && njobs == 1 && jobs_host[0].Qp && items_mode(1, jobs_host[0])) {
         const cudaError_t e =
-            launch_attend_tc_batch(nullptr, jobs_host[0], 1, true, true, num_sms_, job_items(jobs_host[0]), max_T, nullptr, part_, ml_, d_status_, stream_);
+            launch_attend_tc_batch(nullptr, jobs_host[0], 1, true, true, num_sms_, job_items(jobs_host[0]), max_T, nullptr, part_, ml_, d_status_, stream_,
+                                   nullptr, nullptr, stamps());
         if (e == cudaSuccess) {
             launches_ += 2;
             return;
@@ -192,7 +193,7 @@ void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items,
     }
     if (use_tc_ && njobs == 1) {
         const cudaError_t e = launch_attend_tc(jobs_host[0], num_sms_, part_, ml_, work_items_, xmax_, xmax_ + (size_t) NKV * ATT_NCH * xnb_ * AR,
-                                               xnb_, ++epoch_, d_status_, stream_, nullptr, 0, 0, nullptr, nullptr, prof_, tc_done_, &tc_done_seq_);
+                                               xnb_, ++epoch_, d_status_, stream_, nullptr, 0, 0, nullptr, nullptr, stamps(), tc_done_, &tc_done_seq_);
         if (e == cudaSuccess) {
             launches_ += 1;
             return;
@@ -208,7 +209,7 @@ void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items,
             for (int w = 0; w < 2; w++) one_format &= jobs_host[j].kv.s[w].bits == jobs_host[0].kv.s[w].bits;
         }
         const cudaError_t e = staged && items <= work_items_ ? launch_attend_tc_batch(d_jobs_, jobs_host[0], njobs, false, one_format, num_sms_, last.titem0 + job_items(last),
-                                                                                      max_T, batch_next_, part_, ml_, d_status_, stream_)
+                                                                                      max_T, batch_next_, part_, ml_, d_status_, stream_, nullptr, nullptr, stamps())
                                                              : cudaErrorNotSupported;
         if (e == cudaSuccess) {
             launches_ += 2;
@@ -219,7 +220,7 @@ void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items,
     }
     {
         const cudaError_t e = launch_attend_fast(d_jobs_, jobs_host, njobs, items, max_T, num_sms_, part_, ml_, work_items_, xmax_,
-                                                 std::min(xnb_, 64), ++epoch_, d_status_, njobs == 1 ? prof_ : nullptr, true, stream_);
+                                                 std::min(xnb_, 64), ++epoch_, d_status_, njobs == 1 ? stamps() : nullptr, true, stream_);
         if (e == cudaSuccess) {
             launches_ += 2;
             return;
@@ -533,7 +534,7 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
             for (int l = layer0; l < layer0 + nlayers; l++) spill_to(s, l, table.base.ws); // positions that left the window are read in the main format
             table.base.Qp = qp;
             MKKV_CK(launch_attend_tc_batch(d_jobs_, table.base, nlayers, true, layers_one_format(s, layer0, nlayers), num_sms_, nlayers * table.items, T, d_next_,
-                                           part_, ml_, d_status_, stream_));
+                                           part_, ml_, d_status_, stream_, nullptr, nullptr, stamps()));
             launches_ += 2;
             return;
         }
@@ -553,7 +554,6 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
 // Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode (one layer: 22 .. 24 us against 22 .. 24): there the
 // layers' outputs are the same bits one by one and together.
 bool KvEngine::items_mode(int nlayers, const AttnJob & j) const {
-    if (prof_) return false; // (MK_KV_PROFILE stamps the spread kernel)
     if (j.cs <= 128) return true;
     if (nlayers < 2) return false;
     const int sms = std::max(num_sms_, NKV), nit = (j.nch + j.cpi - 1) / j.cpi;
@@ -867,7 +867,7 @@ void KvEngine::step_layers_partial(int seq, int nlayers, int n, int T, const voi
             for (int l = 0; l < nlayers; l++) spill_to(s, l, std::min(table.base.ws, hi)); // rows of this range that left the window
             table.base.Qp = qprep_;
             MKKV_CK(launch_attend_tc_batch(d_jobs_, table.base, nlayers, true, layers_one_format(s, 0, nlayers), num_sms_, nlayers * table.items, T, d_next_, part_,
-                                           ml_, d_status_, stream_, static_cast<float *>(parts), static_cast<float2 *>(mls)));
+                                           ml_, d_status_, stream_, static_cast<float *>(parts), static_cast<float2 *>(mls), stamps()));
             launches_ += 2;
             return;
         }
@@ -1746,6 +1746,12 @@ std::vector<unsigned long long> KvEngine::state_digest(int seq) {
     return out;
 }
 
+// where the launch about to be made leaves its stamps (null: tracing is off), cleared of an earlier launch's: launches differ in CTAs and
+// groups, and tracing changes neither the kernels nor their order
+unsigned long long * KvEngine::stamps() {
+    if (prof_) MKKV_CK(cudaMemsetAsync(prof_, 0, attend_fast_prof_words(num_sms_) * sizeof(unsigned long long), stream_));
+    return prof_;
+}
 std::vector<unsigned long long> KvEngine::profile() {
     use_device();
     std::vector<unsigned long long> v;

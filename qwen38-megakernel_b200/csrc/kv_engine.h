@@ -151,7 +151,7 @@ class KvEngine {
     int bits(int side, int layer) const { return kvb_[side][layer]; }
     bool has_ring(int side, int layer) const { return ring_[side][layer]; }
     size_t device_bytes() const { return dev_bytes_; }
-    std::vector<unsigned long long> profile(); // MK_KV_PROFILE=1: the stamps of the last fast attention launch (else empty)
+    std::vector<unsigned long long> profile(); // MK_KV_PROFILE=1: the stamps of the last attention launch (else empty)
     long long launches() const { return launches_; } // kernels launched so far (every launcher call counts its kernels)
 
   private:
@@ -259,7 +259,8 @@ class KvEngine {
     unsigned * tc_done_ = nullptr; // fused merge of the tensor-core kernel: per kv head, CTAs done over all launches
     unsigned tc_done_seq_ = 0;     // launches that counted on it
     void ensure_xch(int nb);
-    unsigned long long * prof_ = nullptr; // MK_KV_PROFILE=1: phase stamps of the last fast attention launch
+    unsigned long long * prof_ = nullptr; // MK_KV_PROFILE=1: phase stamps of the last attention launch
+    unsigned long long * stamps();
     void launch_attention(const AttnJob * jobs_host, int njobs, int items, int max_T);
 
     // host store

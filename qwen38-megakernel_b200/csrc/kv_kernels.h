@@ -85,7 +85,7 @@ cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, flo
 // un-normalised (m, l, O) goes to raw_part + j * 4 * 48 * 256 floats and raw_ml + j * 4 * 48 instead of its O
 cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & first, int njobs, bool uniform, bool one_format, int num_sms, int nitems, int max_T,
                                    unsigned * next, float * part, float2 * ml, int * status, cudaStream_t stream, float * raw_part = nullptr,
-                                   float2 * raw_ml = nullptr);
+                                   float2 * raw_ml = nullptr, unsigned long long * prof = nullptr);
 size_t attend_tc_smem_bytes();
 // test probe: the tensor-core kernel's unpack step on nrows packed rows -> fp16 operand values [nrows][256] in natural dim order
 cudaError_t launch_unpack_probe(int bits, const uint8_t * rows, const uint16_t * sc, int nrows, uint16_t * out, cudaStream_t stream);

@@ -113,3 +113,23 @@ def test_scratch_of_the_one_launch_step_is_taken_where_it_can_run(mk, torch_cuda
         eng.close()
     partials, rows = 16 * 80 * 48 * 258 * 4, 32 << 20
     assert held["tc", 16] >= partials - (4 << 20) and held["fast", 16] < rows and held["tc", 1] < rows, held
+
+
+@pytest.mark.parametrize("n,layers", [(1000, 1), (3000, 8)])
+def test_tracing_changes_neither_launches_nor_results(mk, torch_cuda, monkeypatch, n, layers):
+    torch = torch_cuda
+    K, V, Q = (torch.from_numpy(x).cuda() for x in rows(layers, 8, n, 3))
+    got = []
+    for traced in (False, True):
+        if traced:
+            monkeypatch.setenv("MK_KV_PROFILE", "1")
+        eng = mk.Engine(layers, n + 64, "K*=5r,V*=6", 2048)
+        for l in range(layers):
+            fill_both(torch, eng, None, l, 0, n, seed=90 + l)
+        O = torch.zeros((layers, 3, 24, 256), dtype=torch.float32, device="cuda")
+        before = eng.launches()
+        eng.step_layers(n, K, V, Q, O)
+        eng.sync()
+        got.append((eng.launches() - before, O.cpu().numpy(), eng.profile() is not None))
+        eng.close()
+    assert got[0][0] == got[1][0] == 3 and np.array_equal(got[0][1], got[1][1]) and (got[0][2], got[1][2]) == (False, True)
