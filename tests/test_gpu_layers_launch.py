@@ -11,6 +11,11 @@ from gpu_util import check_flips, fill_both
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def tensor_core_kernel(monkeypatch):
+    monkeypatch.setenv("MK_KV_ATTN", "tc")  # (the mma.sync kernel has no such mode)
+
+
 def rows(layers, seed, n, T):
     K = np.stack([kvdata.kv_rows(seed, l, n, T)[0] for l in range(layers)])
     V = np.stack([kvdata.kv_rows(seed, l, n, T)[1] for l in range(layers)])
@@ -133,3 +138,26 @@ def test_tracing_changes_neither_launches_nor_results(mk, torch_cuda, monkeypatc
         got.append((eng.launches() - before, O.cpu().numpy(), eng.profile() is not None))
         eng.close()
     assert got[0][0] == got[1][0] == 3 and np.array_equal(got[0][1], got[1][1]) and (got[0][2], got[1][2]) == (False, True)
+
+
+@pytest.mark.parametrize("o_stride", [0, 24 * 256, 24 * 256 + 64])
+def test_layers_whose_outputs_overlap_keep_their_order(mk, torch_cuda, o_stride):
+    """an output stride of less than a layer's rows: layer after layer, the last writer's values stay"""
+    torch = torch_cuda
+    n, T, layers = 1500, 2, 3
+    eng = mk.Engine(layers, n + 64, "K*=5r,V*=6", 2048)
+    for l in range(layers):
+        fill_both(torch, eng, None, l, 0, n, seed=95 + l)
+    K, V, Q = (torch.from_numpy(x).cuda() for x in rows(layers, 9, n, T))
+    want = torch.zeros((layers - 1) * o_stride + T * 24 * 256, dtype=torch.float32, device="cuda")
+    one = torch.zeros((T, 24, 256), dtype=torch.float32, device="cuda")
+    for l in range(layers):
+        eng.step(l, n, K[l], V[l], Q[l], one)
+        eng.sync()
+        want[l * o_stride:l * o_stride + T * 24 * 256] = one.view(-1)
+    for _ in range(5):
+        got = torch.zeros_like(want)
+        eng.step_layers(n, K, V, Q, got.as_strided((layers, T, 24, 256), (o_stride, 24 * 256, 256, 1)))
+        eng.sync()
+        assert torch.equal(got, want)
+    eng.close()
