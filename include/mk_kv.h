@@ -77,13 +77,13 @@ int mk_kv_attend(void * h, int seq, int layer, int n, int T, const void * Q, voi
 /* No counterpart in the reference. mk_kv_attend for callers that must not touch the CUDA allocator while they decode: a
  * plugin inside a server that has already handed every byte of device memory to its own pool (a cudaMalloc there fails or
  * stalls the whole device), or a real-time loop that may not take the allocator's locks and implicit synchronisation.
- * Same arguments, same result. The split-K partials go to a fixed array compiled into the library (3.96 MB on every GPU
- * that loads it, until the process exits) instead of the engine's allocated workspace; the call runs no cudaMalloc /
- * cudaFree or any other allocating routine. Limits: one sequence per call, T <= 8, at most 80 (kv head, chunk) items; a call
- * beyond that returns -1 with a message saying so. The array's device address is looked up when an engine is created on the device
- * (mk_kv_new), not in this call. All handles of a process share the one array per GPU, and it keeps the last
- * call's contents (nothing in it needs clearing: each call writes every partial it reads): two such calls that can
- * overlap on the GPU (different streams or handles) race and must be serialised by the caller. 0 / -1 */
+ * Same arguments; the result is mk_kv_attend's up to rounding. The split-K partials and the staged queries go to two fixed arrays
+ * compiled into the library (3.96 MB and 98 KB on every GPU that loads it, until the process exits) instead of the engine's allocated
+ * workspace; the call runs no cudaMalloc / cudaFree or any other allocating routine. Limits: one sequence per call, T <= 8, at most 80
+ * (kv head, chunk) items; a call beyond that returns -1 with a message saying so. The arrays' device addresses are looked up when an
+ * engine is created on the device (mk_kv_new), not in this call. All handles of a process share the arrays of a GPU, and they keep the
+ * last call's contents (nothing in them needs clearing: each call writes all it reads): two such calls that can overlap on the GPU
+ * (different streams or handles) would mix each other's queries and partials and must be serialised by the caller. 0 / -1 */
 int mk_kv_attend_static(void * h, int seq, int layer, int n, int T, const void * Q, void * O);
 /* ---- one very long sequence split by position over several GPUs (no counterpart in the reference, which is single-GPU: its
  * split-K partials (qwen38_mk.cu:3048-3064) and merge (:4658-4669) are the unit that is exchanged) ----

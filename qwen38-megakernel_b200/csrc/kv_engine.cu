@@ -596,7 +596,7 @@ void KvEngine::ensure_qprep(int slots) {
 void KvEngine::staged_q(AttnJob & j, int slot, bool staged) {
     j.Qp = qprep_ + (size_t) slot * NKV * (QP_HEAD_BYTES / 2);
     if (staged) return;
-    MKKV_CK(launch_qprep(nullptr, &j, 1, stream_));
+    MKKV_CK(launch_qprep(j, stream_));
     launches_++;
 }
 

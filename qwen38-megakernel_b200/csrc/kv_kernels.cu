@@ -137,22 +137,13 @@ __device__ __forceinline__ void qprep_row(const uint16_t * Q, uint16_t * qp, int
     *reinterpret_cast<uint4 *>(dst) = out;
 }
 constexpr int QP_BLOCKS = NKV * AR / 8; // blocks of 8 warps that stage one job's queries
-__global__ void __launch_bounds__(256) qprep_kernel(const __grid_constant__ AttnArgs a) {
+__global__ void __launch_bounds__(256) qprep_kernel(const __grid_constant__ AttnJob J) {
     release_next();
-    const AttnJob & J = a.jobs ? a.jobs[blockIdx.y] : a.one;
     const int lane = threadIdx.x & 31, idx = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (!J.Qp) return;
     qprep_row(J.Q, const_cast<uint16_t *>(J.Qp), J.T, J.kv.s[0].rot, idx / AR, idx % AR, lane);
 }
-cudaError_t launch_qprep(const AttnJob * jobs_dev, const AttnJob * jobs_host, int njobs, cudaStream_t stream) {
-    if (njobs <= 0) return cudaSuccess;
-    AttnArgs a;
-    a.one = jobs_host[0];
-    a.jobs = njobs > 1 ? jobs_dev : nullptr;
-    a.njobs = njobs;
-    a.part = nullptr;
-    a.ml = nullptr;
-    qprep_kernel<<<dim3(QP_BLOCKS, njobs), 256, 0, stream>>>(a);
+cudaError_t launch_qprep(const AttnJob & job, cudaStream_t stream) {
+    qprep_kernel<<<QP_BLOCKS, 256, 0, stream>>>(job);
     return cudaGetLastError();
 }
 
@@ -403,7 +394,7 @@ cudaError_t launch_attend_static(const AttnJob & job, int num_sms, int * status,
         // call has the SMs to itself, one group per CTA instead of two takes 1,000 positions, 1 token from 20.5 us to 18.5 (mma.sync: 21.7)
         // and 2,551, 8 tokens from 21.9 to 20.5 (32.9), and a partial's sum stays as short as the mma.sync kernel's.
         j.Qp = qp;
-        e = launch_qprep(nullptr, &j, 1, stream);
+        e = launch_qprep(j, stream);
         if (e != cudaSuccess) return e;
         const int items = NKV * j.nch;
         return launch_attend_tc_batch(nullptr, j, 1, true, true, std::max(num_sms, items), items, j.T, nullptr, part, ml, status, stream);

@@ -112,7 +112,7 @@ cudaError_t launch_append_batch(const AppendJob * ajobs_dev, const AttnJob * job
 // [dim group 32][row group 6][8 rows][8 dims in the unpacked units' order], rows beyond 6 T zero. One bulk copy brings a head's block
 // into shared memory.
 constexpr int QP_HEAD_BYTES = AR * HD * 2;
-cudaError_t launch_qprep(const AttnJob * jobs_dev, const AttnJob * jobs_host, int njobs, cudaStream_t stream);
+cudaError_t launch_qprep(const AttnJob & job, cudaStream_t stream); // one job's, in a launch of its own
 // rows pos0 .. pos0 + n - 1 of layers 0 .. nlayers - 1 of one sequence in one launch (views_dev: the sequence's device array of views);
 // Q != null: the same launch stages the T query tokens of every layer (Q + l q_stride bytes -> qp + l * 4 * QP_HEAD_BYTES bytes)
 // table (with Q only): it also leaves the layers' attention jobs in table->jobs: base with layer l's view, queries, output (base.O + l
@@ -145,8 +145,8 @@ cudaError_t launch_gather(const CopyRegion * regions, int nregions, int a, int b
 // Decode attention of ONE job whose split partials live in a fixed array inside the library's device image instead of
 // memory obtained from the CUDA allocator. The array holds STATIC_ITEMS (kv head, chunk) items: enough for any single
 // job (the partition never makes more than NKV * ATT_NCH), about 3.96 MB per GPU that loads the library, held until the
-// process exits. The array's device address is looked up (cudaGetSymbolAddress) by preload_kernels, which every engine runs at
-// construction. Returns cudaErrorInvalidValue if the job needs more items than the array holds.
+// process exits; the staged queries have a second one (98 KB). The arrays' device addresses are looked up (cudaGetSymbolAddress) by
+// preload_kernels, which every engine runs at construction. Returns cudaErrorInvalidValue if the job needs more items than the array holds.
 constexpr int STATIC_ITEMS = NKV * ATT_NCH;
 // num_sms > 0: on the tensor-core kernel's batch mode (its staged queries have a fixed array too), else on the mma.sync kernel.
 cudaError_t launch_attend_static(const AttnJob & job, int num_sms, int * status, cudaStream_t stream);
