@@ -49,10 +49,12 @@ for p in (ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests")):
 LAYERS, CTX0, T_STEP, WIN = 16, 101600, 8, 2048
 SPEC = "K*=5r,V*=6"
 NH, NKV, HD = 24, 4, 256
-# dram__bytes_read.sum + dram__bytes_write.sum of one attention launch at this workload's shapes, from an ncu capture of the
-# one-layer case of this benchmark (a launch of the 16-layer run processes the same one layer); NCU_TRAFFIC_FROM says which
-NCU_TRAFFIC_BYTES = 164.2e6
-NCU_TRAFFIC_FROM = "ncu capture of `bench.py --layers 1 --steps 2 --warmup 3 --no-cpu`, kernel attn_tc_kernel<5, 6> (since compiled as the one-job instance attn_tc_kernel<5, 6, false>, same code), one launch"
+# dram__bytes_read.sum + dram__bytes_write.sum at this workload's shapes per layer, from ncu captures of this benchmark with fewer layers; one
+# entry per attention kernel instance, since a launch of one layer and a launch of all layers of a step move different partials
+NCU_TRAFFIC = {
+    "one": (164.2e6, "ncu capture of `bench.py --layers 1 --steps 2 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, false>, one launch (partials and merge in it)"),
+    "batch": (None, None),
+}
 WORKLOAD = "config2: 16 attention layers, 101,600 positions, preset F layout K5r/V6 + q8_0 window 2048, 8 queries/step, streaming append+spill+attend"
 REPEATS = 5  # the timed K-step loop is run this many times; the line's value is the median run
 
@@ -653,17 +655,17 @@ def main():
     if rank == 0:
         peak, peak_src = hbm_peak()
         us_layer = 1e3 * ms / (layers * args.steps)  # per GPU: every rank streams its own sequence, the slowest rank's time
-        # the attention launch's duration: the event pair around a step's launches / layers, or, when smaller, the timed steps' time per
-        # layer (a step of several layers runs their attention as one launch of the kernel's batch mode, with one append and one merge
-        # launch: its time per layer holds all three)
+        # the attention's duration per layer: of a launch per layer (event pair around a step's launches), and of the timed steps, whose layers'
+        # attention is one launch of the kernel's batch mode (the step's append and merge launches included); the smaller one is named
+        one_us, inst = att_us, "one"
         kernel = "attn_tc_kernel<5, 6, false> (the one-job instance; merge in its tail)"
         att_from = "event pair around a step's %d attention launches" % layers
         if us_layer < att_us:
             att_us, att_from = us_layer, "timed steps (time per layer: 1/%d of the step's append, attention and merge launches)" % layers
             if layers > 1:
-                kernel = "attn_tc_kernel<5, 6, true> (the batch instance: all layers in one launch), attn_merge_kernel"
+                kernel, inst = "attn_tc_kernel<5, 6, true> (the batch instance: all layers in one launch), attn_merge_kernel", "batch"
+        traffic, traffic_from = NCU_TRAFFIC[inst] if layers == LAYERS and ctx0 == CTX0 else (None, None)
         achieved = att_bytes / att_us / 1e3  # GB/s
-        full = layers == LAYERS and ctx0 == CTX0
         line = {
             "metric": "decode_attn_us_per_layer", "value": us_layer, "unit": "us/layer", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
@@ -678,8 +680,13 @@ def main():
                         "us_per_layer_max": 1e3 * runs[order[-1]][0] / (layers * args.steps)},
             "hbm_gbs_step": step_bytes / (ms * 1e-3) / 1e9 * world,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "traffic": NCU_TRAFFIC_BYTES if full else None, "traffic_from": NCU_TRAFFIC_FROM if full else None,
-                         "kernel": kernel, "us_per_launch": att_us, "us_per_launch_from": att_from, "bytes_per_launch": att_bytes, "peak_source": peak_src},
+                         "traffic": traffic, "traffic_from": traffic_from, "kernel": kernel,
+                         "us_per_launch": att_us, "us_per_launch_from": att_from, "bytes_per_launch": att_bytes,
+                         "per": "layer (the batch launch serves %d layers: its time and bytes are divided by that)" % layers if inst == "batch" else "launch",
+                         "peak_source": peak_src},
+            # the launch a forward pass makes whose next layer's queries need this layer's output (`value` is of a step that has all layers' queries)
+            "one_layer_launch": {"us": one_us, "achieved": att_bytes / one_us / 1e3, "frac": att_bytes / one_us / 1e3 / peak,
+                                 "what": "mk_kv_attend layer by layer: query staging + attn_tc_kernel<5, 6, false>"},
             "e2e": {"value": 1e3 * ms_e2e / (layers * args.steps), "unit": "us/layer",
                     "h2d_bytes_per_step": int(layers * (2 * T_STEP * NKV * HD * 2 + T_STEP * NH * HD * 2)),
                     "d2h_bytes_per_step": int(layers * T_STEP * NH * HD * 4)},
