@@ -110,13 +110,14 @@ int mk_kv_combine_layers_strided(void * h, int nlayers, int T, int nparts, const
 /* append + attend of one decode step's layer, as the reference's attention phase does in one pass */
 int mk_kv_step(void * h, int seq, int layer, int n, int T, const void * K, const void * V, const void * Q, void * O);
 /* One decode step over layers 0 .. nlayers - 1 in one call: layer l appends T rows at n from K + l kv_stride, V + l kv_stride
- * and attends with Q + l q_stride into O + l o_stride (strides in bytes). What the reference's forward pass does between its
- * layers' attention phases (engine.cu:1353-1413) with the host out of the loop; equal in result to nlayers calls of mk_kv_step (the
- * rows of all layers are appended by one launch before the first layer's attention: every K and V must be complete at the call). */
+ * and attends with Q + l q_stride into O + l o_stride (strides in bytes). K, V and Q of ALL layers are read at the call: for hosts that hold
+ * them (replays, comparisons, attention layers that do not feed one another). In a decoder each layer's queries need the layer
+ * before, as in the reference's forward pass (engine.cu:1353-1413): it calls mk_kv_step once per layer, and a time per layer of this
+ * call is not the time of that one. The rows of all layers are appended by one launch, and the layers' attention may go out as one: outputs
+ * are then those of nlayers calls of mk_kv_step up to rounding (softmax weights are kept against another reference maximum and
+ * summed in another order: relative 2-norm of the difference 2e-6 .. 1.5e-5); up to 2,560 positions they are the same bits. */
 int mk_kv_step_layers(void * h, int seq, int nlayers, int n, int T, const void * K, const void * V, const void * Q, void * O,
                       size_t kv_stride, size_t q_stride, size_t o_stride);
-/* (The layers' attention may go out as one launch: outputs then equal the per-layer calls' up to the order of fp32 sums; up to 2,560
- * positions they are the same bits.) */
 /* The same for layers layer0 .. layer0 + nlayers - 1 (K, V, Q, O point at layer0's rows): a host that receives a step's rows in
  * blocks of layers overlaps the next block's copies with this block's attention. */
 int mk_kv_step_layers_at(void * h, int seq, int layer0, int nlayers, int n, int T, const void * K, const void * V, const void * Q, void * O,

@@ -20,19 +20,19 @@
 //     groups ahead of P, so that a group's own maxima are published long before another CTA needs them), exchange the running
 //     max with the CTAs that hold the chunk's earlier groups through small global arrays (own group maxima and cumulative
 //     maxima, 8-byte {launch tag, value} words, polled with a bound), and write P to shared memory as the B operand. The
-//     accumulator is kept against a per-row reference max that moves rarely (when the running max passes it by more than 10.5;
-//     then the moved rows' accumulator columns are rescaled, one tensor-memory column per row and block): P, after its fp16 rounding, is multiplied by exp(running max - reference) and carried as an fp16
-//     high and low part (one N = 96 MMA per k-step, two 48-column accumulator blocks), so the reference's fp16 P is reproduced
-//     and no per-tile accumulator rescale is needed;
+//     accumulator is kept against a per-row reference max that moves rarely (when the running max passes it by more than 11;
+//     then the moved rows' accumulator columns are rescaled, one tensor-memory column per row and block): P, after its fp16
+//     rounding, is multiplied by exp(running max - reference) and carried as an fp16 high and low part (one N = 96 MMA per k-step, two
+//     48-column accumulator blocks), so the reference's fp16 P is reproduced and no per-tile accumulator rescale is needed;
 //   - a CTA writes one un-normalised partial (m, l, O); when the CTAs of a kv head have all written theirs (arrival count,
 //     bounded wait) each merges one or two of the head's rows in the kernel's tail, four warps to a row;
 //   - batch mode (several jobs: sequences served together, or all layers of a decode step): a plain launch of one persistent CTA per
 //     SM, each running its share of the (job, kv head, run of cpi chunks) items one after another, the chunks' groups in order with
 //     the running max carried in registers and started anew at every chunk, no exchange; attn_merge_kernel afterwards. The copies,
 //     the unpacking and S^T of the next item run on while the softmax warps finish the one before. What bounds it: a group costs
-//     3.8 us of CTA time at any length (the same instruction issue and latency as in the spread mode), an item about 2.5 us more.
-//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 4.0 us against 18.8;
-//     11,701 (K6 / V5), 3 tokens 12.8 against 27.1; 101,600, 8 tokens 84.7 against 96.7.
+//     3.6 us of CTA time at any length (the same instruction issue and latency as in the spread mode), an item about 2.5 us more.
+//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 3.3 us against 18.8;
+//     11,701 (K6 / V5), 3 tokens 12.3 against 27.1; 101,600, 8 tokens 81.5 against 96.7.
 // Every wait is bounded (about two seconds by default; the limits are launch arguments), then the status word and a CTA-wide
 // flag are set, no later wait of the CTA blocks, the producer waits (bounded) for its copies still in flight, and the kernel
 // runs to its end and frees its tensor memory.

@@ -246,7 +246,8 @@ class Engine:
 
     def step_layers(self, n, K, V, Q, O, seq=SEQ_MAIN):
         """one decode step over every layer in one call: K, V [layers][T][4][256], Q [layers][T][24][256], O likewise (fp32).
-        A layer's rows must be contiguous; the layer stride is free (the first T rows of a larger per-layer buffer are fine)."""
+        A layer's rows must be contiguous; the layer stride is free (the first T rows of a larger per-layer buffer are fine). All layers'
+        queries are read at the call: a decoder whose next layer needs this one's output calls step() layer by layer."""
         for x in (K, V, Q, O):
             if not x.is_cuda or not x[0].is_contiguous():
                 raise EngineError("step_layers: expected CUDA tensors whose per-layer rows are contiguous")
