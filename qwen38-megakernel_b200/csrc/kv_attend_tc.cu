@@ -1437,8 +1437,9 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     const TcKernel kern = one_format ? tc_kernel_for(first.kv.s[0].bits, first.kv.s[1].bits, true) : tc::attn_tc_kernel<0, 0, true>;
     // The prologue beside the launch before (22.3 us instead of 26.6 for a 300-position layer with the merge's early launch, 70.2
     // instead of 73.9 for 16 layers of 1,187 positions) pays where a CTA's work is short; 16 layers of 11,701 positions (45 groups per
-    // CTA) took 222 us with it and 217 without, a batch of 32 sequences 3,176 and 3,020. The merge's blocks waiting beside the
-    // attention cost more than they gain as soon as CTAs have more than one item (102 -> 111 us for 16 layers of 4,000 positions).
+    // CTA) took 222 us with it and 217 without, a batch of 32 sequences 3,176 and 3,020 (without it, with the softmax warps' packed
+    // arithmetic, 197 and 2,782). Of jobs that differ, the first and longest one's chunk length stands for all. The merge's blocks waiting
+    // beside the attention cost more than they gain as soon as CTAs have more than one item (102 -> 111 us for 16 layers of 4,000 positions).
     const int grid = std::min(nitems, num_sms), per_cta = (nitems + grid - 1) / grid * std::max(first.cpi, 1) * ((first.cs / ATP + tc::GT - 1) / tc::GT);
     e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(tc::NTHREADS), attend_tc_smem_bytes(), stream, a);
     if (e != cudaSuccess) return e;
