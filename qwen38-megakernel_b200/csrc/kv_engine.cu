@@ -548,10 +548,10 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
 // Whether nlayers layers of one step (job j's shape, each) go out as one launch of the tensor-core kernel's batch mode, or one by one
 // in its spread mode. In tenths of a 128-position group's time on one CTA (3.6 us): the batch launch takes the CTA with the most
 // groups, 7 per item besides (queries, partial, the pipeline's refill) and 50 for itself, its append and its merge; a spread launch
-// deals a layer's groups over all CTAs but takes 42 for itself (exchange of maxima, slowest CTA, merge). Measured when the constants were
-// taken, both modes at 3.8 us a group (us, batch against spread, 3 tokens): 2 layers of 4,000 positions 33 / 44, of 11,701 66 / 60; 4
-// layers of 11,701 87 / 114, of 38,000 198 / 197, of 101,600 472 / 403; 8 layers of 101,600 773 / 802; 16 layers of 1,187 74 / 304, of
-// 101,600 1,381 / 1,596. The batch side since: 16 layers of 1,187 53.5, of 101,600 1,304.
+// deals a layer's groups over all CTAs but takes 42 for itself (exchange of maxima, slowest CTA, merge). Measured (us, batch against
+// spread, 8 tokens): 2 layers of 4,003 positions 30 / 42, of 11,701 56 / 58 (the rule takes spread), of 24,003 93 / 83; 4 layers of
+// 24,003 135 / 162, of 38,000 189 / 200, of 101,600 453 / 389; 8 layers of 101,600 737 / 768; 16 layers of 101,600 1,308 / 1,521. Of 48
+// shapes of 2 .. 16 layers the slower form is taken in one, by 2.7 %.
 // Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode (one layer: 22 .. 24 us against 22 .. 24): there the
 // layers' outputs are the same bits one by one and together.
 bool KvEngine::items_mode(int nlayers, const AttnJob & j) const {
