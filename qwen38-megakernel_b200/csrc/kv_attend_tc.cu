@@ -251,6 +251,13 @@ __device__ __forceinline__ unsigned desc_hi(unsigned sbo) { return ((sbo >> 4) &
 __device__ __forceinline__ void umma_commit(uint64_t * bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// One lane of a converged warp. Code under this test is known to be one thread's, so that the descriptors of its tcgen05.mma (uniform
+// registers) need no search for the lanes that agree.
+__device__ __forceinline__ bool elect_one() {
+    unsigned r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -628,7 +635,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         }
     } else if (warp == W_ISSUE) {
         // ---- issuer: S(0) .. S(NSB - 1), then PV(i), S(i + NSB) ----
-        if (lane == 0) {
+        if (elect_one()) { // (with lane == 0 as the test an instruction took 50 % longer to issue: see elect_one)
             unsigned oseq = 0;
             if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc, a.status); // the queries are staged
             // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S^T of the segment before is
