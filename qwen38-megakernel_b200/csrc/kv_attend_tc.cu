@@ -9,17 +9,19 @@
 //   - 16 unpack warps turn packed rows into exact fp16(d * q) operands in the canonical no-swizzle UMMA layouts (one thread:
 //     one position x 32 dims per step; the fp16 pairs are assembled straight from the nibble words and high-bit fields with one
 //     AND-OR each, kv_unpack.h, which leaves the 8 dims of a 16-byte unit in the order UNIT_PERM: the queries are staged in the
-//     same order and the output dims are mapped back) -- K as the K-major A operand of S^T[128 pos x 48 rows] = K Q^T, V as the
+//     same order and the output dims are mapped back) -- K as the K-major B operand of S[48 (64) rows x 128 pos] = Q K^T, V as the
 //     MN-major A operand of O^T[256 dims x 48 rows] += V^T P^T;
 //   - the queries arrive staged (qprep in kv_kernels.cu: rotated when K is, x 1/16, fp16, in the B operand's layout; made once per
 //     (job, kv head) by the decode step's append launch or a small launch of its own) and are fetched with one bulk copy;
 //   - one issuer thread runs tcgen05.mma on the slots as they fill (mbarrier "full" from the unpack warps, tcgen05.commit
-//     to "empty"), S^T in five tensor-memory buffers (K runs five groups ahead of V), O^T (two 128-dim halves) resident there
-//     for the whole kernel;
-//   - 8 softmax warps read S^T back (tcgen05.ld: a thread owns one position and 24 query rows), take the tile maxima (two
-//     groups ahead of P, so that a group's own maxima are published long before another CTA needs them), exchange the running
+//     to "empty"), S in four tensor-memory buffers (K runs four groups ahead of V; M = 64 takes 16 lanes of each quarter, so two
+//     buffers share their columns), O^T (two 128-dim halves) resident there for the whole kernel;
+//   - 8 softmax warps read S back (tcgen05.ld 16x32bx2: a thread owns one query row and one tile of 32 positions), so that a tile's
+//     maximum and sum are taken inside a thread (with positions on lanes they were 24 warp reductions a warp and group, a barrier and
+//     a hand-out of each row's maxima: 1.9 k more instructions a group); they exchange the running
 //     max with the CTAs that hold the chunk's earlier groups through small global arrays (own group maxima and cumulative
-//     maxima, 8-byte {launch tag, value} words, polled with a bound), and write P to shared memory as the B operand. The
+//     maxima, 8-byte {launch tag, value} words, polled with a bound; maxima two groups ahead of P), and write P to shared memory as
+//     the K-major B operand. The
 //     accumulator is kept against a per-row reference max that moves rarely (when the running max passes it by more than 11;
 //     then the moved rows' accumulator columns are rescaled, one tensor-memory column per row and block): P, after its fp16
 //     rounding, is multiplied by exp(running max - reference) and carried as an fp16 high and low part (one N = 96 MMA per k-step, two
@@ -27,8 +29,9 @@
 //   - a CTA writes one un-normalised partial (m, l, O); when the CTAs of a kv head have all written theirs (arrival count,
 //     bounded wait) each merges one or two of the head's rows in the kernel's tail, four warps to a row;
 //   - batch mode (several jobs: sequences served together, or all layers of a decode step): a plain launch of one persistent CTA per
-//     SM, each running its share of the (job, kv head, run of cpi chunks) items one after another, the chunks' groups in order with
-//     the running max carried in registers and started anew at every chunk, no exchange; attn_merge_kernel afterwards. The copies,
+//     SM, each running its share of the (job, kv head, run of cpi chunks) items one after another, groups of four consecutive tiles in order
+//     with the running max carried in registers and started anew at a chunk's first tile (a group may hold tiles of several chunks: with
+//     groups that ended with their chunk, half of each was padding at 1,187 positions and 16 layers took 47.5 us instead of 37.3), no exchange; attn_merge_kernel afterwards. The copies,
 //     the unpacking and S^T of the next item run on while the softmax warps finish the one before. What bounds it: a group costs
 //     3.6 us of CTA time at any length (the same instruction issue and latency as in the spread mode), an item about 2.5 us more.
 //     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 3.3 us against 18.8;
@@ -53,40 +56,30 @@ namespace tc {
 
 using namespace attn_common;
 
-#ifndef MKKV_TC_NDQ
-#define MKKV_TC_NDQ 16 // unpack warps: 16 (one 32-dim block of a half each, 28 warps per CTA) or 8 (two blocks each, 20 warps: measured
-                       // 115 us against 105 on the one-layer case, the unpack needs the warps)
-#endif
-constexpr int NSL = 2;         // row slices of the softmax warps: 24 query rows each
-constexpr int NSOFT = 4 * NSL; // softmax warps first: warp = 4 c2 + q, tile q (tensor-memory lanes 32 q ..), query rows RS c2 .. + RS - 1
-constexpr int NDQ = MKKV_TC_NDQ; // then the unpack warps: 4 c + q, tile q, 32-dim blocks c, c + NDQ / 4, .. of each 128-dim half
-constexpr int BPW = 16 / NDQ;  // blocks of a half per unpack warp
+constexpr int NSOFT = 8;       // softmax warps first: warp 4 h2 + q, query rows 16 q .. + 15, tiles 2 h2 and 2 h2 + 1 of a group
+constexpr int NDQ = 16;        // then the unpack warps: 4 c + q, tile q, 32-dim block c of each 128-dim half
 constexpr int W_ISSUE = NSOFT + NDQ, W_PROD = W_ISSUE + 1;
 constexpr int NTHREADS = (W_PROD + 3) * 32; // two idle warps complete the last group of four (register reallocation is per group)
-constexpr int GT = 4, GP = GT * ATP;        // tiles / positions per group: the M of one MMA
-constexpr int RS = AR / NSL;                // query rows per softmax warp
+constexpr int GT = 4, GP = GT * ATP;        // tiles / positions per group: the N of an S instruction
 // registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
 // most the CTA's launch allocation -- a larger sum faults)
-#if MKKV_TC_NDQ == 8
-#define MKKV_TC_REGS_SOFT "128"
-#define MKKV_TC_REGS_DQ "80"
-#define MKKV_TC_REGS_CTL "56"
-static_assert(NTHREADS == 640 && 8 * 128 + 8 * 80 + 4 * 56 <= 20 * 96, "register shares");
-#else
-#define MKKV_TC_REGS_SOFT "112"
+#define MKKV_TC_REGS_SOFT "104"
 #define MKKV_TC_REGS_DQ "56"
-#define MKKV_TC_REGS_CTL "56"
-static_assert(NTHREADS == 896 && 8 * 112 + 16 * 56 + 4 * 56 <= 28 * 72, "register shares");
-#endif
+#define MKKV_TC_REGS_CTL "72"
+static_assert(NTHREADS == 896 && 8 * 104 + 16 * 56 + 4 * 72 <= 28 * 72, "register shares");
 constexpr int RAW_SLOT = ATP * HD + ATP * SCALE_ROW; // one tile of the widest format and its scales: 8704 bytes
 constexpr int NRAW = 8;                     // packed tile slots: two side-groups (one being unpacked, one in flight)
 static_assert(NRAW % GT == 0, "whole groups only: a 7-slot ring, tried once, was 20 % slower and its results changed from run to run");
 constexpr int OP_SLOT = GP * 128 * 2;       // fp16 operand: 128 positions x 128 dims
 constexpr int NOP = 3;
-constexpr int NSB = 5;                      // S^T buffers: K runs NSB groups ahead of V
+constexpr int NSB = 4;                      // S buffers: K runs NSB groups ahead of V
 constexpr int NTASK = 16;
-constexpr int Q_BYTES = AR * HD * 2, P_BYTES = AR * GP * 2;
-constexpr unsigned S_COL = 0, S_STRIDE = 64, O_COL0 = NSB * 64, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512; // an O^T half: 48 columns for P's high part, 48 for its low part
+constexpr int Q_BYTES = AR * HD * 2;
+constexpr int P_KGROUP = 2 * AR / 8 * 128;  // P of 8 positions: the 6 row groups of its high part, then those of its low part
+constexpr int P_BYTES = GP / 8 * P_KGROUP;
+// An S buffer is 128 columns (positions) on 16 lanes (query rows) of each quarter of the lanes: two buffers share their columns. An
+// accumulator half is 48 columns for P's high part and 48 for its low part.
+constexpr unsigned S_COL = 0, S_STRIDE = GP, O_COL0 = NSB / 2 * S_STRIDE, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512;
 static_assert(O_COL1 + 2 * AR <= TMEM_COLS, "tensor-memory columns");
 static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
 // The accumulator's reference max of a row is set REF_BELOW below the running max it is taken from and moves when the running max
@@ -97,16 +90,13 @@ static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
 constexpr float REF_SLACK = 11.f, REF_BELOW = 2.f;
 constexpr float LOG2E = 1.4426950408889634f;
 
+template <int V> struct IntC { // an integer as an argument of a generic lambda
+    static constexpr int value = V;
+};
+
 struct WaitCtl { // the launch's wait limits and the CTA's give-up flag
     int dead;
     unsigned hint, rounds, poll; // nanoseconds per failed try, failed tries of an mbarrier wait, failed polls of a global word
-};
-
-struct WarpScratch { // what the row-owner lanes of a softmax warp hand to all its lanes
-    float nm[RS];    // minus the running max of the warp's tile (-inf where nothing is visible yet: exp2 gives 0)
-    float beta[RS];  // exp(running max - reference max)
-    float f[RS];     // factor of a moved reference max
-    unsigned bh[RS / 2], bl[RS / 2]; // beta as fp16 high + low parts, rows (2 j, 2 j + 1) packed
 };
 
 // A group's task record as the producer leaves it for the other roles. The fields behind AttnTask serve the batch mode, where one CTA
@@ -114,8 +104,10 @@ struct WarpScratch { // what the row-owner lanes of a softmax warp hand to all i
 struct GroupRec : AttnTask {
     const uint16_t * q;       // the segment's staged queries
     int n, T, slot, flags;    // of the segment's job; the partial's slot
-    int ring0[2], bits[2];    // K / V: first position read from the q8_0 ring (0x7fffffff: no ring), bits of the main rows
+    unsigned restart;         // bit t: tile t opens a chunk, the running max starts anew
 };
+// What the unpack warps need of one side of one tile: rows that are there | UD_END in the CTA's last group | bits of the rows << 8
+constexpr unsigned UD_ROWS = 0x3fu, UD_END = 0x80u;
 constexpr int REC_FIRST = 1, REC_LAST = 2, REC_END = 4; // first / last group of its segment, last group of the CTA
 struct TileSrc { // where one side of one tile lies: rows, scales, bytes per row, rows
     const uint8_t * val;
@@ -126,12 +118,13 @@ struct TileSrc { // where one side of one tile lies: rows, scales, bytes per row
 struct Smem {
     uint8_t op[NOP][OP_SLOT];   // [dim group 16][position group 16][8 positions][8 dims] fp16
     uint8_t raw[NRAW][RAW_SLOT];
-    uint8_t q[Q_BYTES];         // [dim group 32][row group 6][8 rows][8 dims]
-    uint8_t p[2][P_BYTES];      // high / low part: [row group 6][position group 16][8 positions][8 rows]
-    float tmax[4][GT][AR];      // row maxima of a group's tiles; by group % 4: a group's maxima are read while those of the next two
-                                // groups exist or are being written, and a warp is never a whole group ahead of its slice.
-                                // The first buffer holds the row sums at the end.
-    WarpScratch ws[NSOFT];
+    uint8_t q[Q_BYTES];         // [dim group 32][row group 6][8 rows][8 dims]. (As the A operand of M = 64 rows a dim group is read on
+                                // into the next one, the last into p: rows 48 .. 63 of S are never read)
+    uint8_t p[P_BYTES];         // [position group 16][high part, low part][row group 6][8 rows][8 positions]
+    float tmax[2][GT][AR];      // row maxima of a group's tiles, by group parity
+    float lsum[AR];             // row sums of tiles 2 and 3 on their way to the warps of tiles 0 and 1
+    float resc_f[2][AR];        // factors of the reference maxima that moved, by group parity
+    unsigned resc_rows[2][4];   // and which of each 16 rows they are
     unsigned tmem_base;
     int merge_ok;               // the tail's merge: the head's CTAs have all arrived
     WaitCtl wc;                 // the launch's wait limits; dead: a wait of this CTA gave up, no later wait blocks
@@ -139,9 +132,9 @@ struct Smem {
                                 // the producer's K is at most NSB + 2 groups ahead of the softmax warps' group)
     uint64_t raw_full[NRAW], raw_empty[NRAW], op_full[NOP], op_empty[NOP], s_full[NSB], s_empty[NSB], p_full, p_empty, q_ready, fin;
     AttnJob job;
+    unsigned udesc[NTASK][2][GT]; // K / V tiles of a group, by group % NTASK (see UD_ROWS)
     // batch mode only
     TileSrc vsrc[NTASK][GT];    // the V tiles of the groups whose K the producer has fetched
-    float lsum[2][GT][AR];      // row sums of a segment's four tiles, by segment parity
     uint64_t rec_full[NTASK];   // record (group % NTASK) is written
 };
 
@@ -169,9 +162,6 @@ struct Args {
     unsigned wait_hint_ns, wait_rounds, poll_rounds; // limits of the waits: a failed mbarrier try suspends for up to wait_hint_ns,
                                                      // wait_rounds failed tries (poll_rounds failed polls of an exchange word) give up
 };
-#ifndef MKKV_ABL
-#define MKKV_ABL 0 // experiments only (wrong results): 1 no unpack arithmetic, 2 no P arithmetic, 4 no tile maxima
-#endif
 #ifndef MKKV_TC_PROF
 #define MKKV_TC_PROF 0 // 1: compile the phase stamps in (they cost a few per cent)
 #endif
@@ -202,17 +192,19 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t * bar, unsigned pari
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void tc_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    if (mbar_try_wait_hint(bar, parity, 0u)) return; // (the common case: no limit loaded)
+// Returns whether the phase is complete.
+__device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
+    if (mbar_try_wait_hint(bar, parity, 0u)) return true; // (the common case: no limit loaded)
     const unsigned hint = wc->hint, rounds = wc->rounds;
     for (unsigned it = 0; !mbar_try_wait_hint(bar, parity, hint); it++) {
-        if (wc->dead) return;
+        if (wc->dead) return false;
         if (it >= rounds) {
             wc->dead = 1;
             atomicExch(status, (int) KS_WAIT_TIMEOUT);
-            return;
+            return false;
         }
     }
+    return true;
 }
 // Whether the CTA has given up, the same answer for all the lanes of mask. Another warp may set the flag between two lanes' reads: a
 // warp that leaves a loop with warp-wide operations in it leaves it by this vote (lanes that disagreed would wait for each other, some
@@ -236,9 +228,10 @@ __device__ __forceinline__ void drain_copies(uint64_t * raw_full, unsigned issue
 // Shared-memory matrix descriptors (no swizzle, version 1), as their 32-bit halves: the low half holds the start address and the
 // byte distance between the two 8-element groups along K of one instruction ("leading"), the high half the distance between 8-row
 // groups along M / N ("stride"). Only the low half changes between k-steps.
-// D[128 x 48] (+)= A B, fp16 operands, fp32 accumulate; MN: both operands MN-major, else both K-major
-constexpr unsigned IDESC_K = (1u << 4) | ((unsigned) (AR / 8) << 17) | ((unsigned) (GP / 16) << 24);
-constexpr unsigned IDESC_MN = (1u << 4) | (1u << 15) | (1u << 16) | ((unsigned) (2 * AR / 8) << 17) | ((unsigned) (GP / 16) << 24); // N = 96
+// fp16 operands, fp32 accumulate. S[64 (48 used) query rows x 128 positions] = Q K^T: both K-major; O^T[128 dims x 96] += V^T P^T:
+// V MN-major, P (48 rows' high parts, then their low parts) K-major
+constexpr unsigned IDESC_S = (1u << 4) | ((unsigned) (GP / 8) << 17) | ((unsigned) (64 / 16) << 24);
+constexpr unsigned IDESC_PV = (1u << 4) | (1u << 15) | ((unsigned) (2 * AR / 8) << 17) | ((unsigned) (128 / 16) << 24);
 __device__ __forceinline__ void umma(unsigned d_tmem, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi, unsigned idesc, unsigned accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\tsetp.ne.b32 p, %6, 0;\n\t"
@@ -266,30 +259,25 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// 8 consecutive columns, in flight until tmem_wait8 on the same registers (the wait names them so that no use can move above it)
-__device__ __forceinline__ void tmem_ld8_async(unsigned taddr, unsigned (&r)[8]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_wait8(unsigned (&r)[8]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
-}
-// 8 consecutive columns
-__device__ __forceinline__ void tmem_ld8(unsigned taddr, float (&v)[8]) {
-    unsigned r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+// Scores of two tiles, 64 columns of the 16 lanes from taddr's on: lanes 0 .. 15 get the first tile of their row, lanes 16 .. 31 the
+// second. (One statement with its wait: no use of the registers can move between the two.)
+__device__ __forceinline__ void tmem_scores(unsigned taddr, float (&s)[ATP]) {
+    unsigned r[ATP];
+    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32], 32;\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr)
+                 : "memory");
 #pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+    for (int i = 0; i < ATP; i++) s[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void tmem_st8(unsigned taddr, const float (&v)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(__float_as_uint(v[0])),
-                 "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])),
-                 "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+// 16 consecutive columns at each of two addresses
+__device__ __forceinline__ void tmem_ld16_two(unsigned ta, unsigned tb, unsigned (&v)[16], unsigned (&w)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]), "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+                 : "r"(ta), "r"(tb)
                  : "memory");
 }
 // exp(x), relative error about 2^-21 (scale factors applied alike to the accumulator and the row sums)
@@ -326,13 +314,6 @@ __device__ __forceinline__ float ex2(float x) { // 2^x for x <= 0 (and -inf -> 0
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// max over the warp (sm_100a: redux.sync on fp32)
-__device__ __forceinline__ float warp_max(float x) {
-    float r;
-    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
-    return r;
 }
 
 // bounded poll of an exchange word until it carries this launch's tag
@@ -398,10 +379,10 @@ __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool p) {
 __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int lane) {
     const int grid = (int) gridDim.x;
     int next_item = (int) blockIdx.x, pending = a.nitems; // (pending: lane 0's)
-    // current segment: chunks [c, c_end) of one kv head; current group b of chunk c
+    // current segment: positions [first_pos, end) of one kv head, a run of chunks; the current group starts at pos
     const AttnJob * const jobs = a.jobs ? a.jobs : &a.one;
     const AttnJob * J = jobs;
-    int g = 0, c = 0, c_end = 0, b = 0, slot = 0;
+    int g = 0, first_pos = 0, pos = 0, end = 0, slot = 0;
     auto next_segment = [&]() {
         const int item = next_item;
         if (a.nitems > grid && lane == 0) pending = grid + (int) atomicAdd(a.next, 1u);
@@ -426,9 +407,9 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
             g = rel / nit;
             run = rel - g * nit;
         }
-        c = J->c_lo + run * cpi;
-        c_end = min(c + cpi, J->c_lo + J->nch);
-        b = 0;
+        const int c = J->c_lo + run * cpi;
+        first_pos = pos = max(c * J->cs, J->pos_lo);
+        end = min(min(c + cpi, J->c_lo + J->nch) * J->cs, J->pos_hi);
         slot = J->item0 + g * J->nch + run;
     };
     // A single job comes with the launch's arguments: its first record and addresses are made while the launch before still runs, and
@@ -437,9 +418,8 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
     bool waiting = !a.jobs;
     if (!waiting) wait_previous();
     next_segment();
-    bool first = true;
     SideSrc ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-    int cs = J->cs, lo = J->pos_lo, hi = J->pos_hi, n = J->n, T = J->T;
+    int cs = J->cs, n = J->n, T = J->T;
     const uint16_t * qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
     auto tile_src = [&](const SideSrc & S, int tb, int c1) -> TileSrc {
         TileSrc t;
@@ -464,39 +444,44 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         TileSrc t;
         int nt;
         if (isK) {
-            const int c0 = max(c * cs, lo), c1 = min((c + 1) * cs, hi), ntc = (c1 - c0 + ATP - 1) / ATP, nb = (ntc + GT - 1) / GT;
-            const int pos0 = c0 + b * GP;
-            nt = min(GT, ntc - b * GT);
-            const bool seg_last = b + 1 == nb && c + 1 == c_end;
+            const int pos0 = pos, c1 = end, mine = pos0 + lane * ATP; // (the tiles of a run are consecutive, also across its chunks' bounds)
+            nt = min(GT, (c1 - pos0 + ATP - 1) / ATP);
+            const bool seg_last = c1 - pos0 <= GP;
+            const unsigned restart = __ballot_sync(FULL_MASK, lane < nt && (mine == first_pos || mine % cs == 0));
             if (seg_last) next_item = __shfl_sync(FULL_MASK, pending, 0);
             const bool cta_last = seg_last && next_item >= a.nitems;
             if (lane == 0) {
                 GroupRec & k = sm.tasks[nk % NTASK];
-                k.c = c, k.b = b, k.nb = nb, k.pos0 = pos0, k.c1 = c1, k.nt = nt;
+                k.pos0 = pos0, k.c1 = c1, k.nt = nt;
                 k.q = qp;
                 k.n = n, k.T = T, k.slot = slot;
-                k.flags = (first ? REC_FIRST : 0) | (seg_last ? REC_LAST : 0) | (cta_last ? REC_END : 0);
-                k.ring0[0] = ks.ring0, k.ring0[1] = vs.ring0;
-                k.bits[0] = ks.bits, k.bits[1] = vs.bits;
+                k.flags = (pos0 == first_pos ? REC_FIRST : 0) | (seg_last ? REC_LAST : 0) | (cta_last ? REC_END : 0);
+                k.restart = restart;
             }
-            if (lane < nt) {
-                t = tile_src(ks, pos0 + lane * ATP, c1);
-                sm.vsrc[nk % NTASK][lane] = tile_src(vs, pos0 + lane * ATP, c1);
+            if (lane < GT) {
+                const unsigned last = cta_last ? UD_END : 0u;
+                unsigned dk = last | (unsigned) ks.bits << 8, dv = last | (unsigned) vs.bits << 8; // (no row: any of the side's formats)
+                if (lane < nt) {
+                    t = tile_src(ks, mine, c1);
+                    const TileSrc v = tile_src(vs, mine, c1);
+                    sm.vsrc[nk % NTASK][lane] = v;
+                    dk = last | (unsigned) t.np | ((unsigned) t.rb << 3); // (32 bytes a row and bit: the bits 8 up)
+                    dv = last | (unsigned) v.np | ((unsigned) v.rb << 3);
+                }
+                sm.udesc[nk % NTASK][0][lane] = dk;
+                sm.udesc[nk % NTASK][1][lane] = dv;
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.rec_full[nk % NTASK]);
-            first = seg_last;
             if (cta_last) {
                 G = nk + 1;
             } else if (seg_last) {
                 next_segment();
                 ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-                cs = J->cs, lo = J->pos_lo, hi = J->pos_hi, n = J->n, T = J->T;
+                cs = J->cs, n = J->n, T = J->T;
                 qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
-            } else if (b + 1 == nb) {
-                c++, b = 0;
             } else {
-                b++;
+                pos += GP;
             }
         } else {
             nt = sm.tasks[nv % NTASK].nt;
@@ -518,6 +503,58 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         else nv++;
     }
     if (lane < GT) drain_copies(sm.raw_full, issued, NRAW / GT);
+}
+
+// Spread mode: the merge, in the kernel's tail: when every CTA of kv head g has written its partial, this CTA (kk-th of the head's cph)
+// merges rows kk and kk + cph of the head's 6 T. The softmax warps (mw), four to a row (warp j of the team: partials j, j + 4, ..: all
+// their loads are in flight at once); the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete).
+__device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int kk, int T, int mw, int lane) {
+    __threadfence();
+    named_bar(7, NSOFT * 32);
+    if (mw == 0 && lane == 0) {
+        bool ok = true;
+        atomicAdd(a.done + g, 1u);
+        unsigned it = 0;
+        while ((int) (ld_acquire_u32(a.done + g) - a.done_target) < 0) {
+            __nanosleep(100);
+            if (++it >= (sm.wc.poll << 2) || sm.wc.dead) { // (about a second)
+                atomicExch(a.status, (int) KS_WAIT_TIMEOUT);
+                ok = false;
+                break;
+            }
+        }
+        sm.merge_ok = ok;
+    }
+    named_bar(7, NSOFT * 32);
+#if MKKV_TC_PROF
+    if (mw == 0) TC_STAMP(15, 12);
+#endif
+    const int team = mw >> 2, tj = mw & 3, rr = kk + team * a.cph;
+    const bool has = sm.merge_ok && rr < GQ * T;
+    float * const scratch = reinterpret_cast<float *>(sm.op[0]); // [warp][lane][8 sums], then [warp] weights' sums
+    float num[8], den = 0.f, M = -CUDART_INF_F;
+    if (has) {
+        merge_accumulate<4>(a.part, a.ml, (size_t) g * a.cph, (size_t) AR * HD, (size_t) AR, a.cph, tj, 4, rr, lane, num, den, M);
+        float4 * d = reinterpret_cast<float4 *>(scratch + ((size_t) mw * 32 + lane) * 8);
+        d[0] = make_float4(num[0], num[1], num[2], num[3]);
+        d[1] = make_float4(num[4], num[5], num[6], num[7]);
+        if (lane == 0) scratch[NSOFT * 32 * 8 + mw] = den;
+    }
+    named_bar(7, NSOFT * 32);
+    if (has && tj == 0) {
+#pragma unroll
+        for (int w2 = 1; w2 < 4; w2++) {
+            const float4 * o = reinterpret_cast<const float4 *>(scratch + ((size_t) (mw + w2) * 32 + lane) * 8);
+            const float4 o0 = o[0], o1 = o[1];
+            num[0] += o0.x, num[1] += o0.y, num[2] += o0.z, num[3] += o0.w;
+            num[4] += o1.x, num[5] += o1.y, num[6] += o1.z, num[7] += o1.w;
+            den += scratch[NSOFT * 32 * 8 + mw + w2];
+        }
+        merge_finish(sm.job, g * GQ + rr / T, rr % T, lane, a.raw_part != nullptr, a.raw_part, a.raw_ml, num, den, M);
+    }
+#if MKKV_TC_PROF
+    if (mw == 0) TC_STAMP(15, 13);
+#endif
 }
 
 // KB / VB: the bits of the K / V main rows the instance is compiled for (0: any, decided per tile at run time). A compiled-in
@@ -612,6 +649,10 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                            // the copies' barriers order their reads after this write)
                     k = get_task(kk + nk * tstep);
                     if (lane == 0) static_cast<AttnTask &>(sm.tasks[nk % NTASK]) = k;
+                    const int tp = k.pos0 + lane * ATP;
+                    const unsigned np = lane < k.nt ? (unsigned) min(ATP, k.c1 - tp) : 0u;
+                    sm.udesc[nk % NTASK][0][lane] = np | (unsigned) (tp >= ksrc.ring0 ? 8 : ksrc.bits) << 8;
+                    sm.udesc[nk % NTASK][1][lane] = np | (unsigned) (tp >= vsrc.ring0 ? 8 : vsrc.bits) << 8;
                 } else {
                     k = sm.tasks[nv % NTASK];
                 }
@@ -651,11 +692,11 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 q_flight = true;
             };
             if (batch) fetch_queries(0);
-            const unsigned q_lo = desc_lo(smem_u32(sm.q), AR / 8 * 128), p_lo0 = desc_lo(smem_u32(sm.p[0]), 128);
-            const unsigned hi_k = desc_hi(128), hi_mn = desc_hi(2048); // K-major: 8-row groups 128 bytes apart; MN-major: 2048
+            const unsigned q_lo = desc_lo(smem_u32(sm.q), AR / 8 * 128), p_lo = desc_lo(smem_u32(sm.p), P_KGROUP);
+            const unsigned hi_128 = desc_hi(128), hi_2048 = desc_hi(2048); // K-major: 8-row groups 128 bytes apart; V, MN-major: 2048
             for (int nk = 0, nv = 0; nv < G && !sm.wc.dead;) {
                 const bool isK = nk < G && nk < nv + NSB;
-                if (isK) { // S^T(nk) = K Q^T
+                if (isK) { // S(nk) = Q K^T
                     const int sb = nk % NSB;
                     if (nk >= NSB) tc_wait(&sm.s_empty[sb], ((nk / NSB) - 1) & 1, &sm.wc, a.status);
                     if (batch && q_flight) {
@@ -663,16 +704,16 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                         if (sm.wc.dead) break;
                         q_ph ^= 1, q_flight = false;
                     }
-                    const unsigned dcol = tb + S_COL + S_STRIDE * sb;
+                    const unsigned dcol = tb + S_COL + S_STRIDE * (sb >> 1) + ((unsigned) (16 * (sb & 1)) << 16);
 #pragma unroll 1
                     for (int h = 0; h < 2; h++, oseq++) {
                         const int os = oseq % NOP;
                         tc_wait(&sm.op_full[os], (oseq / NOP) & 1, &sm.wc, a.status);
                         tc_fence_after();
-                        const unsigned a_lo = desc_lo(smem_u32(sm.op[os]), 2048), b_lo = q_lo + ((8 * h) * (2 * AR / 8 * 128) >> 4);
+                        const unsigned k_lo = desc_lo(smem_u32(sm.op[os]), 2048), qh_lo = q_lo + ((8 * h) * (2 * AR / 8 * 128) >> 4);
 #pragma unroll
                         for (int ks = 0; ks < 8; ks++)
-                            umma(dcol, a_lo + (ks * 4096 >> 4), hi_k, b_lo + (ks * (2 * AR / 8 * 128) >> 4), hi_k, IDESC_K, (unsigned) (h | ks));
+                            umma(dcol, qh_lo + (ks * (2 * AR / 8 * 128) >> 4), hi_128, k_lo + (ks * 4096 >> 4), hi_128, IDESC_S, (unsigned) (h | ks));
                         umma_commit(&sm.op_empty[os]);
                     }
                     umma_commit(&sm.s_full[sb]);
@@ -700,10 +741,10 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                         if (h == 0) TC_STAMP(nv, 18);
 #endif
                         tc_fence_after();
-                        const unsigned a_lo = desc_lo(smem_u32(sm.op[os]), 128), dcol = tb + (h ? O_COL1 : O_COL0);
+                        const unsigned v_lo = desc_lo(smem_u32(sm.op[os]), 128), dcol = tb + (h ? O_COL1 : O_COL0);
 #pragma unroll
-                        for (int ks = 0; ks < 8; ks++) // B: the 48 rows of P's high part, then the 48 of its low part (12 row groups)
-                            umma(dcol, a_lo + (ks * 256 >> 4), hi_mn, p_lo0 + (ks * 256 >> 4), hi_mn, IDESC_MN, (unsigned) (!fresh || ks));
+                        for (int ks = 0; ks < 8; ks++)
+                            umma(dcol, v_lo + (ks * 256 >> 4), hi_2048, p_lo + (ks * (2 * P_KGROUP) >> 4), hi_128, IDESC_PV, (unsigned) (!fresh || ks));
                         umma_commit(&sm.op_empty[os]);
                     }
                     umma_commit(&sm.p_empty);
@@ -723,423 +764,377 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
     }
     } else if (warp >= NSOFT) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_DQ ";");
-        // ---- unpack warps: packed rows -> operand slots, both 128-dim halves of one side of a group at a time ----
+        // ---- unpack warps: packed rows -> operand slots, both 128-dim halves of one side of a group at a time, in the producer's order.
+        // They bound the kernel (5,200 of a group's 6,500 cycles at work, 6.4 cycles an instruction), so everything besides the
+        // values' arithmetic is kept out of the loop: a side's body knows its format, a tile is one descriptor word, the bias constants
+        // stay in registers ----
         const int w = warp - NSOFT, q = w & 3, c = w >> 2, prow = ATP * q + lane;
         const unsigned pos_off = (prow >> 3) * 128 + (prow & 7) * 16; // the position's 16-byte unit inside a dim group
+        const UnpackConst uc = unpack_const();
+        const unsigned raw_q = smem_u32(sm.raw[q]), op0 = smem_u32(sm.op[0]) + pos_off;
         const bool st = w == 0;
-        int rs = q, rph = 0, os = 0, oph = 0; // raw slot / phase of this warp's tile, operand slot / phase
-        bool owrap = false;
-        for (int nk = 0, nv = 0; nv < G;) {
-            const bool isK = nk < G && nk < nv + NSB;
-            const int side = isK ? 0 : 1, grp = isK ? nk - NSB : nv;
-            (void) grp; // (the stamps' group index)
-            if (st) TC_STAMP(grp, side ? 8 : 11);
-            tc_wait(&sm.raw_full[rs], rph, &sm.wc, a.status);
-            if (gave_up(FULL_MASK, &sm.wc)) break;
-            if (st) TC_STAMP(grp, side ? 9 : 12);
-            const GroupRec & kr = sm.tasks[(isK ? nk : nv) % NTASK];
-            if (batch && isK && (kr.flags & REC_END)) G = nk + 1;
-            const int k_pos0 = kr.pos0;
-            const int2 kt = *reinterpret_cast<const int2 *>(&kr.c1); // c1, nt
-            const int tbq = k_pos0 + q * ATP;
-            const bool valid = q < kt.y && lane < kt.x - tbq;
-            const int bits = batch ? (tbq >= kr.ring0[side] ? 8 : kr.bits[side]) : (kv.s[side].rval && tbq >= ws) ? 8 : kv.s[side].bits;
-            // which 32-dim blocks of a half this lane unpacks: the warps of a tile cover the four blocks of every row, rotated with
+        (void) st;
+        unsigned rseq = 0, os = 0, oph = 1; // this warp's tiles so far (its two raw slots in turn), operand slot / parity of its "empty" wait
+        auto hand_over = [&]() {
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.op_full[os]);
+            if (++os == NOP) os = 0, oph ^= 1;
+        };
+        auto unpack_tile = [&](auto bits_c, unsigned rawa, bool valid) {
+            constexpr int B = decltype(bits_c)::value;
+            // which 32-dim block of a half this lane unpacks: the warps of a tile cover the four blocks of every row, rotated with
             // the row so that the 16-byte loads of 8 consecutive lanes (rows 32 bits bytes apart) fall into 8 different bank groups
-            const int jr = (c + (lane >> (bits == 6 ? 1 : (bits == 5 || bits == 7) ? 2 : 0))) & 3;
+            const int jr = (c + (lane >> (B == 6 ? 1 : (B == 5 || B == 7) ? 2 : 0))) & 3;
             // the packed bytes of both 128-dim halves are read first (they need no operand slot), then each half is written into its
             // slot as that slot frees up
-            const unsigned rawa = smem_u32(sm.raw[rs]);
-#define MKKV_SIDE(B)                                                                                                   \
-    {                                                                                                                  \
-        PackedBlock<B> b0[BPW], b1[BPW];                                                                               \
-        _Pragma("unroll") for (int k = 0; k < BPW; k++) {                                                              \
-            dq_load<B>(b0[k], rawa, lane, (jr + k * (NDQ / 4)) & 3, valid);                                            \
-            dq_load<B>(b1[k], rawa, lane, 4 + ((jr + k * (NDQ / 4)) & 3), valid);                                      \
-        }                                                                                                              \
-        if (owrap) tc_wait(&sm.op_empty[os], oph ^ 1, &sm.wc, a.status);                                               \
-        if (!(MKKV_ABL & 1))                                                                                           \
-            _Pragma("unroll") for (int k = 0; k < BPW; k++)                                                            \
-                dq_emit<B>(b0[k], smem_u32(sm.op[os]) + 4 * ((jr + k * (NDQ / 4)) & 3) * 2048 + pos_off);              \
-        fence_async_smem();                                                                                            \
-        __syncwarp();                                                                                                  \
-        if (lane == 0) mbar_arrive(&sm.op_full[os]);                                                                   \
-        if (++os == NOP) os = 0, oph ^= 1, owrap = true;                                                               \
-        if (owrap) tc_wait(&sm.op_empty[os], oph ^ 1, &sm.wc, a.status);                                               \
-        if (!(MKKV_ABL & 1))                                                                                           \
-            _Pragma("unroll") for (int k = 0; k < BPW; k++)                                                            \
-                dq_emit<B>(b1[k], smem_u32(sm.op[os]) + 4 * ((jr + k * (NDQ / 4)) & 3) * 2048 + pos_off);              \
-        fence_async_smem();                                                                                            \
-        __syncwarp();                                                                                                  \
-        if (lane == 0) mbar_arrive(&sm.op_full[os]);                                                                   \
-        if (++os == NOP) os = 0, oph ^= 1, owrap = true;                                                               \
-    }
-            const int fixed = side ? VB : KB; // the side's compiled-in main format, or 0: any
-            if (bits == 8) MKKV_SIDE(8)
-            else if (fixed == 4 || (!fixed && bits == 4)) MKKV_SIDE(4)
-            else if (fixed == 5 || (!fixed && bits == 5)) MKKV_SIDE(5)
-            else if (fixed == 6 || (!fixed && bits == 6)) MKKV_SIDE(6)
-            else if (fixed == 7 || !fixed) MKKV_SIDE(7)
-#undef MKKV_SIDE
+            PackedBlock<B> b0, b1;
+            dq_load<B>(b0, rawa, lane, jr, valid);
+            dq_load<B>(b1, rawa, lane, 4 + jr, valid);
+            tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
+            dq_emit<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048);
+            hand_over();
+            tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
+            dq_emit<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048);
+            hand_over();
+        };
+        // one side of group j; false: the CTA has given up
+        auto unpack_side = [&](auto side_c, int j, unsigned & ud) -> bool {
+            constexpr int SIDE = decltype(side_c)::value, FIXED = SIDE ? VB : KB; // the side's compiled-in main format, or 0: any
+            const unsigned rs = q + GT * (rseq & 1);
+            if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 8 : 11);
+            if (!__all_sync(FULL_MASK, tc_wait(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status))) return false;
+            if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 9 : 12);
+            ud = sm.udesc[j % NTASK][SIDE][q];
+            const bool valid = lane < (int) (ud & UD_ROWS);
+            const int bits = (int) (ud >> 8);
+            const unsigned rawa = raw_q + (rseq & 1) * (GT * RAW_SLOT);
+            if (bits == 8) unpack_tile(IntC<8>{}, rawa, valid);
+            else if (FIXED == 4 || (!FIXED && bits == 4)) unpack_tile(IntC<4>{}, rawa, valid);
+            else if (FIXED == 5 || (!FIXED && bits == 5)) unpack_tile(IntC<5>{}, rawa, valid);
+            else if (FIXED == 6 || (!FIXED && bits == 6)) unpack_tile(IntC<6>{}, rawa, valid);
+            else if (FIXED == 7 || !FIXED) unpack_tile(IntC<7>{}, rawa, valid);
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.raw_empty[rs]);
-            if (st) TC_STAMP(grp, side ? 10 : 13);
-            rs += GT;
-            if (rs >= NRAW) rs -= NRAW, rph ^= 1;
-            if (isK) nk++;
-            else nv++;
+            if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 10 : 13);
+            rseq++;
+            return true;
+        };
+        for (int it = -NSB; it < G; it++) { // K(0) .. K(NSB - 1), then V(it), K(it + NSB)
+            unsigned ud;
+            if (it >= 0 && !unpack_side(IntC<1>{}, it, ud)) break;
+            if (it + NSB < G) {
+                if (!unpack_side(IntC<0>{}, it + NSB, ud)) break;
+                if (batch && (ud & UD_END)) G = it + NSB + 1;
+            }
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
 #if MKKV_TC_PROF
         const unsigned long long t_loop = globaltimer_ns();
 #endif
-        // ---- softmax warps: warp = 4 c2 + q: positions 32 q .. + 31 of a group (tensor-memory lanes 32 q ..), query rows
-        // 24 c2 .. + 23. Lanes 0 .. 23 own one row each (its running / reference max; replicated over the four q) ----
-        const int q = warp & 3, c2 = warp >> 2, prow = ATP * q + lane, row0 = RS * c2;
-        const unsigned pos_off = (prow >> 3) * 128 + (prow & 7) * 16;
+        // ---- softmax warps: warp 4 h2 + q holds query rows 16 q .. + 15 of tiles 2 h2 and 2 h2 + 1; a thread owns row r_own and one tile:
+        // the running maxima, the reference max and the row sum are plain registers, kept alike by the four threads of a row. Warps
+        // without a row of the job (rows 48 .. 63 never are one's) only take part in the accumulator's read-out and rescaling, where a
+        // warp's lanes are dims of half h2. (One warp per 16 rows, two tiles a thread: about 650 instructions in a row, 5,100 of a
+        // group's 6,500 cycles.) ----
+        const int q = warp & 3, h2 = warp >> 2, hf = lane >> 4, tile = 2 * h2 + hf, r_own = 16 * q + (lane & 15);
         const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
-        const bool owner = lane < RS, st = warp == 0;
-        const int r_own = row0 + (owner ? lane : 0);
-        WarpScratch & W = sm.ws[warp];
-        F2 l_acc[RS / 2]; // row sums of the thread's position, rows (2 j, 2 j + 1)
-#pragma unroll
-        for (int i = 0; i < RS / 2; i++) l_acc[i] = 0ull;
-        float m_acc = -CUDART_INF_F, carry = -CUDART_INF_F; // (carry: batch mode, the chunk's running max after the previous group)
+        const bool st = warp == 0, lead = h2 == 0 && hf == 0; // (lead: the row's first thread)
+        float l_acc = 0.f, m_acc = -CUDART_INF_F; // row sum over the thread's tiles, reference max
+        float carry = -CUDART_INF_F;              // (batch mode: the running max after the previous group)
         unsigned long long w0 = 0, w1 = 0, w2 = 0;
         auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
         // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
         // producer never reached are not valid) and only inside their bounds
         auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
-        // which of the warp's rows this thread's position must not see in group k: row token t sees positions <= n + t, positions past
-        // the chunk end see nothing (0 for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their
-        // queries are zero, so are their scores, and no one reads what becomes of them. A group that ends its chunk but lies before the
-        // new tokens is one test for all rows: chunks shorter than a group (contexts up to 1,920 positions) have no other groups, and
-        // with the row loop for each of them 16 layers of 1,187 positions took 60.3 us instead of 53.5, one call 2 us more.
-        const int tok0 = batch ? 0 : row0 % T; // token of the warp's first row (row = (head % 6) T + t)
-        auto row_mask = [&](const GroupRec & k) -> unsigned {
-            const int Tk = batch ? k.T : T, nn = batch ? k.n : n;
-            unsigned m = 0u;
-            if (k.pos0 + GP - 1 > min(k.c1 - 1, nn)) { // (the group reaches the chunk's end or the new tokens)
-                const int p_abs = k.pos0 + prow;
-                if (k.c1 - 1 <= nn) return p_abs >= k.c1 ? (1u << RS) - 1u : 0u;
-                int t = batch ? row0 % Tk : tok0;
-#pragma unroll 1
-                for (int i = 0; i < RS; i++) {
-                    if (p_abs > min(k.c1 - 1, nn + t)) m |= 1u << i;
-                    if (++t == Tk) t = 0;
-                }
-            }
-            return m;
+        // the thread's tile (and its neighbour) in the S buffer of group j: rows on 16 lanes of the warp's quarter (the other 16 are the
+        // neighbouring buffer's), positions on columns
+        auto s_addr = [&](int j) -> unsigned {
+            return lane_addr + S_COL + S_STRIDE * ((j % NSB) >> 1) + 2 * ATP * h2 + ((unsigned) (16 * (j & 1)) << 16);
         };
-        // rows row0 + 8 gq .. + 7 of S^T of group j: request, then (after the wait) as masked floats
-        auto scores_request = [&](int j, int gq, unsigned (&r)[8]) { tmem_ld8_async(lane_addr + S_COL + S_STRIDE * (j % NSB) + row0 + 8 * gq, r); };
-        auto scores_take = [&](unsigned (&r)[8], unsigned mask, bool masked, int gq, float (&s)[8]) {
-            tmem_wait8(r);
+        // the last of the tile's positions that the row sees: row token t sees positions <= n + t, nothing is visible past the chunk end
+        // (all of them for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their queries are zero, so
+        // are their scores, and no one reads what becomes of them.
+        auto last_visible = [&](const GroupRec & k, int nn, int Tk) -> int {
+            if (k.pos0 + GP - 1 <= min(k.c1 - 1, nn)) return ATP; // (the group reaches neither the chunk's end nor the new tokens)
+            return min(k.c1 - 1, nn + r_own % Tk) - k.pos0 - ATP * tile;
+        };
+        auto mask_tile = [&](int lim, float (&s)[ATP]) {
+            if (__any_sync(FULL_MASK, lim < ATP)) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) s[i] = __uint_as_float(r[i]);
-            if (masked) {
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    if ((mask >> (8 * gq + i)) & 1u) s[i] = -CUDART_INF_F;
+                for (int c = 0; c < ATP; c++)
+                    if (c > lim) s[c] = -CUDART_INF_F;
             }
         };
-        // tile maxima of group j, its own maxima published, the words its running max will need requested
-        // (batch mode: returns false when a wait of the CTA gave up, the same for all four warps of a slice, which meet at its barrier:
-        // the record and everything derived from it is only used after a true)
-        auto maxima = [&](int j) -> bool {
-            if (st) TC_STAMP(j, 0);
-            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
-            const GroupRec k = sm.tasks[j % NTASK];
-            if (st) TC_STAMP(j, 1);
-            tc_fence_after();
-#if !(MKKV_ABL & 4)
-            unsigned rq[RS / 8][8];
+        // maxima of the four tiles of group j in the thread's row (act: s holds the tile's scores). A barrier of the row's two warps, which
+        // they meet at whatever the group's record says (after a give-up the two may read different records)
+        auto tile_maxima = [&](int j, bool act, const float (&s)[ATP]) -> float4 {
+            float(&tm)[GT][AR] = sm.tmax[j & 1]; // (read again by nobody when group j + 2 writes it: the barrier of j + 1 is between)
+            const float4 none = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+            if (q == AR / 16) return none;
+            if (act) {
+                float x[ATP / 2];
 #pragma unroll
-            for (int gq = 0; gq < RS / 8; gq++) scores_request(j, gq, rq[gq]);
-            const unsigned mask = row_mask(k);
-            const bool masked = __any_sync(FULL_MASK, mask != 0u);
+                for (int c = 0; c < ATP / 2; c++) x[c] = fmaxf(s[2 * c], s[2 * c + 1]);
 #pragma unroll
-            for (int gq = 0; gq < RS / 8; gq++) {
-                float s[8];
-                scores_take(rq[gq], mask, masked, gq, s);
-                float mx[8];
+                for (int o = ATP / 4; o > 0; o >>= 1)
 #pragma unroll
-                for (int i = 0; i < 8; i++) mx[i] = warp_max(s[i]);
-                if (lane == 0) {
-                    float4 * d = reinterpret_cast<float4 *>(&sm.tmax[j & 3][q][row0 + 8 * gq]);
-                    d[0] = make_float4(mx[0], mx[1], mx[2], mx[3]);
-                    d[1] = make_float4(mx[4], mx[5], mx[6], mx[7]);
-                }
+                    for (int c = 0; c < o; c++) x[c] = fmaxf(x[c], x[c + o]);
+                tm[tile][r_own] = x[0];
             }
-#endif
-            if (batch) {
-                if (named_bar_or(1 + c2, GT * 32, sm.wc.dead != 0)) return false;
-                if (k.flags & REC_END) G = j + 1;
-                return true;
-            }
-            named_bar(1 + c2, GT * 32);
-            if (!batch && owner && q == 0 && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k)) {
-                const float(&tm)[GT][AR] = sm.tmax[j & 3];
-                const float gk = fmaxf(fmaxf(tm[0][r_own], tm[1][r_own]), fmaxf(tm[2][r_own], tm[3][r_own]));
-                __stcg(a.xa + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(gk));
-            }
-            if (st) TC_STAMP(j, 2);
-            return true;
-        };
-        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
-        // the chunk's previous groups have most likely published them
-        auto request_words = [&](const Task & k) {
-            if (!batch && owner && k.nb > 1 && exch_ok(k)) {
-                const size_t xb0 = xbase(k);
-                if (k.b >= 1) w1 = __ldcv(a.xa + xb0 + (size_t) (k.b - 1) * AR);
-                if (k.b >= 2) w2 = __ldcv(a.xa + xb0 + (size_t) (k.b - 2) * AR);
-                if (k.b >= 3) w0 = __ldcv(a.xb + xb0 + (size_t) (k.b - 3) * AR);
-            }
+            named_bar(1 + q, 64);
+            return act ? make_float4(tm[0][r_own], tm[1][r_own], tm[2][r_own], tm[3][r_own]) : none;
         };
         // batch mode: the partial of a finished segment (O^T lanes are dims in the unpacked units' order, columns are query rows), read
         // out when its last P V is complete and before the next P allows the MMA that overwrites O^T: between the two the tensor cores
-        // and the unpack warps stand still, so the next group's exponentials are computed first and the loads go out half by half
+        // and the unpack warps stand still, so the next group's exponentials are computed first
         int flush_slot = -1, flush_rows = 0;
-        const int pdim = (prow & ~7) | unit_perm(prow & 7);
-        auto flush = [&]() {
+        const int prow = ATP * q + lane, pdim = (prow & ~7) | unit_perm(prow & 7);
+        auto read_out = [&](int to_slot, int rows, bool any) {
+            const unsigned col0 = lane_addr + (h2 ? O_COL1 : O_COL0);
+            float * dst = a.part + (size_t) to_slot * AR * HD + 128 * h2 + pdim;
 #pragma unroll 1
-            for (int h = 0; h < 2; h++) {
-                unsigned v[RS / 8][8], w[RS / 8][8];
+            for (int r0 = 0; r0 < rows; r0 += 16, dst += 16 * HD) {
+                unsigned v[16], w[16];
+                if (any) tmem_ld16_two(col0 + r0, col0 + r0 + AR, v, w);
 #pragma unroll
-                for (int gq = 0; gq < RS / 8; gq++) {
-                    tmem_ld8_async(lane_addr + (h ? O_COL1 : O_COL0) + row0 + 8 * gq, v[gq]);
-                    tmem_ld8_async(lane_addr + (h ? O_COL1 : O_COL0) + AR + row0 + 8 * gq, w[gq]);
-                }
-                float * dst = a.part + ((size_t) flush_slot * AR + row0) * HD + 128 * h + pdim;
-#pragma unroll
-                for (int gq = 0; gq < RS / 8; gq++) {
-                    tmem_wait8(v[gq]);
-                    tmem_wait8(w[gq]);
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (row0 + 8 * gq + j < flush_rows) dst[(8 * gq + j) * HD] = __uint_as_float(v[gq][j]) + __uint_as_float(w[gq][j]);
-                }
+                for (int j = 0; j < 16; j++)
+                    if (r0 + j < rows) dst[j * HD] = any ? __uint_as_float(v[j]) + __uint_as_float(w[j]) : 0.f;
             }
-            flush_slot = -1;
         };
-        // P of group i
-        auto softmax = [&](int i, const GroupRec & k) {
-            if (st) TC_STAMP(i, 3);
-            float beta = 0.f, f = 1.f;
-            if (owner && !(MKKV_ABL & 8)) {
-                float m_in = batch && k.b > 0 ? carry : -CUDART_INF_F;
-                const size_t xb0 = xbase(k);
-                const bool alive = exch_ok(k);
-                if (alive && !batch && k.nb > 1) {
-                    if (k.b >= 1) m_in = poll_word(a.xa + xb0 + (size_t) (k.b - 1) * AR, w1, a.epoch, &sm.wc, a.status);
-                    if (k.b >= 2) m_in = fmaxf(m_in, poll_word(a.xa + xb0 + (size_t) (k.b - 2) * AR, w2, a.epoch, &sm.wc, a.status));
-                    if (k.b >= 3) m_in = fmaxf(m_in, poll_word(a.xb + xb0 + (size_t) (k.b - 3) * AR, w0, a.epoch, &sm.wc, a.status));
+        // P of group i, whose tile maxima (tm) are known; take(s): the masked scores of the thread's tile. restart: bit t: tile t opens a
+        // chunk, the running max starts anew. Returns false when a wait of the CTA gave up (batch mode; the same answer for all eight
+        // warps: nothing that the group's record says leaves the warp's registers before a true).
+        auto softmax = [&](int i, bool act, float m_in, unsigned restart, const float4 & tm, auto && take) -> bool {
+            // running maxima after each tile; M: the largest of them
+            const float r0 = (restart & 1u) ? tm.x : fmaxf(m_in, tm.x), r1 = (restart & 2u) ? tm.y : fmaxf(r0, tm.y);
+            const float r2 = (restart & 4u) ? tm.z : fmaxf(r1, tm.z), r3 = (restart & 8u) ? tm.w : fmaxf(r2, tm.w);
+            const float M = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
+            carry = r3;
+            bool moved = false;
+            if (act && M != -CUDART_INF_F) {
+                if (m_acc == -CUDART_INF_F) m_acc = M - REF_BELOW;
+                else if (M > m_acc + REF_SLACK) { // the reference max moves: the row sums follow at once, the accumulator when it is at rest (below)
+                    const float f = exp_any(m_acc - (M - REF_BELOW));
+                    m_acc = M - REF_BELOW;
+                    l_acc *= f;
+                    moved = true;
+                    if (lead) sm.resc_f[i & 1][r_own] = f;
                 }
-                if (st) TC_STAMP(i, 7);
-                const float(&tm)[GT][AR] = sm.tmax[i & 3];
-                float mr = m_in; // running max after this warp's tile, M: after the whole group
-#pragma unroll
-                for (int t = 0; t < GT; t++)
-                    if (t <= q) mr = fmaxf(mr, tm[t][r_own]);
-                float M = mr;
-#pragma unroll
-                for (int t = 0; t < GT; t++)
-                    if (t > q) M = fmaxf(M, tm[t][r_own]);
-                if (alive && !batch && q == 0 && k.nb > 1 && k.b + 3 < k.nb) __stcg(a.xb + xb0 + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(M));
-                carry = M;
-                if (M != -CUDART_INF_F) {
-                    if (m_acc == -CUDART_INF_F) m_acc = M - REF_BELOW;
-                    else if (M > m_acc + REF_SLACK) {
-                        f = exp_any(m_acc - (M - REF_BELOW));
-                        m_acc = M - REF_BELOW;
-                    }
-                }
-                beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);
-                W.nm[lane] = mr == -CUDART_INF_F ? -CUDART_INF_F : -mr;
-                W.beta[lane] = beta;
-                W.f[lane] = f;
             }
-            if (st) TC_STAMP(i, 14);
-            const float bnext = __shfl_down_sync(FULL_MASK, beta, 1);
-            if (owner && !(lane & 1)) {
-                const __half2 bh = __floats2half2_rn(beta, bnext);
-                const float2 bf = __half22float2(bh);
-                const __half2 bl = __floats2half2_rn(beta - bf.x, bnext - bf.y);
-                W.bh[lane >> 1] = *reinterpret_cast<const unsigned *>(&bh);
-                W.bl[lane >> 1] = *reinterpret_cast<const unsigned *>(&bl);
-            }
-            const unsigned anyf = __ballot_sync(FULL_MASK, owner && f != 1.f);
-            __syncwarp();
+            const unsigned rows_moved = __ballot_sync(FULL_MASK, moved) & 0xffffu;
+            if (lead && lane == 0) sm.resc_rows[i & 1][q] = rows_moved;
             if (st) TC_STAMP(i, 4);
-            if (anyf) { // a reference max moved: the row sums follow at once, the accumulator when it is at rest (below)
+            unsigned hi[ATP / 2], lo[ATP / 2]; // positions (2 c, 2 c + 1) of the tile
+            if (act) {
+                float s[ATP];
+                take(s);
+                const float mr = tile == 0 ? r0 : tile == 1 ? r1 : tile == 2 ? r2 : r3;
+                const float beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);
+                const float nm = mr == -CUDART_INF_F ? mr : -mr; // (nothing visible yet: exp2 gives 0)
+                const F2 nmv = f2_pack(nm, nm);
+                const __half bhs = __float2half_rn(beta);
+                const __half2 bh = __half2half2(bhs), bl = __half2half2(__float2half_rn(beta - __half2float(bhs)));
+                F2 sum0 = 0ull, sum1 = 0ull;
 #pragma unroll
-                for (int j = 0; j < RS / 2; j++) l_acc[j] = f2_mul(l_acc[j], f2_pack(W.f[2 * j], W.f[2 * j + 1]));
-            }
-            // P of the group into registers: the exponentials do not wait for the P buffer
-            const unsigned mask = row_mask(k);
-            const bool masked = __any_sync(FULL_MASK, mask != 0u);
-            unsigned ra[8], rb[8], hi[RS / 8][4], lo[RS / 8][4];
-            scores_request(i, 0, ra);
-#pragma unroll
-            for (int gq = 0; gq < RS / 8; gq++) { // row groups of 8: one 16-byte unit of each P part; the next group's scores are in
-                                                  // flight while this one's P is computed
-                float s[8];
-                if (gq + 1 < RS / 8) {
-                    if (gq & 1) {
-                        scores_take(rb, mask, masked, gq, s);
-                        scores_request(i, gq + 1, ra);
-                    } else {
-                        scores_take(ra, mask, masked, gq, s);
-                        scores_request(i, gq + 1, rb);
-                    }
-                } else {
-                    scores_take((gq & 1) ? rb : ra, mask, masked, gq, s);
-                }
-                if (gq == RS / 8 - 1) { // the last read of this S^T buffer
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sm.s_empty[i % NSB]);
-                }
-#if MKKV_ABL & 2
-                for (int j = 0; j < 4; j++) hi[gq][j] = lo[gq][j] = __float_as_uint(s[j]);
-                continue;
-#endif
-                const ulonglong2 ma = *reinterpret_cast<const ulonglong2 *>(&W.nm[8 * gq]), mb = *reinterpret_cast<const ulonglong2 *>(&W.nm[8 * gq + 4]);
-                const ulonglong2 ba = *reinterpret_cast<const ulonglong2 *>(&W.beta[8 * gq]), bb = *reinterpret_cast<const ulonglong2 *>(&W.beta[8 * gq + 4]);
-                const uint4 bhv = *reinterpret_cast<const uint4 *>(&W.bh[4 * gq]), blv = *reinterpret_cast<const uint4 *>(&W.bl[4 * gq]);
-                const F2 nm[4] = {ma.x, ma.y, mb.x, mb.y}, be[4] = {ba.x, ba.y, bb.x, bb.y};
-                const unsigned bhw[4] = {bhv.x, bhv.y, bhv.z, bhv.w}, blw[4] = {blv.x, blv.y, blv.z, blv.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
+                for (int c = 0; c < ATP / 2; c++) {
                     float p0, p1;
-                    f2_unpack(f2_mul(f2_add(f2_pack(s[2 * j], s[2 * j + 1]), nm[j]), f2_pack(LOG2E, LOG2E)), p0, p1);
+                    f2_unpack(f2_mul(f2_add(f2_pack(s[2 * c], s[2 * c + 1]), nmv), f2_pack(LOG2E, LOG2E)), p0, p1);
                     p0 = ex2(p0), p1 = ex2(p1);
-                    l_acc[4 * gq + j] = f2_fma(be[j], f2_pack(p0, p1), l_acc[4 * gq + j]);
+                    if (c & 1) sum1 = f2_add(sum1, f2_pack(p0, p1));
+                    else sum0 = f2_add(sum0, f2_pack(p0, p1));
                     const __half2 ph = __floats2half2_rn(p0, p1); // the reference's fp16 P
-                    const __half2 bh = *reinterpret_cast<const __half2 *>(&bhw[j]), bl = *reinterpret_cast<const __half2 *>(&blw[j]);
-                    const __half2 hh = __hmul2(ph, bh);                 // P beta = hh + ll up to 2^-22: the product's exact residual
+                    const __half2 hh = __hmul2(ph, bh);           // P beta = hh + ll up to 2^-22: the product's exact residual
                     const __half2 ll = __hfma2(ph, bl, __hfma2(ph, bh, __hneg2(hh))); // plus the low part of beta
-                    hi[gq][j] = *reinterpret_cast<const unsigned *>(&hh);
-                    lo[gq][j] = *reinterpret_cast<const unsigned *>(&ll);
+                    hi[c] = *reinterpret_cast<const unsigned *>(&hh);
+                    lo[c] = *reinterpret_cast<const unsigned *>(&ll);
                 }
+                float x0, x1;
+                f2_unpack(f2_add(sum0, sum1), x0, x1);
+                l_acc = __fmaf_rn(beta, x0 + x1, l_acc);
+            }
+            if constexpr (!BATCH) { // (the last read of this S buffer)
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.s_empty[i % NSB]);
             }
             if (st && i < 15) TC_STAMP(i, 15);
+            const bool anyf = named_bar_or(5, NSOFT * 32, rows_moved != 0u || (batch && sm.wc.dead != 0));
+            if (batch && anyf && named_bar_or(6, NSOFT * 32, sm.wc.dead != 0)) return false;
             if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
             if (st) TC_STAMP(i, 5);
             tc_fence_after();
 #if MKKV_TC_PROF
-            if (anyf && a.prof && st && lane == 0) a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 15] += 1ull | ((unsigned long long) __popc(anyf) << 32);
+            if (anyf && a.prof && st && lane == 0) a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 15] += 1ull;
 #endif
-            if (batch && flush_slot >= 0) flush(); // (a segment's first group: no reference max moves at it)
-            if (anyf) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference:
-                        // a row is one column in each of the four blocks (two halves x high / low part); the four loads of a row
-                        // are in flight together
-                unsigned left = anyf;
+            if (batch && flush_slot >= 0) { // (a segment's first group: no reference max moves at it)
+                read_out(flush_slot, flush_rows, true);
+                flush_slot = -1;
+            }
+            if (anyf) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference: of a
+                        // row and half, one column of the high and one of the low part
 #pragma unroll 1
-                while (left) {
-                    const int r = __ffs(left) - 1;
-                    left &= left - 1;
-                    const float fr = W.f[r];
-                    const unsigned ad = lane_addr + row0 + r;
-                    unsigned v0, v1, v2, v3;
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v0) : "r"(ad + O_COL0));
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v1) : "r"(ad + O_COL0 + AR));
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v2) : "r"(ad + O_COL1));
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v3) : "r"(ad + O_COL1 + AR));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v0), "+r"(v1), "+r"(v2), "+r"(v3)::"memory");
-                    v0 = __float_as_uint(__uint_as_float(v0) * fr), v1 = __float_as_uint(__uint_as_float(v1) * fr);
-                    v2 = __float_as_uint(__uint_as_float(v2) * fr), v3 = __float_as_uint(__uint_as_float(v3) * fr);
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0), "r"(v0) : "memory");
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0 + AR), "r"(v1) : "memory");
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1), "r"(v2) : "memory");
-                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1 + AR), "r"(v3) : "memory");
+                for (int qq = 0; qq < AR / 16; qq++) {
+                    unsigned left = sm.resc_rows[i & 1][qq];
+#pragma unroll 1
+                    while (left) {
+                        const int r = 16 * qq + __ffs(left) - 1;
+                        left &= left - 1;
+                        const float fr = sm.resc_f[i & 1][r];
+                        const unsigned ad = lane_addr + (h2 ? O_COL1 : O_COL0) + r;
+                        unsigned v0, v1;
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v0) : "r"(ad));
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v1) : "r"(ad + AR));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v0), "+r"(v1)::"memory");
+                        v0 = __float_as_uint(__uint_as_float(v0) * fr), v1 = __float_as_uint(__uint_as_float(v1) * fr);
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad), "r"(v0) : "memory");
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + AR), "r"(v1) : "memory");
+                    }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
+            if (act) {
+                uint8_t * const dst = sm.p + 4 * tile * P_KGROUP + (r_own >> 3) * 128 + (r_own & 7) * 16;
 #pragma unroll
-            for (int gq = 0; gq < RS / 8; gq++) {
-                const unsigned off = (unsigned) ((RS / 8) * c2 + gq) * 2048 + pos_off;
-                *reinterpret_cast<uint4 *>(sm.p[0] + off) = make_uint4(hi[gq][0], hi[gq][1], hi[gq][2], hi[gq][3]);
-                *reinterpret_cast<uint4 *>(sm.p[1] + off) = make_uint4(lo[gq][0], lo[gq][1], lo[gq][2], lo[gq][3]);
+                for (int u = 0; u < 4; u++) { // 8 positions of a row: one 16-byte unit of each part
+                    *reinterpret_cast<uint4 *>(dst + u * P_KGROUP) = make_uint4(hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]);
+                    *reinterpret_cast<uint4 *>(dst + u * P_KGROUP + AR / 8 * 128) = make_uint4(lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]);
+                }
             }
             fence_async_smem();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.p_full);
             if (st) TC_STAMP(i, 6);
+            return true;
         };
 
-        // Tile maxima run ahead of P (tasks: left by the producer, see there), so that a group's own maxima are published well
-        // before the CTAs that hold the chunk's next groups need them: the CTAs of a kv head may drift apart by a group
-        // without a poll having to wait. The lead grows from none (the first P needs only its own group's scores) to two groups.
-        constexpr int MAX_AHEAD = 2;
-        int maxima_done = 0;
+        // the row's sum over the thread's share of the tiles, complete in the row's lead thread
+        auto row_sum = [&]() -> float {
+            float l_row = l_acc + __shfl_xor_sync(FULL_MASK, l_acc, 16);
+            if (q < AR / 16) {
+                if (h2 && !hf) sm.lsum[r_own] = l_row;
+                named_bar(1 + q, 64); // (lsum is written again behind a later barrier of the two warps)
+                if (lead) l_row += sm.lsum[r_own];
+            }
+            return l_row;
+        };
+
         if constexpr (BATCH) {
-            bool alive = true;
-            int par = 0;
-            for (int i = 0; alive && i < G; i++) {
-                while (alive && maxima_done < min(G, i + 1 + min(i, MAX_AHEAD))) alive = maxima(maxima_done++);
-                if (!alive) break;
-                const GroupRec k = sm.tasks[i % NTASK];
-                softmax(i, k);
-                if (!(k.flags & REC_LAST)) continue;
-                // The segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below). A transposing
-                // reduction: each step halves the rows a lane holds; 27 shuffles for the 24 rows instead of 120, the same sums. Lane bits
-                // 4, 3, 2 select the row.
-                static_assert(RS == 24, "12, 6 and 3 rows per step");
+            // a group's scores are read once: S buffer free, maxima, P
+            for (int i = 0; i < G; i++) {
+                if (st) TC_STAMP(i, 0);
+                tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
+                const GroupRec & k = sm.tasks[i % NTASK];
+                if (st) TC_STAMP(i, 1);
+                tc_fence_after();
+                const bool act = 16 * q < GQ * k.T;
+                float s[ATP];
+                if (act) tmem_scores(s_addr(i), s);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sm.s_empty[i % NSB]);
+                if (act) mask_tile(last_visible(k, k.n, k.T), s);
+                const float4 tm = tile_maxima(i, act, s);
+                if (st) TC_STAMP(i, 3);
+                if (!softmax(i, act, carry, k.restart, tm, [&](float (&x)[ATP]) {
+#pragma unroll
+                        for (int c = 0; c < ATP; c++) x[c] = s[c];
+                    }))
+                    break;
+                const int flags = k.flags;
+                if (flags & REC_END) G = i + 1;
+                if (!(flags & REC_LAST)) continue;
+                // the segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below)
                 const int rows = GQ * k.T;
-                float ls[RS], l3[12];
-#pragma unroll
-                for (int j = 0; j < RS / 2; j++) f2_unpack(l_acc[j], ls[2 * j], ls[2 * j + 1]);
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    const int half = 12 >> r, o = 16 >> r;
-                    const bool up = (lane & o) != 0;
-#pragma unroll
-                    for (int j = 0; j < 12; j++)
-                        if (j < half) {
-                            const float x = r ? l3[j] : ls[j], y = r ? l3[j + half < 12 ? j + half : 0] : ls[j + half];
-                            l3[j] = (up ? y : x) + __shfl_xor_sync(FULL_MASK, up ? x : y, o);
-                        }
-                }
-                const int lrow = row0 + 12 * (lane >> 4) + 6 * ((lane >> 3) & 1) + 3 * ((lane >> 2) & 1);
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    float x = l3[j];
-                    x += __shfl_xor_sync(FULL_MASK, x, 2);
-                    x += __shfl_xor_sync(FULL_MASK, x, 1);
-                    if ((lane & 3) == 0) sm.lsum[par][q][lrow + j] = x;
-                }
-#pragma unroll
-                for (int j = 0; j < RS / 2; j++) l_acc[j] = 0ull;
-                named_bar(1 + c2, GT * 32); // (the buffer is written again two segments later, behind the next segment's barrier)
-                if (owner && q == 0 && r_own < rows)
-                    a.ml[(size_t) k.slot * AR + r_own] =
-                        make_float2(m_acc, sm.lsum[par][0][r_own] + sm.lsum[par][1][r_own] + sm.lsum[par][2][r_own] + sm.lsum[par][3][r_own]);
+                const float l_row = row_sum();
+                if (lead && r_own < rows) a.ml[(size_t) k.slot * AR + r_own] = make_float2(m_acc, l_row);
+                l_acc = 0.f;
                 m_acc = -CUDART_INF_F;
-                par ^= 1;
                 flush_slot = k.slot, flush_rows = rows;
             }
             if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
                 tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
                 tc_fence_after();
-                flush();
+                read_out(flush_slot, flush_rows, true);
             }
         } else {
-        if (G > 0) {
-            for (int i = 0; i < G; i++) {
-                const int want = min(G, i + 1 + min(i, MAX_AHEAD));
-                while (maxima_done < want) maxima(maxima_done++);
-                const GroupRec kc = sm.tasks[i % NTASK];
-                softmax(i, kc);
-                if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
-                    const Task kn = sm.tasks[(i + 1) % NTASK];
-                    request_words(kn);
-                } else {
-                    w0 = w1 = w2 = 0ull; // (no early request: the polls fetch the words themselves)
-                }
+        // Tile maxima run ahead of P (tasks: left by the producer, see there), so that a group's own maxima are published well
+        // before the CTAs that hold the chunk's next groups need them: the CTAs of a kv head may drift apart by a group
+        // without a poll having to wait. The lead grows from none (the first P needs only its own group's scores) to MAX_AHEAD groups.
+        const bool act = 16 * q < R, pub = lead && r_own < R, polls = !hf && r_own < R;
+        // tile maxima of group j, its own maxima published
+        auto maxima = [&](int j) -> float4 {
+            if (st) TC_STAMP(j, 0);
+            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
+            const GroupRec & k = sm.tasks[j % NTASK];
+            if (st) TC_STAMP(j, 1);
+            tc_fence_after();
+            float s[ATP];
+            if (act) {
+                tmem_scores(s_addr(j), s);
+                mask_tile(last_visible(k, n, T), s);
             }
+            const float4 tm = tile_maxima(j, act, s);
+            if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
+                __stcg(a.xa + xbase(k) + (size_t) k.b * AR,
+                       ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(fmaxf(fmaxf(tm.x, tm.y), fmaxf(tm.z, tm.w))));
+            if (st) TC_STAMP(j, 2);
+            return tm;
+        };
+        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
+        // the chunk's previous groups have most likely published them
+        auto request_words = [&](const Task & k) {
+            if (polls && k.nb > 1 && exch_ok(k)) {
+                const size_t xb0 = xbase(k);
+                if (k.b >= 1) w1 = __ldcv(a.xa + xb0 + (size_t) (k.b - 1) * AR);
+                if (k.b >= 2) w2 = __ldcv(a.xa + xb0 + (size_t) (k.b - 2) * AR);
+                if (k.b >= 3) w0 = __ldcv(a.xb + xb0 + (size_t) (k.b - 3) * AR);
+            }
+        };
+        constexpr int MAX_AHEAD = 2;
+        static_assert(MAX_AHEAD + 1 < NSB, "S of the groups ahead stays until their P");
+        float4 tm0, tm1, tm2; // of groups i, i + 1, i + 2
+        tm0 = tm1 = tm2 = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+        int maxima_done = 0;
+        for (int i = 0; i < G; i++) {
+            const int want = min(G, i + 1 + min(i, MAX_AHEAD));
+            while (maxima_done < want) {
+                const float4 t = maxima(maxima_done);
+                if (maxima_done == i) tm0 = t;
+                else if (maxima_done == i + 1) tm1 = t;
+                else tm2 = t;
+                maxima_done++;
+            }
+            const GroupRec & k = sm.tasks[i % NTASK];
+            if (st) TC_STAMP(i, 3);
+            float m_in = -CUDART_INF_F;
+            const size_t xb0 = xbase(k);
+            if (polls && k.nb > 1 && exch_ok(k)) {
+                if (k.b >= 1) m_in = poll_word(a.xa + xb0 + (size_t) (k.b - 1) * AR, w1, a.epoch, &sm.wc, a.status);
+                if (k.b >= 2) m_in = fmaxf(m_in, poll_word(a.xa + xb0 + (size_t) (k.b - 2) * AR, w2, a.epoch, &sm.wc, a.status));
+                if (k.b >= 3) m_in = fmaxf(m_in, poll_word(a.xb + xb0 + (size_t) (k.b - 3) * AR, w0, a.epoch, &sm.wc, a.status));
+                if (pub && k.b + 3 < k.nb)
+                    __stcg(a.xb + xb0 + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) |
+                                                               __float_as_uint(fmaxf(fmaxf(m_in, fmaxf(tm0.x, tm0.y)), fmaxf(tm0.z, tm0.w))));
+            }
+            __syncwarp();
+            m_in = __shfl_sync(FULL_MASK, m_in, lane & 15);
+            if (st) TC_STAMP(i, 7);
+            softmax(i, act, m_in, 0u, tm0, [&](float (&x)[ATP]) {
+                tmem_scores(s_addr(i), x);
+                mask_tile(last_visible(k, n, T), x);
+            });
+            tm0 = tm1;
+            tm1 = tm2;
+            if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
+                request_words(sm.tasks[(i + 1) % NTASK]);
+            } else {
+                w0 = w1 = w2 = 0ull; // (no early request: the polls fetch the words themselves)
+            }
+        }
+        if (G > 0) {
             tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
             tc_fence_after();
         }
@@ -1156,95 +1151,13 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         }
 #endif
         // ---- the CTA's partial: O^T lanes are dims (in the unpacked units' order: mapped back here), columns are query rows ----
-#pragma unroll 1
-        for (int hg = 0; hg < 2 * (RS / 8); hg++) {
-            const int h = hg / (RS / 8), gq = hg % (RS / 8);
-            float v[8], w[8];
-            if (G > 0) {
-                tmem_ld8(lane_addr + (h ? O_COL1 : O_COL0) + row0 + 8 * gq, v);
-                tmem_ld8(lane_addr + (h ? O_COL1 : O_COL0) + AR + row0 + 8 * gq, w);
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int r = row0 + 8 * gq + j;
-                if (r < R) a.part[((size_t) slot * AR + r) * HD + 128 * h + pdim] = G > 0 ? v[j] + w[j] : 0.f;
-            }
-        }
-        float ls[RS];
-#pragma unroll
-        for (int j = 0; j < RS / 2; j++) f2_unpack(l_acc[j], ls[2 * j], ls[2 * j + 1]);
-#pragma unroll
-        for (int j = 0; j < RS; j++) {
-            float x = ls[j];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(FULL_MASK, x, o);
-            ls[j] = x;
-        }
-        named_bar(5, NSOFT * 32); // every softmax warp is past its last read of the tile maxima
-        float(&lsum)[GT][AR] = *reinterpret_cast<float(*)[GT][AR]>(&sm.tmax[0][0][0]);
-        if (lane == 0) {
-#pragma unroll
-            for (int j = 0; j < RS; j++) lsum[q][row0 + j] = ls[j];
-        }
-        named_bar(5, NSOFT * 32);
-        if (owner && q == 0 && r_own < R)
-            a.ml[(size_t) slot * AR + r_own] = make_float2(m_acc, lsum[0][r_own] + lsum[1][r_own] + lsum[2][r_own] + lsum[3][r_own]);
+        read_out(slot, R, G > 0);
+        const float l_row = row_sum();
+        if (lead && r_own < R) a.ml[(size_t) slot * AR + r_own] = make_float2(m_acc, l_row);
 #if MKKV_TC_PROF
         if (warp == 0) TC_STAMP(15, 11);
 #endif
-        if (a.done) {
-            // ---- the merge, in the kernel's tail: when every CTA of the kv head has written its partial, this CTA merges rows
-            // kk and kk + cph of the head's 6 T. Four warps share a row (warp j of the team: partials j, j + 4, ..: all their loads
-            // are in flight at once), the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete) ----
-            __threadfence();
-            named_bar(5, NSOFT * 32);
-            if (warp == 0) {
-                bool ok = true;
-                if (lane == 0) {
-                    atomicAdd(a.done + g, 1u);
-                    unsigned it = 0;
-                    while ((int) (ld_acquire_u32(a.done + g) - a.done_target) < 0) {
-                        __nanosleep(100);
-                        if (++it >= (sm.wc.poll << 2) || sm.wc.dead) { // (about a second)
-                            atomicExch(a.status, (int) KS_WAIT_TIMEOUT);
-                            ok = false;
-                            break;
-                        }
-                    }
-                    sm.merge_ok = ok;
-                }
-            }
-            named_bar(5, NSOFT * 32);
-#if MKKV_TC_PROF
-            if (warp == 0) TC_STAMP(15, 12);
-#endif
-            const int team = warp >> 2, tj = warp & 3, rr = kk + team * a.cph;
-            const bool has = sm.merge_ok && rr < GQ * T;
-            float * const scratch = reinterpret_cast<float *>(sm.op[0]); // [warp][lane][8 sums], then [warp] weights' sums
-            float num[8], den = 0.f, M = -CUDART_INF_F;
-            if (has) {
-                merge_accumulate<4>(a.part, a.ml, (size_t) g * a.cph, (size_t) AR * HD, (size_t) AR, a.cph, tj, 4, rr, lane, num, den, M);
-                float4 * d = reinterpret_cast<float4 *>(scratch + ((size_t) warp * 32 + lane) * 8);
-                d[0] = make_float4(num[0], num[1], num[2], num[3]);
-                d[1] = make_float4(num[4], num[5], num[6], num[7]);
-                if (lane == 0) scratch[NSOFT * 32 * 8 + warp] = den;
-            }
-            named_bar(5, NSOFT * 32);
-            if (has && tj == 0) {
-#pragma unroll
-                for (int w2 = 1; w2 < 4; w2++) {
-                    const float4 * o = reinterpret_cast<const float4 *>(scratch + ((size_t) (warp + w2) * 32 + lane) * 8);
-                    const float4 o0 = o[0], o1 = o[1];
-                    num[0] += o0.x, num[1] += o0.y, num[2] += o0.z, num[3] += o0.w;
-                    num[4] += o1.x, num[5] += o1.y, num[6] += o1.z, num[7] += o1.w;
-                    den += scratch[NSOFT * 32 * 8 + warp + w2];
-                }
-                merge_finish(J, g * GQ + rr / T, rr % T, lane, a.raw_part != nullptr, a.raw_part, a.raw_ml, num, den, M);
-            }
-#if MKKV_TC_PROF
-            if (warp == 0) TC_STAMP(15, 13);
-#endif
-        }
+        if (a.done) tail_merge(sm, a, g, kk, T, warp, lane);
         }
     }
     tc_fence_before();

@@ -56,6 +56,17 @@ __device__ __forceinline__ unsigned lds16(unsigned addr) {
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
     return v;
 }
+// The two biases, in registers: an AND-OR has room for one immediate, and constants that the compiler knows are loaded anew for each
+// (an opaque value is not)
+struct UnpackConst {
+    unsigned a, b; // MAGIC_A, MAGIC_B
+};
+__device__ __forceinline__ UnpackConst unpack_const() {
+    UnpackConst u;
+    asm volatile("mov.b32 %0, %1;" : "=r"(u.a) : "n"(MAGIC_A));
+    asm volatile("mov.b32 %0, %1;" : "=r"(u.b) : "n"(MAGIC_B));
+    return u;
+}
 // one unit: the pairs' high-bit words y0 .. y3 (bias included) and the lane word -> four values, stored
 template <int BITS> __device__ __forceinline__ void unit_out(unsigned dst, unsigned word, unsigned y0, unsigned y1, unsigned y2, unsigned y3, unsigned d) {
     constexpr unsigned SA = MAGIC_A + (0x00010001u << (BITS - 1)), SB = MAGIC_B + (0x00100010u << (BITS - 1));
@@ -87,28 +98,28 @@ template <int BITS> __device__ __forceinline__ void dq_load(PackedBlock<BITS> & 
         if constexpr (BITS == 7) b.h[0] = lds32(rp + 128 + 12 * jb), b.h[1] = lds32(rp + 132 + 12 * jb), b.h[2] = lds32(rp + 136 + 12 * jb);
     }
 }
-template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BITS> & b, unsigned dst) {
+template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned dst) {
     const unsigned d = b.d;
     if constexpr (BITS == 8) {
         constexpr unsigned S8 = MAGIC_A + 0x00800080u;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const unsigned lo = b.w[2 * u] ^ 0x80808080u, hi = b.w[2 * u + 1] ^ 0x80808080u; // q + 128
-            sts128(dst + u * 2048, pair_val<S8>(__byte_perm(lo, MAGIC_A, 0x7270), d), // (value 0, value 2) under the exponent of 1024
-                   pair_val<S8>(__byte_perm(hi, MAGIC_A, 0x7270), d),                 // (4, 6)
-                   pair_val<S8>(__byte_perm(lo, MAGIC_A, 0x7371), d),                 // (1, 3)
-                   pair_val<S8>(__byte_perm(hi, MAGIC_A, 0x7371), d));                // (5, 7)
+            sts128(dst + u * 2048, pair_val<S8>(__byte_perm(lo, uc.a, 0x7270), d), // (value 0, value 2) under the exponent of 1024
+                   pair_val<S8>(__byte_perm(hi, uc.a, 0x7270), d),                 // (4, 6)
+                   pair_val<S8>(__byte_perm(lo, uc.a, 0x7371), d),                 // (1, 3)
+                   pair_val<S8>(__byte_perm(hi, uc.a, 0x7371), d));                // (5, 7)
         }
     } else if constexpr (BITS == 4) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) unit_out<4>(dst + u * 2048, b.w[u], MAGIC_A, MAGIC_B, MAGIC_A, MAGIC_B, d);
+        for (int u = 0; u < 4; u++) unit_out<4>(dst + u * 2048, b.w[u], uc.a, uc.b, uc.a, uc.b, d);
     } else if constexpr (BITS == 5) {
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             // bit k of the word's byte of high bits at 4 + k and 18 + k; the copy one lower serves the odd values
             const unsigned hb = __byte_perm(b.h[0], 0u, 0x4440 + u), t = hb * 0x00040010u, t1 = hb * 0x00020008u;
-            unit_out<5>(dst + u * 2048, b.w[u], and_or_imm<0x00100010u>(t, MAGIC_A), and_or_imm<0x01000100u>(t, MAGIC_B),
-                        and_or_imm<0x00100010u>(t1, MAGIC_A), and_or_imm<0x01000100u>(t1, MAGIC_B), d);
+            unit_out<5>(dst + u * 2048, b.w[u], and_or_imm<0x00100010u>(t, uc.a), and_or_imm<0x01000100u>(t, uc.b),
+                        and_or_imm<0x00100010u>(t1, uc.a), and_or_imm<0x01000100u>(t1, uc.b), d);
         }
     } else if constexpr (BITS == 6) {
         const unsigned hw[4] = {b.h[0], b.h[0] >> 16, b.h[1], b.h[1] >> 16};
@@ -116,8 +127,8 @@ template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BI
         for (int u = 0; u < 4; u++) {
             // even values' 2-bit fields at bits 0, 4, 8, 12 of he, odd values' of ho: the gaps keep the shifted copies' sums apart
             const unsigned he = hw[u] & 0x3333u, ho = (hw[u] >> 2) & 0x3333u;
-            unit_out<6>(dst + u * 2048, b.w[u], and_or_imm<0x00300030u>(he * 0x00010010u, MAGIC_A), and_or_imm<0x03000300u>(he * 0x00001001u, MAGIC_B),
-                        and_or_imm<0x00300030u>(ho * 0x00010010u, MAGIC_A), and_or_imm<0x03000300u>(ho * 0x00001001u, MAGIC_B), d);
+            unit_out<6>(dst + u * 2048, b.w[u], and_or_imm<0x00300030u>(he * 0x00010010u, uc.a), and_or_imm<0x03000300u>(he * 0x00001001u, uc.b),
+                        and_or_imm<0x00300030u>(ho * 0x00010010u, uc.a), and_or_imm<0x03000300u>(ho * 0x00001001u, uc.b), d);
         }
     } else { // 7 bits: every pair under the 1024 bias (pair_words7)
         const unsigned hw[4] = {b.h[0], __funnelshift_r(b.h[0], b.h[1], 24), __funnelshift_r(b.h[1], b.h[2], 16), b.h[2] >> 8}; // (bits above 23: not read)
@@ -134,7 +145,7 @@ template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BI
 template <int BITS> __device__ __forceinline__ void dq_item(unsigned raw, int row, int jb, bool valid, unsigned dst) {
     PackedBlock<BITS> b;
     dq_load<BITS>(b, raw, row, jb, valid);
-    dq_emit<BITS>(b, dst);
+    dq_emit<BITS>(b, unpack_const(), dst);
 }
 } // namespace tc
 } // namespace mkkv
