@@ -16,7 +16,7 @@
 //   - one issuer thread runs tcgen05.mma on the slots as they fill (mbarrier "full" from the unpack warps, tcgen05.commit
 //     to "empty"), S in four tensor-memory buffers (K runs four groups ahead of V; M = 64 takes 16 lanes of each quarter, so two
 //     buffers share their columns), O^T (two 128-dim halves) resident there for the whole kernel;
-//   - 8 softmax warps read S back (tcgen05.ld 16x32bx2: a thread owns one query row and one tile of 32 positions), so that a tile's
+//   - four softmax warps read S back (tcgen05.ld 16x32bx2: a thread owns one query row and 64 of its positions), so that a tile's
 //     maximum and sum are taken inside a thread (with positions on lanes they were 24 warp reductions a warp and group, a barrier and
 //     a hand-out of each row's maxima: 1.9 k more instructions a group); they exchange the running
 //     max with the CTAs that hold the chunk's earlier groups through small global arrays (own group maxima and cumulative
@@ -29,13 +29,14 @@
 //   - a CTA writes one un-normalised partial (m, l, O); when the CTAs of a kv head have all written theirs (arrival count,
 //     bounded wait) each merges one or two of the head's rows in the kernel's tail, four warps to a row;
 //   - batch mode (several jobs: sequences served together, or all layers of a decode step): a plain launch of one persistent CTA per
-//     SM, each running its share of the (job, kv head, run of cpi chunks) items one after another, groups of four consecutive tiles in order
-//     with the running max carried in registers and started anew at a chunk's first tile (a group may hold tiles of several chunks: with
-//     groups that ended with their chunk, half of each was padding at 1,187 positions and 16 layers took 47.5 us instead of 37.3), no exchange; attn_merge_kernel afterwards. The copies,
-//     the unpacking and S^T of the next item run on while the softmax warps finish the one before. What bounds it: a group costs
-//     3.6 us of CTA time at any length (the same instruction issue and latency as in the spread mode), an item about 2.5 us more.
-//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 3.3 us against 18.8;
-//     11,701 (K6 / V5), 3 tokens 12.3 against 27.1; 101,600, 8 tokens 81.5 against 96.7.
+//     SM, each running its share of the (job, kv head, run of cpi chunks) items one after another, groups of four consecutive tiles in
+//     order with the running max carried in registers and started anew at a chunk's first tile (a group may hold tiles of several
+//     chunks: with groups that ended with their chunk, half of each was padding at 1,187 positions and 16 layers took 47.5 us instead
+//     of 37.3), no exchange; attn_merge_kernel afterwards. The copies, the unpacking and S of the next item run on while the softmax
+//     warps finish the one before. What bounds it: a group costs 3.0 us of CTA time at any length, most of it the unpack warps'
+//     instructions, an item about 2 us more.
+//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 2.3 us against 18.8;
+//     101,600, 8 tokens 67.3 against 95.
 // Every wait is bounded (about two seconds by default; the limits are launch arguments), then the status word and a CTA-wide
 // flag are set, no later wait of the CTA blocks, the producer waits (bounded) for its copies still in flight, and the kernel
 // runs to its end and frees its tensor memory.
@@ -56,17 +57,19 @@ namespace tc {
 
 using namespace attn_common;
 
-constexpr int NSOFT = 8;       // softmax warps first: warp 4 h2 + q, query rows 16 q .. + 15, tiles 2 h2 and 2 h2 + 1 of a group
+constexpr int NSOFT = 4;       // softmax warps first: warp q, query rows 16 q .. + 15 (the accumulator's read-out: tensor-memory lanes 32 q ..)
 constexpr int NDQ = 16;        // then the unpack warps: 4 c + q, tile q, 32-dim block c of each 128-dim half
-constexpr int W_ISSUE = NSOFT + NDQ, W_PROD = W_ISSUE + 1;
-constexpr int NTHREADS = (W_PROD + 3) * 32; // two idle warps complete the last group of four (register reallocation is per group)
+// then the control warps, two of them idle to complete a group of four (register reallocation is per group). The issuer is the warp on
+// the scheduler whose softmax warp has no query rows.
+constexpr int W_CTL = NSOFT + NDQ, W_PROD = W_CTL + 2, W_ISSUE = W_CTL + 3;
+constexpr int NTHREADS = (W_CTL + 4) * 32;
 constexpr int GT = 4, GP = GT * ATP;        // tiles / positions per group: the N of an S instruction
 // registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
 // most the CTA's launch allocation -- a larger sum faults)
-#define MKKV_TC_REGS_SOFT "104"
+#define MKKV_TC_REGS_SOFT "168"
 #define MKKV_TC_REGS_DQ "56"
-#define MKKV_TC_REGS_CTL "72"
-static_assert(NTHREADS == 896 && 8 * 104 + 16 * 56 + 4 * 72 <= 28 * 72, "register shares");
+#define MKKV_TC_REGS_CTL "80"
+static_assert(NTHREADS == 768 && 4 * 168 + 16 * 56 + 4 * 80 <= 24 * 80, "register shares");
 constexpr int RAW_SLOT = ATP * HD + ATP * SCALE_ROW; // one tile of the widest format and its scales: 8704 bytes
 constexpr int NRAW = 8;                     // packed tile slots: two side-groups (one being unpacked, one in flight)
 static_assert(NRAW % GT == 0, "whole groups only: a 7-slot ring, tried once, was 20 % slower and its results changed from run to run");
@@ -90,6 +93,10 @@ static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
 constexpr float REF_SLACK = 11.f, REF_BELOW = 2.f;
 constexpr float LOG2E = 1.4426950408889634f;
 
+// one arrival of the calling warp: by the lane with `lane` 0, under a predicate (a branch would open a divergent region)
+__device__ __forceinline__ void warp_arrive(uint64_t * bar, int lane) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
+}
 template <int V> struct IntC { // an integer as an argument of a generic lambda
     static constexpr int value = V;
 };
@@ -121,10 +128,8 @@ struct Smem {
     uint8_t q[Q_BYTES];         // [dim group 32][row group 6][8 rows][8 dims]. (As the A operand of M = 64 rows a dim group is read on
                                 // into the next one, the last into p: rows 48 .. 63 of S are never read)
     uint8_t p[P_BYTES];         // [position group 16][high part, low part][row group 6][8 rows][8 positions]
-    float tmax[2][GT][AR];      // row maxima of a group's tiles, by group parity
-    float lsum[AR];             // row sums of tiles 2 and 3 on their way to the warps of tiles 0 and 1
     float resc_f[2][AR];        // factors of the reference maxima that moved, by group parity
-    unsigned resc_rows[2][4];   // and which of each 16 rows they are
+    unsigned resc_rows[2][4];   // and which rows of each softmax warp they are
     unsigned tmem_base;
     int merge_ok;               // the tail's merge: the head's CTAs have all arrived
     WaitCtl wc;                 // the launch's wait limits; dead: a wait of this CTA gave up, no later wait blocks
@@ -177,34 +182,42 @@ struct Args {
     } while (0)
 #endif
 
-// Wait for a phase of an mbarrier. A failed try suspends the thread in hardware for up to the hinted time (it wakes when the phase
-// completes), so waiting warps take next to no issue slots. Bounded: after `rounds` failed tries the status word and the CTA's
-// `dead` flag are set; from then on no wait of this CTA blocks, and the kernel runs to its end.
+// Wait for a phase of an mbarrier. A try suspends the thread in hardware (it wakes when the phase completes, or after a time of the
+// hardware's choosing), so waiting warps take next to no issue slots. (try_wait with a time limit of its own becomes a loop that polls,
+// sleeps and reads the clock.) Bounded: after about hint x rounds nanoseconds the status word and the CTA's `dead` flag are set; from
+// then on no wait of this CTA blocks, and the kernel runs to its end.
 constexpr unsigned WAIT_HINT_NS = 10000u, WAIT_ROUNDS = 200000u, POLL_ROUNDS = 1u << 21; // defaults: about two seconds each
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t * bar, unsigned parity, unsigned hint_ns) {
+__device__ __forceinline__ bool mbar_test_wait(uint64_t * bar, unsigned parity) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
+        : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
 }
 // Returns whether the phase is complete.
 __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    if (mbar_try_wait_hint(bar, parity, 0u)) return true; // (the common case: no limit loaded)
-    const unsigned hint = wc->hint, rounds = wc->rounds;
-    for (unsigned it = 0; !mbar_try_wait_hint(bar, parity, hint); it++) {
+    if (mbar_test_wait(bar, parity)) return true; // (the common case: no limit loaded)
+    const unsigned rounds = wc->rounds;
+    if (rounds && mbar_try_wait(bar, parity)) return true;
+    const unsigned long long limit = (unsigned long long) wc->hint * rounds, t0 = globaltimer_ns();
+    do {
         if (wc->dead) return false;
-        if (it >= rounds) {
+        if (globaltimer_ns() - t0 >= limit) {
             wc->dead = 1;
             atomicExch(status, (int) KS_WAIT_TIMEOUT);
             return false;
         }
-    }
+    } while (!mbar_try_wait(bar, parity));
     return true;
+}
+// at most about 16 ms, for the copies and instructions in flight at the kernel's end
+__device__ __forceinline__ void wait_landed(uint64_t * bar, unsigned parity) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < 16000000ull) {}
 }
 // Whether the CTA has given up, the same answer for all the lanes of mask. Another warp may set the flag between two lanes' reads: a
 // warp that leaves a loop with warp-wide operations in it leaves it by this vote (lanes that disagreed would wait for each other, some
@@ -220,7 +233,7 @@ __device__ __forceinline__ void drain_copies(uint64_t * raw_full, unsigned issue
     for (int j = 0; j < slots; j++) {
         const unsigned e = (issued >> (8 * j)) & 0xffu;
         if (e == NO_COPY) continue;
-        for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&raw_full[e >> 1], e & 1u, 1000u); it++) {}
+        wait_landed(&raw_full[e >> 1], e & 1u);
     }
 }
 
@@ -259,11 +272,23 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// Scores of two tiles, 64 columns of the 16 lanes from taddr's on: lanes 0 .. 15 get the first tile of their row, lanes 16 .. 31 the
-// second. (One statement with its wait: no use of the registers can move between the two.)
-__device__ __forceinline__ void tmem_scores(unsigned taddr, float (&s)[ATP]) {
+// The scores of one S buffer (16 lanes of the warp's quarter from taddr's on): lanes 0 .. 15 get columns 0 .. 63 of their row, lanes
+// 16 .. 31 columns 64 .. 127. (One statement with its wait: no use of the registers can move between the two.)
+__device__ __forceinline__ void tmem_scores(unsigned taddr, float (&s)[2 * ATP]) {
+    unsigned r[2 * ATP];
+    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%64], 64;\n\t"
+                 "tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%65], 64;\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
+                 : "r"(taddr), "r"(taddr + ATP)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 2 * ATP; i++) s[i] = __uint_as_float(r[i]);
+}
+// one tile of the two above
+__device__ __forceinline__ void tmem_scores_tile(unsigned taddr, float (&s)[ATP]) {
     unsigned r[ATP];
-    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32], 32;\n\t"
+    asm volatile("tcgen05.ld.sync.aligned.16x32bx2.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32], 64;\n\t"
                  "tcgen05.wait::ld.sync.aligned;"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr)
@@ -506,11 +531,12 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
 }
 
 // Spread mode: the merge, in the kernel's tail: when every CTA of kv head g has written its partial, this CTA (kk-th of the head's cph)
-// merges rows kk and kk + cph of the head's 6 T. The softmax warps (mw), four to a row (warp j of the team: partials j, j + 4, ..: all
-// their loads are in flight at once); the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete).
+// merges rows kk and kk + cph of the head's 6 T. Eight warps (mw; the softmax warps and the first four unpack warps), four
+// to a row (warp j of the team: partials j, j + 4, ..: all their loads are in flight at once); the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete).
+constexpr int MERGE_WARPS = 8;
 __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int kk, int T, int mw, int lane) {
     __threadfence();
-    named_bar(7, NSOFT * 32);
+    named_bar(5, MERGE_WARPS * 32);
     if (mw == 0 && lane == 0) {
         bool ok = true;
         atomicAdd(a.done + g, 1u);
@@ -525,7 +551,7 @@ __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int
         }
         sm.merge_ok = ok;
     }
-    named_bar(7, NSOFT * 32);
+    named_bar(5, MERGE_WARPS * 32);
 #if MKKV_TC_PROF
     if (mw == 0) TC_STAMP(15, 12);
 #endif
@@ -538,9 +564,9 @@ __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int
         float4 * d = reinterpret_cast<float4 *>(scratch + ((size_t) mw * 32 + lane) * 8);
         d[0] = make_float4(num[0], num[1], num[2], num[3]);
         d[1] = make_float4(num[4], num[5], num[6], num[7]);
-        if (lane == 0) scratch[NSOFT * 32 * 8 + mw] = den;
+        if (lane == 0) scratch[MERGE_WARPS * 32 * 8 + mw] = den;
     }
-    named_bar(7, NSOFT * 32);
+    named_bar(5, MERGE_WARPS * 32);
     if (has && tj == 0) {
 #pragma unroll
         for (int w2 = 1; w2 < 4; w2++) {
@@ -548,7 +574,7 @@ __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int
             const float4 o0 = o[0], o1 = o[1];
             num[0] += o0.x, num[1] += o0.y, num[2] += o0.z, num[3] += o0.w;
             num[4] += o1.x, num[5] += o1.y, num[6] += o1.z, num[7] += o1.w;
-            den += scratch[NSOFT * 32 * 8 + mw + w2];
+            den += scratch[MERGE_WARPS * 32 * 8 + mw + w2];
         }
         merge_finish(sm.job, g * GQ + rr / T, rr % T, lane, a.raw_part != nullptr, a.raw_part, a.raw_ml, num, den, M);
     }
@@ -592,7 +618,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         sm.wc.poll = a.poll_rounds;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == W_ISSUE) { // tensor memory: S^T five times, O^T in two halves
+    if (warp == W_ISSUE) { // tensor memory: four S buffers, O^T in two halves
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         tc_fence_before();
@@ -626,7 +652,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
     // The kv head's query rows come staged (qprep: fp16 -> fp32 -> K's rotation -> x 1/16 -> fp16 in the K-major B operand's layout,
     // row = (head % 6) T + t): the producer fetches the block with one bulk copy, the issuer waits for it.
     // registers move from the unpack / control warps to the softmax warps
-    if (warp >= W_ISSUE) {
+    if (warp >= W_CTL) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
     if (warp == W_PROD) {
         if constexpr (BATCH) {
@@ -670,7 +696,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 else nv++;
             }
             if (lane == 0) // (the query block too: the issuer may give up on it)
-                for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.q_ready, 0u, 1000u); it++) {}
+                wait_landed(&sm.q_ready, 0u);
             drain_copies(sm.raw_full, issued, NRAW / GT);
         }
         }
@@ -679,7 +705,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         if (elect_one()) { // (with lane == 0 as the test an instruction took 50 % longer to issue: see elect_one)
             unsigned oseq = 0;
             if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc, a.status); // the queries are staged
-            // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S^T of the segment before is
+            // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S of the segment before is
             // complete: they arrive while P V of an earlier group runs
             bool q_flight = false;
             unsigned q_ph = 0;
@@ -757,9 +783,9 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             // every instruction issued above is complete before the tensor memory is freed and the CTA's shared memory released
             // (bounded; in a normal run the softmax warps have already waited for the last one)
             if (batch && q_flight) // (given up with the query block in flight: it lands before the CTA's shared memory is released)
-                for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.q_ready, q_ph, 1000u); it++) {}
+                wait_landed(&sm.q_ready, q_ph);
             umma_commit(&sm.fin);
-            for (unsigned it = 0; it < (1u << 14) && !mbar_try_wait_hint(&sm.fin, 0u, 1000u); it++) {}
+            wait_landed(&sm.fin, 0u);
         }
     }
     } else if (warp >= NSOFT) {
@@ -778,7 +804,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         auto hand_over = [&]() {
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.op_full[os]);
+            warp_arrive(&sm.op_full[os], lane);
             if (++os == NOP) os = 0, oph ^= 1;
         };
         auto unpack_tile = [&](auto bits_c, unsigned rawa, bool valid) {
@@ -815,7 +841,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             else if (FIXED == 6 || (!FIXED && bits == 6)) unpack_tile(IntC<6>{}, rawa, valid);
             else if (FIXED == 7 || !FIXED) unpack_tile(IntC<7>{}, rawa, valid);
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.raw_empty[rs]);
+            warp_arrive(&sm.raw_empty[rs], lane);
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 10 : 13);
             rseq++;
             return true;
@@ -828,63 +854,60 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 if (batch && (ud & UD_END)) G = it + NSB + 1;
             }
         }
+        if constexpr (!BATCH)
+            if (a.done && w < MERGE_WARPS - NSOFT) tail_merge(sm, a, g, kk, T, NSOFT + w, lane);
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
 #if MKKV_TC_PROF
         const unsigned long long t_loop = globaltimer_ns();
 #endif
-        // ---- softmax warps: warp 4 h2 + q holds query rows 16 q .. + 15 of tiles 2 h2 and 2 h2 + 1; a thread owns row r_own and one tile:
-        // the running maxima, the reference max and the row sum are plain registers, kept alike by the four threads of a row. Warps
-        // without a row of the job (rows 48 .. 63 never are one's) only take part in the accumulator's read-out and rescaling, where a
-        // warp's lanes are dims of half h2. (One warp per 16 rows, two tiles a thread: about 650 instructions in a row, 5,100 of a
-        // group's 6,500 cycles.) ----
-        const int q = warp & 3, h2 = warp >> 2, hf = lane >> 4, tile = 2 * h2 + hf, r_own = 16 * q + (lane & 15);
+        // ---- softmax warps: warp q holds query rows 16 q .. + 15; a thread owns row r_own and one half of a group's positions (tiles
+        // 2 hf, 2 hf + 1): the running maxima, the reference max and the row sums are plain registers, kept alike by the two threads of
+        // a row. Warps without a row of the job (rows 48 .. 63 never are one's) only take part in the accumulator's read-out and
+        // rescaling, where a warp's lanes are dims. (Eight warps, a tile a thread, halve a warp's work but not the SM's: 101,600 positions
+        // 1,165 us instead of 1,073.) ----
+        const int q = warp, hf = lane >> 4, r_own = 16 * q + (lane & 15);
         const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
-        const bool st = warp == 0, lead = h2 == 0 && hf == 0; // (lead: the row's first thread)
-        float l_acc = 0.f, m_acc = -CUDART_INF_F; // row sum over the thread's tiles, reference max
+        const bool st = warp == 0;
+        float l_acc = 0.f, m_acc = -CUDART_INF_F; // row sum over the thread's positions, reference max
         float carry = -CUDART_INF_F;              // (batch mode: the running max after the previous group)
         unsigned long long w0 = 0, w1 = 0, w2 = 0;
         auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
         // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
         // producer never reached are not valid) and only inside their bounds
         auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
-        // the thread's tile (and its neighbour) in the S buffer of group j: rows on 16 lanes of the warp's quarter (the other 16 are the
-        // neighbouring buffer's), positions on columns
-        auto s_addr = [&](int j) -> unsigned {
-            return lane_addr + S_COL + S_STRIDE * ((j % NSB) >> 1) + 2 * ATP * h2 + ((unsigned) (16 * (j & 1)) << 16);
-        };
-        // the last of the tile's positions that the row sees: row token t sees positions <= n + t, nothing is visible past the chunk end
-        // (all of them for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their queries are zero, so
-        // are their scores, and no one reads what becomes of them.
+        // S buffer of group j: rows on 16 lanes of the warp's quarter (the other 16 are the neighbouring buffer's), positions on columns
+        auto s_addr = [&](int j) -> unsigned { return lane_addr + S_COL + S_STRIDE * ((j % NSB) >> 1) + ((unsigned) (16 * (j & 1)) << 16); };
+        // the last of the thread's 64 positions that its row sees: row token t sees positions <= n + t, nothing is visible past the
+        // chunk end (all of them for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their queries are
+        // zero, so are their scores, and no one reads what becomes of them.
         auto last_visible = [&](const GroupRec & k, int nn, int Tk) -> int {
-            if (k.pos0 + GP - 1 <= min(k.c1 - 1, nn)) return ATP; // (the group reaches neither the chunk's end nor the new tokens)
-            return min(k.c1 - 1, nn + r_own % Tk) - k.pos0 - ATP * tile;
+            if (k.pos0 + GP - 1 <= min(k.c1 - 1, nn)) return 2 * ATP; // (the group reaches neither the chunk's end nor the new tokens)
+            return min(k.c1 - 1, nn + r_own % Tk) - k.pos0 - 2 * ATP * hf;
         };
-        auto mask_tile = [&](int lim, float (&s)[ATP]) {
-            if (__any_sync(FULL_MASK, lim < ATP)) {
+        auto mask_tile = [&](int t, int lim, float * s) {
+            if (lim < 2 * ATP) {
 #pragma unroll
                 for (int c = 0; c < ATP; c++)
-                    if (c > lim) s[c] = -CUDART_INF_F;
+                    if (ATP * t + c > lim) s[c] = -CUDART_INF_F;
             }
         };
-        // maxima of the four tiles of group j in the thread's row (act: s holds the tile's scores). A barrier of the row's two warps, which
-        // they meet at whatever the group's record says (after a give-up the two may read different records)
-        auto tile_maxima = [&](int j, bool act, const float (&s)[ATP]) -> float4 {
-            float(&tm)[GT][AR] = sm.tmax[j & 1]; // (read again by nobody when group j + 2 writes it: the barrier of j + 1 is between)
-            const float4 none = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
-            if (q == AR / 16) return none;
-            if (act) {
+        // maxima of the group's four tiles (the same in both threads of a row)
+        auto tile_maxima = [&](const float (&s)[2 * ATP]) -> float4 {
+            float m[2];
+#pragma unroll
+            for (int t = 0; t < 2; t++) {
                 float x[ATP / 2];
 #pragma unroll
-                for (int c = 0; c < ATP / 2; c++) x[c] = fmaxf(s[2 * c], s[2 * c + 1]);
+                for (int c = 0; c < ATP / 2; c++) x[c] = fmaxf(s[ATP * t + 2 * c], s[ATP * t + 2 * c + 1]);
 #pragma unroll
                 for (int o = ATP / 4; o > 0; o >>= 1)
 #pragma unroll
                     for (int c = 0; c < o; c++) x[c] = fmaxf(x[c], x[c + o]);
-                tm[tile][r_own] = x[0];
+                m[t] = x[0];
             }
-            named_bar(1 + q, 64);
-            return act ? make_float4(tm[0][r_own], tm[1][r_own], tm[2][r_own], tm[3][r_own]) : none;
+            const float o0 = __shfl_xor_sync(FULL_MASK, m[0], 16), o1 = __shfl_xor_sync(FULL_MASK, m[1], 16);
+            return hf ? make_float4(o0, o1, m[0], m[1]) : make_float4(m[0], m[1], o0, o1);
         };
         // batch mode: the partial of a finished segment (O^T lanes are dims in the unpacked units' order, columns are query rows), read
         // out when its last P V is complete and before the next P allows the MMA that overwrites O^T: between the two the tensor cores
@@ -892,20 +915,24 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         int flush_slot = -1, flush_rows = 0;
         const int prow = ATP * q + lane, pdim = (prow & ~7) | unit_perm(prow & 7);
         auto read_out = [&](int to_slot, int rows, bool any) {
-            const unsigned col0 = lane_addr + (h2 ? O_COL1 : O_COL0);
-            float * dst = a.part + (size_t) to_slot * AR * HD + 128 * h2 + pdim;
 #pragma unroll 1
-            for (int r0 = 0; r0 < rows; r0 += 16, dst += 16 * HD) {
+            for (int hg = 0; hg < 2 * (AR / 16); hg++) {
+                const int h = hg & 1, r0 = 16 * (hg >> 1);
+                if (r0 >= rows) break;
                 unsigned v[16], w[16];
-                if (any) tmem_ld16_two(col0 + r0, col0 + r0 + AR, v, w);
+                if (any) {
+                    const unsigned col = lane_addr + (h ? O_COL1 : O_COL0) + r0;
+                    tmem_ld16_two(col, col + AR, v, w);
+                }
+                float * dst = a.part + ((size_t) to_slot * AR + r0) * HD + 128 * h + pdim;
 #pragma unroll
                 for (int j = 0; j < 16; j++)
                     if (r0 + j < rows) dst[j * HD] = any ? __uint_as_float(v[j]) + __uint_as_float(w[j]) : 0.f;
             }
         };
-        // P of group i, whose tile maxima (tm) are known; take(s): the masked scores of the thread's tile. restart: bit t: tile t opens a
-        // chunk, the running max starts anew. Returns false when a wait of the CTA gave up (batch mode; the same answer for all eight
-        // warps: nothing that the group's record says leaves the warp's registers before a true).
+        // P of group i, whose tile maxima (tm) are known; take(t, s): the masked scores of tile t of the thread's two. restart: bit t: tile
+        // t opens a chunk, the running max starts anew. Returns false when a wait of the CTA gave up (batch mode; the same answer for all
+        // four warps: the group's record and everything derived from it is only used after a true).
         auto softmax = [&](int i, bool act, float m_in, unsigned restart, const float4 & tm, auto && take) -> bool {
             // running maxima after each tile; M: the largest of them
             const float r0 = (restart & 1u) ? tm.x : fmaxf(m_in, tm.x), r1 = (restart & 2u) ? tm.y : fmaxf(r0, tm.y);
@@ -920,48 +947,51 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                     m_acc = M - REF_BELOW;
                     l_acc *= f;
                     moved = true;
-                    if (lead) sm.resc_f[i & 1][r_own] = f;
+                    if (!hf) sm.resc_f[i & 1][r_own] = f;
                 }
             }
             const unsigned rows_moved = __ballot_sync(FULL_MASK, moved) & 0xffffu;
-            if (lead && lane == 0) sm.resc_rows[i & 1][q] = rows_moved;
+            if (lane == 0) sm.resc_rows[i & 1][q] = rows_moved;
             if (st) TC_STAMP(i, 4);
-            unsigned hi[ATP / 2], lo[ATP / 2]; // positions (2 c, 2 c + 1) of the tile
+            const bool anyf = named_bar_or(1, NSOFT * 32, rows_moved != 0u || (batch && sm.wc.dead != 0));
+            if (batch && anyf && named_bar_or(2, NSOFT * 32, sm.wc.dead != 0)) return false;
+            unsigned hi[ATP], lo[ATP]; // positions (2 c, 2 c + 1) of the thread's half
             if (act) {
-                float s[ATP];
-                take(s);
-                const float mr = tile == 0 ? r0 : tile == 1 ? r1 : tile == 2 ? r2 : r3;
-                const float beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);
-                const float nm = mr == -CUDART_INF_F ? mr : -mr; // (nothing visible yet: exp2 gives 0)
-                const F2 nmv = f2_pack(nm, nm);
-                const __half bhs = __float2half_rn(beta);
-                const __half2 bh = __half2half2(bhs), bl = __half2half2(__float2half_rn(beta - __half2float(bhs)));
-                F2 sum0 = 0ull, sum1 = 0ull;
 #pragma unroll
-                for (int c = 0; c < ATP / 2; c++) {
-                    float p0, p1;
-                    f2_unpack(f2_mul(f2_add(f2_pack(s[2 * c], s[2 * c + 1]), nmv), f2_pack(LOG2E, LOG2E)), p0, p1);
-                    p0 = ex2(p0), p1 = ex2(p1);
-                    if (c & 1) sum1 = f2_add(sum1, f2_pack(p0, p1));
-                    else sum0 = f2_add(sum0, f2_pack(p0, p1));
-                    const __half2 ph = __floats2half2_rn(p0, p1); // the reference's fp16 P
-                    const __half2 hh = __hmul2(ph, bh);           // P beta = hh + ll up to 2^-22: the product's exact residual
-                    const __half2 ll = __hfma2(ph, bl, __hfma2(ph, bh, __hneg2(hh))); // plus the low part of beta
-                    hi[c] = *reinterpret_cast<const unsigned *>(&hh);
-                    lo[c] = *reinterpret_cast<const unsigned *>(&ll);
+                for (int t = 0; t < 2; t++) {
+                    float s[ATP];
+                    take(t, s);
+                    const float mr = t ? (hf ? r3 : r1) : (hf ? r2 : r0);
+                    const float beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);
+                    const float nm = mr == -CUDART_INF_F ? mr : -mr; // (nothing visible yet: exp2 gives 0)
+                    const F2 nmv = f2_pack(nm, nm);
+                    const __half bhs = __float2half_rn(beta);
+                    const __half2 bh = __half2half2(bhs), bl = __half2half2(__float2half_rn(beta - __half2float(bhs)));
+                    F2 sum0 = 0ull, sum1 = 0ull;
+#pragma unroll
+                    for (int c = 0; c < ATP / 2; c++) {
+                        float p0, p1;
+                        f2_unpack(f2_mul(f2_add(f2_pack(s[2 * c], s[2 * c + 1]), nmv), f2_pack(LOG2E, LOG2E)), p0, p1);
+                        p0 = ex2(p0), p1 = ex2(p1);
+                        if (c & 1) sum1 = f2_add(sum1, f2_pack(p0, p1));
+                        else sum0 = f2_add(sum0, f2_pack(p0, p1));
+                        const __half2 ph = __floats2half2_rn(p0, p1); // the reference's fp16 P
+                        const __half2 hh = __hmul2(ph, bh);           // P beta = hh + ll up to 2^-22: the product's exact residual
+                        const __half2 ll = __hfma2(ph, bl, __hfma2(ph, bh, __hneg2(hh))); // plus the low part of beta
+                        hi[ATP / 2 * t + c] = *reinterpret_cast<const unsigned *>(&hh);
+                        lo[ATP / 2 * t + c] = *reinterpret_cast<const unsigned *>(&ll);
+                    }
+                    float x0, x1;
+                    f2_unpack(f2_add(sum0, sum1), x0, x1);
+                    l_acc = __fmaf_rn(beta, x0 + x1, l_acc);
                 }
-                float x0, x1;
-                f2_unpack(f2_add(sum0, sum1), x0, x1);
-                l_acc = __fmaf_rn(beta, x0 + x1, l_acc);
             }
             if constexpr (!BATCH) { // (the last read of this S buffer)
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.s_empty[i % NSB]);
+                warp_arrive(&sm.s_empty[i % NSB], lane);
             }
             if (st && i < 15) TC_STAMP(i, 15);
-            const bool anyf = named_bar_or(5, NSOFT * 32, rows_moved != 0u || (batch && sm.wc.dead != 0));
-            if (batch && anyf && named_bar_or(6, NSOFT * 32, sm.wc.dead != 0)) return false;
             if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
             if (st) TC_STAMP(i, 5);
             tc_fence_after();
@@ -972,8 +1002,9 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 read_out(flush_slot, flush_rows, true);
                 flush_slot = -1;
             }
-            if (anyf) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference: of a
-                        // row and half, one column of the high and one of the low part
+            if (anyf) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference:
+                        // a row is one column in each of the four blocks (two halves x high / low part); the four loads of a row
+                        // are in flight together
 #pragma unroll 1
                 for (int qq = 0; qq < AR / 16; qq++) {
                     unsigned left = sm.resc_rows[i & 1][qq];
@@ -982,22 +1013,27 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                         const int r = 16 * qq + __ffs(left) - 1;
                         left &= left - 1;
                         const float fr = sm.resc_f[i & 1][r];
-                        const unsigned ad = lane_addr + (h2 ? O_COL1 : O_COL0) + r;
-                        unsigned v0, v1;
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v0) : "r"(ad));
-                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v1) : "r"(ad + AR));
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v0), "+r"(v1)::"memory");
+                        const unsigned ad = lane_addr + r;
+                        unsigned v0, v1, v2, v3;
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v0) : "r"(ad + O_COL0));
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v1) : "r"(ad + O_COL0 + AR));
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v2) : "r"(ad + O_COL1));
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v3) : "r"(ad + O_COL1 + AR));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v0), "+r"(v1), "+r"(v2), "+r"(v3)::"memory");
                         v0 = __float_as_uint(__uint_as_float(v0) * fr), v1 = __float_as_uint(__uint_as_float(v1) * fr);
-                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad), "r"(v0) : "memory");
-                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + AR), "r"(v1) : "memory");
+                        v2 = __float_as_uint(__uint_as_float(v2) * fr), v3 = __float_as_uint(__uint_as_float(v3) * fr);
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0), "r"(v0) : "memory");
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0 + AR), "r"(v1) : "memory");
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1), "r"(v2) : "memory");
+                        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1 + AR), "r"(v3) : "memory");
                     }
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
             if (act) {
-                uint8_t * const dst = sm.p + 4 * tile * P_KGROUP + (r_own >> 3) * 128 + (r_own & 7) * 16;
+                uint8_t * const dst = sm.p + 8 * hf * P_KGROUP + (r_own >> 3) * 128 + (r_own & 7) * 16;
 #pragma unroll
-                for (int u = 0; u < 4; u++) { // 8 positions of a row: one 16-byte unit of each part
+                for (int u = 0; u < 8; u++) { // 8 positions of a row: one 16-byte unit of each part
                     *reinterpret_cast<uint4 *>(dst + u * P_KGROUP) = make_uint4(hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]);
                     *reinterpret_cast<uint4 *>(dst + u * P_KGROUP + AR / 8 * 128) = make_uint4(lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]);
                 }
@@ -1005,20 +1041,9 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             fence_async_smem();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.p_full);
+            warp_arrive(&sm.p_full, lane);
             if (st) TC_STAMP(i, 6);
             return true;
-        };
-
-        // the row's sum over the thread's share of the tiles, complete in the row's lead thread
-        auto row_sum = [&]() -> float {
-            float l_row = l_acc + __shfl_xor_sync(FULL_MASK, l_acc, 16);
-            if (q < AR / 16) {
-                if (h2 && !hf) sm.lsum[r_own] = l_row;
-                named_bar(1 + q, 64); // (lsum is written again behind a later barrier of the two warps)
-                if (lead) l_row += sm.lsum[r_own];
-            }
-            return l_row;
         };
 
         if constexpr (BATCH) {
@@ -1030,17 +1055,22 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 if (st) TC_STAMP(i, 1);
                 tc_fence_after();
                 const bool act = 16 * q < GQ * k.T;
-                float s[ATP];
+                float s[2 * ATP];
                 if (act) tmem_scores(s_addr(i), s);
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&sm.s_empty[i % NSB]);
-                if (act) mask_tile(last_visible(k, k.n, k.T), s);
-                const float4 tm = tile_maxima(i, act, s);
+                warp_arrive(&sm.s_empty[i % NSB], lane);
+                float4 tm = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+                if (act) {
+                    const int lim = last_visible(k, k.n, k.T);
+                    mask_tile(0, lim, s);
+                    mask_tile(1, lim, s + ATP);
+                    tm = tile_maxima(s);
+                }
                 if (st) TC_STAMP(i, 3);
-                if (!softmax(i, act, carry, k.restart, tm, [&](float (&x)[ATP]) {
+                if (!softmax(i, act, carry, k.restart, tm, [&](int t, float (&x)[ATP]) {
 #pragma unroll
-                        for (int c = 0; c < ATP; c++) x[c] = s[c];
+                        for (int c = 0; c < ATP; c++) x[c] = s[ATP * t + c];
                     }))
                     break;
                 const int flags = k.flags;
@@ -1048,8 +1078,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 if (!(flags & REC_LAST)) continue;
                 // the segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below)
                 const int rows = GQ * k.T;
-                const float l_row = row_sum();
-                if (lead && r_own < rows) a.ml[(size_t) k.slot * AR + r_own] = make_float2(m_acc, l_row);
+                const float l_row = l_acc + __shfl_xor_sync(FULL_MASK, l_acc, 16);
+                if (!hf && r_own < rows) a.ml[(size_t) k.slot * AR + r_own] = make_float2(m_acc, l_row);
                 l_acc = 0.f;
                 m_acc = -CUDART_INF_F;
                 flush_slot = k.slot, flush_rows = rows;
@@ -1063,7 +1093,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         // Tile maxima run ahead of P (tasks: left by the producer, see there), so that a group's own maxima are published well
         // before the CTAs that hold the chunk's next groups need them: the CTAs of a kv head may drift apart by a group
         // without a poll having to wait. The lead grows from none (the first P needs only its own group's scores) to MAX_AHEAD groups.
-        const bool act = 16 * q < R, pub = lead && r_own < R, polls = !hf && r_own < R;
+        const bool act = 16 * q < R, pub = act && !hf && r_own < R;
         // tile maxima of group j, its own maxima published
         auto maxima = [&](int j) -> float4 {
             if (st) TC_STAMP(j, 0);
@@ -1071,12 +1101,15 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             const GroupRec & k = sm.tasks[j % NTASK];
             if (st) TC_STAMP(j, 1);
             tc_fence_after();
-            float s[ATP];
+            float4 tm = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
             if (act) {
+                float s[2 * ATP];
                 tmem_scores(s_addr(j), s);
-                mask_tile(last_visible(k, n, T), s);
+                const int lim = last_visible(k, n, T);
+                mask_tile(0, lim, s);
+                mask_tile(1, lim, s + ATP);
+                tm = tile_maxima(s);
             }
-            const float4 tm = tile_maxima(j, act, s);
             if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
                 __stcg(a.xa + xbase(k) + (size_t) k.b * AR,
                        ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(fmaxf(fmaxf(tm.x, tm.y), fmaxf(tm.z, tm.w))));
@@ -1086,7 +1119,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
         // the chunk's previous groups have most likely published them
         auto request_words = [&](const Task & k) {
-            if (polls && k.nb > 1 && exch_ok(k)) {
+            if (pub && k.nb > 1 && exch_ok(k)) {
                 const size_t xb0 = xbase(k);
                 if (k.b >= 1) w1 = __ldcv(a.xa + xb0 + (size_t) (k.b - 1) * AR);
                 if (k.b >= 2) w2 = __ldcv(a.xa + xb0 + (size_t) (k.b - 2) * AR);
@@ -1111,20 +1144,21 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             if (st) TC_STAMP(i, 3);
             float m_in = -CUDART_INF_F;
             const size_t xb0 = xbase(k);
-            if (polls && k.nb > 1 && exch_ok(k)) {
+            if (pub && k.nb > 1 && exch_ok(k)) {
                 if (k.b >= 1) m_in = poll_word(a.xa + xb0 + (size_t) (k.b - 1) * AR, w1, a.epoch, &sm.wc, a.status);
                 if (k.b >= 2) m_in = fmaxf(m_in, poll_word(a.xa + xb0 + (size_t) (k.b - 2) * AR, w2, a.epoch, &sm.wc, a.status));
                 if (k.b >= 3) m_in = fmaxf(m_in, poll_word(a.xb + xb0 + (size_t) (k.b - 3) * AR, w0, a.epoch, &sm.wc, a.status));
-                if (pub && k.b + 3 < k.nb)
+                if (k.b + 3 < k.nb)
                     __stcg(a.xb + xb0 + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) |
                                                                __float_as_uint(fmaxf(fmaxf(m_in, fmaxf(tm0.x, tm0.y)), fmaxf(tm0.z, tm0.w))));
             }
             __syncwarp();
             m_in = __shfl_sync(FULL_MASK, m_in, lane & 15);
             if (st) TC_STAMP(i, 7);
-            softmax(i, act, m_in, 0u, tm0, [&](float (&x)[ATP]) {
-                tmem_scores(s_addr(i), x);
-                mask_tile(last_visible(k, n, T), x);
+            const int lim = act ? last_visible(k, n, T) : 0;
+            softmax(i, act, m_in, 0u, tm0, [&](int t, float (&x)[ATP]) {
+                tmem_scores_tile(s_addr(i) + ATP * t, x);
+                mask_tile(t, lim, x);
             });
             tm0 = tm1;
             tm1 = tm2;
@@ -1152,8 +1186,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
 #endif
         // ---- the CTA's partial: O^T lanes are dims (in the unpacked units' order: mapped back here), columns are query rows ----
         read_out(slot, R, G > 0);
-        const float l_row = row_sum();
-        if (lead && r_own < R) a.ml[(size_t) slot * AR + r_own] = make_float2(m_acc, l_row);
+        const float l_row = l_acc + __shfl_xor_sync(FULL_MASK, l_acc, 16);
+        if (!hf && r_own < R) a.ml[(size_t) slot * AR + r_own] = make_float2(m_acc, l_row);
 #if MKKV_TC_PROF
         if (warp == 0) TC_STAMP(15, 11);
 #endif
