@@ -311,30 +311,6 @@ __device__ __forceinline__ float exp_any(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, LOG2E)));
     return y;
 }
-// pairs of fp32 in one instruction (sm_100a), each half rounded as the scalar form: with them, the masks of padding rows left out and one
-// vote per pass instead of three, 16 layers of 101,600 positions 1,334 -> 1,310 us, 32 sequences x 4 layers 2,885 -> 2,807
-typedef unsigned long long F2;
-__device__ __forceinline__ F2 f2_pack(float a, float b) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(F2 x, float & a, float & b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x)); }
-__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
-    F2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-    F2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-    F2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 __device__ __forceinline__ float ex2(float x) { // 2^x for x <= 0 (and -inf -> 0)
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -481,8 +481,11 @@ void KvEngine::append(int seq, int layer, int pos0, int n, const void * K, const
         // run is cut into pieces of at most one ring so no piece displaces its own rows
         for (int done = 0; done < n;) {
             const int p = pos0 + done, m = std::min(n - done, rc_);
-            spill_to(s, layer, std::min(p, p + m - rc_));
-            MKKV_CK(launch_append(s.views[layer], k + (size_t) done * NKV * HD, v + (size_t) done * NKV * HD, p, m, stream_));
+            const int from = s.spilled[layer], upto = std::min(p, p + m - rc_);
+            const bool together = upto > from && from >= p - rc_; // every row to be spilled is displaced by one of these
+            if (!together) spill_to(s, layer, upto);
+            MKKV_CK(launch_append(s.views[layer], k + (size_t) done * NKV * HD, v + (size_t) done * NKV * HD, p, m, stream_, together ? from : 0, together ? upto : 0));
+            if (together) s.spilled[layer] = upto;
             launches_++;
             done += m;
         }

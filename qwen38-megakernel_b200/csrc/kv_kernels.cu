@@ -20,6 +20,8 @@ namespace mkkv {
 // --------------------------------------------------------------------------------------------------------------------
 // append / spill / refill: one warp per row
 // --------------------------------------------------------------------------------------------------------------------
+constexpr int MANY_ROWS = 64; // more positions than these: four rows share a warp (fewer: a row a warp is the shorter chain)
+
 struct AppendArgs {
     KvView kv;
     const uint16_t * K;
@@ -65,21 +67,73 @@ __global__ void __launch_bounds__(256) append_kernel(const __grid_constant__ App
     append_row(a.kv, w, g, pos, (w ? a.V : a.K) + ((size_t) t * NKV + g) * HD, lane);
 }
 
-// rows [p0, p1) x layers x ring sides x kv heads, one warp per row: fp16 shadow row -> main-format row
+// ---- many rows: four to a warp, the four kv heads of one (position, side) ----
+__device__ __forceinline__ void load_block_f16(const uint16_t * src, float (&v)[32]) {
+    uint4 raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) raw[i] = reinterpret_cast<const uint4 *>(src)[i];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __half2 * h = reinterpret_cast<const __half2 *>(&raw[i]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const float2 f = __half22float2(h[k]);
+            v[8 * i + 2 * k] = f.x, v[8 * i + 2 * k + 1] = f.y;
+        }
+    }
+}
+// main-format rows of position pos, side w, from the fp16 shadow
+__device__ __forceinline__ void spill_rows4(const KvView & kv, int w, int pos, int lane) {
+    const KvSide & s = kv.s[w];
+    const int g = lane >> 3, sub = lane & 7;
+    float v[32];
+    load_block_f16(s.shadow + ((size_t) g * kv.rc + pos % kv.rc) * HD + 32 * sub, v);
+    if (s.rot) fwht256_block(v, sub);
+    const size_t row = (size_t) g * kv.ctxp + (pos - kv.base);
+    store_row_block(s.val + row * row_bytes(s.bits), s.sc + row * 8, v, s.bits, sub);
+}
+// rows pos0 .. of K and V, warp = (row, side). What bounds it: the quantizer's instructions; with a row a warp each division and extreme
+// was computed by all four lanes of a block and 40 values crossed lanes in a row's transform instead of 24. A prompt of 6,001 rows in
+// 16 layers and a step: 1,145 us with a row a warp and a spill launch before each append that displaces rows, 846 so.
+// Spill mode: the row whose ring and shadow slot this one takes (position - rc) is made in its main format first if it lies in
+// [spill0, spill1) (every one of those is displaced by a row of this launch).
+__global__ void __launch_bounds__(256) append_many_kernel(const __grid_constant__ AppendArgs a, int spill0, int spill1) {
+    const int lane = threadIdx.x & 31, idx = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (idx >= a.n * 2) return;
+    const int t = idx >> 1, w = idx & 1, pos = a.pos0 + t, g = lane >> 3, sub = lane & 7;
+    const KvView & kv = a.kv;
+    const KvSide & s = kv.s[w];
+    const uint16_t * src = (w ? a.V : a.K) + (size_t) t * NKV * HD;
+    if (s.shadow) {
+        const int old = pos - kv.rc;
+        if (old >= spill0 && old < spill1) spill_rows4(kv, w, old, lane);
+        __syncwarp(); // (the old row has been read by every lane)
+#pragma unroll
+        for (int h = 0; h < NKV; h++) { // (a row at a time: full sectors)
+            const size_t rr = (size_t) h * kv.rc + pos % kv.rc;
+            *reinterpret_cast<uint4 *>(s.shadow + rr * HD + lane * 8) = *reinterpret_cast<const uint4 *>(src + h * HD + lane * 8);
+        }
+    }
+    float v[32];
+    load_block_f16(src + (size_t) g * HD + 32 * sub, v);
+    if (s.rot) fwht256_block(v, sub);
+    if (kv.eager || !s.rval) {
+        const size_t row = (size_t) g * kv.ctxp + (pos - kv.base);
+        store_row_block(s.val + row * row_bytes(s.bits), s.sc + row * 8, v, s.bits, sub);
+    }
+    if (s.rval) {
+        const size_t rr = (size_t) g * kv.rc + pos % kv.rc;
+        store_q8_block(s.rval + rr * HD, s.rsc + rr * 8, v, sub);
+    }
+}
+
+// rows [p0, p1) x layers x ring sides: fp16 shadow rows -> main-format rows
 __global__ void __launch_bounds__(256) spill_kernel(const KvView * views, int layers, int p0, int p1) {
     const int lane = threadIdx.x & 31;
-    const long long total = (long long) (p1 - p0) * layers * 2 * NKV;
+    const long long total = (long long) (p1 - p0) * layers * 2;
     for (long long i = (long long) blockIdx.x * 8 + (threadIdx.x >> 5); i < total; i += (long long) gridDim.x * 8) {
-        const int g = (int) (i % NKV), w = (int) ((i / NKV) & 1), l = (int) ((i / (2 * NKV)) % layers);
-        const int pos = p0 + (int) (i / ((long long) 2 * NKV * layers));
-        const KvView & kv = views[l];
-        const KvSide & s = kv.s[w];
-        if (!s.shadow) continue;
-        float v[8];
-        load_row_f16(s.shadow + ((size_t) g * kv.rc + pos % kv.rc) * HD, lane, v);
-        if (s.rot) fwht256(v, lane);
-        const size_t row = (size_t) g * kv.ctxp + (pos - kv.base);
-        store_row(s.val + row * row_bytes(s.bits), s.sc + row * 8, v, s.bits, lane);
+        const int w = (int) (i & 1), l = (int) ((i >> 1) % layers);
+        if (views[l].s[w].shadow) spill_rows4(views[l], w, p0 + (int) ((i >> 1) / layers), lane);
     }
 }
 
@@ -220,16 +274,20 @@ cudaError_t launch_append_batch(const AppendJob * ajobs_dev, const AttnJob * job
     return cudaGetLastError();
 }
 
-cudaError_t launch_append(const KvView & kv, const uint16_t * K, const uint16_t * V, int pos0, int n, cudaStream_t stream) {
+cudaError_t launch_append(const KvView & kv, const uint16_t * K, const uint16_t * V, int pos0, int n, cudaStream_t stream, int spill0, int spill1) {
     if (n <= 0) return cudaSuccess;
     AppendArgs a{kv, K, V, pos0, n};
+    if (n > MANY_ROWS || spill1 > spill0) {
+        append_many_kernel<<<(n * 2 + 7) / 8, 256, 0, stream>>>(a, spill0, spill1);
+        return cudaGetLastError();
+    }
     append_kernel<<<(n * 2 * NKV + 7) / 8, 256, 0, stream>>>(a);
     return cudaGetLastError();
 }
 static int row_grid(long long rows) { return (int) std::min<long long>((rows + 7) / 8, 148 * 8); }
 cudaError_t launch_spill(const KvView * views, int layers, int p0, int p1, cudaStream_t stream) {
     if (p1 <= p0) return cudaSuccess;
-    spill_kernel<<<row_grid((long long) (p1 - p0) * layers * 2 * NKV), 256, 0, stream>>>(views, layers, p0, p1);
+    spill_kernel<<<row_grid((long long) (p1 - p0) * layers * 2), 256, 0, stream>>>(views, layers, p0, p1);
     return cudaGetLastError();
 }
 cudaError_t launch_refill(const KvView * views, int layers, int p0, int p1, cudaStream_t stream) {
@@ -338,7 +396,7 @@ static float2 * g_static_ml_addr[64] = {};
 static uint16_t * g_static_qp_addr[64] = {};
 cudaError_t preload_kernels() {
     cudaFuncAttributes fa;
-    const void * fns[] = {(const void *) append_kernel, (const void *) spill_kernel, (const void *) refill_kernel, (const void *) append_batch_kernel, (const void *) append_layers_kernel, (const void *) qprep_kernel,
+    const void * fns[] = {(const void *) append_kernel, (const void *) append_many_kernel, (const void *) spill_kernel, (const void *) refill_kernel, (const void *) append_batch_kernel, (const void *) append_layers_kernel, (const void *) qprep_kernel,
                           (const void *) gather_kernel, (const void *) attn_merge_kernel};
     for (const void * f : fns) {
         const cudaError_t e = cudaFuncGetAttributes(&fa, f);

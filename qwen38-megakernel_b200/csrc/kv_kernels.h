@@ -37,7 +37,9 @@ enum KernelStatus : int { KS_OK = 0, KS_WAIT_TIMEOUT = 1 };
 
 // rows pos0 .. pos0 + n - 1 of one (sequence, layer): K, V fp16 [n][4][256] -> ring q8 row (+ fp16 shadow) and, in eager
 // mode or for a side without a ring, the main-format row
-cudaError_t launch_append(const KvView & kv, const uint16_t * K, const uint16_t * V, int pos0, int n, cudaStream_t stream);
+// [spill0, spill1), spill mode: displaced positions (their slots are taken by this launch's rows, n <= ring rows) that still need
+// their main-format row, made by the same launch
+cudaError_t launch_append(const KvView & kv, const uint16_t * K, const uint16_t * V, int pos0, int n, cudaStream_t stream, int spill0 = 0, int spill1 = 0);
 // spill mode: main-format rows of positions [p0, p1) of the layers' ring sides, quantized from the fp16 shadow.
 // views: device array of KvView, one per layer
 cudaError_t launch_spill(const KvView * views, int layers, int p0, int p1, cudaStream_t stream);

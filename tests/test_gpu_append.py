@@ -219,3 +219,63 @@ def test_per_layer_spec_items_match_oracle(mk, torch_cuda):
         eng.sync()
         assert np.abs(O.cpu().numpy() - orc.attend(layer, n, Q)).max() <= 2e-3, layer
     eng.close()
+
+
+@pytest.mark.parametrize("bits", [4, 5, 6, 7, 8])
+@pytest.mark.parametrize("rot", [False, True])
+def test_many_rows_at_once_give_the_same_bytes(mk, torch_cuda, bits, rot):
+    """From 65 positions on four rows share a warp. The corner-case rows (zeros of both signs, ties, the type's extremes, subnormals) and
+    random ones, 65 and 97 positions at once, against the same rows in calls of 64 or fewer: every stored byte."""
+    torch = torch_cuda
+    edge = kvdata.edge_rows().astype(np.float16)
+    rng = np.random.default_rng(bits)
+    for n in (65, 97):
+        rows = (rng.standard_normal((n, 4, 256)) * rng.uniform(0.01, 30, (n, 4, 1))).astype(np.float16)
+        for i in range(len(edge)):
+            rows[(i * 5) % n, i % 4] = edge[i]
+        K, V = torch.from_numpy(rows).cuda(), torch.from_numpy(rows[::-1].copy()).cuda()
+        spec = "K*=%d%s,V*=%d%s" % (bits, "r" if rot else "", bits, "" if rot else "r")
+        engs = [mk.Engine(1, 256, spec, 640 if bits < 8 else 0) for _ in range(2)]
+        engs[0].append(0, 3, K, V)
+        for a in range(0, n, 40):
+            engs[1].append(0, 3 + a, K[a:a + 40].contiguous(), V[a:a + 40].contiguous())
+        for e in engs:
+            e.sync()
+        for w in range(2):
+            for g in range(4):
+                for p in range(3, 3 + n):
+                    for ring in (False, True) if engs[0].has_ring(w, 0) else (False,):
+                        (a, sa), (b, sb) = (e.read_row(0, w, g, p, ring=ring) for e in engs)
+                        assert np.array_equal(a, b) and np.array_equal(sa, sb), (n, w, g, p, ring)
+        for e in engs:
+            e.close()
+
+
+@pytest.mark.parametrize("first", [640, 3000, 3232, 3300])
+def test_displaced_rows_spill_with_the_rows_that_displace_them(mk, torch_cuda, first):
+    """Spill mode: an append past the ring's end makes the displaced rows' main-format rows in its own launch; 1 and 100 rows at a time,
+    from a fresh sequence, at the first displacement and after a rewind: the eager bytes"""
+    torch = torch_cuda
+    spec, win, L = "K*=5r,V*=6", 2048, 7000
+    eng, eager = (mk.Engine(1, L + 16, spec, win, spill=s) for s in (True, False))
+    K, V = (torch.from_numpy(x).cuda() for x in kvdata.kv_rows(9, 0, 0, L))
+    sizes, p, i = [first, 1, 100, 2, 65, 3232, 7], 0, 0
+    while p < L:
+        m = min(sizes[i % len(sizes)], L - p)
+        for e in (eng, eager):
+            e.append(0, p, K[p:p + m].contiguous(), V[p:p + m].contiguous())
+            e.commit(p + m)
+        p, i = p + m, i + 1
+        if i == 4:
+            for e in (eng, eager):
+                e.truncate(p - 5)
+            p -= 5
+    for e in (eng, eager):
+        e.sync()
+    for w in range(2):
+        for g in (0, 3):
+            for q in list(range(0, L - eng.ring_rows(), 53)) + [L - eng.ring_rows() - 1]:
+                (a, sa), (b, sb) = (e.read_row(0, w, g, q) for e in (eng, eager))
+                assert np.array_equal(a, b) and np.array_equal(sa, sb), (w, g, q)
+    for e in (eng, eager):
+        e.close()
