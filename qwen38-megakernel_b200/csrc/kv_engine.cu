@@ -951,10 +951,14 @@ void KvEngine::step_batch(int njobs, const int * seqs, int layer, const int * n,
     check_layer(layer);
     if (njobs < 1) return;
     if (njobs > work_jobs_) throw std::runtime_error("step_batch: call reserve_batch(" + std::to_string(njobs) + ") first");
-    // the job tables are reused by every call: the previous call's upload must have been consumed
-    MKKV_CK(cudaEventSynchronize(ev_compute_));
+    // Up to TABLE_JOBS jobs go along with the append launch, which leaves the table on the device; more are uploaded, and as the pinned
+    // table is reused by every call, the previous upload must have been consumed
+    const bool in_args = use_tc_ && njobs <= TABLE_JOBS && njobs <= qprep_slots_;
+    BatchTable table;
+    if (!in_args) MKKV_CK(cudaEventSynchronize(ev_compute_));
     static_assert(alignof(AppendJob) <= alignof(AttnJob), "append jobs behind attention jobs");
-    AppendJob * aj = reinterpret_cast<AppendJob *>(h_jobs_ + njobs);
+    AttnJob * const jobs = in_args ? table.job : h_jobs_;
+    AppendJob * const aj = reinterpret_cast<AppendJob *>(h_jobs_ + njobs);
     int items = 0, maxT = 0;
     size_t row = 0;
     for (int j = 0; j < njobs; j++) {
@@ -969,31 +973,43 @@ void KvEngine::step_batch(int njobs, const int * seqs, int layer, const int * n,
         wait_copies(s);
         if (do_append && cfg_.spill && rc_ > 0) spill_to(s, layer, n[j] + T[j] - rc_);
         if (do_append) s.kv_top = std::max(s.kv_top, n[j] + T[j]);
-        AttnJob & a = h_jobs_[j];
+        AttnJob & a = jobs[j];
         a = whole_job(s, "step_batch", layer, n[j], T[j], static_cast<const uint16_t *>(Q) + row * NH * HD, static_cast<float *>(O) + row * NH * HD);
         if (use_tc_ && j < qprep_slots_) a.Qp = qprep_ + (size_t) j * NKV * (QP_HEAD_BYTES / 2); // (staged below, every job in one launch)
         items += NKV * a.nch;
         maxT = std::max(maxT, T[j]);
-        aj[j].kv = a.kv;
-        aj[j].K = static_cast<const uint16_t *>(K) + row * NKV * HD;
-        aj[j].V = static_cast<const uint16_t *>(V) + row * NKV * HD;
-        aj[j].pos0 = n[j];
-        aj[j].n = T[j];
+        if (!in_args) {
+            aj[j].kv = a.kv;
+            aj[j].K = static_cast<const uint16_t *>(K) + row * NKV * HD;
+            aj[j].V = static_cast<const uint16_t *>(V) + row * NKV * HD;
+            aj[j].pos0 = n[j];
+            aj[j].n = T[j];
+        }
         row += T[j];
         spill_to(s, layer, a.ws);
     }
     if (items > work_items_) throw std::runtime_error("step_batch: call reserve_batch first");
-    plan_items(h_jobs_, njobs);
-    const size_t up = (sizeof(AttnJob) + (do_append ? sizeof(AppendJob) : 0)) * njobs; // (a multiple of 8)
-    *reinterpret_cast<unsigned *>(reinterpret_cast<char *>(h_jobs_) + up) = 0u;
-    batch_next_ = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(d_jobs_) + up);
-    MKKV_CK(cudaMemcpyAsync(d_jobs_, h_jobs_, up + sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
-    MKKV_CK(cudaEventRecord(ev_compute_, stream_));
-    if (do_append || use_tc_) {
-        MKKV_CK(launch_append_batch(do_append ? reinterpret_cast<const AppendJob *>(d_jobs_ + njobs) : nullptr, d_jobs_, njobs, maxT, stream_));
+    plan_items(jobs, njobs);
+    if (in_args) {
+        for (int j = 0; j < njobs; j++) table.row[j] = (int) ((jobs[j].Q - static_cast<const uint16_t *>(Q)) / (NH * HD)); // (plan_items has sorted them)
+        table.K = static_cast<const uint16_t *>(K);
+        table.V = static_cast<const uint16_t *>(V);
+        table.jobs = d_jobs_;
+        table.next = batch_next_ = d_next_;
+        MKKV_CK(launch_append_table(table, njobs, maxT, do_append, stream_));
         launches_++;
+    } else {
+        const size_t up = (sizeof(AttnJob) + (do_append ? sizeof(AppendJob) : 0)) * njobs; // (a multiple of 8)
+        *reinterpret_cast<unsigned *>(reinterpret_cast<char *>(h_jobs_) + up) = 0u;
+        batch_next_ = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(d_jobs_) + up);
+        MKKV_CK(cudaMemcpyAsync(d_jobs_, h_jobs_, up + sizeof(unsigned), cudaMemcpyHostToDevice, stream_));
+        MKKV_CK(cudaEventRecord(ev_compute_, stream_));
+        if (do_append || use_tc_) {
+            MKKV_CK(launch_append_batch(do_append ? reinterpret_cast<const AppendJob *>(d_jobs_ + njobs) : nullptr, d_jobs_, njobs, maxT, stream_));
+            launches_++;
+        }
     }
-    launch_attention(h_jobs_, njobs, items, maxT);
+    launch_attention(jobs, njobs, items, maxT);
 }
 
 // ---- rewind ----

@@ -218,6 +218,34 @@ __global__ void __launch_bounds__(256) append_batch_kernel(const AppendJob * ajo
     append_row(j.kv, w, g, pos, (w ? j.V : j.K) + ((size_t) t * NKV + g) * HD, lane);
 }
 
+// the same with the jobs in the launch's arguments, which leaves them in the device's table for the attention launch (the last block of a
+// job's row of blocks): no upload before it, no host wait for the one before
+__global__ void __launch_bounds__(256) append_table_kernel(const __grid_constant__ BatchTable b, int nab) {
+    release_next();
+    const AttnJob & J = b.job[blockIdx.y];
+    const int lane = threadIdx.x & 31;
+    if (blockIdx.x == gridDim.x - 1) {
+        static_assert(sizeof(AttnJob) % 4 == 0 && sizeof(AttnJob) / 4 < 255, "copied word by word");
+        const int i = threadIdx.x;
+        if (i < (int) (sizeof(AttnJob) / 4)) reinterpret_cast<unsigned *>(b.jobs + blockIdx.y)[i] = reinterpret_cast<const unsigned *>(&J)[i];
+        if (i == 255 && blockIdx.y == 0) *b.next = 0u;
+    }
+    if ((int) blockIdx.x >= nab) {
+        const int idx = ((int) blockIdx.x - nab) * 8 + (threadIdx.x >> 5);
+        qprep_row(J.Q, const_cast<uint16_t *>(J.Qp), J.T, J.kv.s[0].rot, idx / AR, idx % AR, lane);
+        return;
+    }
+    const int idx = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (idx >= J.T * 2 * NKV) return;
+    const int t = idx / (2 * NKV), w = (idx / NKV) & 1, g = idx % NKV;
+    append_row(J.kv, w, g, J.n + t, (w ? b.V : b.K) + ((size_t) (b.row[blockIdx.y] + t) * NKV + g) * HD, lane);
+}
+cudaError_t launch_append_table(const BatchTable & b, int njobs, int max_n, bool rows, cudaStream_t stream) {
+    const int nab = rows ? (max_n * 2 * NKV + 7) / 8 : 0;
+    append_table_kernel<<<dim3(nab + QP_BLOCKS, njobs), 256, 0, stream>>>(b, nab);
+    return cudaGetLastError();
+}
+
 // the same rows for every layer of one sequence in one launch: layer = blockIdx.y, its K / V rows kv_stride bytes after the previous
 // layer's (the views are the sequence's device-resident array, so a decode step uploads nothing). Blocks beyond the rows' stage the
 // layer's queries for the attention launch that follows (Q != null).
@@ -396,7 +424,7 @@ static float2 * g_static_ml_addr[64] = {};
 static uint16_t * g_static_qp_addr[64] = {};
 cudaError_t preload_kernels() {
     cudaFuncAttributes fa;
-    const void * fns[] = {(const void *) append_kernel, (const void *) append_many_kernel, (const void *) spill_kernel, (const void *) refill_kernel, (const void *) append_batch_kernel, (const void *) append_layers_kernel, (const void *) qprep_kernel,
+    const void * fns[] = {(const void *) append_kernel, (const void *) append_many_kernel, (const void *) spill_kernel, (const void *) refill_kernel, (const void *) append_batch_kernel, (const void *) append_table_kernel, (const void *) append_layers_kernel, (const void *) qprep_kernel,
                           (const void *) gather_kernel, (const void *) attn_merge_kernel};
     for (const void * f : fns) {
         const cudaError_t e = cudaFuncGetAttributes(&fa, f);

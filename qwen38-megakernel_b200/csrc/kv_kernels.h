@@ -109,6 +109,18 @@ struct AppendJob {
 };
 // the rows of append job j (ajobs_dev null: none) and the queries of attention job j (those with a Qp) in one launch
 cudaError_t launch_append_batch(const AppendJob * ajobs_dev, const AttnJob * jobs_dev, int njobs, int max_n, cudaStream_t stream);
+// The same for up to TABLE_JOBS jobs whose table travels as a kernel argument (6.6 KB): job j appends its T rows at position n, rows
+// row[j] .. of K / V (rows: false: none), and is copied to jobs[j] on the device; every job has a Qp. *next is zeroed.
+constexpr int TABLE_JOBS = 32;
+struct BatchTable {
+    AttnJob job[TABLE_JOBS];
+    int row[TABLE_JOBS];
+    const uint16_t * K;
+    const uint16_t * V;
+    AttnJob * jobs;
+    unsigned * next;
+};
+cudaError_t launch_append_table(const BatchTable & b, int njobs, int max_n, bool rows, cudaStream_t stream);
 // Queries staged for the tensor-core attention kernel (qwen38_mk.cu:2876-2883: fp16 -> fp32 -> K's rotation -> x 1/16 -> fp16), once
 // per (job, kv head) instead of once per CTA: QP_HEAD_BYTES bytes per kv head in that kernel's B-operand layout
 // [dim group 32][row group 6][8 rows][8 dims in the unpacked units' order], rows beyond 6 T zero. One bulk copy brings a head's block
