@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256) append_many_kernel(const __grid_constant_
         const size_t row = (size_t) g * kv.ctxp + (pos - kv.base);
         store_row_block(s.val + row * row_bytes(s.bits), s.sc + row * 8, v, s.bits, sub);
     }
-    if (s.rval) {
+    if (s.rval && pos + kv.rc >= a.pos0 + a.n) { // (more rows than the ring has: one of the last takes this one's slot, in any order)
         const size_t rr = (size_t) g * kv.rc + pos % kv.rc;
         store_q8_block(s.rval + rr * HD, s.rsc + rr * 8, v, sub);
     }

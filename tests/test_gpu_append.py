@@ -279,3 +279,15 @@ def test_displaced_rows_spill_with_the_rows_that_displace_them(mk, torch_cuda, f
                 assert np.array_equal(a, b) and np.array_equal(sa, sb), (w, g, q)
     for e in (eng, eager):
         e.close()
+
+
+@pytest.mark.parametrize("n", [1312, 1313, 1889, 4000])
+def test_more_rows_at_once_than_the_ring_has(mk, torch_cuda, n):
+    """Eager mode takes any number of rows in one launch: a ring slot keeps the last row that falls on it (1,312 rows for a 640 window)"""
+    torch = torch_cuda
+    eng, orc = mk.Engine(1, n + 8, "K*=5r,V*=6", 640), ko.Cache(1, n + 8, "K*=5r,V*=6", 640)
+    assert eng.ring_rows() == 1312
+    for rep in range(4):
+        fill_both(torch, eng, orc, 0, 0, n, seed=n + rep, chunk=n)
+        assert_rows_equal(eng, orc, 0, [0, n - 1], ring_positions=list(range(n - 1312, n, 41)) + [n - 1])
+    eng.close()
