@@ -791,13 +791,12 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
             // the packed bytes of both 128-dim halves are read first (they need no operand slot), then each half is written into its
             // slot as that slot frees up
             PackedBlock<B> b0, b1;
-            dq_load<B>(b0, rawa, lane, jr, valid);
-            dq_load<B>(b1, rawa, lane, 4 + jr, valid);
+            dq_load<B>(b0, b1, rawa, lane, jr, valid);
             tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            dq_emit<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048);
+            dq_emit<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
             hand_over();
             tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            dq_emit<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048);
+            dq_emit<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
             hand_over();
         };
         // one side of group j; false: the CTA has given up

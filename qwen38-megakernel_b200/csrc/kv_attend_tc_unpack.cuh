@@ -51,11 +51,6 @@ __device__ __forceinline__ unsigned lds32(unsigned addr) {
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ unsigned lds16(unsigned addr) {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
-    return v;
-}
 // The two biases, in registers: an AND-OR has room for one immediate, and constants that the compiler knows are loaded anew for each
 // (an opaque value is not)
 struct UnpackConst {
@@ -80,32 +75,49 @@ template <int BITS> struct PackedBlock {
     unsigned h[3];                 // the block's high bits: 4 (5 bits), 8 (6 bits) or 12 bytes (7 bits)
     unsigned d;                    // the block's scale as an fp16 pair (0 for a row past the chunk end)
 };
-template <int BITS> __device__ __forceinline__ void dq_load(PackedBlock<BITS> & b, unsigned raw, int row, int jb, bool valid) {
-    const unsigned sc = valid ? lds16(raw + TILE_SC_OFF + (row * 8 + jb) * 2) : 0u;
-    b.d = sc | (sc << 16);
+// 8 bits: which half of a block row `row`'s lane holds in w[0 .. 3]: with the blocks rotated by the row, the 16-byte loads of eight lanes then
+// fall into eight different bank groups
+__device__ __forceinline__ unsigned half_swap(int row) { return (row >> 2) & 1; }
+// Blocks jr and 4 + jr (jr 0 .. 3) of row `row` of a staged tile. The row's eight scales come with one load: fetched one by one, 16 bytes
+// apart from lane to lane, they took four shared-memory cycles each, and shared memory is the scarcest pipe here (an unpack loop alone
+// takes 29 cycles a unit and scheduler, 26 of them its loads and stores).
+template <int BITS> __device__ __forceinline__ void dq_load(PackedBlock<BITS> & b0, PackedBlock<BITS> & b1, unsigned raw, int row, int jr, bool valid) {
+    const uint4 sc = lds128(raw + TILE_SC_OFF + row * SCALE_ROW);
+    const unsigned s0 = (jr & 2) ? sc.y : sc.x, s1 = (jr & 2) ? sc.w : sc.z, pick = (jr & 1) ? 0x3232u : 0x1010u;
+    b0.d = valid ? __byte_perm(s0, 0u, pick) : 0u;
+    b1.d = valid ? __byte_perm(s1, 0u, pick) : 0u;
     const unsigned rp = raw + row * (32 * BITS);
-    if constexpr (BITS == 8) {
-        const uint4 v0 = lds128(rp + 32 * jb), v1 = lds128(rp + 32 * jb + 16);
-        b.w[0] = v0.x, b.w[1] = v0.y, b.w[2] = v0.z, b.w[3] = v0.w, b.w[4] = v1.x, b.w[5] = v1.y, b.w[6] = v1.z, b.w[7] = v1.w;
-    } else {
-        const uint4 nv = lds128(rp + 16 * jb);
-        b.w[0] = nv.x, b.w[1] = nv.y, b.w[2] = nv.z, b.w[3] = nv.w;
-        if constexpr (BITS == 5) b.h[0] = lds32(rp + 128 + 4 * jb);
-        if constexpr (BITS == 6) {
-            const uint2 h = lds64(rp + 128 + 8 * jb);
-            b.h[0] = h.x, b.h[1] = h.y;
+    PackedBlock<BITS> * const bs[2] = {&b0, &b1};
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        PackedBlock<BITS> & b = *bs[h];
+        const int jb = jr + 4 * h;
+        if constexpr (BITS == 8) { // (rows 256 bytes apart: lanes 4 .. 7 of eight start with the block's second 16 bytes, see half_swap)
+            const unsigned first = 16u * half_swap(row);
+            const uint4 v0 = lds128(rp + 32 * jb + first), v1 = lds128(rp + 32 * jb + (16u - first));
+            b.w[0] = v0.x, b.w[1] = v0.y, b.w[2] = v0.z, b.w[3] = v0.w, b.w[4] = v1.x, b.w[5] = v1.y, b.w[6] = v1.z, b.w[7] = v1.w;
+        } else {
+            const uint4 nv = lds128(rp + 16 * jb);
+            b.w[0] = nv.x, b.w[1] = nv.y, b.w[2] = nv.z, b.w[3] = nv.w;
+            if constexpr (BITS == 5) b.h[0] = lds32(rp + 128 + 4 * jb);
+            if constexpr (BITS == 6) {
+                const uint2 hw = lds64(rp + 128 + 8 * jb);
+                b.h[0] = hw.x, b.h[1] = hw.y;
+            }
+            if constexpr (BITS == 7) b.h[0] = lds32(rp + 128 + 12 * jb), b.h[1] = lds32(rp + 132 + 12 * jb), b.h[2] = lds32(rp + 136 + 12 * jb);
         }
-        if constexpr (BITS == 7) b.h[0] = lds32(rp + 128 + 12 * jb), b.h[1] = lds32(rp + 132 + 12 * jb), b.h[2] = lds32(rp + 136 + 12 * jb);
     }
 }
-template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned dst) {
+// row: the block's row (8 bits only)
+template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned dst, int row) {
     const unsigned d = b.d;
     if constexpr (BITS == 8) {
         constexpr unsigned S8 = MAGIC_A + 0x00800080u;
+        const unsigned half[2] = {dst + half_swap(row) * 4096u, dst + 4096u - half_swap(row) * 4096u};
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const unsigned lo = b.w[2 * u] ^ 0x80808080u, hi = b.w[2 * u + 1] ^ 0x80808080u; // q + 128
-            sts128(dst + u * 2048, pair_val<S8>(__byte_perm(lo, uc.a, 0x7270), d), // (value 0, value 2) under the exponent of 1024
+            sts128(half[u >> 1] + (u & 1) * 2048, pair_val<S8>(__byte_perm(lo, uc.a, 0x7270), d), // (value 0, value 2) under the exponent of 1024
                    pair_val<S8>(__byte_perm(hi, uc.a, 0x7270), d),                 // (4, 6)
                    pair_val<S8>(__byte_perm(lo, uc.a, 0x7371), d),                 // (1, 3)
                    pair_val<S8>(__byte_perm(hi, uc.a, 0x7371), d));                // (5, 7)
@@ -143,9 +155,10 @@ template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BI
 }
 // one block
 template <int BITS> __device__ __forceinline__ void dq_item(unsigned raw, int row, int jb, bool valid, unsigned dst) {
-    PackedBlock<BITS> b;
-    dq_load<BITS>(b, raw, row, jb, valid);
-    dq_emit<BITS>(b, unpack_const(), dst);
+    PackedBlock<BITS> b0, b1;
+    dq_load<BITS>(b0, b1, raw, row, jb & 3, valid);
+    if (jb < 4) dq_emit<BITS>(b0, unpack_const(), dst, row);
+    else dq_emit<BITS>(b1, unpack_const(), dst, row);
 }
 } // namespace tc
 } // namespace mkkv
