@@ -18,14 +18,14 @@
 //     buffers share their columns), O^T (two 128-dim halves) resident there for the whole kernel;
 //   - four softmax warps read S back (tcgen05.ld 16x32bx2: a thread owns one query row and 64 of its positions), so that a tile's
 //     maximum and sum are taken inside a thread (with positions on lanes they were 24 warp reductions a warp and group, a barrier and
-//     a hand-out of each row's maxima: 1.9 k more instructions a group); they exchange the running
-//     max with the CTAs that hold the chunk's earlier groups through small global arrays (own group maxima and cumulative
-//     maxima, 8-byte {launch tag, value} words, polled with a bound; maxima two groups ahead of P), and write P to shared memory as
-//     the K-major B operand. The
+//     a hand-out of each row's maxima: 1.9 k more instructions a group), and write P to shared memory as the K-major B operand. The
 //     accumulator is kept against a per-row reference max that moves rarely (when the running max passes it by more than 11;
 //     then the moved rows' accumulator columns are rescaled, one tensor-memory column per row and block): P, after its fp16
 //     rounding, is multiplied by exp(running max - reference) and carried as an fp16 high and low part (one N = 96 MMA per k-step, two
 //     48-column accumulator blocks), so the reference's fp16 P is reproduced and no per-tile accumulator rescale is needed;
+//   - spread mode: four more warps take the tile maxima two groups ahead of P and exchange the running max with the CTAs that hold the
+//     chunk's earlier groups through small global arrays (own group maxima and cumulative maxima, 8-byte {launch tag, value} words,
+//     polled with a bound, the missing ones together);
 //   - a CTA writes one un-normalised partial (m, l, O); when the CTAs of a kv head have all written theirs (arrival count,
 //     bounded wait) each merges one or two of the head's rows in the kernel's tail, four warps to a row;
 //   - batch mode (several jobs: sequences served together, or all layers of a decode step): a plain launch of one persistent CTA per
@@ -62,14 +62,18 @@ constexpr int NDQ = 16;        // then the unpack warps: 4 c + q, tile q, 32-dim
 // then the control warps, two of them idle to complete a group of four (register reallocation is per group). The issuer is the warp on
 // the scheduler whose softmax warp has no query rows.
 constexpr int W_CTL = NSOFT + NDQ, W_PROD = W_CTL + 2, W_ISSUE = W_CTL + 3;
-constexpr int NTHREADS = (W_CTL + 4) * 32;
+constexpr int W_MAX = W_CTL + 4;      // spread mode only: four warps that take the tile maxima and exchange the running maxima
+constexpr int NTHREADS = W_MAX * 32, NTHREADS_SPREAD = (W_MAX + 4) * 32;
 constexpr int GT = 4, GP = GT * ATP;        // tiles / positions per group: the N of an S instruction
 // registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
 // most the CTA's launch allocation -- a larger sum faults)
-#define MKKV_TC_REGS_SOFT "168"
+#define MKKV_TC_REGS_SOFT "176"
 #define MKKV_TC_REGS_DQ "56"
-#define MKKV_TC_REGS_CTL "80"
-static_assert(NTHREADS == 768 && 4 * 168 + 16 * 56 + 4 * 80 <= 24 * 80, "register shares");
+#define MKKV_TC_REGS_CTL "72"
+static_assert(NTHREADS == 768 && 4 * 176 + 16 * 56 + 4 * 72 <= 24 * 80, "register shares");
+#define MKKV_TC_REGS_SOFT_SPREAD "152"
+#define MKKV_TC_REGS_CTL_SPREAD "56" // (the maxima warps keep the launch's 72)
+static_assert(NTHREADS_SPREAD == 896 && 4 * 152 + 16 * 56 + 4 * 56 + 4 * 72 <= 28 * 72, "register shares");
 constexpr int RAW_SLOT = ATP * HD + ATP * SCALE_ROW; // one tile of the widest format and its scales: 8704 bytes
 constexpr int NRAW = 8;                     // packed tile slots: two side-groups (one being unpacked, one in flight)
 static_assert(NRAW % GT == 0, "whole groups only: a 7-slot ring, tried once, was 20 % slower and its results changed from run to run");
@@ -141,6 +145,10 @@ struct Smem {
     // batch mode only
     TileSrc vsrc[NTASK][GT];    // the V tiles of the groups whose K the producer has fetched
     uint64_t rec_full[NTASK];   // record (group % NTASK) is written
+    // spread mode only
+    float tmax[NSB][GT][AR];    // row maxima of a group's tiles and the running max before it, by group % NSB
+    float m_in[NSB][AR];
+    uint64_t m_full[NSB];
 };
 
 struct Args {
@@ -317,21 +325,22 @@ __device__ __forceinline__ float ex2(float x) { // 2^x for x <= 0 (and -inf -> 0
     return y;
 }
 
-// bounded poll of an exchange word until it carries this launch's tag
-__device__ __forceinline__ float poll_word(const unsigned long long * src, unsigned long long w, int epoch, volatile WaitCtl * wc, int * status) {
-    if ((unsigned) (w >> 32) != (unsigned) epoch) {
-        const unsigned rounds = wc->poll;
-        for (unsigned it = 0; (unsigned) (w >> 32) != (unsigned) epoch; it++) {
-            if (wc->dead) break;
-            if (it >= rounds) { // (a round is a trip to the L2)
-                wc->dead = 1;
-                atomicExch(status, (int) KS_WAIT_TIMEOUT);
-                break;
-            }
-            w = __ldcv(src);
+// bounded poll of up to three exchange words until each carries this launch's tag (null: not needed); what is missing is asked for together
+__device__ __forceinline__ void poll_words(const unsigned long long * (&src)[3], unsigned long long (&w)[3], int epoch, volatile WaitCtl * wc, int * status) {
+    for (unsigned it = 0;; it++) {
+        bool ready = true;
+#pragma unroll
+        for (int x = 0; x < 3; x++) ready = ready && (!src[x] || (unsigned) (w[x] >> 32) == (unsigned) epoch);
+        if (ready || wc->dead) return;
+        if (it >= wc->poll) { // (a round is a trip to the L2)
+            wc->dead = 1;
+            atomicExch(status, (int) KS_WAIT_TIMEOUT);
+            return;
         }
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+            if (src[x] && (unsigned) (w[x] >> 32) != (unsigned) epoch) w[x] = __ldcv(src[x]);
     }
-    return __uint_as_float((unsigned) w);
 }
 // task t of a kv head (group-major over its chunks), 4 tiles per task; mul_*: ceil(2^32 / divisor) (exact quotients for t < 2^26)
 struct Geo4 {
@@ -559,12 +568,40 @@ __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int
 #endif
 }
 
+// ---- scores of one row on one thread (hf 0: tiles 0 and 1 of the group, 1: tiles 2 and 3) ----
+// S buffer of group j: rows on 16 lanes of the warp's quarter (the other 16 are the neighbouring buffer's), positions on columns
+__device__ __forceinline__ unsigned s_buffer(unsigned lane_addr, int j) { return lane_addr + S_COL + S_STRIDE * ((j % NSB) >> 1) + ((unsigned) (16 * (j & 1)) << 16); }
+// the last of the thread's 64 positions that its row sees: row token t sees positions <= n + t, nothing is visible past the chunk end
+// (all of them for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their queries are zero, so are their
+// scores, and no one reads what becomes of them.
+__device__ __forceinline__ int last_visible_of(const GroupRec & k, int n, int t, int hf) {
+    if (k.pos0 + GP - 1 <= min(k.c1 - 1, n)) return 2 * ATP; // (the group reaches neither the chunk's end nor the new tokens)
+    return min(k.c1 - 1, n + t) - k.pos0 - 2 * ATP * hf;
+}
+__device__ __forceinline__ void mask_tile_of(int t, int lim, float * s) {
+    if (lim < 2 * ATP) {
+#pragma unroll
+        for (int c = 0; c < ATP; c++)
+            if (ATP * t + c > lim) s[c] = -CUDART_INF_F;
+    }
+}
+__device__ __forceinline__ float tile_max(const float * s) {
+    float x[ATP / 2];
+#pragma unroll
+    for (int c = 0; c < ATP / 2; c++) x[c] = fmaxf(s[2 * c], s[2 * c + 1]);
+#pragma unroll
+    for (int o = ATP / 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < o; c++) x[c] = fmaxf(x[c], x[c + o]);
+    return x[0];
+}
+
 // KB / VB: the bits of the K / V main rows the instance is compiled for (0: any, decided per tile at run time). A compiled-in
 // format leaves two unpack bodies per side (the format and the q8_0 ring) instead of five: a smaller instruction footprint.
 // BATCH: the instance for several jobs (persistent CTAs over runs of chunks, no exchange between CTAs); the instance for one
 // job spread over the SMs carries none of that mode's code (with both modes in one body the spread mode's loops came out 1.7 %
 // slower).
-template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS, 1) attn_tc_kernel(const __grid_constant__ Args a) {
+template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? NTHREADS : NTHREADS_SPREAD, 1) attn_tc_kernel(const __grid_constant__ Args a) {
     // (the dynamic shared memory starts on a 128-byte boundary -- there is no static shared memory in this kernel --, which is all the
     // bulk copies, matrix descriptors and barriers need; no pointer arithmetic here, so every access below is a shared-space one)
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -576,12 +613,12 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
     if (!BATCH) {
         const unsigned * src = reinterpret_cast<const unsigned *>(&a.one);
         unsigned * dst = reinterpret_cast<unsigned *>(&sm.job);
-        for (int i = tid; i < (int) (sizeof(AttnJob) / 4); i += NTHREADS) dst[i] = src[i];
+        for (int i = tid; i < (int) (sizeof(AttnJob) / 4); i += NTHREADS_SPREAD) dst[i] = src[i];
     }
     if (tid == 0) {
         for (int s = 0; s < NRAW; s++) { mbar_init(&sm.raw_full[s], 1); mbar_init(&sm.raw_empty[s], NDQ / GT); }
         for (int s = 0; s < NOP; s++) { mbar_init(&sm.op_full[s], NDQ); mbar_init(&sm.op_empty[s], 1); }
-        for (int s = 0; s < NSB; s++) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.s_empty[s], NSOFT); }
+        for (int s = 0; s < NSB; s++) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.s_empty[s], BATCH ? NSOFT : NSOFT + 4); mbar_init(&sm.m_full[s], 4); }
         mbar_init(&sm.p_full, NSOFT);
         mbar_init(&sm.p_empty, 1);
         mbar_init(&sm.fin, 1);
@@ -628,8 +665,106 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
     // The kv head's query rows come staged (qprep: fp16 -> fp32 -> K's rotation -> x 1/16 -> fp16 in the K-major B operand's layout,
     // row = (head % 6) T + t): the producer fetches the block with one bulk copy, the issuer waits for it.
     // registers move from the unpack / control warps to the softmax warps
-    if (warp >= W_CTL) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
+    if (!BATCH && warp >= W_MAX) {
+        // ---- spread mode, maxima warps: warp W_MAX + q takes the tile maxima of query rows 16 q .. + 15 (a thread: one row, two of the tiles),
+        // publishes each group's, collects the running max before it and leaves both for the softmax warp of the same rows. Tile maxima
+        // run ahead of P, so that a group's own maxima are published well before the CTAs that hold the chunk's next groups need them: the
+        // CTAs of a kv head may drift apart by a group without a poll having to wait. The lead grows from none (the first P needs only
+        // its own group's scores) to MAX_AHEAD groups. (In the softmax warps, between one P and the next, maxima and polls took 2,900 of a
+        // group's 7,800 cycles: one layer of 101,600 positions 111 us, 103 with warps of their own, 99.6 with the words polled together.) ----
+        const int q = warp & 3, hf = lane >> 4, r_own = 16 * q + (lane & 15);
+        const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
+        const bool st = q == 0, act = 16 * q < R, pub = act && !hf && r_own < R;
+        (void) st;
+        auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
+        // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
+        // producer never reached are not valid) and only inside their bounds
+        auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
+        unsigned long long w[3] = {0ull, 0ull, 0ull};
+        // the words of the groups one and two before, and the cumulative one of the group three before
+        auto words = [&](const Task & k, const unsigned long long * (&src)[3]) {
+            const size_t xb0 = xbase(k);
+            src[0] = k.b >= 1 ? a.xa + xb0 + (size_t) (k.b - 1) * AR : nullptr;
+            src[1] = k.b >= 2 ? a.xa + xb0 + (size_t) (k.b - 2) * AR : nullptr;
+            src[2] = k.b >= 3 ? a.xb + xb0 + (size_t) (k.b - 3) * AR : nullptr;
+        };
+        // tile maxima of group j, its own maxima published
+        auto maxima = [&](int j) {
+            if (st) TC_STAMP(j, 0);
+            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
+            const GroupRec & k = sm.tasks[j % NTASK];
+            if (st) TC_STAMP(j, 1);
+            tc_fence_after();
+            float m[2] = {-CUDART_INF_F, -CUDART_INF_F};
+            if (act) {
+                const int lim = last_visible_of(k, n, r_own % T, hf);
+                const unsigned sa = s_buffer(lane_addr, j);
+#pragma unroll
+                for (int t = 0; t < 2; t++) {
+                    float s[ATP];
+                    tmem_scores_tile(sa + ATP * t, s);
+                    mask_tile_of(t, lim, s);
+                    m[t] = tile_max(s);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            warp_arrive(&sm.s_empty[j % NSB], lane);
+            if (act) {
+                sm.tmax[j % NSB][2 * hf][r_own] = m[0];
+                sm.tmax[j % NSB][2 * hf + 1][r_own] = m[1];
+            }
+            __syncwarp();
+            const float mine = fmaxf(m[0], m[1]), group = fmaxf(mine, __shfl_xor_sync(FULL_MASK, mine, 16));
+            if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
+                __stcg(a.xa + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(group));
+            if (st) TC_STAMP(j, 2);
+        };
+        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
+        // the chunk's previous groups have most likely published them
+        auto request_words = [&](const Task & k) {
+            if (pub && k.nb > 1 && exch_ok(k)) {
+                const unsigned long long * src[3];
+                words(k, src);
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+                    if (src[x]) w[x] = __ldcv(src[x]);
+            }
+        };
+        constexpr int MAX_AHEAD = 2;
+        static_assert(MAX_AHEAD + 1 < NSB, "S of the groups ahead stays until their P");
+        int maxima_done = 0;
+        for (int i = 0; i < G; i++) {
+            const int want = min(G, i + 1 + min(i, MAX_AHEAD));
+            while (maxima_done < want) maxima(maxima_done++);
+            const GroupRec & k = sm.tasks[i % NTASK];
+            float m_in = -CUDART_INF_F;
+            if (pub && k.nb > 1 && exch_ok(k)) {
+                const unsigned long long * src[3];
+                words(k, src);
+                poll_words(src, w, a.epoch, &sm.wc, a.status);
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+                    if (src[x]) m_in = fmaxf(m_in, __uint_as_float((unsigned) w[x]));
+                if (k.b + 3 < k.nb) {
+                    const float(&x)[GT][AR] = sm.tmax[i % NSB];
+                    const float M = fmaxf(fmaxf(m_in, fmaxf(x[0][r_own], x[1][r_own])), fmaxf(x[2][r_own], x[3][r_own]));
+                    __stcg(a.xb + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(M));
+                }
+            }
+            if (st) TC_STAMP(i, 7);
+            if (act && !hf) sm.m_in[i % NSB][r_own] = m_in;
+            __syncwarp();
+            warp_arrive(&sm.m_full[i % NSB], lane);
+            if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
+                request_words(sm.tasks[(i + 1) % NTASK]);
+            } else {
+                w[0] = w[1] = w[2] = 0ull; // (no early request: the polls fetch the words themselves)
+            }
+        }
+    } else if (warp >= W_CTL) {
+    if constexpr (BATCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL_SPREAD ";");
     if (warp == W_PROD) {
         if constexpr (BATCH) {
             batch_producer(sm, a, lane);
@@ -832,7 +967,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         if constexpr (!BATCH)
             if (a.done && w < MERGE_WARPS - NSOFT) tail_merge(sm, a, g, kk, T, NSOFT + w, lane);
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
+        if constexpr (BATCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT_SPREAD ";");
 #if MKKV_TC_PROF
         const unsigned long long t_loop = globaltimer_ns();
 #endif
@@ -846,41 +982,12 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
         const bool st = warp == 0;
         float l_acc = 0.f, m_acc = -CUDART_INF_F; // row sum over the thread's positions, reference max
         float carry = -CUDART_INF_F;              // (batch mode: the running max after the previous group)
-        unsigned long long w0 = 0, w1 = 0, w2 = 0;
-        auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
-        // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
-        // producer never reached are not valid) and only inside their bounds
-        auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
-        // S buffer of group j: rows on 16 lanes of the warp's quarter (the other 16 are the neighbouring buffer's), positions on columns
-        auto s_addr = [&](int j) -> unsigned { return lane_addr + S_COL + S_STRIDE * ((j % NSB) >> 1) + ((unsigned) (16 * (j & 1)) << 16); };
-        // the last of the thread's 64 positions that its row sees: row token t sees positions <= n + t, nothing is visible past the
-        // chunk end (all of them for almost every group: uniform test first). Rows beyond the job's 6 T need no mask: their queries are
-        // zero, so are their scores, and no one reads what becomes of them.
-        auto last_visible = [&](const GroupRec & k, int nn, int Tk) -> int {
-            if (k.pos0 + GP - 1 <= min(k.c1 - 1, nn)) return 2 * ATP; // (the group reaches neither the chunk's end nor the new tokens)
-            return min(k.c1 - 1, nn + r_own % Tk) - k.pos0 - 2 * ATP * hf;
-        };
-        auto mask_tile = [&](int t, int lim, float * s) {
-            if (lim < 2 * ATP) {
-#pragma unroll
-                for (int c = 0; c < ATP; c++)
-                    if (ATP * t + c > lim) s[c] = -CUDART_INF_F;
-            }
-        };
+        auto s_addr = [&](int j) -> unsigned { return s_buffer(lane_addr, j); };
+        auto last_visible = [&](const GroupRec & k, int nn, int Tk) -> int { return last_visible_of(k, nn, r_own % Tk, hf); };
+        auto mask_tile = [&](int t, int lim, float * s) { mask_tile_of(t, lim, s); };
         // maxima of the group's four tiles (the same in both threads of a row)
         auto tile_maxima = [&](const float (&s)[2 * ATP]) -> float4 {
-            float m[2];
-#pragma unroll
-            for (int t = 0; t < 2; t++) {
-                float x[ATP / 2];
-#pragma unroll
-                for (int c = 0; c < ATP / 2; c++) x[c] = fmaxf(s[ATP * t + 2 * c], s[ATP * t + 2 * c + 1]);
-#pragma unroll
-                for (int o = ATP / 4; o > 0; o >>= 1)
-#pragma unroll
-                    for (int c = 0; c < o; c++) x[c] = fmaxf(x[c], x[c + o]);
-                m[t] = x[0];
-            }
+            const float m[2] = {tile_max(s), tile_max(s + ATP)};
             const float o0 = __shfl_xor_sync(FULL_MASK, m[0], 16), o1 = __shfl_xor_sync(FULL_MASK, m[1], 16);
             return hf ? make_float4(o0, o1, m[0], m[1]) : make_float4(m[0], m[1], o0, o1);
         };
@@ -1065,83 +1172,26 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(NTHREADS
                 read_out(flush_slot, flush_rows, true);
             }
         } else {
-        // Tile maxima run ahead of P (tasks: left by the producer, see there), so that a group's own maxima are published well
-        // before the CTAs that hold the chunk's next groups need them: the CTAs of a kv head may drift apart by a group
-        // without a poll having to wait. The lead grows from none (the first P needs only its own group's scores) to MAX_AHEAD groups.
-        const bool act = 16 * q < R, pub = act && !hf && r_own < R;
-        // tile maxima of group j, its own maxima published
-        auto maxima = [&](int j) -> float4 {
-            if (st) TC_STAMP(j, 0);
-            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
-            const GroupRec & k = sm.tasks[j % NTASK];
-            if (st) TC_STAMP(j, 1);
-            tc_fence_after();
-            float4 tm = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
-            if (act) {
-                float s[2 * ATP];
-                tmem_scores(s_addr(j), s);
-                const int lim = last_visible(k, n, T);
-                mask_tile(0, lim, s);
-                mask_tile(1, lim, s + ATP);
-                tm = tile_maxima(s);
-            }
-            if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
-                __stcg(a.xa + xbase(k) + (size_t) k.b * AR,
-                       ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(fmaxf(fmaxf(tm.x, tm.y), fmaxf(tm.z, tm.w))));
-            if (st) TC_STAMP(j, 2);
-            return tm;
-        };
-        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
-        // the chunk's previous groups have most likely published them
-        auto request_words = [&](const Task & k) {
-            if (pub && k.nb > 1 && exch_ok(k)) {
-                const size_t xb0 = xbase(k);
-                if (k.b >= 1) w1 = __ldcv(a.xa + xb0 + (size_t) (k.b - 1) * AR);
-                if (k.b >= 2) w2 = __ldcv(a.xa + xb0 + (size_t) (k.b - 2) * AR);
-                if (k.b >= 3) w0 = __ldcv(a.xb + xb0 + (size_t) (k.b - 3) * AR);
-            }
-        };
-        constexpr int MAX_AHEAD = 2;
-        static_assert(MAX_AHEAD + 1 < NSB, "S of the groups ahead stays until their P");
-        float4 tm0, tm1, tm2; // of groups i, i + 1, i + 2
-        tm0 = tm1 = tm2 = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
-        int maxima_done = 0;
+        // tile maxima and incoming running max come from the maxima warps (above)
+        const bool act = 16 * q < R;
         for (int i = 0; i < G; i++) {
-            const int want = min(G, i + 1 + min(i, MAX_AHEAD));
-            while (maxima_done < want) {
-                const float4 t = maxima(maxima_done);
-                if (maxima_done == i) tm0 = t;
-                else if (maxima_done == i + 1) tm1 = t;
-                else tm2 = t;
-                maxima_done++;
-            }
+            tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
+            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
+            tc_fence_after();
             const GroupRec & k = sm.tasks[i % NTASK];
             if (st) TC_STAMP(i, 3);
+            float4 tm = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
             float m_in = -CUDART_INF_F;
-            const size_t xb0 = xbase(k);
-            if (pub && k.nb > 1 && exch_ok(k)) {
-                if (k.b >= 1) m_in = poll_word(a.xa + xb0 + (size_t) (k.b - 1) * AR, w1, a.epoch, &sm.wc, a.status);
-                if (k.b >= 2) m_in = fmaxf(m_in, poll_word(a.xa + xb0 + (size_t) (k.b - 2) * AR, w2, a.epoch, &sm.wc, a.status));
-                if (k.b >= 3) m_in = fmaxf(m_in, poll_word(a.xb + xb0 + (size_t) (k.b - 3) * AR, w0, a.epoch, &sm.wc, a.status));
-                if (k.b + 3 < k.nb)
-                    __stcg(a.xb + xb0 + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) |
-                                                               __float_as_uint(fmaxf(fmaxf(m_in, fmaxf(tm0.x, tm0.y)), fmaxf(tm0.z, tm0.w))));
+            if (act) {
+                const float(&x)[GT][AR] = sm.tmax[i % NSB];
+                tm = make_float4(x[0][r_own], x[1][r_own], x[2][r_own], x[3][r_own]);
+                m_in = sm.m_in[i % NSB][r_own];
             }
-            __syncwarp();
-            m_in = __shfl_sync(FULL_MASK, m_in, lane & 15);
-            if (st) TC_STAMP(i, 7);
             const int lim = act ? last_visible(k, n, T) : 0;
-            softmax(i, act, m_in, 0u, tm0, [&](int t, float (&x)[ATP]) {
+            softmax(i, act, m_in, 0u, tm, [&](int t, float (&x)[ATP]) {
                 tmem_scores_tile(s_addr(i) + ATP * t, x);
                 mask_tile(t, lim, x);
             });
-            tm0 = tm1;
-            tm1 = tm2;
-            if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
-                request_words(sm.tasks[(i + 1) % NTASK]);
-            } else {
-                w0 = w1 = w2 = 0ull; // (no early request: the polls fetch the words themselves)
-            }
         }
         if (G > 0) {
             tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
@@ -1317,7 +1367,7 @@ cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, flo
     a.done = fused ? done : nullptr;
     a.done_target = fused ? (*done_seq + 1u) * (unsigned) a.cph : 0u;
     void * args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *) tc_kernel_for(job.kv.s[0].bits, job.kv.s[1].bits, false), dim3(NKV * a.cph), dim3(tc::NTHREADS), args, attend_tc_smem_bytes(), stream);
+    e = cudaLaunchCooperativeKernel((const void *) tc_kernel_for(job.kv.s[0].bits, job.kv.s[1].bits, false), dim3(NKV * a.cph), dim3(tc::NTHREADS_SPREAD), args, attend_tc_smem_bytes(), stream);
     if (e != cudaSuccess) return e;
     if (fused) {
         *done_seq += 1u;
