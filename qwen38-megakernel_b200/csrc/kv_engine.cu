@@ -549,35 +549,32 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
 }
 
 // Whether nlayers layers of one step (job j's shape, each) go out as one launch of the tensor-core kernel's batch mode, or one by one
-// in its spread mode. In tenths of a 128-position group's time on one CTA (3.6 us): the batch launch takes the CTA with the most
-// groups, 7 per item besides (queries, partial, the pipeline's refill) and 50 for itself, its append and its merge; a spread launch
-// deals a layer's groups over all CTAs but takes 42 for itself (exchange of maxima, slowest CTA, merge). Measured (us, batch against
-// spread, 8 tokens): 2 layers of 4,003 positions 30 / 42, of 11,701 56 / 58 (the rule takes spread), of 24,003 93 / 83; 4 layers of
-// 24,003 135 / 162, of 38,000 189 / 200, of 101,600 453 / 389; 8 layers of 101,600 737 / 768; 16 layers of 101,600 1,308 / 1,521. Of 48
-// shapes of 2 .. 16 layers the slower form is taken in one, by 2.7 %.
-// Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode (one layer: 22 .. 24 us against 22 .. 24): there the
-// layers' outputs are the same bits one by one and together.
+// in its spread mode. In tenths of a 128-position group's time on one CTA of the batch launch (3.0 us): it takes the CTA with the most
+// groups, 7 per item besides (queries, partial, the pipeline's refill) and 43 for itself, its append and its merge; a spread launch
+// deals a layer's groups over all CTAs, a group there takes 12 (exchange of maxima) and the launch 54 (slowest CTA, merge). Measured (us,
+// batch against spread, 8 tokens): 1 layer of 4,096 positions 22.0 / 22.7, of 6,003 24.8 / 24.7, of 9,003 28.8 / 26.9, of 24,003
+// 45.2 / 39.0, of 101,600 134 / 103; 2 layers of 13,003 55.5 / 58.5, of 38,000 112 / 99, of 101,600 258 / 201; 4 layers of 38,000
+// 156 / 193, of 101,600 368 / 396; 8 layers of 101,600 598 / 785.
+// Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode (one layer of 2,600: 20.7 us against 20.7 ..
+// 24.5): there the layers' outputs are the same bits one by one and together.
 bool KvEngine::items_mode(int nlayers, const AttnJob & j) const {
     if (j.cs <= 128) return true;
-    if (nlayers < 2) return false;
     const int sms = std::max(num_sms_, NKV), nit = (j.nch + j.cpi - 1) / j.cpi;
     std::vector<int> load(sms, 0);
     long long item = 0, groups = 0;
     for (int k = 0; k < nit; k++) {
         const int run = batch_run(j, j.cpi, nit, k);
-        int len = 7;
-        for (int c = j.c_lo + run * j.cpi; c < std::min(j.c_lo + j.nch, j.c_lo + (run + 1) * j.cpi); c++) {
-            const int n = std::min((c + 1) * j.cs, j.pos_hi) - std::max(c * j.cs, j.pos_lo), nb = (n + 4 * ATP - 1) / (4 * ATP);
-            len += 10 * nb;
-            groups += nb;
-        }
+        const int c = j.c_lo + run * j.cpi, lo = std::max(c * j.cs, j.pos_lo), hi = std::min((c + j.cpi) * j.cs, j.pos_hi);
+        const int len = 7 + 10 * ((hi - lo + 4 * ATP - 1) / (4 * ATP));
+        for (int d = c; d < std::min(j.c_lo + j.nch, c + j.cpi); d++) // (the spread mode's groups end with their chunk)
+            groups += (std::min((d + 1) * j.cs, j.pos_hi) - std::max(d * j.cs, j.pos_lo) + 4 * ATP - 1) / (4 * ATP);
         for (int h = 0; h < nlayers * NKV; h++, item++) { // (items of descending length: back and forth over the CTAs is close to what they take)
             const int r = (int) (item / sms), b = (int) (item % sms);
             load[r & 1 ? sms - 1 - b : b] += len;
         }
     }
     const long long spread = (groups + sms / NKV - 1) / (sms / NKV);
-    return *std::max_element(load.begin(), load.end()) + 50 < nlayers * (10 * spread + 42);
+    return *std::max_element(load.begin(), load.end()) + 43 < nlayers * (12 * spread + 54);
 }
 int KvEngine::job_items(const AttnJob & j) { return NKV * ((j.nch + std::max(j.cpi, 1) - 1) / std::max(j.cpi, 1)); }
 bool KvEngine::layers_one_format(const Seq & s, int layer0, int nlayers) const {
