@@ -429,7 +429,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
     if (!waiting) wait_previous();
     next_segment();
     SideSrc ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-    int cs = J->cs, n = J->n, T = J->T;
+    int chunk = J->restart, n = J->n, T = J->T;
     const uint16_t * qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
     auto tile_src = [&](const SideSrc & S, int tb, int c1) -> TileSrc {
         TileSrc t;
@@ -457,7 +457,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
             const int pos0 = pos, c1 = end, mine = pos0 + lane * ATP; // (the tiles of a run are consecutive, also across its chunks' bounds)
             nt = min(GT, (c1 - pos0 + ATP - 1) / ATP);
             const bool seg_last = c1 - pos0 <= GP;
-            const unsigned restart = __ballot_sync(FULL_MASK, lane < nt && (mine == first_pos || mine % cs == 0));
+            const unsigned restart = __ballot_sync(FULL_MASK, lane < nt && (mine == first_pos || mine % chunk == 0));
             if (seg_last) next_item = __shfl_sync(FULL_MASK, pending, 0);
             const bool cta_last = seg_last && next_item >= a.nitems;
             if (lane == 0) {
@@ -488,7 +488,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
             } else if (seg_last) {
                 next_segment();
                 ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-                cs = J->cs, n = J->n, T = J->T;
+                chunk = J->restart, n = J->n, T = J->T;
                 qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
             } else {
                 pos += GP;

@@ -82,6 +82,8 @@ struct AttnJob {
     float * O;          // fp32 [T][24][256]
     int n, T;
     int nch, cs, ws;    // partition and window start of L = n + T
+    int restart;        // batch mode: the running max starts anew at multiples of this (the partition's chunk length; cs, which cuts the items, may
+                        // differ from it in a position range's job)
     int item0;          // first (kv head, chunk) item of this job in the call's partial buffers
     int cpi, titem0;    // the tensor-core kernel's batch mode: an item is a run of cpi consecutive chunks of a kv head, so a head has
                         // ceil(nch / cpi) partials, in slots item0 + g nch + 0 ..; titem0: the job's first item

@@ -162,3 +162,40 @@ def test_layers_whose_outputs_overlap_keep_their_order(mk, torch_cuda, o_stride)
         eng.sync()
         assert torch.equal(got, want)
     eng.close()
+
+
+def test_long_ranges_are_cut_into_even_items(mk, torch_cuda):
+    """16 layers of a 45,000-position sequence on two ranges: the range's items are pieces of its chunks (the first range ends inside a chunk,
+    the second holds the window and the new rows); the oracle has the uncut chunks"""
+    torch = torch_cuda
+    spec, win, n, T, layers, cuts = "K*=5r,V*=6", 2048, 45003, 3, 16, [0, 23008, 45056]
+    used = (0, layers - 1)  # (the layers with rows of their own; the others share layer 0's)
+    orc = ko.Cache(2, n + 64, spec, win)
+    engs = [mk.Engine(layers, b - a + 64, spec, win) for a, b in zip(cuts, cuts[1:])]
+    for a, eng in zip(cuts, engs):
+        eng.set_base(a)
+    for i, l in enumerate(used):
+        Kl, Vl = kvdata.kv_rows(80 + i, 0, 0, n)
+        orc.append(i, 0, Kl, Vl)
+        for a, b, eng in zip(cuts, cuts[1:], engs):
+            b = min(b, n)
+            for m in range(layers) if i == 0 else [l]:
+                eng.append(m, a, torch.from_numpy(Kl[a:b]).cuda(), torch.from_numpy(Vl[a:b]).cuda())
+            eng.sync()
+    K, V, Q = rows(layers, 6, n, T)
+    Kd, Vd, Qd = (torch.from_numpy(x).cuda() for x in (K, V, Q))
+    parts = torch.zeros((2, layers, 4, 48, 256), dtype=torch.float32, device="cuda")
+    mls = torch.zeros((2, layers, 4, 48, 2), dtype=torch.float32, device="cuda")
+    for r, (a, b, eng) in enumerate(zip(cuts, cuts[1:], engs)):
+        before = eng.launches()
+        eng.step_layers_partial(n, Kd, Vd, Qd, a, b, a, b, parts[r], mls[r])
+        assert eng.launches() - before == 3
+        eng.sync()
+    O = torch.empty((layers, T, 24, 256), dtype=torch.float32, device="cuda")
+    engs[0].combine_layers(T, 2, parts, mls, O)
+    engs[0].sync()
+    for i, l in enumerate(used):
+        orc.append(i, n, K[l], V[l])
+        assert np.abs(O[l].cpu().numpy() - orc.attend(i, n, Q[l])).max() <= 2e-3
+    for eng in engs:
+        eng.close()
