@@ -53,8 +53,8 @@ int mk_kv_set_stream(void * h, void * cuda_stream);
 /* Waits for the engine's streams; -1 if a kernel reported a wait that ran out (the engine is reset), the reference's error-word
  * convention (mk_shared.cuh:170-203, capi.cpp:219-244) */
 int mk_kv_sync(void * h);
-/* Every device-side wait of the decode-attention kernel is bounded: a failed try of a shared-memory barrier suspends the thread for
- * up to hint_ns, after `rounds` failed tries (or `polls` failed reads of another CTA's exchange word) the CTA gives up: it sets the
+/* Every device-side wait of the decode-attention kernel is bounded: after `rounds` times hint_ns (a hint below 100 counts as 100) at a
+ * shared-memory barrier (or `polls` failed reads of another CTA's exchange words) the CTA gives up: it sets the
  * status word mk_kv_sync reports, stops waiting, lets its copies in flight land, frees its tensor memory and returns. These calls
  * set the limits for the launches that follow, process-wide (defaults: 10,000 ns, 200,000, 2,097,152: about two seconds;
  * (0, 0, 0) restores them). mk_kv_wait_limits_expire_now makes the first wait that does not succeed at once give up: the

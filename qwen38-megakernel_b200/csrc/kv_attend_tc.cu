@@ -107,7 +107,7 @@ template <int V> struct IntC { // an integer as an argument of a generic lambda
 
 struct WaitCtl { // the launch's wait limits and the CTA's give-up flag
     int dead;
-    unsigned hint, rounds, poll; // nanoseconds per failed try, failed tries of an mbarrier wait, failed polls of a global word
+    unsigned hint, rounds, poll; // an mbarrier wait lasts rounds times hint nanoseconds (a hint below 100 counts as 100), a global word is polled so often
 };
 
 // A group's task record as the producer leaves it for the other roles. The fields behind AttnTask serve the batch mode, where one CTA
@@ -172,8 +172,8 @@ struct Args {
     unsigned done_target;   // the count that means "every CTA of the head, this launch"; done == null: separate merge launch
     unsigned long long * prof; // optional: [CTA][16 groups][20] globaltimer stamps: softmax warp 0 (0 .. 7), unpack warp 8 (8 .. 15),
                                // issuer (16 .. 19)
-    unsigned wait_hint_ns, wait_rounds, poll_rounds; // limits of the waits: a failed mbarrier try suspends for up to wait_hint_ns,
-                                                     // wait_rounds failed tries (poll_rounds failed polls of an exchange word) give up
+    unsigned wait_hint_ns, wait_rounds, poll_rounds; // limits of the waits: an mbarrier wait gives up after wait_rounds times
+                                                     // wait_hint_ns, one for exchange words after poll_rounds failed polls
 };
 #ifndef MKKV_TC_PROF
 #define MKKV_TC_PROF 0 // 1: compile the phase stamps in (they cost a few per cent)
@@ -211,7 +211,7 @@ __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatil
     if (mbar_test_wait(bar, parity)) return true; // (the common case: no limit loaded)
     const unsigned rounds = wc->rounds;
     if (rounds && mbar_try_wait(bar, parity)) return true;
-    const unsigned long long limit = (unsigned long long) wc->hint * rounds, t0 = globaltimer_ns();
+    const unsigned long long limit = (unsigned long long) max(wc->hint, 100u) * rounds, t0 = globaltimer_ns();
     do {
         if (wc->dead) return false;
         if (globaltimer_ns() - t0 >= limit) {

@@ -475,8 +475,8 @@ cudaError_t launch_attend_static(const AttnJob & job, int num_sms, int * status,
     j.cpi = 1;
     j.titem0 = 0;
     if (num_sms > 0) {
-        // One CTA per (kv head, chunk) either way, but the unpack and the MMAs of this kernel take 3.6 us per 128 positions against about
-        // 6 of the mma.sync one: 20,011 positions, 2 tokens: 43.5 us against 69.8. Short chunks are not paired here (chunks_per_item): the
+        // One CTA per (kv head, chunk) either way, but the unpack and the MMAs of this kernel take 3.0 us per 128 positions against about
+        // 6 of the mma.sync one: 20,011 positions, 2 tokens: 36.9 us against 69.8. Short chunks are not paired here (chunks_per_item): the
         // call has the SMs to itself, one group per CTA instead of two takes 1,000 positions, 1 token from 20.5 us to 18.5 (mma.sync: 21.7)
         // and 2,551, 8 tokens from 21.9 to 20.5 (32.9), and a partial's sum stays as short as the mma.sync kernel's.
         j.Qp = qp;

@@ -96,7 +96,7 @@ cudaError_t preload_kernels();
 cudaError_t preload_attend_fast();
 cudaError_t preload_attend_tc();
 // Wait limits of the tensor-core kernel's launches that follow (process-wide; for diagnostics and the failure-path test): a failed
-// mbarrier try suspends for up to hint_ns, `rounds` failed tries or `polls` failed polls of an exchange word make a CTA give up.
+// mbarrier wait gives up after `rounds` times hint_ns (at least 100), one for an exchange word after `polls` failed polls.
 void attend_tc_set_wait_limits(unsigned hint_ns, unsigned rounds, unsigned polls);
 void attend_tc_default_wait_limits();
 
