@@ -53,7 +53,7 @@ NH, NKV, HD = 24, 4, 256
 # entry per attention kernel instance, since a launch of one layer and a launch of all layers of a step move different partials
 NCU_TRAFFIC = {
     "one": (164.2e6, "ncu capture of `bench.py --layers 1 --steps 2 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, false>, one launch (partials and merge in it)"),
-    "batch": (166.8e6, "ncu capture of `bench.py --layers 8 --steps 1 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, true> and attn_merge_kernel of one step, divided by 8"),
+    "batch": (166.6e6, "ncu capture of `bench.py --layers 8 --steps 1 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, true> and attn_merge_kernel of one step, divided by 8"),
 }
 WORKLOAD = "config2: 16 attention layers, 101,600 positions, preset F layout K5r/V6 + q8_0 window 2048, 8 queries/step, streaming append+spill+attend"
 REPEATS = 5  # the timed K-step loop is run this many times; the line's value is the median run
