@@ -222,6 +222,11 @@ __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatil
     } while (!mbar_try_wait(bar, parity));
     return true;
 }
+// The same for a whole warp that goes on with warp-wide instructions (tcgen05.ld and .st, votes): its lanes may leave the wait by different
+// paths and meet again here. True: every lane's wait succeeded.
+__device__ __forceinline__ bool tc_wait_warp(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
+    return __all_sync(FULL_MASK, tc_wait(bar, parity, wc, status)) != 0;
+}
 // at most about 16 ms, for the copies and instructions in flight at the kernel's end
 __device__ __forceinline__ void wait_landed(uint64_t * bar, unsigned parity) {
     const unsigned long long t0 = globaltimer_ns();
@@ -691,7 +696,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // tile maxima of group j, its own maxima published
         auto maxima = [&](int j) {
             if (st) TC_STAMP(j, 0);
-            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
+            tc_wait_warp(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
             const GroupRec & k = sm.tasks[j % NTASK];
             if (st) TC_STAMP(j, 1);
             tc_fence_after();
@@ -939,7 +944,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             constexpr int SIDE = decltype(side_c)::value, FIXED = SIDE ? VB : KB; // the side's compiled-in main format, or 0: any
             const unsigned rs = q + GT * (rseq & 1);
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 8 : 11);
-            if (!__all_sync(FULL_MASK, tc_wait(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status))) return false;
+            if (!tc_wait_warp(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status)) return false;
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 9 : 12);
             ud = sm.udesc[j % NTASK][SIDE][q];
             const bool valid = lane < (int) (ud & UD_ROWS);
@@ -1014,7 +1019,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         };
         // P of group i, whose tile maxima (tm) are known; take(t, s): the masked scores of tile t of the thread's two. restart: bit t: tile
         // t opens a chunk, the running max starts anew. Returns false when a wait of the CTA gave up (batch mode; the same answer for all
-        // four warps: the group's record and everything derived from it is only used after a true).
+        // four warps). Before that a warp uses the group's record only where its own wait for it succeeded (act), after a true all may.
         auto softmax = [&](int i, bool act, float m_in, unsigned restart, const float4 & tm, auto && take) -> bool {
             // running maxima after each tile; M: the largest of them
             const float r0 = (restart & 1u) ? tm.x : fmaxf(m_in, tm.x), r1 = (restart & 2u) ? tm.y : fmaxf(r0, tm.y);
@@ -1074,7 +1079,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 warp_arrive(&sm.s_empty[i % NSB], lane);
             }
             if (st && i < 15) TC_STAMP(i, 15);
-            if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
+            if (i > 0) tc_wait_warp(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
             if (st) TC_STAMP(i, 5);
             tc_fence_after();
 #if MKKV_TC_PROF
@@ -1132,11 +1137,14 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             // a group's scores are read once: S buffer free, maxima, P
             for (int i = 0; i < G; i++) {
                 if (st) TC_STAMP(i, 0);
-                tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
+                // After a wait that gave up the group's record may not be written: the wait's result is voted on, so that the warp-wide
+                // instructions under `act` are executed by all lanes or none, and a warp without a record has nothing to do but the barriers
+                // that carry the flag (softmax).
+                const bool there = tc_wait_warp(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
                 const GroupRec & k = sm.tasks[i % NTASK];
                 if (st) TC_STAMP(i, 1);
                 tc_fence_after();
-                const bool act = 16 * q < GQ * k.T;
+                const bool act = there && 16 * q < GQ * k.T;
                 float s[2 * ATP];
                 if (act) tmem_scores(s_addr(i), s);
                 tc_fence_before();
@@ -1167,7 +1175,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 flush_slot = k.slot, flush_rows = rows;
             }
             if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
-                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+                tc_wait_warp(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
                 tc_fence_after();
                 read_out(flush_slot, flush_rows, true);
             }
@@ -1176,7 +1184,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         const bool act = 16 * q < R;
         for (int i = 0; i < G; i++) {
             tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
-            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
+            tc_wait_warp(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
             tc_fence_after();
             const GroupRec & k = sm.tasks[i % NTASK];
             if (st) TC_STAMP(i, 3);
@@ -1194,7 +1202,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             });
         }
         if (G > 0) {
-            tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+            tc_wait_warp(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
             tc_fence_after();
         }
 #if MKKV_TC_PROF

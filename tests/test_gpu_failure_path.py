@@ -109,6 +109,55 @@ def test_expired_wait_in_every_mode(mk, torch_cuda, monkeypatch, entry, layers, 
     eng.close()
 
 
+@pytest.mark.parametrize("ns,Ts", [((3000, 2590, 1500, 300), (8, 1, 3, 6)), ((40, 70), (1, 8))])
+def test_expired_wait_of_jobs_with_different_rows(mk, torch_cuda, monkeypatch, ns, Ts):
+    """step_batch of 1 to 8 tokens a sequence: which softmax warps have rows (6, 18, 36 or 48 of them) is in a group's record, and a warp whose
+    wait gave up may look at the record of an earlier group or at one that is being written. The launch ends and the next one is right."""
+    torch = torch_cuda
+    monkeypatch.setenv("MK_KV_ATTN", "tc")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(len(ns))
+    rows = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    eng = mk.Engine(1, 64, "K*=5r,V*=6", 2048)
+    eng.slots_open(len(ns), max(ns) + 64)
+    eng.reserve_batch(len(ns))
+    K, V = rows(max(ns), 4, 256), rows(max(ns), 4, 256)
+    Kt, Vt, Q = (rows(sum(Ts), h, 256) for h in (4, 4, 24))
+
+    def call():
+        O = torch.zeros((sum(Ts), 24, 256), dtype=torch.float32, device="cuda")
+        eng.step_batch(list(range(len(ns))), 0, list(ns), list(Ts), Kt, Vt, Q, O)
+        return O
+
+    def fill():
+        for s, m in enumerate(ns):
+            eng.append(0, 0, K[:m], V[:m], seq=s)
+        eng.sync()
+
+    fill()
+    good = call()
+    eng.sync()
+    for limits in (None, (20, 2, 2), (20, 20, 20), (20, 100, 100), (100, 100, 100)):
+        try:
+            eng.wait_limits(*limits) if limits else eng.wait_limits_expire_now()
+            O = call()
+            try:
+                eng.sync()
+                gave_up = False
+            except mk.EngineError as e:
+                assert "gave up waiting" in str(e)
+                gave_up = True
+        finally:
+            eng.wait_limits()
+        assert gave_up or limits
+        if gave_up:
+            fill()
+            O = call()
+            eng.sync()
+        assert torch.equal(O, good), (limits, gave_up)
+    eng.close()
+
+
 def test_split_sequence_refuses_whole_sequence_calls(mk, torch_cuda):
     torch = torch_cuda
     eng = mk.Engine(1, 4096, "K*=5r,V*=6", 2048)
