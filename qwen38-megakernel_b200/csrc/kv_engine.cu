@@ -10,6 +10,8 @@
 #include <cstring>
 #include <unistd.h>
 
+#include "kv_plan.h"
+
 namespace mkkv {
 
 // A sticky error means the context is lost: nothing can be reset, the process ends with code 4 as the reference does
@@ -180,7 +182,7 @@ void KvEngine::ensure_xch(int nb) {
 // the decode-attention launches of one call: the tensor-core kernel, else the mma.sync one (spread over the grid, or, for shapes
 // that mode does not take, one CTA per (kv head, chunk) item)
 void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items, int max_T) {
-    if (use_tc_ && njobs == 1 && jobs_host[0].Qp && items_mode(1, jobs_host[0])) {
+    if (use_tc_ && njobs == 1 && jobs_host[0].Qp && items_mode(1, jobs_host[0], num_sms_)) {
         const cudaError_t e =
             launch_attend_tc_batch(nullptr, jobs_host[0], 1, true, true, num_sms_, job_items(jobs_host[0]), max_T, nullptr, part_, ml_, d_status_, stream_,
                                    nullptr, nullptr, stamps());
@@ -525,7 +527,7 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
             table.o_stride = o_stride;
             table.items = job_items(table.base);
             table.next = d_next_;
-            whole = items_mode(nlayers, table.base);
+            whole = items_mode(nlayers, table.base, num_sms_);
         }
         uint16_t * const qp = qprep_ + (size_t) layer0 * NKV * (QP_HEAD_BYTES / 2);
         MKKV_CK(launch_append_layers(s.d_views + layer0, nlayers, static_cast<const uint16_t *>(K), static_cast<const uint16_t *>(V), kv_stride, n, T, stream_,
@@ -548,39 +550,6 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
     }
 }
 
-// Whether nlayers layers of one step (job j's shape, each) go out as one launch of the tensor-core kernel's batch mode, or one by one
-// in its spread mode. In tenths of a 128-position group's time on one CTA of the batch launch (3.0 us): it takes the CTA with the most
-// groups, 7 per item besides (queries, partial, the pipeline's refill) and 43 for itself, its append and its merge; a spread launch
-// deals a layer's groups over all CTAs, a group there takes 12 (exchange of maxima) and the launch 54 (slowest CTA, merge). Measured (us,
-// batch against spread, 8 tokens): 1 layer of 4,096 positions 22.0 / 22.7, of 6,003 24.8 / 24.7, of 9,003 28.8 / 26.9, of 24,003
-// 45.2 / 39.0, of 101,600 134 / 103; 2 layers of 13,003 55.5 / 58.5, of 38,000 112 / 99, of 101,600 258 / 201; 4 layers of 38,000
-// 156 / 193, of 101,600 368 / 396; 8 layers of 101,600 598 / 785.
-// Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode (one layer of 2,600: 20.7 us against 20.7 ..
-// 24.5): there the layers' outputs are the same bits one by one and together.
-bool KvEngine::items_mode(int nlayers, const AttnJob & j) const {
-    if (j.restart <= 128) return true;
-    const int sms = std::max(num_sms_, NKV);
-    long long groups = 0;
-    for (int c = j.c_lo; c < j.c_lo + j.nch; c++) // (the spread mode's groups end with their chunk)
-        groups += (std::min((c + 1) * j.cs, j.pos_hi) - std::max(c * j.cs, j.pos_lo) + 4 * ATP - 1) / (4 * ATP);
-    const long long spread = (NKV * groups + sms / NKV * NKV - 1) / (sms / NKV * NKV);
-    return items_load(nlayers, j) + 43 < nlayers * (12 * spread + 54);
-}
-// the busiest CTA's groups and items in the batch launch, in tenths of a group's time
-int KvEngine::items_load(int nlayers, const AttnJob & j) const {
-    const int sms = std::max(num_sms_, NKV), nit = (j.nch + j.cpi - 1) / j.cpi;
-    std::vector<int> load(sms, 0);
-    long long item = 0;
-    for (int k = 0; k < nit; k++) {
-        const int c = j.c_lo + batch_run(j, j.cpi, nit, k) * j.cpi, lo = std::max(c * j.cs, j.pos_lo), hi = std::min((c + j.cpi) * j.cs, j.pos_hi);
-        const int len = 7 + 10 * ((hi - lo + 4 * ATP - 1) / (4 * ATP));
-        for (int h = 0; h < nlayers * NKV; h++, item++) { // (items of descending length: back and forth over the CTAs is close to what they take)
-            const int r = (int) (item / sms), b = (int) (item % sms);
-            load[r & 1 ? sms - 1 - b : b] += len;
-        }
-    }
-    return *std::max_element(load.begin(), load.end());
-}
 // A position range of nlayers layers (its job: pos_lo, pos_hi and the partition set): the items' length. A range holds few, long chunks
 // and its ends cut into two of them anyway; where cutting the chunks further (each piece with its own running max, as at the range's ends;
 // at most as many pieces as a context has chunks) evens out the CTAs' loads, it is cut at multiples of that length instead. One of 8
@@ -589,7 +558,7 @@ void KvEngine::cut_range(int nlayers, AttnJob & j) const {
     j.c_lo = j.pos_lo / j.cs;
     j.nch = (j.pos_hi + j.cs - 1) / j.cs - j.c_lo;
     if (j.restart < 2048) return; // (contexts up to 40,320 positions: chunks enough, and a cut's other rounding of P weighs more)
-    int best = items_load(nlayers, j) * 97 / 100; // (a gain of 3 % at least)
+    int best = busiest_cta(nlayers, j, std::max(num_sms_, NKV)) * 97 / 100; // (a gain of 3 % at least)
     const AttnJob whole_chunks = j;
     for (int pieces = 1; pieces <= ATT_NCH; pieces++) {
         AttnJob t = whole_chunks;
@@ -598,7 +567,7 @@ void KvEngine::cut_range(int nlayers, AttnJob & j) const {
         t.c_lo = t.pos_lo / t.cs;
         t.nch = (t.pos_hi + t.cs - 1) / t.cs - t.c_lo;
         if (t.nch > ATT_NCH) continue;
-        const int load = items_load(nlayers, t);
+        const int load = busiest_cta(nlayers, t, std::max(num_sms_, NKV));
         if (load < best) best = load, j = t;
     }
 }
@@ -880,7 +849,7 @@ void KvEngine::step_layers_partial(int seq, int nlayers, int n, int T, const voi
             table.jobs = d_jobs_;
             table.items = job_items(table.base);
             table.next = d_next_;
-            whole = items_mode(nlayers, table.base);
+            whole = items_mode(nlayers, table.base, num_sms_);
         }
         if (m > 0 || stage) {
             const size_t skip = (size_t) (m > 0 ? a - n : 0) * NKV * HD * 2;

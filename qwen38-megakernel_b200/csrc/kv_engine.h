@@ -197,8 +197,6 @@ class KvEngine {
     bool ring_overwritten(int L, int kv_top) const;
     static void plan_items(AttnJob * jobs, int njobs);
     static int job_items(const AttnJob & j);
-    bool items_mode(int nlayers, const AttnJob & j) const;
-    int items_load(int nlayers, const AttnJob & j) const;
     void cut_range(int nlayers, AttnJob & j) const;
     bool layers_one_format(const Seq & s, int layer0, int nlayers) const;
     void staged_q(AttnJob & j, int slot, bool staged); // j.Qp = the slot; staged false: filled by a launch of its own (true: the step's

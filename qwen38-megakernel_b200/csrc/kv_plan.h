@@ -1,0 +1,61 @@
+// Host rules of the tensor-core kernel: which of its two modes a call runs in. They see a context's or range's end rounded up
+// to the partition's 640 positions (plan_end), so that what they choose, like the partition itself, does not depend on the number of
+// query tokens (as long as these share one partition).
+#pragma once
+#include <algorithm>
+#include <vector>
+
+#include "kv_format.h"
+
+namespace mkkv {
+
+constexpr int GROUP = 4 * ATP; // positions of the kernel's unit of work
+
+// The job's end as the rules see it: rounded up where it lies in the last 640 positions of the context. (A range that ends before
+// them ends there for any number of tokens.)
+inline int plan_end(const AttnJob & j) {
+    const int last = (j.n + j.T + ATT_BUCKET - 1) / ATT_BUCKET;
+    return (j.pos_hi + ATT_BUCKET - 1) / ATT_BUCKET == last ? last * ATT_BUCKET : j.pos_hi;
+}
+
+// Batch mode, nlayers layers of job j (its c_lo, nch, cs, cpi and range): the groups and items of the busiest of `ctas` CTAs, in tenths of a
+// group's time: 10 a group, 7 an item besides (queries, partial, the pipeline's refill).
+inline int busiest_cta(int nlayers, const AttnJob & j, int ctas) {
+    const int nit = (j.nch + j.cpi - 1) / j.cpi;
+    std::vector<int> load(ctas, 0);
+    int at = 0, dir = 1; // (items of descending length: back and forth over the CTAs is close to what they take)
+    for (int k = 0; k < nit; k++) {
+        const int c = j.c_lo + batch_run(j, j.cpi, nit, k) * j.cpi, lo = std::max(c * j.cs, j.pos_lo), hi = std::min((c + j.cpi) * j.cs, j.pos_hi);
+        const int len = 7 + 10 * ((hi - lo + GROUP - 1) / GROUP);
+        for (int h = 0; h < nlayers * NKV; h++) {
+            load[at] += len;
+            if (at + dir < 0 || at + dir >= ctas) dir = -dir;
+            else at += dir;
+        }
+    }
+    return *std::max_element(load.begin(), load.end());
+}
+
+// Whether nlayers layers of one step (job j's shape, each) go out as one launch of the tensor-core kernel's batch mode, or one by one
+// in its spread mode. In tenths of a 128-position group's time on one CTA of the batch launch (3.0 us): it takes the busiest CTA's and 43
+// for itself, its append and its merge; a spread launch deals a layer's groups over all CTAs, a group there takes 12 (exchange of maxima)
+// and the launch 54 (slowest CTA, merge). Measured (us, batch against spread, K5r / V6, 8 tokens unless said otherwise):
+//   1 layer: 2,900 positions 22.0 / 22.6, 3,700 20.6 / 24.6, 4,096 (q8_0, 1 token) 20.5 / 20.5, 4,097 22.4 / 22.6, 4,900 20.5 / 24.6, 5,111
+//     20.6 / 24.6; from 5,121 on the rule takes the spread mode: 5,130 24.6 / 24.6, 6,390 23.3 / 24.6, 7,600 23.3 / 24.6, 9,003 28.8 / 26.9,
+//     24,003 45.2 / 39.0, 101,600 134 / 103 (two or three groups a chunk: the batch launch is never slower, by up to 1.4 us faster beyond the line)
+//   2 layers: 13,003 55.5 / 58.5, 38,000 112 / 99, 101,600 258 / 201; 4 layers: 38,000 156 / 193, 101,600 368 / 396; 8 layers: 101,600 598 / 785.
+// Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode: there the layers' outputs are the same bits one
+// by one and together. Beyond, the two modes' outputs differ by rounding (about 1e-7, relative 2-norm).
+inline bool items_mode(int nlayers, AttnJob j, int sms) {
+    if (j.cs <= GROUP) return true;
+    sms = std::max(sms, NKV);
+    j.pos_hi = plan_end(j);
+    j.nch = (j.pos_hi + j.cs - 1) / j.cs - j.c_lo;
+    long long groups = 0;
+    for (int c = j.c_lo; c < j.c_lo + j.nch; c++) // (the spread mode's groups end with their chunk)
+        groups += (std::min((c + 1) * j.cs, j.pos_hi) - std::max(c * j.cs, j.pos_lo) + GROUP - 1) / GROUP;
+    const long long spread = (NKV * groups + sms / NKV * NKV - 1) / (sms / NKV * NKV);
+    return busiest_cta(nlayers, j, sms) + 43 < nlayers * (12 * spread + 54);
+}
+
+} // namespace mkkv

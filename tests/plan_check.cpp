@@ -1,0 +1,52 @@
+// Host rules of csrc/kv_plan.h: what they choose is the same for every length of one 640-position bucket, so the number of query tokens
+// cannot change it.
+#include <cstdio>
+#include <cstring>
+
+#include "kv_plan.h"
+
+using namespace mkkv;
+
+static AttnJob job(int L, int T, int lo, int hi) {
+    AttnJob j{};
+    j.n = L - T;
+    j.T = T;
+    attn_dims(L, j.nch, j.cs);
+    j.cpi = chunks_per_item(j.cs);
+    j.pos_lo = lo;
+    j.pos_hi = std::min(L, hi);
+    j.c_lo = lo / j.cs;
+    j.nch = (j.pos_hi + j.cs - 1) / j.cs - j.c_lo;
+    return j;
+}
+
+// which mode a call takes: one answer per bucket, for whole contexts and for ranges; one layer leaves the one launch once
+static int modes() {
+    int bad = 0;
+    for (int nlayers : {1, 2, 3, 4, 8, 16}) {
+        int switches = 0, before = -1;
+        for (int bucket = 1; bucket <= 262144 / ATT_BUCKET; bucket += bucket < 40 ? 1 : 7) {
+            const int top = bucket * ATT_BUCKET, starts[3] = {0, top / 3 / ATP * ATP, (top - 1) / ATT_BUCKET * ATT_BUCKET};
+            for (int lo : starts) {
+                const int ends[3] = {1 << 30, std::max(lo + ATP, top - 5 * ATP), std::max(lo + ATP, top / 2 / ATP * ATP)};
+                for (int hi : ends) {
+                    int first = -1;
+                    for (int L = top - ATT_BUCKET + 1; L <= top; L += top - L < 10 ? 1 : 9) {
+                        if (std::min(L, hi) <= lo) continue;
+                        for (int T : {1, 8}) {
+                            if (L < T) continue;
+                            const int m = items_mode(nlayers, job(L, T, lo, hi), 148);
+                            if (first >= 0 && m != first) bad++ < 5 ? std::printf("%d layers, length %d, range %d .. %d: %d\n", nlayers, L, lo, hi, m) : 0;
+                            first = m;
+                        }
+                    }
+                    if (lo == 0 && hi == 1 << 30) switches += before >= 0 && first != before, before = first;
+                }
+            }
+        }
+        if (nlayers == 1 && switches != 1) bad++, std::printf("one layer: %d switches\n", switches);
+    }
+    return bad;
+}
+
+int main() { return modes() != 0; }

@@ -199,3 +199,23 @@ def test_long_ranges_are_cut_into_even_items(mk, torch_cuda):
         assert np.abs(O[l].cpu().numpy() - orc.attend(i, n, Q[l])).max() <= 2e-3
     for eng in engs:
         eng.close()
+
+
+@pytest.mark.parametrize("n", [3004, 3580, 4157, 4733, 5112, 5121])
+def test_tokens_of_a_call_do_not_change_its_mode(mk, torch_cuda, n):
+    """one layer just below and at the lengths where the number of a chunk's groups or of the launch's items changes: a 1-token and an 8-token
+    call take the same launches, and the first token's output is the same up to the order of fp32 sums"""
+    torch = torch_cuda
+    eng = mk.Engine(1, n + 64, "K*=5r,V*=6", 2048)
+    fill_both(torch, eng, None, 0, 0, n + 8, seed=33)
+    Q = torch.from_numpy(kvdata.q_rows(33, 0, n, 8)).cuda()
+    O = torch.zeros((2, 8, 24, 256), dtype=torch.float32, device="cuda")
+    counts = []
+    for i, T in enumerate((1, 8)):
+        before = eng.launches()
+        eng.attend(0, n, Q[:T], O[i, :T])
+        counts.append(eng.launches() - before)
+    eng.sync()
+    assert counts[0] == counts[1] == (3 if n < 5120 else 2)  # staging, attention and, behind the batch launch, the merge
+    assert float((O[0, 0] - O[1, 0]).abs().max()) <= 1e-6 * float(O[1, 0].abs().max())
+    eng.close()
