@@ -98,7 +98,9 @@ int mk_kv_combine(void * h, int layer, int T, int nparts, const void * parts, co
 /* The two calls above for every layer of one decode step, so that the ranks exchange once per step instead of once per layer:
  * mk_kv_step_layers_partial: layer l appends those of the T rows at n that fall into [own_lo, own_hi) (K, V + l kv_stride bytes, the
  * step's T rows) and attends with Q + l q_stride over [pos_lo, min(pos_hi, n + T)); its partial goes to parts + l * 4 * 48 * 256
- * floats and mls + l * 4 * 48 * 2 floats. mk_kv_combine_layers: parts [nparts][nlayers][4][48][256] and mls [nparts][nlayers][4][48][2]
+ * floats and mls + l * 4 * 48 * 2 floats. In contexts of more than 40,320 positions a range's chunks may be cut into shorter, even pieces,
+ * each with a running max of its own; where is a function of the context's 640-bucket, the range and the engine's layers, not of T
+ * or nlayers. mk_kv_combine_layers: parts [nparts][nlayers][4][48][256] and mls [nparts][nlayers][4][48][2]
  * (the ranks' arrays gathered in rank order) -> O + l o_stride bytes, every layer in one launch. */
 int mk_kv_step_layers_partial(void * h, int seq, int nlayers, int n, int T, const void * K, const void * V, const void * Q, size_t kv_stride,
                               size_t q_stride, int own_lo, int own_hi, int pos_lo, int pos_hi, void * parts, void * mls);

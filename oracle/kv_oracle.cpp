@@ -452,7 +452,7 @@ int orc_append(void * h, int layer, int pos0, int n, const uint16_t * K, const u
 // rotated). split > 1 cuts every chunk of the reference partition into that many pieces (partition-sensitivity probe).
 // Prologue qwen38_mk.cu:2876-2883, partition :2548-2573, merge :4658-4685.
 static int attend_impl(void * h, int layer, int n, int T, const uint16_t * Q, float * O, int nthreads, int split, float * out_m,
-                       float * out_l, float * out_O, int ncuts = 0, const int * cuts = nullptr) {
+                       float * out_l, float * out_O, int ncuts = 0, const int * cuts = nullptr, bool pieces = false) {
     Cache & c = *static_cast<Cache *>(h);
     if (layer < 0 || layer >= c.layers || T < 1 || T > 8 || n < 0 || n + T > c.ctxp) { g_err = "orc_attend: out of range"; return -1; }
     const int L = n + T, R = GQ * T, ws = kv_ws(L, c.win);
@@ -460,7 +460,16 @@ static int attend_impl(void * h, int layer, int n, int T, const uint16_t * Q, fl
     attn_dims(L, nch, cs);
     // chunk list per kv head
     std::vector<std::pair<int, int>> ch;
-    for (int k = 0; k < nch; k++) {
+    if (pieces) { // the cuts are the whole partition, the reference's chunk bounds are none
+        int a = 0;
+        for (int i = 0; i < ncuts; i++)
+            if (cuts[i] > a && cuts[i] < L) {
+                ch.push_back({a, cuts[i]});
+                a = cuts[i];
+            }
+        ch.push_back({a, L});
+    }
+    for (int k = 0; k < nch && !pieces; k++) {
         const int c0 = k * cs, c1 = std::min(L, c0 + cs);
         if (ncuts > 0) { // the chunk cut again at the given positions (multiples of 32): a sequence split by position over GPUs
             int a = c0;
@@ -543,6 +552,11 @@ int orc_attend_parts(void * h, int layer, int n, int T, const uint16_t * Q, floa
 // position over several GPUs computes (every piece starts its running max afresh; the merge is the reference's).
 int orc_attend_cuts(void * h, int layer, int n, int T, const uint16_t * Q, float * O, int nthreads, int ncuts, const int * cuts) {
     return attend_impl(h, layer, n, T, Q, O, nthreads, 1, nullptr, nullptr, nullptr, ncuts, cuts) < 0 ? -1 : 0;
+}
+// The same attention over pieces that end at `bounds` (ascending positions, multiples of 32) and nowhere else: the evenly cut ranges of a
+// split sequence's step.
+int orc_attend_pieces(void * h, int layer, int n, int T, const uint16_t * Q, float * O, int nthreads, int nbounds, const int * bounds) {
+    return attend_impl(h, layer, n, T, Q, O, nthreads, 1, nullptr, nullptr, nullptr, nbounds, bounds, true) < 0 ? -1 : 0;
 }
 // The merge alone (qwen38_mk.cu:4658-4685) over given partials of nc chunks per kv head in the layout above: O fp32 [T][24][256]
 void orc_merge_parts(int T, int nc, int rot_v, const float * pm, const float * pl, const float * pO, float * O) {

@@ -43,6 +43,7 @@ def lib():
         L.orc_append.argtypes = [vp, ip, ip, ip, vp, vp]
         L.orc_attend.argtypes = [vp, ip, ip, ip, vp, vp, ip, ip]
         L.orc_attend_cuts.argtypes = [vp, ip, ip, ip, vp, vp, ip, ip, vp]
+        L.orc_attend_pieces.argtypes = [vp, ip, ip, ip, vp, vp, ip, ip, vp]
         L.orc_attend_parts.argtypes = [vp, ip, ip, ip, vp, vp, ip, vp, vp, vp]
         L.orc_merge_parts.restype = None
         L.orc_merge_parts.argtypes = [ip, ip, ip, vp, vp, vp, vp]
@@ -197,6 +198,16 @@ class Cache:
         O = np.zeros((T, NH, HD), dtype=np.float32)
         c = np.ascontiguousarray(sorted(int(x) for x in cuts), dtype=np.int32)
         if lib().orc_attend_cuts(self.h, layer, n, T, _p(Q), _p(O), threads, len(c), _p(c)) != 0:
+            raise ValueError(err())
+        return O
+
+    def attend_pieces(self, layer, n, Q, bounds, threads=8):
+        """attend() over the pieces between the positions `bounds`, whatever chunks they lie in (a split sequence's evenly cut ranges)"""
+        Q = np.ascontiguousarray(Q, dtype=np.float16)
+        T = Q.shape[0]
+        O = np.zeros((T, NH, HD), dtype=np.float32)
+        b = np.ascontiguousarray(sorted(int(x) for x in bounds), dtype=np.int32)
+        if lib().orc_attend_pieces(self.h, layer, n, T, _p(Q), _p(O), threads, len(b), _p(b)) != 0:
             raise ValueError(err())
         return O
 

@@ -642,11 +642,11 @@ int build_range_tasks(const AttnJob & J, int B, std::vector<AttnTask> & out) {
     struct Ch { int c, c0, c1, ntc, nb; };
     std::vector<Ch> chs;
     int max_nb = 0;
-    for (int c = 0; c < J.nch; c++) {
+    for (int c = J.c_lo; c < J.c_lo + J.nch; c++) {
         const int c0 = std::max(c * J.cs, J.pos_lo), c1 = std::min(std::min(L, (c + 1) * J.cs), J.pos_hi);
         if (c1 <= c0) continue;
         const int ntc = (c1 - c0 + ATP - 1) / ATP, nb = (ntc + B - 1) / B;
-        chs.push_back({c, c0, c1, ntc, nb});
+        chs.push_back({c - J.c_lo, c0, c1, ntc, nb}); // (the exchange arrays have room for ATT_NCH)
         max_nb = std::max(max_nb, nb);
     }
     for (int b = 0; b < max_nb; b++)

@@ -434,7 +434,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
     if (!waiting) wait_previous();
     next_segment();
     SideSrc ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-    int chunk = J->restart, n = J->n, T = J->T;
+    int chunk = J->cs, n = J->n, T = J->T;
     const uint16_t * qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
     auto tile_src = [&](const SideSrc & S, int tb, int c1) -> TileSrc {
         TileSrc t;
@@ -493,7 +493,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
             } else if (seg_last) {
                 next_segment();
                 ks = make_src(J->kv, 0, g, J->ws), vs = make_src(J->kv, 1, g, J->ws);
-                chunk = J->restart, n = J->n, T = J->T;
+                chunk = J->cs, n = J->n, T = J->T;
                 qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
             } else {
                 pos += GP;

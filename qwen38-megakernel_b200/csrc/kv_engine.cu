@@ -550,26 +550,11 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
     }
 }
 
-// A position range of nlayers layers (its job: pos_lo, pos_hi and the partition set): the items' length. A range holds few, long chunks
-// and its ends cut into two of them anyway; where cutting the chunks further (each piece with its own running max, as at the range's ends;
-// at most as many pieces as a context has chunks) evens out the CTAs' loads, it is cut at multiples of that length instead. One of 8
-// GPUs' part of 262,136 positions, 16 layers: 192 items of 102 or 52 groups on 148 CTAs, the busiest with 154 of a mean of 111.
-void KvEngine::cut_range(int nlayers, AttnJob & j) const {
+// the pieces of a split sequence's range (j: its bounds set, the partition the context's)
+void KvEngine::cut_range(AttnJob & j) const {
+    j.cs = range_piece(cfg_.layers, j);
     j.c_lo = j.pos_lo / j.cs;
     j.nch = (j.pos_hi + j.cs - 1) / j.cs - j.c_lo;
-    if (j.restart < 2048) return; // (contexts up to 40,320 positions: chunks enough, and a cut's other rounding of P weighs more)
-    int best = busiest_cta(nlayers, j, std::max(num_sms_, NKV)) * 97 / 100; // (a gain of 3 % at least)
-    const AttnJob whole_chunks = j;
-    for (int pieces = 1; pieces <= ATT_NCH; pieces++) {
-        AttnJob t = whole_chunks;
-        t.cs = ((j.pos_hi - j.pos_lo + pieces - 1) / pieces + 4 * ATP - 1) / (4 * ATP) * (4 * ATP);
-        if (t.cs >= t.restart) continue;
-        t.c_lo = t.pos_lo / t.cs;
-        t.nch = (t.pos_hi + t.cs - 1) / t.cs - t.c_lo;
-        if (t.nch > ATT_NCH) continue;
-        const int load = busiest_cta(nlayers, t, std::max(num_sms_, NKV));
-        if (load < best) best = load, j = t;
-    }
 }
 int KvEngine::job_items(const AttnJob & j) { return NKV * ((j.nch + std::max(j.cpi, 1) - 1) / std::max(j.cpi, 1)); }
 bool KvEngine::layers_one_format(const Seq & s, int layer0, int nlayers) const {
@@ -666,7 +651,6 @@ AttnJob KvEngine::job_of(const Seq & s, int layer, int n, int T, const void * Q,
     j.n = n;
     j.T = T;
     attn_dims(n + T, j.nch, j.cs);
-    j.restart = j.cs;
     j.ws = kv_ws(n + T, cfg_.win);
     j.item0 = 0;
     j.cpi = chunks_per_item(j.cs);
@@ -705,10 +689,10 @@ void KvEngine::set_base(int seq, int base) {
 }
 
 void KvEngine::attend_partial(int seq, int layer, int n, int T, const void * Q, int pos_lo, int pos_hi, void * part_out, void * ml_out) {
-    attend_partial_impl(seq, layer, n, T, Q, pos_lo, pos_hi, part_out, ml_out, false);
+    attend_partial_impl(seq, layer, n, T, Q, pos_lo, pos_hi, part_out, ml_out, false, false);
 }
 void KvEngine::attend_partial_impl(int seq, int layer, int n, int T, const void * Q, int pos_lo, int pos_hi, void * part_out, void * ml_out,
-                                   bool q_staged) {
+                                   bool q_staged, bool pieces) {
     use_device();
     check_layer(layer);
     Seq & s = seq_ref(seq);
@@ -729,7 +713,6 @@ void KvEngine::attend_partial_impl(int seq, int layer, int n, int T, const void 
     j.n = n;
     j.T = T;
     attn_dims(L, j.nch, j.cs);
-    j.restart = j.cs;
     j.ws = kv_ws(L, cfg_.win);
     j.item0 = 0;
     j.cpi = 1;
@@ -741,16 +724,18 @@ void KvEngine::attend_partial_impl(int seq, int layer, int n, int T, const void 
     j.rstride = 0;
     if (pos_hi > pos_lo) spill_to(s, layer, std::min(j.ws, pos_hi)); // rows of this range that left the window
     if (use_tc_) staged_q(j, layer, q_staged);
+    AttnJob cut = j; // the partition of the task list; the launch's own job keeps the context's
+    if (pieces && pos_hi > pos_lo) cut_range(cut);
     std::vector<AttnTask> tasks;
     bool tc = use_tc_;
     for (;; tc = false) { // the tensor-core kernel first (4 tiles per task), else the fast kernel (8)
         // the task list depends on the partition and the range only: a rank whose range does not end at the context's end keeps
         // the list of the previous step (no rebuild, no upload)
         const int B = tc ? 4 : 8;
-        const long long key[5] = {j.nch, j.cs, pos_lo, pos_hi, B};
+        const long long key[5] = {cut.nch, cut.cs, pos_lo, pos_hi, B};
         int nt = tasks_n_;
         if (memcmp(key, tasks_key_, sizeof(key)) != 0 || tasks_n_ < 0) {
-            const int max_nb = build_range_tasks(j, B, tasks);
+            const int max_nb = build_range_tasks(cut, B, tasks);
             if (tc) ensure_xch(max_nb);
             else if (max_nb > std::min(xnb_, 64)) throw std::runtime_error("attend_partial: the context is too long for the exchange buffers");
             nt = (int) tasks.size();
@@ -799,7 +784,7 @@ void KvEngine::combine(int layer, int T, int nparts, const void * parts, const v
     j.n = 0;
     j.T = T;
     j.nch = nparts;
-    j.cs = j.restart = 0;
+    j.cs = 0;
     j.ws = 0;
     j.item0 = 0;
     j.cpi = 1;
@@ -845,7 +830,7 @@ void KvEngine::step_layers_partial(int seq, int nlayers, int n, int T, const voi
             table.base = job_of(s, 0, n, T, Q, nullptr);
             table.base.pos_lo = pos_lo;
             table.base.pos_hi = hi;
-            cut_range(nlayers, table.base);
+            cut_range(table.base);
             table.jobs = d_jobs_;
             table.items = job_items(table.base);
             table.next = d_next_;
@@ -872,7 +857,7 @@ void KvEngine::step_layers_partial(int seq, int nlayers, int n, int T, const voi
     }
     for (int l = 0; l < nlayers; l++) {
         attend_partial_impl(seq, l, n, T, static_cast<const char *>(Q) + l * q_stride, pos_lo, hi > pos_lo ? hi : pos_lo,
-                            static_cast<float *>(parts) + (size_t) l * NKV * AR * HD, static_cast<float *>(mls) + (size_t) l * NKV * AR * 2, staged);
+                            static_cast<float *>(parts) + (size_t) l * NKV * AR * HD, static_cast<float *>(mls) + (size_t) l * NKV * AR * 2, staged, true);
     }
 }
 
@@ -895,7 +880,7 @@ void KvEngine::combine_layers(int nlayers, int T, int nparts, const void * parts
         j.n = 0;
         j.T = T;
         j.nch = nparts;
-        j.cs = j.restart = 0;
+        j.cs = 0;
         j.ws = 0;
         j.item0 = l * NKV;          // partial p of kv head g of layer l is slot (p * nlayers + l) * 4 + g
         j.cpi = 1;

@@ -197,12 +197,12 @@ class KvEngine {
     bool ring_overwritten(int L, int kv_top) const;
     static void plan_items(AttnJob * jobs, int njobs);
     static int job_items(const AttnJob & j);
-    void cut_range(int nlayers, AttnJob & j) const;
+    void cut_range(AttnJob & j) const;
     bool layers_one_format(const Seq & s, int layer0, int nlayers) const;
     void staged_q(AttnJob & j, int slot, bool staged); // j.Qp = the slot; staged false: filled by a launch of its own (true: the step's
                                                        // append launch has just done it)
     void attend_impl(int seq, int layer, int n, int T, const void * Q, void * O, bool q_staged);
-    void attend_partial_impl(int seq, int layer, int n, int T, const void * Q, int pos_lo, int pos_hi, void * part_out, void * ml_out, bool q_staged);
+    void attend_partial_impl(int seq, int layer, int n, int T, const void * Q, int pos_lo, int pos_hi, void * part_out, void * ml_out, bool q_staged, bool pieces);
     std::vector<std::pair<char *, size_t>> state_regions(Seq & s, int hend) const;
     void spill_to(Seq & s, int layer, int upto);
     void ring_rewind(Seq & s, int P);

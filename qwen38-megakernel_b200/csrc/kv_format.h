@@ -42,7 +42,7 @@ MKKV_HD void attn_dims(int L, int & nch, int & cs) {
     const int n = (L + cs - 1) / cs;
     nch = n > 1 ? n : 1;
 }
-// Chunks per item of the tensor-core kernel's batch mode: the partials, and so the order of the sums, depend on the context's length
+// Chunks per item of the tensor-core kernel's batch mode: a whole context's partials, and so the order of the sums, depend on its length
 // only. A chunk of one 128-position group (contexts up to 2,560 positions) shares an item with its neighbour: an item costs about 0.7 of
 // a group's time besides its groups.
 MKKV_HD int chunks_per_item(int cs) { return cs <= 128 ? 2 : 1; }
@@ -81,9 +81,7 @@ struct AttnJob {
                          // (head % 6) T + t, rotated when K is, x 1/16, fp16, in the operand layout; null: not staged
     float * O;          // fp32 [T][24][256]
     int n, T;
-    int nch, cs, ws;    // partition and window start of L = n + T
-    int restart;        // batch mode: the running max starts anew at multiples of this (the partition's chunk length; cs, which cuts the items, may
-                        // differ from it in a position range's job)
+    int nch, cs, ws;    // partition (chunks of cs positions; of a split sequence's range: its pieces, range_piece) and window start of L = n + T
     int item0;          // first (kv head, chunk) item of this job in the call's partial buffers
     int cpi, titem0;    // the tensor-core kernel's batch mode: an item is a run of cpi consecutive chunks of a kv head, so a head has
                         // ceil(nch / cpi) partials, in slots item0 + g nch + 0 ..; titem0: the job's first item

@@ -1,4 +1,4 @@
-// Host rules of the tensor-core kernel: which of its two modes a call runs in. They see a context's or range's end rounded up
+// Host rules of the tensor-core kernel: which of its two modes a call runs in, and how a split sequence's range is cut. They see a context's or range's end rounded up
 // to the partition's 640 positions (plan_end), so that what they choose, like the partition itself, does not depend on the number of
 // query tokens (as long as these share one partition).
 #pragma once
@@ -10,6 +10,7 @@
 namespace mkkv {
 
 constexpr int GROUP = 4 * ATP; // positions of the kernel's unit of work
+constexpr int B200_SMS = 148;
 
 // The job's end as the rules see it: rounded up where it lies in the last 640 positions of the context. (A range that ends before
 // them ends there for any number of tokens.)
@@ -56,6 +57,39 @@ inline bool items_mode(int nlayers, AttnJob j, int sms) {
         groups += (std::min((c + 1) * j.cs, j.pos_hi) - std::max(c * j.cs, j.pos_lo) + GROUP - 1) / GROUP;
     const long long spread = (NKV * groups + sms / NKV * NKV - 1) / (sms / NKV * NKV);
     return busiest_cta(nlayers, j, sms) + 43 < nlayers * (12 * spread + 54);
+}
+
+// The pieces of a position range in a split sequence's step (job j: the range's bounds and the context's partition): cut at multiples of
+// the length returned, each with a running max of its own, in either mode. j.cs: the range keeps its chunks.
+// A range holds few, long chunks and its ends cut into two of them anyway, so the busiest CTA of the batch launch had much more than the
+// mean: one of 8 GPUs' part of 262,136 positions, 16 layers: 192 items of 102 or 52 groups on 148 CTAs, the busiest with 154 of a mean of 111;
+// 490 us uncut, 419 with pieces of 2,816 positions; 1 layer 47.9 uncut, 43.2 so, 2 and 4 of the 16 82 and 155 (69 and 136 with pieces of
+// their own, which is what a result that depends on the call would buy). What is computed must not depend on how it is run: the length is a function of the
+// partition, the range (its end as plan_end has it) and the engine's layers, taken for a B200 whole, not of the layers or tokens of a call or
+// the SMs at hand. At most as many pieces as a context has chunks (the partials' scratch), and only for a gain of 3 % in the busiest CTA's load.
+// Contexts up to 40,320 positions keep their chunks. Against 64 bits pieces are no worse than chunks on either side of that line (the oracle,
+// one range in two, relative 2-norm, chunks / pieces: 20,003 positions 1.9e-5 / 1.3e-5, 38,003 2.0e-5 / 2.0e-5, 40,003 3.8e-5 / 3.0e-5, 45,003 2.6e-5 /
+// 2.1e-5, 60,003 3.2e-5 / 1.4e-5, 101,608 1.9e-5 / 2.2e-5), but the shorter a context, the further from the reference's partition they are: largest difference
+// 1e-3 at 8,003 positions, 3e-4 .. 5e-4 from 20,003 on (2e-3, the bar, at 60,003, where the chunks are 1.9e-3 off 64 bits and the pieces 5e-4).
+inline int range_piece(int layers, const AttnJob & j) {
+    if (j.cs < 2048) return j.cs;
+    AttnJob t = j;
+    t.pos_hi = plan_end(j);
+    t.cpi = 1;
+    auto load_of = [&](int len) {
+        t.cs = len;
+        t.c_lo = t.pos_lo / len;
+        t.nch = (t.pos_hi + len - 1) / len - t.c_lo;
+        return t.nch > ATT_NCH ? 0x7fffffff : busiest_cta(layers, t, B200_SMS);
+    };
+    int best = (int) (load_of(j.cs) * 97ll / 100), piece = j.cs;
+    for (int pieces = 1; pieces <= ATT_NCH; pieces++) {
+        const int len = ((t.pos_hi - t.pos_lo + pieces - 1) / pieces + GROUP - 1) / GROUP * GROUP;
+        if (len >= j.cs) continue;
+        const int load = load_of(len);
+        if (load < best) best = load, piece = len;
+    }
+    return piece;
 }
 
 } // namespace mkkv

@@ -1,7 +1,7 @@
 // Host rules of csrc/kv_plan.h: what they choose is the same for every length of one 640-position bucket, so the number of query tokens
-// cannot change it.
+// cannot change it. With arguments n, T, pos_lo, pos_hi, layers: prints the length of a range's pieces.
 #include <cstdio>
-#include <cstring>
+#include <cstdlib>
 
 #include "kv_plan.h"
 
@@ -49,4 +49,36 @@ static int modes() {
     return bad;
 }
 
-int main() { return modes() != 0; }
+// a range's pieces: one length per bucket, whole groups, no longer than a chunk, no more of them than the partials' scratch holds
+static int pieces() {
+    int bad = 0, cut = 0;
+    for (int layers : {1, 8, 16})
+        for (int bucket = 1; bucket <= 262144 / ATT_BUCKET; bucket += bucket < 70 ? 3 : 13)
+            for (int world : {1, 2, 3, 8})
+                for (int rank = 0; rank < world; rank++) {
+                    const int top = bucket * ATT_BUCKET, share = (top + 64 + world - 1) / world / ATP * ATP + ATP, lo = rank * share, hi = lo + share;
+                    int first = -1;
+                    for (int L = top - ATT_BUCKET + 1; L <= top; L += top - L < 10 ? 1 : 61)
+                        for (int T : {1, 8}) {
+                            if (L < T || std::min(L, hi) <= lo) continue;
+                            AttnJob j = job(L, T, lo, hi);
+                            const int p = range_piece(layers, j);
+                            const int n = (j.pos_hi + p - 1) / p - lo / p;
+                            const bool ok = (first < 0 || p == first) && p <= j.cs && (p == j.cs || p % GROUP == 0) && n <= ATT_NCH && (bucket > 63 || p == j.cs);
+                            if (!ok) bad++ < 5 ? std::printf("%d layers, length %d, range %d .. %d: pieces of %d, chunks of %d\n", layers, L, lo, hi, p, j.cs) : 0;
+                            first = p;
+                            cut += p != j.cs;
+                        }
+                }
+    if (!cut) bad++, std::printf("no range was cut\n");
+    return bad;
+}
+
+int main(int argc, char ** argv) {
+    if (argc == 6) {
+        const int n = atoi(argv[1]), T = atoi(argv[2]);
+        std::printf("%d\n", range_piece(atoi(argv[5]), job(n + T, T, atoi(argv[3]), atoi(argv[4]))));
+        return 0;
+    }
+    return modes() + pieces() != 0;
+}

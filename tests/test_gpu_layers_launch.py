@@ -1,11 +1,14 @@
 """A decode step's layers in one attention launch (the tensor-core kernel's batch mode) against the oracle, at the partition's edges:
 one chunk, short last chunks, chunks of 1, 2 and 3 groups of 128 positions, the first length past each, mixed formats per layer; and
 the same for a position range whose cuts fall inside chunks. Tolerance: the path's 2e-3 (gpu_util.check_flips)."""
+import subprocess
+
 import numpy as np
 import pytest
 
 import kv_oracle as ko
 import kvdata
+import test_plan_cpu
 from gpu_util import check_flips, fill_both
 
 pytestmark = pytest.mark.gpu
@@ -164,10 +167,13 @@ def test_layers_whose_outputs_overlap_keep_their_order(mk, torch_cuda, o_stride)
     eng.close()
 
 
-def test_long_ranges_are_cut_into_even_items(mk, torch_cuda):
-    """16 layers of a 45,000-position sequence on two ranges: the range's items are pieces of its chunks (the first range ends inside a chunk,
-    the second holds the window and the new rows); the oracle has the uncut chunks"""
+def test_long_ranges_are_cut_into_even_items(mk, torch_cuda, tmp_path):
+    """16 layers of a 45,000-position sequence on two ranges, cut into even pieces (the first range ends inside a chunk, the second holds the
+    window and the new rows). Against the oracle with the chunks, whose P is rounded against other maxima, the path's 2e-3; the oracle with
+    the same pieces must be at least four times nearer (there P differs only where the last bits of a score turn its rounding, a
+    few values in a thousand against all)."""
     torch = torch_cuda
+    plan = test_plan_cpu.build(tmp_path)
     spec, win, n, T, layers, cuts = "K*=5r,V*=6", 2048, 45003, 3, 16, [0, 23008, 45056]
     used = (0, layers - 1)  # (the layers with rows of their own; the others share layer 0's)
     orc = ko.Cache(2, n + 64, spec, win)
@@ -194,11 +200,58 @@ def test_long_ranges_are_cut_into_even_items(mk, torch_cuda):
     O = torch.empty((layers, T, 24, 256), dtype=torch.float32, device="cuda")
     engs[0].combine_layers(T, 2, parts, mls, O)
     engs[0].sync()
+    bounds = []
+    for a, b in zip(cuts, cuts[1:]):
+        p = int(subprocess.run([plan] + [str(x) for x in (n, T, a, b, layers)], capture_output=True, text=True, check=True).stdout)
+        assert p < ko.attn_dims(n + T)[1]
+        bounds += [a] + list(range((a // p + 1) * p, min(b, n + T), p))
     for i, l in enumerate(used):
         orc.append(i, n, K[l], V[l])
-        assert np.abs(O[l].cpu().numpy() - orc.attend(i, n, Q[l])).max() <= 2e-3
+        got, chunks, pieces = O[l].cpu().numpy(), orc.attend(i, n, Q[l]), orc.attend_pieces(i, n, Q[l], bounds[1:])
+        assert np.abs(got - chunks).max() <= 2e-3
+        assert np.linalg.norm(got - pieces) <= np.linalg.norm(got - chunks) / 4
     for eng in engs:
         eng.close()
+
+
+@pytest.mark.parametrize("n,lo,hi", [(230009, 196608, 262144), (262136, 98304, 131072)])
+def test_pieces_of_a_range_are_those_of_every_call(mk, torch_cuda, n, lo, hi):
+    """A range's partial must not depend on how many layers or tokens share the call: 16 layers in the one launch, 2 layers and 1 layer in the
+    spread mode, 8 tokens and 1, over the same rows, 1e-5 (a P rounded against another maximum moves the output by 2e-5 .. 4e-5); and
+    the layers of a call, given the same rows, the same bits. The context's end, with the new rows, and an inner range."""
+    torch = torch_cuda
+    layers, T, end = 16, 8, min(hi, n)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    scale = torch.rand((4, 256), generator=g, device="cuda") * 1.5 + 0.5
+    rows = lambda m, h=4: torch.randn((m, h, 256), generator=g, device="cuda")
+    eng = mk.Engine(layers, hi - lo + 64, "K*=5r,V*=6", 2048)
+    eng.set_base(lo)
+    for a in range(lo, end, 16384):
+        m = min(16384, end - a)
+        K, V = ((rows(m) * scale).half() for _ in range(2))
+        for l in range(layers):
+            eng.append(l, a, K, V)
+    K, V = ((rows(T) * scale).half().expand(layers, T, 4, 256).contiguous() for _ in range(2))
+    Q = rows(T, 24).half().expand(layers, T, 24, 256).contiguous()
+
+    def call(nlayers, tokens):
+        part = torch.zeros((nlayers, 4, 48, 256), dtype=torch.float32, device="cuda")
+        ml = torch.zeros((nlayers, 4, 48, 2), dtype=torch.float32, device="cuda")
+        O = torch.zeros((nlayers, tokens, 24, 256), dtype=torch.float32, device="cuda")
+        eng.step_layers_partial(n, *(x[:nlayers, :tokens].contiguous() for x in (K, V, Q)), lo, hi, lo, hi, part, ml)
+        eng.combine_layers(tokens, 1, part, ml, O)
+        eng.sync()
+        return O
+
+    want = call(layers, T)
+    for l in range(1, layers):
+        assert torch.equal(want[l], want[0]), l
+    for nlayers, tokens in ((2, T), (1, T), (layers, 1), (2, 1), (1, 1)):
+        got = call(nlayers, tokens)
+        rel = float((got[0] - want[0, :tokens]).norm() / want[0, :tokens].norm())
+        assert rel <= 1e-5, (nlayers, tokens, rel)
+    eng.close()
 
 
 @pytest.mark.parametrize("n", [3004, 3580, 4157, 4733, 5112, 5121])

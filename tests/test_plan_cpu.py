@@ -1,4 +1,4 @@
-"""CPU check of the rules that choose a call's kernel mode (csrc/kv_plan.h, host code)."""
+"""CPU check of the rules that choose a call's kernel mode and a range's pieces (csrc/kv_plan.h, host code)."""
 import os
 import subprocess
 
@@ -12,6 +12,6 @@ def build(tmp_path):
     return exe
 
 
-def test_mode_depends_on_the_bucket_only(tmp_path):
+def test_mode_and_pieces_depend_on_the_bucket_only(tmp_path):
     r = subprocess.run([build(tmp_path)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
