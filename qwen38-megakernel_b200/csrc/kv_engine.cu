@@ -10,8 +10,6 @@
 #include <cstring>
 #include <unistd.h>
 
-#include "kv_plan.h"
-
 namespace mkkv {
 
 // A sticky error means the context is lost: nothing can be reset, the process ends with code 4 as the reference does
@@ -182,7 +180,7 @@ void KvEngine::ensure_xch(int nb) {
 // the decode-attention launches of one call: the tensor-core kernel, else the mma.sync one (spread over the grid, or, for shapes
 // that mode does not take, one CTA per (kv head, chunk) item)
 void KvEngine::launch_attention(const AttnJob * jobs_host, int njobs, int items, int max_T) {
-    if (use_tc_ && njobs == 1 && jobs_host[0].Qp && items_mode(1, jobs_host[0], num_sms_)) {
+    if (use_tc_ && njobs == 1 && jobs_host[0].Qp && items_launch(1, jobs_host[0])) {
         const cudaError_t e =
             launch_attend_tc_batch(nullptr, jobs_host[0], 1, true, true, num_sms_, job_items(jobs_host[0]), max_T, nullptr, part_, ml_, d_status_, stream_,
                                    nullptr, nullptr, stamps());
@@ -527,7 +525,7 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
             table.o_stride = o_stride;
             table.items = job_items(table.base);
             table.next = d_next_;
-            whole = items_mode(nlayers, table.base, num_sms_);
+            whole = items_launch(nlayers, table.base);
         }
         uint16_t * const qp = qprep_ + (size_t) layer0 * NKV * (QP_HEAD_BYTES / 2);
         MKKV_CK(launch_append_layers(s.d_views + layer0, nlayers, static_cast<const uint16_t *>(K), static_cast<const uint16_t *>(V), kv_stride, n, T, stream_,
@@ -550,9 +548,14 @@ void KvEngine::step_layers(int seq, int nlayers, int n, int T, const void * K, c
     }
 }
 
+// the rules of kv_plan.h; the jobs' other fields follow from the keys (a job of more than one group a chunk has one chunk an item)
+bool KvEngine::items_launch(int nlayers, const AttnJob & j) {
+    if (j.cs <= GROUP) return true;
+    return mode_plan_.get({nlayers, j.cs, j.pos_lo, plan_end(j)}, [&] { return items_mode(nlayers, j, num_sms_); }) != 0;
+}
 // the pieces of a split sequence's range (j: its bounds set, the partition the context's)
-void KvEngine::cut_range(AttnJob & j) const {
-    j.cs = range_piece(cfg_.layers, j);
+void KvEngine::cut_range(AttnJob & j) {
+    j.cs = piece_plan_.get({cfg_.layers, j.cs, j.pos_lo, plan_end(j)}, [&] { return range_piece(cfg_.layers, j); });
     j.c_lo = j.pos_lo / j.cs;
     j.nch = (j.pos_hi + j.cs - 1) / j.cs - j.c_lo;
 }
@@ -834,7 +837,7 @@ void KvEngine::step_layers_partial(int seq, int nlayers, int n, int T, const voi
             table.jobs = d_jobs_;
             table.items = job_items(table.base);
             table.next = d_next_;
-            whole = items_mode(nlayers, table.base, num_sms_);
+            whole = items_launch(nlayers, table.base);
         }
         if (m > 0 || stage) {
             const size_t skip = (size_t) (m > 0 ? a - n : 0) * NKV * HD * 2;

@@ -12,6 +12,7 @@
 
 #include "kv_format.h"
 #include "kv_kernels.h"
+#include "kv_plan.h"
 
 namespace mkkv {
 
@@ -197,7 +198,8 @@ class KvEngine {
     bool ring_overwritten(int L, int kv_top) const;
     static void plan_items(AttnJob * jobs, int njobs);
     static int job_items(const AttnJob & j);
-    void cut_range(AttnJob & j) const;
+    bool items_launch(int nlayers, const AttnJob & j);
+    void cut_range(AttnJob & j);
     bool layers_one_format(const Seq & s, int layer0, int nlayers) const;
     void staged_q(AttnJob & j, int slot, bool staged); // j.Qp = the slot; staged false: filled by a launch of its own (true: the step's
                                                        // append launch has just done it)
@@ -247,6 +249,7 @@ class KvEngine {
     int tasks_cap_ = 0;
     long long tasks_key_[5] = {-1, -1, -1, -1, -1}; // (partition, range, tiles per task) of the list d_tasks_ holds
     int tasks_n_ = -1;
+    PlanMemo mode_plan_, piece_plan_;
     int * h_status_ = nullptr; // mapped pinned word the kernels write
     int * d_status_ = nullptr;
     // fast attention path: exchange of row maxima between the CTAs of one chunk

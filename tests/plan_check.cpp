@@ -74,11 +74,28 @@ static int pieces() {
     return bad;
 }
 
+// 2,000 decode steps of 1 to 8 tokens, then another sequence's: the rules are evaluated once per bucket, with the same answers
+static int memo() {
+    PlanMemo mode, piece;
+    int runs = 0, bad = 0, T = 1;
+    for (int n : {60000, 90000})
+        for (int i = 0, at = n; i < 2000; i++, at += T) {
+            T = att_cap_T(at, 1 + i % 8);
+            const AttnJob j = job(at + T, T, 32768, 65536);
+            const std::array<int, 4> key = {16, j.cs, j.pos_lo, plan_end(j)};
+            bad += piece.get(key, [&] { return runs++, range_piece(16, j); }) != range_piece(16, j);
+            bad += mode.get(key, [&] { return runs++, (int) items_mode(16, j, 148); }) != (int) items_mode(16, j, 148);
+        }
+    const int buckets = 2 * (2000 * 9 / 2 / ATT_BUCKET + 2);
+    if (bad || runs > 2 * buckets) std::printf("%d answers differ, %d evaluations\n", bad, runs);
+    return bad + (runs > 2 * buckets);
+}
+
 int main(int argc, char ** argv) {
     if (argc == 6) {
         const int n = atoi(argv[1]), T = atoi(argv[2]);
         std::printf("%d\n", range_piece(atoi(argv[5]), job(n + T, T, atoi(argv[3]), atoi(argv[4]))));
         return 0;
     }
-    return modes() + pieces() != 0;
+    return modes() + pieces() + memo() != 0;
 }
