@@ -225,13 +225,9 @@ __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatil
     } while (!mbar_try_wait(bar, parity));
     return true;
 }
-// The same for a whole warp that goes on with warp-wide instructions (tcgen05.ld and .st, votes): its lanes may leave the wait by different
-// paths and meet again here. _all: whether every lane's wait succeeded.
-__device__ __forceinline__ void tc_wait_warp(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    tc_wait(bar, parity, wc, status);
-    __syncwarp();
-}
-__device__ __forceinline__ bool tc_wait_warp_all(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
+// The same for a warp whose lanes must agree on the result: whether every lane's wait succeeded. (Warp-wide instructions that stand behind a
+// wait whatever its result need no such vote; a __syncwarp before each of them cost 16 calls of 24,003 positions 1.3 %.)
+__device__ __forceinline__ bool tc_wait_all(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
     return __all_sync(FULL_MASK, tc_wait(bar, parity, wc, status)) != 0;
 }
 // at most about 16 ms, for the copies and instructions in flight at the kernel's end
@@ -702,7 +698,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // tile maxima of group j, its own maxima published
         auto maxima = [&](int j) {
             if (st) TC_STAMP(j, 0);
-            tc_wait_warp(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
+            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
             const GroupRec & k = sm.tasks[j % NTASK];
             if (st) TC_STAMP(j, 1);
             tc_fence_after();
@@ -913,8 +909,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
     } else if (warp >= NSOFT) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_DQ ";");
         // ---- unpack warps: packed rows -> operand slots, both 128-dim halves of one side of a group at a time, in the producer's order.
-        // They bound the kernel (5,200 of a group's 6,500 cycles at work, 6.4 cycles an instruction), so everything besides the
-        // values' arithmetic is kept out of the loop: a side's body knows its format, a tile is one descriptor word, the bias constants
+        // They bound the kernel (4,370 of a group's 5,840 cycles at work, the rest waiting for tiles and operand slots), so everything besides
+        // the values' arithmetic is kept out of the loop: a side's body knows its format, a tile is one descriptor word, the bias constants
         // stay in registers ----
         const int w = warp - NSOFT, q = w & 3, c = w >> 2, prow = ATP * q + lane;
         const unsigned pos_off = (prow >> 3) * 128 + (prow & 7) * 16; // the position's 16-byte unit inside a dim group
@@ -950,7 +946,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             constexpr int SIDE = decltype(side_c)::value, FIXED = SIDE ? VB : KB; // the side's compiled-in main format, or 0: any
             const unsigned rs = q + GT * (rseq & 1);
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 8 : 11);
-            if (!tc_wait_warp_all(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status)) return false;
+            if (!tc_wait_all(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status)) return false;
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 9 : 12);
             ud = sm.udesc[j % NTASK][SIDE][q];
             const bool valid = lane < (int) (ud & UD_ROWS);
@@ -1085,7 +1081,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 warp_arrive(&sm.s_empty[i % NSB], lane);
             }
             if (st && i < 15) TC_STAMP(i, 15);
-            if (i > 0) tc_wait_warp(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
+            if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
             if (st) TC_STAMP(i, 5);
             tc_fence_after();
 #if MKKV_TC_PROF
@@ -1146,7 +1142,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 // After a wait that gave up the group's record may not be written: the wait's result is voted on, so that the warp-wide
                 // instructions under `act` are executed by all lanes or none, and a warp without a record has nothing to do but the barriers
                 // that carry the flag (softmax).
-                const bool there = tc_wait_warp_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
+                const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
                 const GroupRec & k = sm.tasks[i % NTASK];
                 if (st) TC_STAMP(i, 1);
                 tc_fence_after();
@@ -1181,7 +1177,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 flush_slot = k.slot, flush_rows = rows;
             }
             if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
-                tc_wait_warp(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
                 tc_fence_after();
                 read_out(flush_slot, flush_rows, true);
             }
@@ -1190,7 +1186,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         const bool act = 16 * q < R;
         for (int i = 0; i < G; i++) {
             tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
-            tc_wait_warp(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
+            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
             tc_fence_after();
             const GroupRec & k = sm.tasks[i % NTASK];
             if (st) TC_STAMP(i, 3);
@@ -1208,7 +1204,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             });
         }
         if (G > 0) {
-            tc_wait_warp(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+            tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
             tc_fence_after();
         }
 #if MKKV_TC_PROF
