@@ -20,7 +20,12 @@ namespace mkkv {
 // --------------------------------------------------------------------------------------------------------------------
 // append / spill / refill: one warp per row
 // --------------------------------------------------------------------------------------------------------------------
-constexpr int MANY_ROWS = 64; // more positions than these: four rows share a warp (fewer: a row a warp is the shorter chain)
+// More positions than these: four rows share a warp. Up to there a row a warp is the shorter chain: a position is one block, and the lines lie
+// where the blocks of rows that are quantized twice (main format and ring) no longer have an SM each, of those quantized once where there
+// are more than three to an SM. us per call, queued (4.14: the rate of empty launches), a row a warp / four: K5r / V6, window 2,048, eager, 64
+// rows 4.2 / 4.4, 128 4.2 / 5.0, 144 4.2 / 5.1, 160 5.2 / 5.1, 256 5.7 / 5.2, 512 6.2 / 5.8; K6 / V5 144 4.2 / 4.2, 160 4.8 / 4.2; K5r / V6, spill, 128 4.2 / 4.7,
+// 416 4.2 / 5.2, 448 4.6 / 5.2, 512 5.6 / 5.2; without a window 416 4.2 / 4.2, 448 5.3 / 4.2, 640 6.2 / 5.0; K8 / V6, spill, 640 4.2 / 4.8; q8_0 equal throughout.
+constexpr int MANY_ROWS_TWICE = 148, MANY_ROWS_ONCE = 3 * 148;
 
 struct AppendArgs {
     KvView kv;
@@ -305,7 +310,7 @@ cudaError_t launch_append_batch(const AppendJob * ajobs_dev, const AttnJob * job
 cudaError_t launch_append(const KvView & kv, const uint16_t * K, const uint16_t * V, int pos0, int n, cudaStream_t stream, int spill0, int spill1) {
     if (n <= 0) return cudaSuccess;
     AppendArgs a{kv, K, V, pos0, n};
-    if (n > MANY_ROWS || spill1 > spill0) {
+    if (n > (kv.eager && kv.rc > 0 ? MANY_ROWS_TWICE : MANY_ROWS_ONCE) || spill1 > spill0) {
         append_many_kernel<<<(n * 2 + 7) / 8, 256, 0, stream>>>(a, spill0, spill1);
         return cudaGetLastError();
     }

@@ -224,18 +224,18 @@ def test_per_layer_spec_items_match_oracle(mk, torch_cuda):
 @pytest.mark.parametrize("bits", [4, 5, 6, 7, 8])
 @pytest.mark.parametrize("rot", [False, True])
 def test_many_rows_at_once_give_the_same_bytes(mk, torch_cuda, bits, rot):
-    """From 65 positions on four rows share a warp. The corner-case rows (zeros of both signs, ties, the type's extremes, subnormals) and
-    random ones, 65 and 97 positions at once, against the same rows in calls of 64 or fewer: every stored byte."""
+    """From 149 positions on (with a window, eager) or 445 (else) four rows share a warp. The corner-case rows (zeros of both signs, ties, the
+    type's extremes, subnormals) and random ones, at once, against the same rows in calls of 40: every stored byte."""
     torch = torch_cuda
     edge = kvdata.edge_rows().astype(np.float16)
     rng = np.random.default_rng(bits)
-    for n in (65, 97):
+    for n in (65, 97, 149, 174) if bits < 8 else (97, 445, 473):
         rows = (rng.standard_normal((n, 4, 256)) * rng.uniform(0.01, 30, (n, 4, 1))).astype(np.float16)
         for i in range(len(edge)):
             rows[(i * 5) % n, i % 4] = edge[i]
         K, V = torch.from_numpy(rows).cuda(), torch.from_numpy(rows[::-1].copy()).cuda()
         spec = "K*=%d%s,V*=%d%s" % (bits, "r" if rot else "", bits, "" if rot else "r")
-        engs = [mk.Engine(1, 256, spec, 640 if bits < 8 else 0) for _ in range(2)]
+        engs = [mk.Engine(1, n + 8, spec, 640 if bits < 8 else 0) for _ in range(2)]
         engs[0].append(0, 3, K, V)
         for a in range(0, n, 40):
             engs[1].append(0, 3 + a, K[a:a + 40].contiguous(), V[a:a + 40].contiguous())
