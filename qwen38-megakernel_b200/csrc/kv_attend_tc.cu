@@ -35,8 +35,8 @@
 //     of 37.3), no exchange; attn_merge_kernel afterwards. The copies, the unpacking and S of the next item run on while the softmax
 //     warps finish the one before. What bounds it: a group costs 3.0 us of CTA time at any length, most of it the unpack warps'
 //     instructions, an item about 2 us more.
-//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 2.3 us against 18.8;
-//     101,600, 8 tokens 67.3 against 95.
+//     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 2.2 us against 18.8;
+//     101,600, 8 tokens 69 (the same cache in every step) .. 74 (another cache each step) against 100.
 // Every wait is bounded (about two seconds by default; the limits are launch arguments), then the status word and a CTA-wide
 // flag are set, no later wait of the CTA blocks, the producer waits (bounded) for its copies still in flight, and the kernel
 // runs to its end and frees its tensor memory.
@@ -1423,11 +1423,12 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     if (e != cudaSuccess) return e;
     // (the jobs of one batch may differ in format: the any-format instance unless they all share a compiled-in pair)
     const TcKernel kern = one_format ? tc_kernel_for(first.kv.s[0].bits, first.kv.s[1].bits, true) : tc::attn_tc_kernel<0, 0, true>;
-    // The prologue beside the launch before (22.3 us instead of 26.6 for a 300-position layer with the merge's early launch, 70.2
-    // instead of 73.9 for 16 layers of 1,187 positions) pays where a CTA's work is short; 16 layers of 11,701 positions (45 groups per
-    // CTA) took 222 us with it and 217 without, a batch of 32 sequences 3,176 and 3,020 (without it, with the softmax warps' packed
-    // arithmetic, 197 and 2,782). Of jobs that differ, the first and longest one's chunk length stands for all. The merge's blocks waiting
-    // beside the attention cost more than they gain as soon as CTAs have more than one item (102 -> 111 us for 16 layers of 4,000 positions).
+    // The prologue beside the launch before saves 2 .. 3 us a launch, which counts where a CTA's work is short (us, without / with): 16
+    // layers of 700 positions 30.9 / 28.8, of 2,000 51.0 / 47.6, of 4,000 84.9 / 81.5, 6 sequences in 16 layers 520 / 486. Long steps gain the
+    // same 2 us (16 layers of 24,000 298.7 / 296.4, of 101,600 1,104.6 / 1,101.7), but a batch of 32 sequences in 4 layers lost 11 (2,350 / 2,361): the
+    // next layer's CTAs wait beside the last items of this one's. The limit of 20 groups a CTA keeps such batches without it. Of jobs
+    // that differ, the first and longest one's chunk length stands for all. The merge's blocks waiting beside the attention cost more than
+    // they gain as soon as CTAs have more than one item (an earlier build: 102 -> 111 us for 16 layers of 4,000 positions).
     const int grid = std::min(nitems, num_sms), per_cta = (nitems + grid - 1) / grid * std::max(first.cpi, 1) * ((first.cs / ATP + tc::GT - 1) / tc::GT);
     e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(tc::NTHREADS), attend_tc_smem_bytes(), stream, a);
     if (e != cudaSuccess) return e;

@@ -214,11 +214,11 @@ def test_long_ranges_are_cut_into_even_items(mk, torch_cuda, tmp_path):
         eng.close()
 
 
-@pytest.mark.parametrize("n,lo,hi", [(230009, 196608, 262144), (262136, 98304, 131072)])
+@pytest.mark.parametrize("n,lo,hi", [(230009, 196608, 262144), (262136, 98304, 131072), (262136, 120000, 130016)])
 def test_pieces_of_a_range_are_those_of_every_call(mk, torch_cuda, n, lo, hi):
     """A range's partial must not depend on how many layers or tokens share the call: 16 layers in the one launch, 2 layers and 1 layer in the
     spread mode, 8 tokens and 1, over the same rows, 1e-5 (a P rounded against another maximum moves the output by 2e-5 .. 4e-5); and
-    the layers of a call, given the same rows, the same bits. The context's end, with the new rows, and an inner range."""
+    the layers of a call, given the same rows, the same bits. The context's end, with the new rows, an inner range and one that lies in a single chunk."""
     torch = torch_cuda
     layers, T, end = 16, 8, min(hi, n)
     g = torch.Generator(device="cuda")
@@ -272,3 +272,28 @@ def test_tokens_of_a_call_do_not_change_its_mode(mk, torch_cuda, n):
     assert counts[0] == counts[1] == (3 if n < 5120 else 2)  # staging, attention and, behind the batch launch, the merge
     assert float((O[0, 0] - O[1, 0]).abs().max()) <= 1e-6 * float(O[1, 0].abs().max())
     eng.close()
+
+
+def test_pieces_are_those_of_the_other_kernel(mk, torch_cuda, monkeypatch):
+    """the mma.sync kernel runs a range's pieces too: its result over the last range of 45,000 positions is the tensor-core kernel's, 1e-5"""
+    torch = torch_cuda
+    n, T, layers, lo, hi = 45003, 3, 2, 23008, 45056
+    got = []
+    for kernel in ("tc", "fast"):
+        monkeypatch.setenv("MK_KV_ATTN", kernel)
+        eng = mk.Engine(layers, hi - lo + 64, "K*=5r,V*=6", 2048)
+        eng.set_base(lo)
+        Kl, Vl = (torch.from_numpy(x).cuda() for x in kvdata.kv_rows(85, 0, lo, n - lo))
+        for l in range(layers):
+            eng.append(l, lo, Kl, Vl)
+        K, V, Q = (torch.from_numpy(x).cuda() for x in rows(layers, 6, n, T))
+        part = torch.zeros((layers, 4, 48, 256), dtype=torch.float32, device="cuda")
+        ml = torch.zeros((layers, 4, 48, 2), dtype=torch.float32, device="cuda")
+        O = torch.zeros((layers, T, 24, 256), dtype=torch.float32, device="cuda")
+        eng.step_layers_partial(n, K, V, Q, lo, hi, lo, hi, part, ml)
+        eng.combine_layers(T, 1, part, ml, O)
+        eng.sync()
+        got.append(O)
+        eng.close()
+    rel = float((got[0] - got[1]).norm() / got[0].norm())
+    assert rel <= 1e-5, rel
