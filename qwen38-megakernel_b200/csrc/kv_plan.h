@@ -1,6 +1,6 @@
-// Host rules of the tensor-core kernel: which of its two modes a call runs in, and how a split sequence's range is cut. They see a context's or range's end rounded up
-// to the partition's 640 positions (plan_end), so that what they choose, like the partition itself, does not depend on the number of
-// query tokens (as long as these share one partition).
+// Host rules of the tensor-core kernel: which of its two modes a call runs in, and how a split sequence's range is cut. They see a
+// context's or range's end rounded up to the partition's 640 positions (plan_end), so that what they choose, like the partition itself,
+// does not depend on the number of query tokens (as long as these share one partition).
 #pragma once
 #include <algorithm>
 #include <array>
@@ -45,6 +45,7 @@ inline int busiest_cta(int nlayers, const AttnJob & j, int ctas) {
 //   1 layer: 2,900 positions 22.0 / 22.6, 3,700 20.6 / 24.6, 4,096 (q8_0, 1 token) 20.5 / 20.5, 4,097 22.4 / 22.6, 4,900 20.5 / 24.6, 5,111
 //     20.6 / 24.6; from 5,121 on the rule takes the spread mode: 5,130 24.6 / 24.6, 6,390 23.3 / 24.6, 7,600 23.3 / 24.6, 9,003 28.8 / 26.9,
 //     24,003 45.2 / 39.0, 101,600 134 / 103 (two or three groups a chunk: the batch launch is never slower, by up to 1.4 us faster beyond the line)
+//   (9,003 and longer and several layers: measured when the rule was made, two builds earlier.)
 //   2 layers: 13,003 55.5 / 58.5, 38,000 112 / 99, 101,600 258 / 201; 4 layers: 38,000 156 / 193, 101,600 368 / 396; 8 layers: 101,600 598 / 785.
 // Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode: there the layers' outputs are the same bits one
 // by one and together. Beyond, the two modes' outputs differ by rounding (about 1e-7, relative 2-norm).
@@ -65,13 +66,15 @@ inline bool items_mode(int nlayers, AttnJob j, int sms) {
 // A range holds few, long chunks and its ends cut into two of them anyway, so the busiest CTA of the batch launch had much more than the
 // mean: one of 8 GPUs' part of 262,136 positions, 16 layers: 192 items of 102 or 52 groups on 148 CTAs, the busiest with 154 of a mean of 111;
 // 490 us uncut, 419 with pieces of 2,816 positions; 1 layer 47.9 uncut, 43.2 so, 2 and 4 of the 16 82 and 155 (69 and 136 with pieces of
-// their own, which is what a result that depends on the call would buy). What is computed must not depend on how it is run: the length is a function of the
-// partition, the range (its end as plan_end has it) and the engine's layers, taken for a B200 whole, not of the layers or tokens of a call or
-// the SMs at hand. At most as many pieces as a context has chunks (the partials' scratch), and only for a gain of 3 % in the busiest CTA's load.
+// their own, which is what a result that depends on the call would buy). What is computed must not depend on how it is run: the length is
+// a function of the partition, the range (its end as plan_end has it) and the engine's layers, taken for a B200 whole, not of the layers
+// or tokens of a call or the SMs at hand. At most as many pieces as a context has chunks (the partials' scratch), and only for a gain of 3 % in the busiest CTA's load.
 // Contexts up to 40,320 positions keep their chunks. Against 64 bits pieces are no worse than chunks on either side of that line (the oracle,
-// one range in two, relative 2-norm, chunks / pieces: 20,003 positions 1.9e-5 / 1.3e-5, 38,003 2.0e-5 / 2.0e-5, 40,003 3.8e-5 / 3.0e-5, 45,003 2.6e-5 /
-// 2.1e-5, 60,003 3.2e-5 / 1.4e-5, 101,608 1.9e-5 / 2.2e-5), but the shorter a context, the further from the reference's partition they are: largest difference
-// 1e-3 at 8,003 positions, 3e-4 .. 5e-4 from 20,003 on (2e-3, the bar, at 60,003, where the chunks are 1.9e-3 off 64 bits and the pieces 5e-4).
+// two ranges, relative 2-norm, chunks / pieces: 20,003 positions 1.9e-5 / 1.3e-5, 38,003 2.0e-5 / 2.0e-5, 40,003 3.8e-5 / 3.0e-5, 45,003 2.6e-5 /
+// 2.1e-5, 60,003 3.2e-5 / 1.4e-5, 101,608 1.9e-5 / 2.2e-5), but the shorter a context, the further from the reference's partition they are:
+// largest difference 1e-3 at 8,003 positions, 3e-4 .. 5e-4 from 20,003 on (2e-3, the bar, at 60,003, where the chunks are 1.9e-3 off 64 bits
+// and the pieces 5e-4). What the line costs (us, 16 layers, the second of 2 / of 4 ranges, uncut against cut): 12,000 positions 103 / 95 and 69 / 61,
+// 20,000 139 / 137 and 93 / 85, 38,000 238 / 239 and 153 / 131; beyond it 45,000 280 / 265 and 179 / 149, 60,000 370 / 342 and 232 / 188.
 inline int range_piece(int layers, const AttnJob & j) {
     if (j.cs < 2048) return j.cs;
     AttnJob t = j;
