@@ -44,12 +44,9 @@
 #include <cuda_fp16.h>
 #include <math_constants.h>
 
-#include "kv_attend_common.cuh"
-#include "kv_kernels.h"
-#include "kv_merge.cuh"
-#include "kv_quant.cuh"
-#include "kv_unpack.h"
+#include "kv_attend_tc_parts.cuh"
 #include "kv_attend_tc_unpack.cuh"
+#include "kv_unpack.h"
 
 namespace mkkv {
 
@@ -64,7 +61,6 @@ constexpr int NDQ = 16;        // then the unpack warps: 4 c + q, tile q, 32-dim
 constexpr int W_CTL = NSOFT + NDQ, W_PROD = W_CTL + 2, W_ISSUE = W_CTL + 3;
 constexpr int W_MAX = W_CTL + 4;      // spread mode only: four warps that take the tile maxima and exchange the running maxima
 constexpr int NTHREADS = W_MAX * 32, NTHREADS_SPREAD = (W_MAX + 4) * 32;
-constexpr int GT = 4, GP = GT * ATP;        // tiles / positions per group: the N of an S instruction
 // registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
 // most the CTA's launch allocation -- a larger sum faults)
 #define MKKV_TC_REGS_SOFT "176"
@@ -89,28 +85,6 @@ constexpr int P_BYTES = GP / 8 * P_KGROUP;
 constexpr unsigned S_COL = 0, S_STRIDE = GP, O_COL0 = NSB / 2 * S_STRIDE, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512;
 static_assert(O_COL1 + 2 * AR <= TMEM_COLS, "tensor-memory columns");
 static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
-// The accumulator's reference max of a row is set REF_BELOW below the running max it is taken from and moves when the running max
-// passes it by more than REF_SLACK: beta = exp(running - reference) of the row's largest terms stays within [e^2, e^11 < fp16 max].
-// P beta is held as two fp16 parts, whose step is 2^-24 for small products: e^-2 2^-24 of the row's largest term, below P's own
-// rounding. (With the reference 3 above the running max the parts of weights under e^-7 were subnormal: rows with one position 14 above
-// the others came out 2e-6 .. 7e-6 off 64 bits, relative 2-norm, where P's rounding gives 3e-7; now 2e-7 .. 6e-7.)
-constexpr float REF_SLACK = 11.f, REF_BELOW = 2.f;
-constexpr float LOG2E = 1.4426950408889634f;
-
-// one arrival of the calling warp: by the lane with `lane` 0, under a predicate (a branch would open a divergent region)
-__device__ __forceinline__ void warp_arrive(uint64_t * bar, int lane) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
-}
-template <int V> struct IntC { // an integer as an argument of a generic lambda
-    static constexpr int value = V;
-};
-
-struct WaitCtl { // the launch's wait limits and the CTA's give-up flag
-    int dead;
-    unsigned poll;              // a global word is polled so often
-    unsigned long long limit;   // an mbarrier wait lasts so many nanoseconds
-};
-
 // A group's task record as the producer leaves it for the other roles. The fields behind AttnTask serve the batch mode, where one CTA
 // works for several (job, kv head) pairs in turn: a segment is a run of chunks of one pair, with its own queries, partial and row sums.
 struct GroupRec : AttnTask {
@@ -121,12 +95,6 @@ struct GroupRec : AttnTask {
 // What the unpack warps need of one side of one tile: rows that are there | UD_END in the CTA's last group | bits of the rows << 8
 constexpr unsigned UD_ROWS = 0x3fu, UD_END = 0x80u;
 constexpr int REC_FIRST = 1, REC_LAST = 2, REC_END = 4; // first / last group of its segment, last group of the CTA
-struct TileSrc { // where one side of one tile lies: rows, scales, bytes per row, rows
-    const uint8_t * val;
-    const uint16_t * sc;
-    int rb, np;
-};
-
 struct Smem {
     uint8_t op[NOP][OP_SLOT];   // [dim group 16][position group 16][8 positions][8 dims] fp16
     uint8_t raw[NRAW][RAW_SLOT];
@@ -152,63 +120,12 @@ struct Smem {
     uint64_t m_full[NSB];
 };
 
-struct Args {
-    AttnJob one;
-    const AttnJob * jobs;   // batch mode: device array of njobs jobs (null: the one job); spread mode: not used, the one job runs on cph
-    int njobs;              // CTAs per kv head with the exchange of row maxima
-    int nitems;             // batch mode: (job, kv head, cpi chunks) items of all jobs, dealt to the CTAs in turn
-    int uniform;            // batch mode: the jobs differ in view, queries and output only (the layers of one step): items run by run
-    unsigned * next;        // batch mode, more items than CTAs: items handed out so far beyond every CTA's first (zeroed before the launch)
-    int cph, ntasks;        // CTAs per kv head; tasks per kv head when a host-built list is given
-    const AttnTask * tasks; // optional list (position-range jobs)
-    float * part;           // [CTA][AR][HD]
-    float2 * ml;            // [CTA][AR]
-    unsigned long long * xa; // [kv head][chunk][group][AR]: the group's own row maxima {tag, value}
-    unsigned long long * xb; // same shape: row maxima of the chunk up to and including the group
-    int nbmax, epoch;
-    int * status;
-    float * raw_part;       // fused merge, optional: the merged but un-normalised (m, l, O) per kv head goes here instead of O
-    float2 * raw_ml;        // ([4][48][256] / [4][48]: the input of a later merge across GPUs)
-    unsigned * done;        // fused merge: [kv head] count of CTAs whose partial is written, over all launches (wraps)
-    unsigned done_target;   // the count that means "every CTA of the head, this launch"; done == null: separate merge launch
-    unsigned long long * prof; // optional: [CTA][16 groups][20] globaltimer stamps: softmax warp 0 (0 .. 7), unpack warp 8 (8 .. 15),
-                               // issuer (16 .. 19)
-    unsigned long long wait_limit_ns; // limits of the waits: an mbarrier wait gives up after so long, one for exchange words after
-    unsigned poll_rounds;             // so many failed polls
-};
-#ifndef MKKV_TC_PROF
-#define MKKV_TC_PROF 0 // 1: compile the phase stamps in (they cost a few per cent)
-#endif
-#if MKKV_TC_PROF
-#define TC_STAMP(grp, k)                                                                                               \
-    do {                                                                                                               \
-        if (a.prof && lane == 0 && (grp) >= 0 && (grp) < 16)                                                           \
-            a.prof[((size_t) blockIdx.x * 16 + (grp)) * 20 + (k)] = globaltimer_ns();                                  \
-    } while (0)
-#else
-#define TC_STAMP(grp, k)                                                                                               \
-    do {                                                                                                               \
-    } while (0)
-#endif
-
 // Wait for a phase of an mbarrier. A try suspends the thread in hardware (it wakes when the phase completes, or after a time of the
 // hardware's choosing), so waiting warps take next to no issue slots. (try_wait with a time limit of its own becomes a loop that polls,
 // sleeps and reads the clock.) Bounded: after the limit the status word and the CTA's `dead` flag are set; from then on no wait of this
 // CTA blocks, and the kernel runs to its end. The limit, hint x rounds nanoseconds, is multiplied on the host: this code stands at every
 // wait, and with the product made here a one-layer call of 101,600 positions took 101.3 us instead of 99.9, of 100,000 in q8_0 91.8 instead
 // of 89.8.
-constexpr unsigned WAIT_HINT_NS = 10000u, WAIT_ROUNDS = 200000u, POLL_ROUNDS = 1u << 21; // defaults: about two seconds each
-__device__ __forceinline__ bool mbar_test_wait(uint64_t * bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Returns whether the phase is complete.
 __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
     if (mbar_test_wait(bar, parity)) return true; // (the common case: no limit loaded)
@@ -230,16 +147,6 @@ __device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatil
 __device__ __forceinline__ bool tc_wait_all(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
     return __all_sync(FULL_MASK, tc_wait(bar, parity, wc, status)) != 0;
 }
-// at most about 16 ms, for the copies and instructions in flight at the kernel's end
-__device__ __forceinline__ void wait_landed(uint64_t * bar, unsigned parity) {
-    const unsigned long long t0 = globaltimer_ns();
-    while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < 16000000ull) {}
-}
-// Whether the CTA has given up, the same answer for all the lanes of mask. Another warp may set the flag between two lanes' reads: a
-// warp that leaves a loop with warp-wide operations in it leaves it by this vote (lanes that disagreed would wait for each other, some
-// at such an operation, the others at the kernel's last barrier, and neither wait is bounded).
-__device__ __forceinline__ bool gave_up(unsigned mask, const volatile WaitCtl * wc) { return __any_sync(mask, wc->dead != 0) != 0; }
-
 // The last copies of a producer lane, newest first, as bytes (slot << 1 | phase parity; 0xff: nothing was copied for that slot's turn):
 // they must land before the CTA's shared memory is released, also when a consumer gives up after the producer has fetched everything
 // and left its loop. Only the last turn of each of the lane's slots can be in flight (the one before it was waited for before the slot
@@ -261,33 +168,6 @@ __device__ __forceinline__ void drain_copies(uint64_t * raw_full, unsigned issue
 // V MN-major, P (48 rows' high parts, then their low parts) K-major
 constexpr unsigned IDESC_S = (1u << 4) | ((unsigned) (GP / 8) << 17) | ((unsigned) (64 / 16) << 24);
 constexpr unsigned IDESC_PV = (1u << 4) | (1u << 15) | ((unsigned) (2 * AR / 8) << 17) | ((unsigned) (128 / 16) << 24);
-__device__ __forceinline__ void umma(unsigned d_tmem, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi, unsigned idesc, unsigned accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\tsetp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ unsigned desc_lo(unsigned addr, unsigned lbo) { return ((addr >> 4) & 0x3fffu) | (((lbo >> 4) & 0x3fffu) << 16); }
-__device__ __forceinline__ unsigned desc_hi(unsigned sbo) { return ((sbo >> 4) & 0x3fffu) | (1u << 14); }
-__device__ __forceinline__ void umma_commit(uint64_t * bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// One lane of a converged warp. Code under this test is known to be one thread's, so that the descriptors of its tcgen05.mma (uniform
-// registers) need no search for the lanes that agree.
-__device__ __forceinline__ bool elect_one() {
-    unsigned r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r != 0;
-}
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // The scores of one S buffer (16 lanes of the warp's quarter from taddr's on): lanes 0 .. 15 get columns 0 .. 63 of their row, lanes
 // 16 .. 31 columns 64 .. 127. (One statement with its wait: no use of the registers can move between the two.)
 __device__ __forceinline__ void tmem_scores(unsigned taddr, float (&s)[2 * ATP]) {
@@ -321,71 +201,6 @@ __device__ __forceinline__ void tmem_ld16_two(unsigned ta, unsigned tb, unsigned
                  : "r"(ta), "r"(tb)
                  : "memory");
 }
-// exp(x), relative error about 2^-21 (scale factors applied alike to the accumulator and the row sums)
-__device__ __forceinline__ float exp_any(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, LOG2E)));
-    return y;
-}
-__device__ __forceinline__ float ex2(float x) { // 2^x for x <= 0 (and -inf -> 0)
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-// bounded poll of up to three exchange words until each carries this launch's tag (null: not needed); what is missing is asked for together
-__device__ __forceinline__ void poll_words(const unsigned long long * (&src)[3], unsigned long long (&w)[3], int epoch, volatile WaitCtl * wc, int * status) {
-    for (unsigned it = 0;; it++) {
-        bool ready = true;
-#pragma unroll
-        for (int x = 0; x < 3; x++) ready = ready && (!src[x] || (unsigned) (w[x] >> 32) == (unsigned) epoch);
-        if (ready || wc->dead) return;
-        if (it >= wc->poll) { // (a round is a trip to the L2)
-            wc->dead = 1;
-            atomicExch(status, (int) KS_WAIT_TIMEOUT);
-            return;
-        }
-#pragma unroll
-        for (int x = 0; x < 3; x++)
-            if (src[x] && (unsigned) (w[x] >> 32) != (unsigned) epoch) w[x] = __ldcv(src[x]);
-    }
-}
-// task t of a kv head (group-major over its chunks), 4 tiles per task; mul_*: ceil(2^32 / divisor) (exact quotients for t < 2^26)
-struct Geo4 {
-    Geo g;
-    unsigned mul_nch, mul_nch1;
-};
-__device__ __forceinline__ Task make_task4(const Geo4 & G4, int t) {
-    const Geo & g = G4.g;
-    Task k;
-    const int first = g.nb_last * g.nch;
-    if (t < first) {
-        k.b = g.nch > 1 ? (int) __umulhi((unsigned) t, G4.mul_nch) : t;
-        k.c = t - k.b * g.nch;
-    } else {
-        const int u = t - first;
-        const int qd = g.nch > 2 ? (int) __umulhi((unsigned) u, G4.mul_nch1) : u;
-        k.b = g.nb_last + qd;
-        k.c = u - qd * (g.nch - 1);
-    }
-    const int ntc = k.c == g.nch - 1 ? g.nt_last : g.nt_full;
-    k.nb = (ntc + GT - 1) / GT;
-    k.c1 = min(g.L, (k.c + 1) * g.cs);
-    k.pos0 = k.c * g.cs + k.b * GP;
-    k.nt = min(GT, ntc - k.b * GT);
-    return k;
-}
-
-// bar.sync with an OR over the threads' predicates (the same answer for all)
-__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool p) {
-    unsigned r;
-    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                 : "=r"(r)
-                 : "r"(id), "r"(nthreads), "r"((unsigned) p)
-                 : "memory");
-    return r != 0;
-}
-
 // ---- batch mode: the producer warp ----
 // Walks the CTA's segments and their groups, fetches K(0) .. K(NSB - 1), then V(i), K(i + NSB) -- the order the unpack warps consume
 // -- and leaves every group's record before its K. Lanes 0 .. 3 fetch one tile of the group each. An item is a run of cpi chunks of one
@@ -521,59 +336,6 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         else nv++;
     }
     if (lane < GT) drain_copies(sm.raw_full, issued, NRAW / GT);
-}
-
-// Spread mode: the merge, in the kernel's tail: when every CTA of kv head g has written its partial, this CTA (kk-th of the head's cph)
-// merges rows kk and kk + cph of the head's 6 T. Eight warps (mw; the softmax warps and the first four unpack warps), four
-// to a row (warp j of the team: partials j, j + 4, ..: all their loads are in flight at once); the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete).
-constexpr int MERGE_WARPS = 8;
-__device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int kk, int T, int mw, int lane) {
-    __threadfence();
-    named_bar(5, MERGE_WARPS * 32);
-    if (mw == 0 && lane == 0) {
-        bool ok = true;
-        atomicAdd(a.done + g, 1u);
-        unsigned it = 0;
-        while ((int) (ld_acquire_u32(a.done + g) - a.done_target) < 0) {
-            __nanosleep(100);
-            if (++it >= (sm.wc.poll << 2) || sm.wc.dead) { // (about a second)
-                atomicExch(a.status, (int) KS_WAIT_TIMEOUT);
-                ok = false;
-                break;
-            }
-        }
-        sm.merge_ok = ok;
-    }
-    named_bar(5, MERGE_WARPS * 32);
-#if MKKV_TC_PROF
-    if (mw == 0) TC_STAMP(15, 12);
-#endif
-    const int team = mw >> 2, tj = mw & 3, rr = kk + team * a.cph;
-    const bool has = sm.merge_ok && rr < GQ * T;
-    float * const scratch = reinterpret_cast<float *>(sm.op[0]); // [warp][lane][8 sums], then [warp] weights' sums
-    float num[8], den = 0.f, M = -CUDART_INF_F;
-    if (has) {
-        merge_accumulate<4>(a.part, a.ml, (size_t) g * a.cph, (size_t) AR * HD, (size_t) AR, a.cph, tj, 4, rr, lane, num, den, M);
-        float4 * d = reinterpret_cast<float4 *>(scratch + ((size_t) mw * 32 + lane) * 8);
-        d[0] = make_float4(num[0], num[1], num[2], num[3]);
-        d[1] = make_float4(num[4], num[5], num[6], num[7]);
-        if (lane == 0) scratch[MERGE_WARPS * 32 * 8 + mw] = den;
-    }
-    named_bar(5, MERGE_WARPS * 32);
-    if (has && tj == 0) {
-#pragma unroll
-        for (int w2 = 1; w2 < 4; w2++) {
-            const float4 * o = reinterpret_cast<const float4 *>(scratch + ((size_t) (mw + w2) * 32 + lane) * 8);
-            const float4 o0 = o[0], o1 = o[1];
-            num[0] += o0.x, num[1] += o0.y, num[2] += o0.z, num[3] += o0.w;
-            num[4] += o1.x, num[5] += o1.y, num[6] += o1.z, num[7] += o1.w;
-            den += scratch[MERGE_WARPS * 32 * 8 + mw + w2];
-        }
-        merge_finish(sm.job, g * GQ + rr / T, rr % T, lane, a.raw_part != nullptr, a.raw_part, a.raw_ml, num, den, M);
-    }
-#if MKKV_TC_PROF
-    if (mw == 0) TC_STAMP(15, 13);
-#endif
 }
 
 // ---- scores of one row on one thread (hf 0: tiles 0 and 1 of the group, 1: tiles 2 and 3) ----
@@ -935,10 +697,10 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             PackedBlock<B> b0, b1;
             dq_load<B>(b0, b1, rawa, lane, jr, valid);
             tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            dq_emit<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
+            store_block<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
             hand_over();
             tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            dq_emit<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
+            store_block<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
             hand_over();
         };
         // one side of group j; false: the CTA has given up
@@ -1236,7 +998,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 
 // ---- test probe of the unpack step ----
 // nrows packed rows of BITS bits (values [nrows][32 BITS] bytes, scales [nrows][8] fp16) through the very code the unpack warps run
-// (dq_load / dq_emit on a staged tile), back in natural dim order: out [nrows][256] fp16 bit patterns. One warp per 32-row tile.
+// (dq_load / store_block on a staged tile), back in natural dim order: out [nrows][256] fp16 bit patterns. One warp per 32-row tile.
 template <int BITS> __global__ void __launch_bounds__(32) unpack_probe_kernel(const uint8_t * rows, const uint16_t * sc, int nrows, uint16_t * out) {
     __shared__ __align__(128) uint8_t raw[RAW_SLOT];
     __shared__ __align__(128) uint8_t op[4 * 2048]; // one 32-dim block: four dim groups of 128 positions x 16 bytes

@@ -1,0 +1,260 @@
+// What a kernel of the tensor-core decode attention is built from: launch arguments, mbarrier and tcgen05 wrappers, exponentials, the exchange of running maxima between CTAs, the
+// tasks of a job spread over the grid and the merge in the kernel's tail.
+#pragma once
+#include <cuda_fp16.h>
+#include <math_constants.h>
+
+#include "kv_attend_common.cuh"
+#include "kv_kernels.h"
+#include "kv_merge.cuh"
+#include "kv_quant.cuh"
+
+namespace mkkv {
+namespace tc {
+
+using namespace attn_common;
+
+constexpr int GT = 4, GP = GT * ATP; // tiles / positions per group: the unit of work
+// The accumulator's reference max of a row is set REF_BELOW below the running max it is taken from and moves when the running max
+// passes it by more than REF_SLACK: beta = exp(running - reference) of the row's largest terms stays within [e^2, e^11 < fp16 max].
+// P beta is held as two fp16 parts, whose step is 2^-24 for small products: e^-2 2^-24 of the row's largest term, below P's own
+// rounding. (With the reference 3 above the running max the parts of weights under e^-7 were subnormal: rows with one position 14 above
+// the others came out 2e-6 .. 7e-6 off 64 bits, relative 2-norm, where P's rounding gives 3e-7; now 2e-7 .. 6e-7.)
+constexpr float REF_SLACK = 11.f, REF_BELOW = 2.f;
+constexpr float LOG2E = 1.4426950408889634f;
+
+
+// one arrival of the calling warp: by the lane with `lane` 0, under a predicate (a branch would open a divergent region)
+__device__ __forceinline__ void warp_arrive(uint64_t * bar, int lane) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane) : "memory");
+}
+template <int V> struct IntC { // an integer as an argument of a generic lambda
+    static constexpr int value = V;
+};
+
+struct WaitCtl { // the launch's wait limits and the CTA's give-up flag
+    int dead;
+    unsigned poll;              // a global word is polled so often
+    unsigned long long limit;   // an mbarrier wait lasts so many nanoseconds
+};
+
+struct TileSrc { // where one side of one tile lies: rows, scales, bytes per row, rows
+    const uint8_t * val;
+    const uint16_t * sc;
+    int rb, np;
+};
+
+
+struct Args {
+    AttnJob one;
+    const AttnJob * jobs;   // batch mode: device array of njobs jobs (null: the one job); spread mode: not used, the one job runs on cph
+    int njobs;              // CTAs per kv head with the exchange of row maxima
+    int nitems;             // batch mode: (job, kv head, cpi chunks) items of all jobs, dealt to the CTAs in turn
+    int uniform;            // batch mode: the jobs differ in view, queries and output only (the layers of one step): items run by run
+    unsigned * next;        // batch mode, more items than CTAs: items handed out so far beyond every CTA's first (zeroed before the launch)
+    int cph, ntasks;        // CTAs per kv head; tasks per kv head when a host-built list is given
+    const AttnTask * tasks; // optional list (position-range jobs)
+    float * part;           // [CTA][AR][HD]
+    float2 * ml;            // [CTA][AR]
+    unsigned long long * xa; // [kv head][chunk][group][AR]: the group's own row maxima {tag, value}
+    unsigned long long * xb; // same shape: row maxima of the chunk up to and including the group
+    int nbmax, epoch;
+    int * status;
+    float * raw_part;       // fused merge, optional: the merged but un-normalised (m, l, O) per kv head goes here instead of O
+    float2 * raw_ml;        // ([4][48][256] / [4][48]: the input of a later merge across GPUs)
+    unsigned * done;        // fused merge: [kv head] count of CTAs whose partial is written, over all launches (wraps)
+    unsigned done_target;   // the count that means "every CTA of the head, this launch"; done == null: separate merge launch
+    unsigned long long * prof; // optional: [CTA][16 groups][20] globaltimer stamps: softmax warp 0 (0 .. 7), unpack warp 8 (8 .. 15),
+                               // issuer (16 .. 19)
+    unsigned long long wait_limit_ns; // limits of the waits: an mbarrier wait gives up after so long, one for exchange words after
+    unsigned poll_rounds;             // so many failed polls
+};
+#ifndef MKKV_TC_PROF
+#define MKKV_TC_PROF 0 // 1: compile the phase stamps in (they cost a few per cent)
+#endif
+#if MKKV_TC_PROF
+#define TC_STAMP(grp, k)                                                                                               \
+    do {                                                                                                               \
+        if (a.prof && lane == 0 && (grp) >= 0 && (grp) < 16)                                                           \
+            a.prof[((size_t) blockIdx.x * 16 + (grp)) * 20 + (k)] = globaltimer_ns();                                  \
+    } while (0)
+#else
+#define TC_STAMP(grp, k)                                                                                               \
+    do {                                                                                                               \
+    } while (0)
+#endif
+
+
+constexpr unsigned WAIT_HINT_NS = 10000u, WAIT_ROUNDS = 200000u, POLL_ROUNDS = 1u << 21; // defaults: about two seconds each
+__device__ __forceinline__ bool mbar_test_wait(uint64_t * bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// at most about 16 ms, for the copies and instructions in flight at the kernel's end
+__device__ __forceinline__ void wait_landed(uint64_t * bar, unsigned parity) {
+    const unsigned long long t0 = globaltimer_ns();
+    while (!mbar_try_wait(bar, parity) && globaltimer_ns() - t0 < 16000000ull) {}
+}
+// Whether the CTA has given up, the same answer for all the lanes of mask. Another warp may set the flag between two lanes' reads: a
+// warp that leaves a loop with warp-wide operations in it leaves it by this vote (lanes that disagreed would wait for each other, some
+// at such an operation, the others at the kernel's last barrier, and neither wait is bounded).
+__device__ __forceinline__ bool gave_up(unsigned mask, const volatile WaitCtl * wc) { return __any_sync(mask, wc->dead != 0) != 0; }
+
+
+// ---- tcgen05 ----
+__device__ __forceinline__ void umma(unsigned d_tmem, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ unsigned desc_lo(unsigned addr, unsigned lbo) { return ((addr >> 4) & 0x3fffu) | (((lbo >> 4) & 0x3fffu) << 16); }
+__device__ __forceinline__ unsigned desc_hi(unsigned sbo) { return ((sbo >> 4) & 0x3fffu) | (1u << 14); }
+__device__ __forceinline__ void umma_commit(uint64_t * bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// One lane of a converged warp. Code under this test is known to be one thread's, so that the descriptors of its tcgen05.mma (uniform
+// registers) need no search for the lanes that agree.
+__device__ __forceinline__ bool elect_one() {
+    unsigned r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned * p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// exp(x), relative error about 2^-21 (scale factors applied alike to the accumulator and the row sums)
+__device__ __forceinline__ float exp_any(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, LOG2E)));
+    return y;
+}
+__device__ __forceinline__ float ex2(float x) { // 2^x for x <= 0 (and -inf -> 0)
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+
+// bounded poll of up to three exchange words until each carries this launch's tag (null: not needed); what is missing is asked for together
+__device__ __forceinline__ void poll_words(const unsigned long long * (&src)[3], unsigned long long (&w)[3], int epoch, volatile WaitCtl * wc, int * status) {
+    for (unsigned it = 0;; it++) {
+        bool ready = true;
+#pragma unroll
+        for (int x = 0; x < 3; x++) ready = ready && (!src[x] || (unsigned) (w[x] >> 32) == (unsigned) epoch);
+        if (ready || wc->dead) return;
+        if (it >= wc->poll) { // (a round is a trip to the L2)
+            wc->dead = 1;
+            atomicExch(status, (int) KS_WAIT_TIMEOUT);
+            return;
+        }
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+            if (src[x] && (unsigned) (w[x] >> 32) != (unsigned) epoch) w[x] = __ldcv(src[x]);
+    }
+}
+// task t of a kv head (group-major over its chunks), 4 tiles per task; mul_*: ceil(2^32 / divisor) (exact quotients for t < 2^26)
+struct Geo4 {
+    Geo g;
+    unsigned mul_nch, mul_nch1;
+};
+__device__ __forceinline__ Task make_task4(const Geo4 & G4, int t) {
+    const Geo & g = G4.g;
+    Task k;
+    const int first = g.nb_last * g.nch;
+    if (t < first) {
+        k.b = g.nch > 1 ? (int) __umulhi((unsigned) t, G4.mul_nch) : t;
+        k.c = t - k.b * g.nch;
+    } else {
+        const int u = t - first;
+        const int qd = g.nch > 2 ? (int) __umulhi((unsigned) u, G4.mul_nch1) : u;
+        k.b = g.nb_last + qd;
+        k.c = u - qd * (g.nch - 1);
+    }
+    const int ntc = k.c == g.nch - 1 ? g.nt_last : g.nt_full;
+    k.nb = (ntc + GT - 1) / GT;
+    k.c1 = min(g.L, (k.c + 1) * g.cs);
+    k.pos0 = k.c * g.cs + k.b * GP;
+    k.nt = min(GT, ntc - k.b * GT);
+    return k;
+}
+
+// bar.sync with an OR over the threads' predicates (the same answer for all)
+__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool p) {
+    unsigned r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r)
+                 : "r"(id), "r"(nthreads), "r"((unsigned) p)
+                 : "memory");
+    return r != 0;
+}
+
+// Spread mode: the merge, in the kernel's tail: when every CTA of kv head g has written its partial, this CTA (kk-th of the head's cph)
+// merges rows kk and kk + cph of the head's 6 T. Eight warps (mw; the softmax warps and the first four unpack warps), four
+// to a row (warp j of the team: partials j, j + 4, ..: all their loads are in flight at once); the team's sums meet in shared memory (an operand slot: every MMA of the CTA is complete).
+constexpr int MERGE_WARPS = 8;
+template <class Smem> __device__ __forceinline__ void tail_merge(Smem & sm, const Args & a, int g, int kk, int T, int mw, int lane) {
+    __threadfence();
+    named_bar(5, MERGE_WARPS * 32);
+    if (mw == 0 && lane == 0) {
+        bool ok = true;
+        atomicAdd(a.done + g, 1u);
+        unsigned it = 0;
+        while ((int) (ld_acquire_u32(a.done + g) - a.done_target) < 0) {
+            __nanosleep(100);
+            if (++it >= (sm.wc.poll << 2) || sm.wc.dead) { // (about a second)
+                atomicExch(a.status, (int) KS_WAIT_TIMEOUT);
+                ok = false;
+                break;
+            }
+        }
+        sm.merge_ok = ok;
+    }
+    named_bar(5, MERGE_WARPS * 32);
+#if MKKV_TC_PROF
+    if (mw == 0) TC_STAMP(15, 12);
+#endif
+    const int team = mw >> 2, tj = mw & 3, rr = kk + team * a.cph;
+    const bool has = sm.merge_ok && rr < GQ * T;
+    float * const scratch = reinterpret_cast<float *>(sm.op[0]); // [warp][lane][8 sums], then [warp] weights' sums
+    float num[8], den = 0.f, M = -CUDART_INF_F;
+    if (has) {
+        merge_accumulate<4>(a.part, a.ml, (size_t) g * a.cph, (size_t) AR * HD, (size_t) AR, a.cph, tj, 4, rr, lane, num, den, M);
+        float4 * d = reinterpret_cast<float4 *>(scratch + ((size_t) mw * 32 + lane) * 8);
+        d[0] = make_float4(num[0], num[1], num[2], num[3]);
+        d[1] = make_float4(num[4], num[5], num[6], num[7]);
+        if (lane == 0) scratch[MERGE_WARPS * 32 * 8 + mw] = den;
+    }
+    named_bar(5, MERGE_WARPS * 32);
+    if (has && tj == 0) {
+#pragma unroll
+        for (int w2 = 1; w2 < 4; w2++) {
+            const float4 * o = reinterpret_cast<const float4 *>(scratch + ((size_t) (mw + w2) * 32 + lane) * 8);
+            const float4 o0 = o[0], o1 = o[1];
+            num[0] += o0.x, num[1] += o0.y, num[2] += o0.z, num[3] += o0.w;
+            num[4] += o1.x, num[5] += o1.y, num[6] += o1.z, num[7] += o1.w;
+            den += scratch[MERGE_WARPS * 32 * 8 + mw + w2];
+        }
+        merge_finish(sm.job, g * GQ + rr / T, rr % T, lane, a.raw_part != nullptr, a.raw_part, a.raw_ml, num, den, M);
+    }
+#if MKKV_TC_PROF
+    if (mw == 0) TC_STAMP(15, 13);
+#endif
+}
+
+
+} // namespace tc
+} // namespace mkkv

@@ -62,12 +62,13 @@ __device__ __forceinline__ UnpackConst unpack_const() {
     asm volatile("mov.b32 %0, %1;" : "=r"(u.b) : "n"(MAGIC_B));
     return u;
 }
-// one unit: the pairs' high-bit words y0 .. y3 (bias included) and the lane word -> four values, stored
-template <int BITS> __device__ __forceinline__ void unit_out(unsigned dst, unsigned word, unsigned y0, unsigned y1, unsigned y2, unsigned y3, unsigned d) {
+// one unit: the pairs' high-bit words y0 .. y3 (bias included) and the lane word -> four value pairs, handed to put(u, ..)
+template <int BITS, class Put>
+__device__ __forceinline__ void unit_out(int u, unsigned word, unsigned y0, unsigned y1, unsigned y2, unsigned y3, unsigned d, Put && put) {
     constexpr unsigned SA = MAGIC_A + (0x00010001u << (BITS - 1)), SB = MAGIC_B + (0x00100010u << (BITS - 1));
     const unsigned w8 = word >> 8;
-    sts128(dst, pair_val<SA>(and_or_imm<NIB_A>(word, y0), d), pair_val<SB>(and_or_imm<NIB_B>(word, y1), d),
-           pair_val<SA>(and_or_imm<NIB_A>(w8, y2), d), pair_val<SB>(and_or_imm<NIB_B>(w8, y3), d));
+    put(u, pair_val<SA>(and_or_imm<NIB_A>(word, y0), d), pair_val<SB>(and_or_imm<NIB_B>(word, y1), d), pair_val<SA>(and_or_imm<NIB_A>(w8, y2), d),
+        pair_val<SB>(and_or_imm<NIB_B>(w8, y3), d));
 }
 // the packed bytes of one (position, 32-dim block): lane words, high-bit words, scale pair
 template <int BITS> struct PackedBlock {
@@ -75,63 +76,29 @@ template <int BITS> struct PackedBlock {
     unsigned h[3];                 // the block's high bits: 4 (5 bits), 8 (6 bits) or 12 bytes (7 bits)
     unsigned d;                    // the block's scale as an fp16 pair (0 for a row past the chunk end)
 };
-// 8 bits: which half of a block row `row`'s lane holds in w[0 .. 3]: with the blocks rotated by the row, the 16-byte loads of eight lanes then
-// fall into eight different bank groups
-__device__ __forceinline__ unsigned half_swap(int row) { return (row >> 2) & 1; }
-// Blocks jr and 4 + jr (jr 0 .. 3) of row `row` of a staged tile. The row's eight scales come with one load: fetched one by one, 16 bytes
-// apart from lane to lane, they took four shared-memory cycles each, and shared memory is the scarcest pipe here (an unpack loop alone
-// takes 29 cycles a unit and scheduler, 26 of them its loads and stores).
-template <int BITS> __device__ __forceinline__ void dq_load(PackedBlock<BITS> & b0, PackedBlock<BITS> & b1, unsigned raw, int row, int jr, bool valid) {
-    const uint4 sc = lds128(raw + TILE_SC_OFF + row * SCALE_ROW);
-    const unsigned s0 = (jr & 2) ? sc.y : sc.x, s1 = (jr & 2) ? sc.w : sc.z, pick = (jr & 1) ? 0x3232u : 0x1010u;
-    b0.d = valid ? __byte_perm(s0, 0u, pick) : 0u;
-    b1.d = valid ? __byte_perm(s1, 0u, pick) : 0u;
-    const unsigned rp = raw + row * (32 * BITS);
-    PackedBlock<BITS> * const bs[2] = {&b0, &b1};
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        PackedBlock<BITS> & b = *bs[h];
-        const int jb = jr + 4 * h;
-        if constexpr (BITS == 8) { // (rows 256 bytes apart: lanes 4 .. 7 of eight start with the block's second 16 bytes, see half_swap)
-            const unsigned first = 16u * half_swap(row);
-            const uint4 v0 = lds128(rp + 32 * jb + first), v1 = lds128(rp + 32 * jb + (16u - first));
-            b.w[0] = v0.x, b.w[1] = v0.y, b.w[2] = v0.z, b.w[3] = v0.w, b.w[4] = v1.x, b.w[5] = v1.y, b.w[6] = v1.z, b.w[7] = v1.w;
-        } else {
-            const uint4 nv = lds128(rp + 16 * jb);
-            b.w[0] = nv.x, b.w[1] = nv.y, b.w[2] = nv.z, b.w[3] = nv.w;
-            if constexpr (BITS == 5) b.h[0] = lds32(rp + 128 + 4 * jb);
-            if constexpr (BITS == 6) {
-                const uint2 hw = lds64(rp + 128 + 8 * jb);
-                b.h[0] = hw.x, b.h[1] = hw.y;
-            }
-            if constexpr (BITS == 7) b.h[0] = lds32(rp + 128 + 12 * jb), b.h[1] = lds32(rp + 132 + 12 * jb), b.h[2] = lds32(rp + 136 + 12 * jb);
-        }
-    }
-}
-// row: the block's row (8 bits only)
-template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned dst, int row) {
+// the block's units in turn: put(u, four words of pairs), u 0 .. 3
+template <int BITS, class Put> __device__ __forceinline__ void block_units(const PackedBlock<BITS> & b, const UnpackConst & uc, Put && put) {
     const unsigned d = b.d;
     if constexpr (BITS == 8) {
         constexpr unsigned S8 = MAGIC_A + 0x00800080u;
-        const unsigned half[2] = {dst + half_swap(row) * 4096u, dst + 4096u - half_swap(row) * 4096u};
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const unsigned lo = b.w[2 * u] ^ 0x80808080u, hi = b.w[2 * u + 1] ^ 0x80808080u; // q + 128
-            sts128(half[u >> 1] + (u & 1) * 2048, pair_val<S8>(__byte_perm(lo, uc.a, 0x7270), d), // (value 0, value 2) under the exponent of 1024
-                   pair_val<S8>(__byte_perm(hi, uc.a, 0x7270), d),                 // (4, 6)
-                   pair_val<S8>(__byte_perm(lo, uc.a, 0x7371), d),                 // (1, 3)
-                   pair_val<S8>(__byte_perm(hi, uc.a, 0x7371), d));                // (5, 7)
+            put(u, pair_val<S8>(__byte_perm(lo, uc.a, 0x7270), d), // (value 0, value 2) under the exponent of 1024
+                pair_val<S8>(__byte_perm(hi, uc.a, 0x7270), d),    // (4, 6)
+                pair_val<S8>(__byte_perm(lo, uc.a, 0x7371), d),    // (1, 3)
+                pair_val<S8>(__byte_perm(hi, uc.a, 0x7371), d));   // (5, 7)
         }
     } else if constexpr (BITS == 4) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) unit_out<4>(dst + u * 2048, b.w[u], uc.a, uc.b, uc.a, uc.b, d);
+        for (int u = 0; u < 4; u++) unit_out<4>(u, b.w[u], uc.a, uc.b, uc.a, uc.b, d, put);
     } else if constexpr (BITS == 5) {
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             // bit k of the word's byte of high bits at 4 + k and 18 + k; the copy one lower serves the odd values
             const unsigned hb = __byte_perm(b.h[0], 0u, 0x4440 + u), t = hb * 0x00040010u, t1 = hb * 0x00020008u;
-            unit_out<5>(dst + u * 2048, b.w[u], and_or_imm<0x00100010u>(t, uc.a), and_or_imm<0x01000100u>(t, uc.b),
-                        and_or_imm<0x00100010u>(t1, uc.a), and_or_imm<0x01000100u>(t1, uc.b), d);
+            unit_out<5>(u, b.w[u], and_or_imm<0x00100010u>(t, uc.a), and_or_imm<0x01000100u>(t, uc.b), and_or_imm<0x00100010u>(t1, uc.a),
+                        and_or_imm<0x01000100u>(t1, uc.b), d, put);
         }
     } else if constexpr (BITS == 6) {
         const unsigned hw[4] = {b.h[0], b.h[0] >> 16, b.h[1], b.h[1] >> 16};
@@ -139,8 +106,8 @@ template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BI
         for (int u = 0; u < 4; u++) {
             // even values' 2-bit fields at bits 0, 4, 8, 12 of he, odd values' of ho: the gaps keep the shifted copies' sums apart
             const unsigned he = hw[u] & 0x3333u, ho = (hw[u] >> 2) & 0x3333u;
-            unit_out<6>(dst + u * 2048, b.w[u], and_or_imm<0x00300030u>(he * 0x00010010u, uc.a), and_or_imm<0x03000300u>(he * 0x00001001u, uc.b),
-                        and_or_imm<0x00300030u>(ho * 0x00010010u, uc.a), and_or_imm<0x03000300u>(ho * 0x00001001u, uc.b), d);
+            unit_out<6>(u, b.w[u], and_or_imm<0x00300030u>(he * 0x00010010u, uc.a), and_or_imm<0x03000300u>(he * 0x00001001u, uc.b),
+                        and_or_imm<0x00300030u>(ho * 0x00010010u, uc.a), and_or_imm<0x03000300u>(ho * 0x00001001u, uc.b), d, put);
         }
     } else { // 7 bits: every pair under the 1024 bias (pair_words7)
         const unsigned hw[4] = {b.h[0], __funnelshift_r(b.h[0], b.h[1], 24), __funnelshift_r(b.h[1], b.h[2], 16), b.h[2] >> 8}; // (bits above 23: not read)
@@ -149,16 +116,56 @@ template <int BITS> __device__ __forceinline__ void dq_emit(const PackedBlock<BI
         for (int u = 0; u < 4; u++) {
             unsigned x[4];
             pair_words7(b.w[u], hw[u], x);
-            sts128(dst + u * 2048, pair_val<S7>(x[0], d), pair_val<S7>(x[1], d), pair_val<S7>(x[2], d), pair_val<S7>(x[3], d));
+            put(u, pair_val<S7>(x[0], d), pair_val<S7>(x[1], d), pair_val<S7>(x[2], d), pair_val<S7>(x[3], d));
         }
     }
+}
+// 8 bits: which half of a block row `row`'s lane holds in w[0 .. 3]: the loads of eight lanes then fall into eight different bank groups
+__device__ __forceinline__ unsigned half_swap(int row) { return (row >> 2) & 1; }
+// packed bytes of block jb (0 .. 7) of row `row` of a staged tile
+template <int BITS> __device__ __forceinline__ void load_block(PackedBlock<BITS> & b, unsigned raw, int row, int jb) {
+    const unsigned rp = raw + row * (32 * BITS);
+    if constexpr (BITS == 8) { // (rows 256 bytes apart: lanes 4 .. 7 of eight start with the block's second 16 bytes, see half_swap)
+        const unsigned first = 16u * half_swap(row);
+        const uint4 v0 = lds128(rp + 32 * jb + first), v1 = lds128(rp + 32 * jb + (16u - first));
+        b.w[0] = v0.x, b.w[1] = v0.y, b.w[2] = v0.z, b.w[3] = v0.w, b.w[4] = v1.x, b.w[5] = v1.y, b.w[6] = v1.z, b.w[7] = v1.w;
+    } else {
+        const uint4 nv = lds128(rp + 16 * jb);
+        b.w[0] = nv.x, b.w[1] = nv.y, b.w[2] = nv.z, b.w[3] = nv.w;
+        if constexpr (BITS == 5) b.h[0] = lds32(rp + 128 + 4 * jb);
+        if constexpr (BITS == 6) {
+            const uint2 hw = lds64(rp + 128 + 8 * jb);
+            b.h[0] = hw.x, b.h[1] = hw.y;
+        }
+        if constexpr (BITS == 7) b.h[0] = lds32(rp + 128 + 12 * jb), b.h[1] = lds32(rp + 132 + 12 * jb), b.h[2] = lds32(rp + 136 + 12 * jb);
+    }
+}
+// the block's four units into shared memory: dst the thread's unit of the block's first dim group, the next ones 2048 bytes apart
+template <int BITS> __device__ __forceinline__ void store_block(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned dst, int row) {
+    const unsigned second = BITS == 8 ? half_swap(row) * 4096u : 0u; // (8 bits: the half of the block that w[0 .. 3] hold)
+    block_units<BITS>(b, uc, [&](int u, unsigned p0, unsigned p1, unsigned p2, unsigned p3) {
+        sts128(BITS == 8 ? dst + (u >> 1 ? 4096u - second : second) + (u & 1) * 2048 : dst + u * 2048, p0, p1, p2, p3);
+    });
+}
+
+// Blocks jr and 4 + jr (jr 0 .. 3) of row `row` of a staged tile. The row's eight scales come with one load: fetched one by one, 16 bytes
+// apart from lane to lane, they took four shared-memory cycles each, and shared memory is the scarcest pipe here (an unpack loop alone
+// takes 29 cycles a unit and scheduler, 26 of them its loads and stores).
+__device__ __forceinline__ uint4 row_scales(unsigned raw, int row) { return lds128(raw + TILE_SC_OFF + row * SCALE_ROW); }
+template <int BITS> __device__ __forceinline__ void dq_load(PackedBlock<BITS> & b0, PackedBlock<BITS> & b1, unsigned raw, int row, int jr, bool valid) {
+    const uint4 sc = row_scales(raw, row);
+    const unsigned s0 = (jr & 2) ? sc.y : sc.x, s1 = (jr & 2) ? sc.w : sc.z, pick = (jr & 1) ? 0x3232u : 0x1010u;
+    b0.d = valid ? __byte_perm(s0, 0u, pick) : 0u;
+    b1.d = valid ? __byte_perm(s1, 0u, pick) : 0u;
+    load_block<BITS>(b0, raw, row, jr);
+    load_block<BITS>(b1, raw, row, jr + 4);
 }
 // one block
 template <int BITS> __device__ __forceinline__ void dq_item(unsigned raw, int row, int jb, bool valid, unsigned dst) {
     PackedBlock<BITS> b0, b1;
     dq_load<BITS>(b0, b1, raw, row, jb & 3, valid);
-    if (jb < 4) dq_emit<BITS>(b0, unpack_const(), dst, row);
-    else dq_emit<BITS>(b1, unpack_const(), dst, row);
+    if (jb < 4) store_block<BITS>(b0, unpack_const(), dst, row);
+    else store_block<BITS>(b1, unpack_const(), dst, row);
 }
 } // namespace tc
 } // namespace mkkv
