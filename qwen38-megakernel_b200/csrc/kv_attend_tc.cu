@@ -45,6 +45,7 @@
 #include <math_constants.h>
 
 #include "kv_attend_tc_parts.cuh"
+#include "kv_plan.h"
 #include "kv_attend_tc_unpack.cuh"
 #include "kv_unpack.h"
 
@@ -1045,7 +1046,7 @@ cudaError_t launch_unpack_probe(int bits, const uint8_t * rows, const uint16_t *
 static_assert(sizeof(tc::Smem) + 128 <= 232448, "shared memory of one CTA");
 size_t attend_tc_smem_bytes() { return sizeof(tc::Smem) + 128; }
 // the kernel instance for a job's main formats: the served presets are compiled in, anything else runs the any-format instance
-typedef void (*TcKernel)(const tc::Args);
+using tc::TcKernel;
 static TcKernel tc_kernel_for(int kb, int vb, bool batch) {
     if (batch) {
         if (kb == 5 && vb == 6) return tc::attn_tc_kernel<5, 6, true>;
@@ -1075,6 +1076,8 @@ static cudaError_t tc_prepare() {
             e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) attend_tc_smem_bytes());
             if (e != cudaSuccess) return e;
         }
+        e = tc::ts_for_each([](TcKernel k, size_t smem) { return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem); });
+        if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
     return cudaSuccess;
@@ -1094,9 +1097,24 @@ cudaError_t preload_attend_tc() {
         const cudaError_t e = cudaFuncGetAttributes(&fa, (const void *) k);
         if (e != cudaSuccess) return e;
     }
-    return tc_prepare();
+    const cudaError_t e = tc::ts_for_each([](TcKernel k, size_t) {
+        cudaFuncAttributes attr;
+        return cudaFuncGetAttributes(&attr, (const void *) k);
+    });
+    return e != cudaSuccess ? e : tc_prepare();
 }
 
+// Which kernel: attn_ts_kernel (kv_attend_ts.cu) has the compiled-in low-bit pairs and wins where a CTA has work for a while; it starts slower, and of
+// q8_0 alone (8 layers of 60,000 positions, 8 tokens: 357 us against 396) attn_tc_kernel stays the faster.
+// Spread over the SMs (groups a CTA, of the context's end rounded up to 640 positions, so that T does not matter; us, attn_tc_kernel / attn_ts_kernel, per
+// layer): 5 groups (20,000 positions, K5r / V5, 5 tokens) 36.2 / 36.3, 6 (24,003, 4 tokens) 37.2 / 36.9, 9 (38,000, K5r / V6, 8) 52.5 / 48.4.
+// Item by item (groups of a CTA's items): 2 (3,000, K6 / V5, 5 tokens, one layer) 20.6 / 22.6, up to 3 (6 sequences of 442 .. 4,469) 29.9 / 30.8, 8 (20,011, 2 tokens,
+// one layer) 37.4 / 35.5, 17 (16 layers of 3,000, 2 tokens) 82.6 / 80.2, 20 sequences of 900 .. 12,000 (4 layers) 277 / 267.
+// Contexts whose chunks are one group (up to 2,560 positions) stay: there the layers' outputs are the same bits one by one and together.
+constexpr int TS_GROUPS_SPREAD = 6, TS_GROUPS_BATCH = 5;
+static TcKernel ts_long(int kb, int vb, bool batch, int groups) {
+    return groups >= (batch ? TS_GROUPS_BATCH : TS_GROUPS_SPREAD) ? tc::ts_kernel_for(kb, vb, batch) : nullptr;
+}
 cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, float2 * ml, int part_slots, unsigned long long * xa,
                              unsigned long long * xb, int nbmax, int epoch, int * status, cudaStream_t stream, const AttnTask * tasks_dev,
                              int ntasks, int tasks_B, float * raw_part, float2 * raw_ml, unsigned long long * prof, unsigned * done,
@@ -1139,7 +1157,10 @@ cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, flo
     a.done = fused ? done : nullptr;
     a.done_target = fused ? (*done_seq + 1u) * (unsigned) a.cph : 0u;
     void * args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *) tc_kernel_for(job.kv.s[0].bits, job.kv.s[1].bits, false), dim3(NKV * a.cph), dim3(tc::NTHREADS_SPREAD), args, attend_tc_smem_bytes(), stream);
+    const int kb = job.kv.s[0].bits, vb = job.kv.s[1].bits, groups = (plan_end(job) - job.pos_lo + tc::GP - 1) / tc::GP;
+    const TcKernel ts = ts_long(kb, vb, false, (groups + a.cph - 1) / a.cph), kern = ts ? ts : tc_kernel_for(kb, vb, false);
+    e = cudaLaunchCooperativeKernel((const void *) kern, dim3(NKV * a.cph), dim3(ts ? tc::TS_THREADS_SPREAD : tc::NTHREADS_SPREAD), args,
+                                    ts ? tc::ts_smem_bytes() : attend_tc_smem_bytes(), stream);
     if (e != cudaSuccess) return e;
     if (fused) {
         *done_seq += 1u;
@@ -1184,7 +1205,6 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     cudaError_t e = tc_prepare();
     if (e != cudaSuccess) return e;
     // (the jobs of one batch may differ in format: the any-format instance unless they all share a compiled-in pair)
-    const TcKernel kern = one_format ? tc_kernel_for(first.kv.s[0].bits, first.kv.s[1].bits, true) : tc::attn_tc_kernel<0, 0, true>;
     // The prologue beside the launch before saves 2 .. 3 us a launch, which counts where a CTA's work is short (us, without / with): 16
     // layers of 700 positions 30.9 / 28.8, of 2,000 51.0 / 47.6, of 4,000 84.9 / 81.5, 6 sequences in 16 layers 520 / 486. Long steps gain the
     // same 2 us (16 layers of 24,000 298.7 / 296.4, of 101,600 1,104.6 / 1,101.7), but a batch of 32 sequences in 4 layers lost 11 (2,350 / 2,361): the
@@ -1192,7 +1212,10 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     // that differ, the first and longest one's chunk length stands for all. The merge's blocks waiting beside the attention cost more than
     // they gain as soon as CTAs have more than one item (an earlier build: 102 -> 111 us for 16 layers of 4,000 positions).
     const int grid = std::min(nitems, num_sms), per_cta = (nitems + grid - 1) / grid * std::max(first.cpi, 1) * ((first.cs / ATP + tc::GT - 1) / tc::GT);
-    e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(tc::NTHREADS), attend_tc_smem_bytes(), stream, a);
+    const int kb = first.kv.s[0].bits, vb = first.kv.s[1].bits;
+    const TcKernel ts = one_format && first.cs > tc::GP ? ts_long(kb, vb, true, per_cta) : nullptr;
+    const TcKernel kern = ts ? ts : one_format ? tc_kernel_for(kb, vb, true) : tc::attn_tc_kernel<0, 0, true>;
+    e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(ts ? tc::TS_THREADS_BATCH : tc::NTHREADS), ts ? tc::ts_smem_bytes() : attend_tc_smem_bytes(), stream, a);
     if (e != cudaSuccess) return e;
     return launch_merge(jobs_dev, &first, njobs, max_T, part, ml, stream, raw_part, raw_ml, true, nitems <= num_sms);
 }

@@ -167,5 +167,61 @@ template <int BITS> __device__ __forceinline__ void dq_item(unsigned raw, int ro
     if (jb < 4) store_block<BITS>(b0, unpack_const(), dst, row);
     else store_block<BITS>(b1, unpack_const(), dst, row);
 }
+
+// ---- for the kernel whose K operand lies in tensor memory (kv_attend_ts.cu) ----
+// The scales of blocks jr (of pair x, y: the row's first four, of z, w: its last four) as fp16 pairs: one byte permute, by a selector that a warp keeps
+__device__ __forceinline__ unsigned scale_pick(int jr) { return 0x1010u + 0x2222u * (unsigned) jr; }
+// ---- V: the warps of a tile cover the four 32-dim blocks of a half, and which of them a lane takes rotates with the row, so that the
+// 16-byte loads of 8 consecutive lanes (rows 32 bits bytes apart) fall into 8 different bank groups ----
+template <int BITS> __device__ __forceinline__ int v_rotation(int row) { return row >> (BITS == 6 ? 1 : (BITS == 5 || BITS == 7) ? 2 : 0); }
+// ---- K: a tensor-memory store writes the same columns of every lane, so all lanes of a warp take the same two blocks 2 c2, 2 c2 + 1
+// of half h. Rows that meet in a bank group load the two blocks (8 bits: the pair's four 16-byte pieces) in another order ----
+template <int BITS> __device__ __forceinline__ void load_pair(PackedBlock<BITS> & b0, PackedBlock<BITS> & b1, unsigned raw, int row, int c2, int h) {
+    const unsigned rp = raw + row * (32 * BITS);
+    if constexpr (BITS == 8) {
+        const unsigned at = rp + 128 * h + 64 * c2;
+        uint4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = lds128(at + 16 * ((i + row) & 3)); // piece p is v[(p - row) & 3]
+        auto sel = [](bool c, const uint4 & a, const uint4 & b) { return make_uint4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w); };
+        const bool r1 = row & 1, r2 = row & 2;
+        const uint4 x0 = sel(r1, v[3], v[0]), x1 = sel(r1, v[0], v[1]), x2 = sel(r1, v[1], v[2]), x3 = sel(r1, v[2], v[3]);
+        const uint4 p0 = sel(r2, x2, x0), p1 = sel(r2, x3, x1), p2 = sel(r2, x0, x2), p3 = sel(r2, x1, x3);
+        b0.w[0] = p0.x, b0.w[1] = p0.y, b0.w[2] = p0.z, b0.w[3] = p0.w, b0.w[4] = p1.x, b0.w[5] = p1.y, b0.w[6] = p1.z, b0.w[7] = p1.w;
+        b1.w[0] = p2.x, b1.w[1] = p2.y, b1.w[2] = p2.z, b1.w[3] = p2.w, b1.w[4] = p3.x, b1.w[5] = p3.y, b1.w[6] = p3.z, b1.w[7] = p3.w;
+    } else {
+        const bool swap = (row >> (BITS == 6 ? 1 : BITS == 4 ? 0 : 2)) & 1;
+        const unsigned at = rp + 64 * h + 32 * c2, first = swap ? 16u : 0u;
+        const uint4 v0 = lds128(at + first), v1 = lds128(at + (16u - first));
+        b0.w[0] = swap ? v1.x : v0.x, b0.w[1] = swap ? v1.y : v0.y, b0.w[2] = swap ? v1.z : v0.z, b0.w[3] = swap ? v1.w : v0.w;
+        b1.w[0] = swap ? v0.x : v1.x, b1.w[1] = swap ? v0.y : v1.y, b1.w[2] = swap ? v0.z : v1.z, b1.w[3] = swap ? v0.w : v1.w;
+        const int pair = 2 * h + c2;
+        if constexpr (BITS == 5) {
+            const uint2 hw = lds64(rp + 128 + 8 * pair);
+            b0.h[0] = hw.x, b1.h[0] = hw.y;
+        }
+        if constexpr (BITS == 6) {
+            const uint4 hw = lds128(rp + 128 + 16 * pair);
+            b0.h[0] = hw.x, b0.h[1] = hw.y, b1.h[0] = hw.z, b1.h[1] = hw.w;
+        }
+        if constexpr (BITS == 7) {
+            const uint2 x = lds64(rp + 128 + 24 * pair), y = lds64(rp + 136 + 24 * pair), z = lds64(rp + 144 + 24 * pair);
+            b0.h[0] = x.x, b0.h[1] = x.y, b0.h[2] = y.x, b1.h[0] = y.y, b1.h[1] = z.x, b1.h[2] = z.y;
+        }
+    }
+}
+// 16 columns of every lane
+__device__ __forceinline__ void tmem_st16(unsigned taddr, const unsigned (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
+                 "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+// one block's 32 values of every lane's row into 16 columns of its tensor-memory lane
+template <int BITS> __device__ __forceinline__ void block_to_tmem(const PackedBlock<BITS> & b, const UnpackConst & uc, unsigned taddr) {
+    unsigned r[16];
+    block_units<BITS>(b, uc, [&](int u, unsigned p0, unsigned p1, unsigned p2, unsigned p3) { r[4 * u] = p0, r[4 * u + 1] = p1, r[4 * u + 2] = p2, r[4 * u + 3] = p3; });
+    tmem_st16(taddr, r);
+}
 } // namespace tc
 } // namespace mkkv

@@ -1,0 +1,1082 @@
+// The tensor-core decode attention for long contexts in the low-bit formats: the arithmetic, the modes, the records and the merge are those of
+// attn_tc_kernel (kv_attend_tc.cu); what differs is where operands and scores lie and which warps wait for one another.
+//   - K's operand lies in tensor memory: its 8 unpack warps write a position's fp16(d q) into the position's lane (tcgen05.st, 16 columns a
+//     block), and S^T[128 positions x 48 rows] = K Q^T takes it from there (Q, K-major, is the B operand). That is 128 KB less through shared
+//     memory a group, no proxy fence, and 26 cycles an instruction instead of the 68 of M = 64, N = 128.
+//   - K and V have unpack warps, raw slots, operand slots, a producer and an issuer of their own; neither side waits for the other. A warp
+//     unpacks a quarter of a tile's side (2 blocks of either half) instead of an eighth of both sides: half the waits and hand-overs.
+//   - S^T has positions on lanes, so a softmax thread owns a position and 24 of the query rows (8 warps: tile q, half of the rows). A row's tile maximum is
+//     one redux.sync; what belongs to a row (running and reference max, factors) is computed by the thread lane = row from the four tiles' maxima
+//     and read back by all. P is the B operand of P V with rows contiguous.
+// What bounds it: the softmax warps (5,000 of a group's 5,400 cycles busy at 8 tokens, 4,400 at 1, in a chain of short steps), V's unpack warps
+// (4,300 .. 4,700) and behind both the instruction cache, 32 KB: straight code of 32 KB and more runs at a third of the rate (3.1 cycles an
+// instruction and warp against 1.07 below), and the first form of this kernel, with both halves of a side, all waits with their clocks and 48 rows
+// in a softmax warp unrolled, missed it in 44 % of its requests (1,050 lines a group) and took 1,643 us for the step below; with loops over the halves, waits of five
+// instructions and 24 rows a warp 6 % are missed. Hence what looks like thrift: one body for both halves, one for both sides of 8-bit tiles,
+// issue loops unrolled twice, one place for every wait.
+// Measured against attn_tc_kernel (us): 16 layers of 101,600 positions, K5r / V6, 8 tokens 1,076 -> 967, 1 token 1,045 -> 926; 8 layers K5r / V5, 8
+// tokens 593 -> 545, K6 / V5 600 -> 580; one layer of 38,000, 8 tokens, 52.5 -> 48.4. It starts slower (a side's tile has 8 warps, not 16): see
+// the rules at ts_long.
+#include <cuda_fp16.h>
+#include <math_constants.h>
+
+#include "kv_attend_tc_parts.cuh"
+#include "kv_attend_tc_unpack.cuh"
+#include "kv_unpack.h"
+
+namespace mkkv {
+namespace tc {
+namespace ts {
+
+constexpr int RS = AR / 2;     // softmax warps first: warp 4 c + q, tile q of a group (tensor-memory lanes 32 q ..) and query rows RS c .. + RS - 1
+constexpr int NSOFT = 8;
+constexpr int NDQ = 16;        // then the unpack warps: 8 c2 + 4 side + q: side (0 K, 1 V) of tile q, blocks 2 c2 and 2 c2 + 1 of each 128-dim half
+constexpr int NSIDE = NDQ / 2; // unpack warps of a side
+// then the control warps: a producer and an issuer for either side of the pipeline, which share nothing but the groups' records
+constexpr int W_CTL = NSOFT + NDQ, W_KPROD = W_CTL, W_VPROD = W_CTL + 1, W_SISSUE = W_CTL + 2, W_OISSUE = W_CTL + 3;
+constexpr int W_MAX = W_CTL + 4;      // spread mode only: four warps that take the tile maxima and exchange the running maxima
+constexpr int NTHREADS = TS_THREADS_BATCH, NTHREADS_SPREAD = TS_THREADS_SPREAD;
+static_assert(NTHREADS == W_MAX * 32 && NTHREADS_SPREAD == (W_MAX + 4) * 32, "warps");
+// registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
+// most the CTA's launch allocation -- a larger sum faults)
+#define MKKV_TC_REGS_SOFT "112"
+#define MKKV_TC_REGS_DQ "56"
+#define MKKV_TC_REGS_CTL "56"
+static_assert(NTHREADS == 896 && 8 * 112 + 16 * 56 + 4 * 56 <= 28 * 72, "register shares");
+#define MKKV_TC_REGS_SOFT_SPREAD "88"
+#define MKKV_TC_REGS_CTL_SPREAD "56"
+#define MKKV_TC_REGS_MAX "56"
+static_assert(NTHREADS_SPREAD == 1024 && 8 * 88 + 16 * 56 + 4 * 56 + 4 * 56 <= 32 * 64, "register shares");
+constexpr int TROWS = RS + 32;              // (a warp's lanes reach beyond the last row)
+constexpr int RAW_SLOT = ATP * HD + ATP * SCALE_ROW; // one tile of the widest format and its scales: 8704 bytes
+constexpr int OP_SLOT = GP * 128 * 2;       // V's fp16 operand: 128 positions x 128 dims
+constexpr int NOP = 3;
+constexpr int NKS = 2;                      // K's operand slots in tensor memory: 128 positions (lanes) x 128 dims (64 columns)
+constexpr int NSB = 4;                      // S buffers: S runs up to NSB groups ahead of P
+constexpr int NTASK = 16;
+constexpr int Q_BYTES = AR * HD * 2;
+constexpr int P_PART = AR * GP * 2;         // P's high part, then its low part: [row group 6][position group 16][8 positions][8 rows]
+constexpr int P_ROWGROUP = GP * 16;
+// An S buffer is 48 columns (query rows), positions on lanes. An accumulator half is 48 columns for P's high part and 48 for its low part.
+constexpr unsigned S_COL = 0, K_COL = S_COL + NSB * AR, K_STRIDE = 64, O_COL0 = K_COL + NKS * K_STRIDE, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512;
+static_assert(O_COL1 + 2 * AR <= TMEM_COLS, "tensor-memory columns");
+static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
+// A group's task record as K's producer leaves it for the other roles. The fields behind AttnTask serve the batch mode, where one CTA works for
+// several (job, kv head) pairs in turn: a segment is a run of chunks of one pair, with its own queries, partial and row sums.
+struct alignas(16) GroupRec : AttnTask {
+    const uint16_t * q;       // the segment's staged queries
+    int n, T;                 // of the segment's job
+    alignas(16) int flags;    // what the softmax warps need for every group, in one load: REC_* and, from bit REC_RESTART on, a bit per tile: the tile opens a
+    int slot, rows;           // chunk, the running max starts anew; the partial's slot; 6 T
+};
+// What the unpack warps need of one side of one tile: rows that are there | UD_END in the CTA's last group | bits of the rows << 8
+constexpr unsigned UD_ROWS = 0x3fu, UD_END = 0x80u;
+constexpr int REC_FIRST = 1, REC_LAST = 2, REC_END = 4; // first / last group of its segment, last group of the CTA
+constexpr int REC_MASK = 8, REC_RESTART = 8;             // the group reaches the chunk's end or the new tokens: some scores are masked; see flags
+struct Smem {
+    uint8_t op[NOP][OP_SLOT];   // V: [dim group 16][position group 16][8 positions][8 dims] fp16
+    uint8_t raw[2][GT][RAW_SLOT]; // packed tiles of K and of V, a slot per tile of a group
+    uint8_t q[Q_BYTES];         // [dim group 32][row group 6][8 rows][8 dims]
+    uint8_t p[2][P_PART];       // high part, low part: [row group 6][position group 16][8 positions][8 rows]
+    unsigned tmem_base;
+    int merge_ok;               // the tail's merge: the head's CTAs have all arrived
+    WaitCtl wc;                 // the launch's wait limits; dead: a wait of this CTA gave up, no later wait blocks
+    GroupRec tasks[NTASK];      // the CTA's groups as K's producer reaches them, by group % NTASK (no role is that far from it: its group j + 1
+                                // is fetched when K(j) has been read, which is behind S(j - 3), which is behind the softmax of j - 3 - NSB)
+    uint64_t raw_full[2][GT], raw_empty[2][GT], k_full[NKS], k_empty[NKS], op_full[NOP], op_empty[NOP], s_full[NSB], s_empty[NSB], p_full, p_empty, q_ready, fin[2];
+    AttnJob job;
+    unsigned udesc[NTASK][2][GT]; // K / V tiles of a group, by group % NTASK (see UD_ROWS)
+    TileSrc vsrc[NTASK][GT];    // the V tiles of the groups whose K has been fetched
+    uint64_t rec_full[NTASK];   // record (group % NTASK) is written
+    alignas(16) float tmax[NSB][GT][TROWS]; // row maxima of a group's tiles, by group % NSB
+    struct alignas(16) {        // what a softmax warp's threads (a position each) need of the rows of its tile: minus the running max, exp(running max -
+        float nm[32], beta[32], f[32]; // reference), the factor of a reference max that moved,
+        uint16_t bh[32], bl[32];       // and beta as two fp16 parts
+    } row[NSOFT];
+    float lsum[GT][AR];         // a finished segment's row sums over a warp's positions
+    // spread mode only
+    float m_in[NSB][TROWS];        // the running max before a group, by group % NSB
+    uint64_t m_full[NSB];
+};
+
+// Waits for a phase of an mbarrier. A try suspends the thread in hardware (it wakes when the phase completes, or after a time of the hardware's
+// choosing), so waiting warps take next to no issue slots. Every wait is bounded: K's producer warp, which waits for someone as long as the
+// CTA has work (watched_wait), measures its waits, and after the limit (hint x rounds nanoseconds, multiplied on the host) sets the status word
+// and the CTA's `dead` flag; from then on no wait of this CTA blocks, and the kernel runs to its end. The other warps' waits only look at the
+// flag: this code stands at some twenty places of the hot loops, and what bounds these is the instruction cache.
+// Returns whether the phase is complete.
+__device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, const volatile WaitCtl * wc) {
+    while (!mbar_try_wait(bar, parity))
+        if (wc->dead) return false;
+    return true;
+}
+// The same for a warp whose lanes must agree on the result: whether every lane's wait succeeded. (Warp-wide instructions that stand behind a
+// wait whatever its result need no such vote; a __syncwarp before each of them cost 16 calls of 24,003 positions 1.3 %.)
+__device__ __forceinline__ bool tc_wait_all(uint64_t * bar, unsigned parity, const volatile WaitCtl * wc) {
+    return __all_sync(FULL_MASK, tc_wait(bar, parity, wc)) != 0;
+}
+__device__ __forceinline__ void watched_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
+    if (mbar_test_wait(bar, parity)) return;
+    const unsigned long long limit = wc->limit, t0 = globaltimer_ns();
+    do {
+        if (wc->dead) return;
+        if (globaltimer_ns() - t0 >= limit) {
+            wc->dead = 1;
+            atomicExch(status, (int) KS_WAIT_TIMEOUT);
+            return;
+        }
+    } while (!mbar_try_wait(bar, parity));
+}
+// The last copy of a producer lane must land before the CTA's shared memory is released, also when a consumer gives up after the producer
+// has fetched everything and left its loop. Only the lane's last turn can be in flight (the one before it was waited for before the slot
+// was filled again). Bounded; in a normal run the producer has nothing else to do and every copy lands.
+struct LastCopy {
+    unsigned parity = 0u;
+    bool any = false; // (a turn without rows copies nothing)
+};
+__device__ __forceinline__ void drain_copy(uint64_t * raw_full, const LastCopy & c) {
+    if (c.any) wait_landed(raw_full, c.parity);
+}
+
+// ---- tcgen05 ----
+// Shared-memory matrix descriptors (no swizzle, version 1), as their 32-bit halves: the low half holds the start address and the
+// byte distance between the two 8-element groups along K of one instruction ("leading"), the high half the distance between 8-row
+// groups along M / N ("stride"). Only the low half changes between k-steps.
+// fp16 operands, fp32 accumulate. S^T[128 positions x 48 query rows] = K Q^T: K in tensor memory, Q K-major; O^T[128 dims x 96] += V^T P^T:
+// both MN-major, P as 48 rows' high parts, then their low parts
+constexpr unsigned IDESC_S = (1u << 4) | ((unsigned) (AR / 8) << 17) | ((unsigned) (GP / 16) << 24);
+constexpr unsigned IDESC_PV = (1u << 4) | (1u << 15) | (1u << 16) | ((unsigned) (2 * AR / 8) << 17) | ((unsigned) (128 / 16) << 24);
+__device__ __forceinline__ void umma_ta(unsigned d_tmem, unsigned a_tmem, unsigned b_lo, unsigned b_hi, unsigned idesc, unsigned accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tmov.b64 db, {%2, %3};\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The scores of RS query rows (columns from taddr on) of the thread's position. (One statement with its wait: no use of the registers can move
+// between the two.)
+__device__ __forceinline__ void tmem_scores(unsigned taddr, float (&s)[RS]) {
+    unsigned r[RS];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%24];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%25];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23])
+                 : "r"(taddr), "r"(taddr + 16)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < RS; i++) s[i] = __uint_as_float(r[i]);
+}
+// 8 consecutive columns at each of two addresses
+__device__ __forceinline__ void tmem_ld8_two(unsigned ta, unsigned tb, unsigned (&v)[8], unsigned (&w)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n\t"
+                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "r"(ta), "r"(tb)
+                 : "memory");
+}
+// maximum over the warp's lanes, in all of them
+__device__ __forceinline__ float warp_max(float x) {
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+// by the lane with `lane` 0, under a predicate (see warp_arrive)
+__device__ __forceinline__ void lane0_sts128(unsigned addr, int lane, float a, float b, float c, float d) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %5, 0;\n\t@p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(lane)
+                 : "memory");
+}
+__device__ __forceinline__ TileSrc tile_source(const SideSrc & S, int tb, int c1) {
+    TileSrc t;
+    t.np = min(ATP, c1 - tb);
+    if (tb >= S.ring0) { // rc is a multiple of 32: a tile never wraps
+        const int r = tb % S.rc;
+        t.val = S.rval + (size_t) r * HD;
+        t.sc = S.rsc + (size_t) r * 8;
+        t.rb = HD;
+    } else {
+        t.val = S.mval + (ptrdiff_t) tb * S.rb;
+        t.sc = S.msc + (ptrdiff_t) tb * 8;
+        t.rb = S.rb;
+    }
+    return t;
+}
+// One side of group j into its raw slots: lanes 0 .. 3 a tile each, t for the first nt of them. A whole producer warp calls this; false: the
+// CTA has given up (nothing is fetched into a slot that may still be read, no barrier is over-subscribed).
+__device__ __forceinline__ bool fetch_tile(Smem & sm, const Args & a, int side, int j, int nt, const TileSrc & t, int lane, LastCopy & last) {
+    if (lane < GT && j > 0) {
+        if (side) tc_wait(&sm.raw_empty[side][lane], (j - 1) & 1, &sm.wc);
+        else watched_wait(&sm.raw_empty[side][lane], (j - 1) & 1, &sm.wc, a.status);
+    }
+    if (gave_up(FULL_MASK, &sm.wc)) return false;
+    if (lane < GT) {
+        uint64_t * full = &sm.raw_full[side][lane];
+        last.any = lane < nt, last.parity = j & 1;
+        if (lane < nt) issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[side][lane], full);
+        else mbar_arrive(full);
+    }
+    __syncwarp();
+    return true;
+}
+// lanes 0 .. 7 of K's producer: one side (the lane's src) of one tile of group j described for the other roles, V's source among them
+__device__ __forceinline__ TileSrc describe_tile(Smem & sm, int j, const SideSrc & src, int side, int tile, int tb, int nt, int c1, unsigned last, int lane) {
+    TileSrc t;
+    if (lane < 2 * GT) {
+        unsigned d = last | (unsigned) src.bits << 8; // (no row: any of the side's formats)
+        if (tile < nt) {
+            t = tile_source(src, tb, c1);
+            if (side) sm.vsrc[j % NTASK][tile] = t;
+            d = last | (unsigned) t.np | ((unsigned) t.rb << 3); // (32 bytes a row and bit: the bits 8 up)
+        }
+        sm.udesc[j % NTASK][side][tile] = d;
+    }
+    return t;
+}
+// K's producer has fetched everything: it watches over the rest (both issuers' last commits stand behind every other wait of the CTA)
+__device__ __forceinline__ void watch_end(Smem & sm, const Args & a, int lane) {
+    if (lane == 0) {
+        watched_wait(&sm.fin[0], 0u, &sm.wc, a.status);
+        watched_wait(&sm.fin[1], 0u, &sm.wc, a.status);
+    }
+}
+// V's producer warp, either mode
+__device__ __forceinline__ void v_producer(Smem & sm, const Args & a, int G, int lane) {
+    LastCopy last_copy;
+    for (int j = 0; j < G; j++) {
+        tc_wait(&sm.rec_full[j % NTASK], (j / NTASK) & 1, &sm.wc);
+        if (gave_up(FULL_MASK, &sm.wc)) break; // (the record may not be written)
+        const int nt = sm.tasks[j % NTASK].nt;
+        const bool end = (sm.tasks[j % NTASK].flags & REC_END) != 0;
+        TileSrc t;
+        if (lane < nt) t = sm.vsrc[j % NTASK][lane];
+        if (!fetch_tile(sm, a, 1, j, nt, t, lane, last_copy) || end) break;
+    }
+    if (lane < GT) drain_copy(&sm.raw_full[1][lane], last_copy);
+}
+
+// ---- batch mode: K's producer warp ----
+// Walks the CTA's segments and their groups, fetches K and leaves every group's record before it; lanes 0 .. 3 fetch one tile of the group
+// each. V's producer follows the records. An item is a run of cpi chunks of one
+// kv head of one job and makes one segment and one partial (slot: the job's item0 + g nch + run). Items come in descending order of
+// length (jobs longest first; jobs of one shape: run by run, the clipped runs at the ends of the range last): CTA b starts with item b
+// and takes the next one from a counter whenever it starts one, so that the number is there when the item's last record is written.
+// (Dealt in a fixed snake order instead, 32 sequences of 3,063 .. 83,693 positions left the busiest CTA 7 % above the mean.) What an item
+// computes does not depend on which CTA runs it or on the jobs beside it.
+__device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int lane) {
+    const int grid = (int) gridDim.x;
+    int next_item = (int) blockIdx.x, pending = a.nitems; // (pending: lane 0's)
+    // current segment: positions [first_pos, end) of one kv head, a run of chunks; the current group starts at pos
+    const AttnJob * const jobs = a.jobs ? a.jobs : &a.one;
+    const AttnJob * const J = a.jobs ? &sm.job : &a.one; // (a job of the table is copied: field after field would be one trip to the L2 after another)
+    int which = -1;
+    int g = 0, first_pos = 0, pos = 0, end = 0, slot = 0;
+    auto use_job = [&](int j) {
+        if (a.jobs && j != which) {
+            __syncwarp();
+            for (int i = lane; i < (int) (sizeof(AttnJob) / 4); i += 32) reinterpret_cast<unsigned *>(&sm.job)[i] = reinterpret_cast<const unsigned *>(jobs + j)[i];
+            __syncwarp();
+            which = j;
+        }
+    };
+    auto next_segment = [&]() {
+        const int item = next_item;
+        if (a.nitems > grid && lane == 0) pending = grid + (int) atomicAdd(a.next, 1u);
+        int cpi, run;
+        if (a.uniform) {
+            const int heads = a.njobs * NKV, k = item / heads, hh = item - k * heads;
+            use_job(hh / NKV);
+            g = hh % NKV;
+            cpi = max(a.one.cpi, 1);
+            const int nit = (a.one.nch + cpi - 1) / cpi;
+            run = batch_run(a.one, cpi, nit, k);
+        } else {
+            int below = 0; // jobs whose first item is <= item (titem0 ascends): the last of them owns it
+            for (int j0 = 0; j0 < a.njobs; j0 += 32) {
+                const unsigned m = __ballot_sync(FULL_MASK, j0 + lane < a.njobs && jobs[j0 + lane].titem0 <= item);
+                below += __popc(m);
+                if (m != FULL_MASK) break;
+            }
+            use_job(below - 1);
+            cpi = max(J->cpi, 1);
+            const int nit = (J->nch + cpi - 1) / cpi, rel = item - J->titem0;
+            g = rel / nit;
+            run = rel - g * nit;
+        }
+        const int c = J->c_lo + run * cpi;
+        first_pos = pos = max(c * J->cs, J->pos_lo);
+        end = min(min(c + cpi, J->c_lo + J->nch) * J->cs, J->pos_hi);
+        slot = J->item0 + g * J->nch + run;
+    };
+    // A single job comes with the launch's arguments: its first record and addresses are made while the launch before still runs, and
+    // the wait for that launch stands before the first copy. (One call of 1,700 positions, 8 tokens: 24.1 .. 24.6 us with all of it
+    // behind the wait, 22.6 so.) A table of jobs and the items' counter are that launch's work.
+    bool waiting = !a.jobs, fresh = true;
+    if (!waiting) wait_previous();
+    SideSrc src; // of the lane's side
+    int chunk, n, T;
+    const uint16_t * qp;
+    LastCopy last_copy;
+    const int side = (lane >> 2) & 1, tile = lane & 3; // lanes 0 .. 3: K's tiles, 4 .. 7: V's
+    for (int nk = 0;; nk++) {
+        if (fresh) {
+            next_segment();
+            src = make_src(J->kv, side, g, J->ws);
+            chunk = J->cs, n = J->n, T = J->T;
+            qp = J->Qp + (size_t) g * (QP_HEAD_BYTES / 2);
+        }
+        const int pos0 = pos, c1 = end, mine = pos0 + tile * ATP; // (the tiles of a run are consecutive, also across its chunks' bounds)
+        const int nt = min(GT, (c1 - pos0 + ATP - 1) / ATP);
+        const bool seg_last = c1 - pos0 <= GP;
+        const unsigned restart = __ballot_sync(FULL_MASK, lane < nt && (mine == first_pos || mine % chunk == 0));
+        if (seg_last) next_item = __shfl_sync(FULL_MASK, pending, 0);
+        const bool cta_last = seg_last && next_item >= a.nitems;
+        if (lane == 0) {
+            GroupRec & k = sm.tasks[nk % NTASK];
+            k.pos0 = pos0, k.c1 = c1, k.nt = nt;
+            k.q = qp;
+            k.n = n, k.T = T, k.slot = slot, k.rows = GQ * T;
+            k.flags = (pos0 == first_pos ? REC_FIRST : 0) | (seg_last ? REC_LAST : 0) | (cta_last ? REC_END : 0) | (pos0 + GP > min(c1, n + 1) ? REC_MASK : 0) |
+                      (int) (restart << REC_RESTART);
+        }
+        const TileSrc t = describe_tile(sm, nk, src, side, tile, mine, nt, c1, cta_last ? UD_END : 0u, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.rec_full[nk % NTASK]);
+        if (waiting) wait_previous(), waiting = false;
+        if (!fetch_tile(sm, a, 0, nk, nt, t, lane, last_copy)) break;
+        if (cta_last) break;
+        fresh = seg_last;
+        pos += GP;
+    }
+    watch_end(sm, a, lane);
+    if (lane < GT) drain_copy(&sm.raw_full[0][lane], last_copy);
+}
+
+// ---- scores: a thread owns one position (tile q of the group, lane) and RS query rows from row0 on ----
+// A row is token r % T and sees positions <= n + r % T; nothing is visible past the chunk end. For almost every group the answer is "all of
+// it" (REC_MASK is not set). Rows beyond the job's 6 T need no mask: their queries are zero, so are their scores, and no one reads what becomes
+// of them.
+__device__ __forceinline__ void mask_scores(const GroupRec & k, int n, int T, int q, int row0, int lane, float (&s)[RS]) {
+    const int pos = k.pos0 + ATP * q + lane, late = pos >= k.c1 ? MAXT : pos - n; // tokens before `late` do not see the position
+    int t = row0 % T;
+#pragma unroll
+    for (int r = 0; r < RS; r++) {
+        if (t < late) s[r] = -CUDART_INF_F;
+        if (++t == T) t = 0;
+    }
+}
+// maxima of the tile's rows (the first `rows` of the RS, in whole groups of eight) into out
+__device__ __forceinline__ void tile_maxima(const float (&s)[RS], int rows, int lane, float * out) {
+    const unsigned dst = smem_u32(out);
+#pragma unroll
+    for (int b = 0; b < RS / 8; b++)
+        if (8 * b < rows) {
+            float m[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) m[i] = warp_max(s[8 * b + i]);
+            lane0_sts128(dst + 32 * b, lane, m[0], m[1], m[2], m[3]);
+            lane0_sts128(dst + 32 * b + 16, lane, m[4], m[5], m[6], m[7]);
+        }
+}
+
+// KB / VB: the bits of the K / V main rows the instance is compiled for (0: any, decided per tile at run time). A compiled-in
+// format leaves two unpack bodies per side (the format and the q8_0 ring) instead of five: a smaller instruction footprint.
+// BATCH: the instance for several jobs (persistent CTAs over runs of chunks, no exchange between CTAs); the instance for one
+// job spread over the SMs carries none of that mode's code (with both modes in one body the spread mode's loops came out 1.7 %
+// slower).
+template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? NTHREADS : NTHREADS_SPREAD, 1) attn_ts_kernel(const __grid_constant__ Args a) {
+    // (the dynamic shared memory starts on a 128-byte boundary -- there is no static shared memory in this kernel --, which is all the
+    // bulk copies, matrix descriptors and barriers need; no pointer arithmetic here, so every access below is a shared-space one)
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    Smem & sm = *reinterpret_cast<Smem *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#if MKKV_TC_PROF
+    const unsigned long long t_entry = globaltimer_ns();
+#endif
+    if (!BATCH) {
+        const unsigned * src = reinterpret_cast<const unsigned *>(&a.one);
+        unsigned * dst = reinterpret_cast<unsigned *>(&sm.job);
+        for (int i = tid; i < (int) (sizeof(AttnJob) / 4); i += NTHREADS_SPREAD) dst[i] = src[i];
+    }
+    if (tid == 0) {
+        for (int s = 0; s < 2 * GT; s++) { mbar_init(&sm.raw_full[s / GT][s % GT], 1); mbar_init(&sm.raw_empty[s / GT][s % GT], NSIDE / GT); }
+        for (int s = 0; s < NKS; s++) { mbar_init(&sm.k_full[s], NSIDE); mbar_init(&sm.k_empty[s], 1); }
+        for (int s = 0; s < NOP; s++) { mbar_init(&sm.op_full[s], NSIDE); mbar_init(&sm.op_empty[s], 1); }
+        for (int s = 0; s < NSB; s++) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.s_empty[s], BATCH ? NSOFT : NSOFT + 4); mbar_init(&sm.m_full[s], 4); }
+        mbar_init(&sm.p_full, NSOFT);
+        mbar_init(&sm.p_empty, 1);
+        for (int s = 0; s < 2; s++) mbar_init(&sm.fin[s], 1);
+        mbar_init(&sm.q_ready, 1);
+        for (int s = 0; s < NTASK; s++) mbar_init(&sm.rec_full[s], 1);
+        sm.wc.dead = 0;
+        sm.wc.limit = a.wait_limit_ns;
+        sm.wc.poll = a.poll_rounds;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == W_SISSUE) { // tensor memory: S buffers, K's operand slots, O^T in two halves
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sm.tmem_base)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    if (BATCH) { // (the prologue above ran beside the launch before this one; every CTA of this launch is resident: at most one per SM)
+        release_next();
+        if (warp != W_KPROD) wait_previous(); // (K's producer warp: batch_producer)
+    }
+    const unsigned tb = sm.tmem_base;
+    const AttnJob & J = sm.job;
+    const KvView & kv = J.kv;
+    // spread mode: CTA kk of kv head g runs tasks kk, kk + cph, .. of the head; batch mode: the producer walks the CTA's segments
+    // (runs of chunks of one (job, kv head), the groups of a chunk in order with the running max carried in registers) and leaves a
+    // record per group, from which the other roles take everything they need, the end of the CTA's work included
+    constexpr bool batch = BATCH;
+    const int g = batch ? 0 : (int) blockIdx.x / a.cph, kk = batch ? 0 : (int) blockIdx.x % a.cph;
+    const int slot = (int) blockIdx.x, tstep = batch ? 1 : a.cph;
+    const int T = J.T, n = J.n, R = GQ * T, ws = J.ws;
+    Geo4 geo4;
+    geo4.g = make_geo(J, GT);
+    geo4.mul_nch = geo4.g.nch > 1 ? 0xffffffffu / (unsigned) geo4.g.nch + 1u : 0u;
+    geo4.mul_nch1 = geo4.g.nch > 2 ? 0xffffffffu / (unsigned) (geo4.g.nch - 1) + 1u : 0u;
+    const AttnTask * const ttab = a.tasks;
+    const int t_end = ttab ? a.ntasks : geo4.g.ntasks_head;
+    auto get_task = [&](int t) -> Task { return ttab ? ttab[t] : make_task4(geo4, t); };
+    // this CTA's groups: tasks kk, kk + tstep, .. (batch mode: known to a role once it has read the record with REC_END)
+    int G = batch ? 0x7fffffff : kk < t_end ? (t_end - kk + tstep - 1) / tstep : 0;
+
+    // The kv head's query rows come staged (qprep: fp16 -> fp32 -> K's rotation -> x 1/16 -> fp16 in the K-major B operand's layout,
+    // row = (head % 6) T + t): the producer fetches the block with one bulk copy, the issuer waits for it.
+    // registers move from the unpack / control warps to the softmax warps
+    if (!BATCH && warp >= W_MAX) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_MAX ";");
+        // ---- spread mode, maxima warps: warp W_MAX + q takes the tile maxima of query rows 16 q .. + 15 (a thread: one row, two of the tiles),
+        // publishes each group's, collects the running max before it and leaves both for the softmax warp of the same rows. Tile maxima
+        // run ahead of P, so that a group's own maxima are published well before the CTAs that hold the chunk's next groups need them: the
+        // CTAs of a kv head may drift apart by a group without a poll having to wait. The lead grows from none (the first P needs only
+        // its own group's scores) to MAX_AHEAD groups. (In the softmax warps, between one P and the next, maxima and polls took 2,900 of a
+        // group's 7,800 cycles: one layer of 101,600 positions 111 us, 103 with warps of their own, 99.6 with the words polled together.) ----
+        const int q = warp & 3, hf = lane >> 4, r_own = 16 * q + (lane & 15);
+        const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
+        const bool st = q == 0, act = q < 3 && 16 * q < R, pub = act && !hf && r_own < R;
+        (void) st;
+        auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
+        // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
+        // producer never reached are not valid) and only inside their bounds
+        auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
+        unsigned long long w[3] = {0ull, 0ull, 0ull};
+        // the words of the groups one and two before, and the cumulative one of the group three before
+        auto words = [&](const Task & k, const unsigned long long * (&src)[3]) {
+            const size_t xb0 = xbase(k);
+            src[0] = k.b >= 1 ? a.xa + xb0 + (size_t) (k.b - 1) * AR : nullptr;
+            src[1] = k.b >= 2 ? a.xa + xb0 + (size_t) (k.b - 2) * AR : nullptr;
+            src[2] = k.b >= 3 ? a.xb + xb0 + (size_t) (k.b - 3) * AR : nullptr;
+        };
+        // tile maxima of group j, its own maxima published
+        auto maxima = [&](int j) {
+            if (st) TC_STAMP(j, 0);
+            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc);
+            const GroupRec & k = sm.tasks[j % NTASK];
+            if (st) TC_STAMP(j, 1);
+            tc_fence_after();
+#pragma unroll 1
+            for (int row0 = 0; row0 < R; row0 += RS) {
+                float s[RS];
+                tmem_scores(lane_addr + S_COL + AR * (j % NSB) + row0, s);
+                if (k.flags & REC_MASK) mask_scores(k, n, T, q, row0, lane, s);
+                tile_maxima(s, R - row0, lane, &sm.tmax[j % NSB][q][row0]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            warp_arrive(&sm.s_empty[j % NSB], lane);
+            named_bar(3, 4 * 32); // (the four tiles' maxima are there)
+            const float(&x)[GT][TROWS] = sm.tmax[j % NSB];
+            const float group = pub ? fmaxf(fmaxf(x[0][r_own], x[1][r_own]), fmaxf(x[2][r_own], x[3][r_own])) : 0.f;
+            if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
+                __stcg(a.xa + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(group));
+            if (st) TC_STAMP(j, 2);
+        };
+        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
+        // the chunk's previous groups have most likely published them
+        auto request_words = [&](const Task & k) {
+            if (pub && k.nb > 1 && exch_ok(k)) {
+                const unsigned long long * src[3];
+                words(k, src);
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+                    if (src[x]) w[x] = __ldcv(src[x]);
+            }
+        };
+        constexpr int MAX_AHEAD = 2;
+        static_assert(MAX_AHEAD + 1 < NSB, "S of the groups ahead stays until their P");
+        int maxima_done = 0;
+        for (int i = 0; i < G; i++) {
+            const int want = min(G, i + 1 + min(i, MAX_AHEAD));
+            while (maxima_done < want) maxima(maxima_done++);
+            const GroupRec & k = sm.tasks[i % NTASK];
+            float m_in = -CUDART_INF_F;
+            if (pub && k.nb > 1 && exch_ok(k)) {
+                const unsigned long long * src[3];
+                words(k, src);
+                poll_words(src, w, a.epoch, &sm.wc, a.status);
+#pragma unroll
+                for (int x = 0; x < 3; x++)
+                    if (src[x]) m_in = fmaxf(m_in, __uint_as_float((unsigned) w[x]));
+                if (k.b + 3 < k.nb) {
+                    const float(&x)[GT][TROWS] = sm.tmax[i % NSB];
+                    const float M = fmaxf(fmaxf(m_in, fmaxf(x[0][r_own], x[1][r_own])), fmaxf(x[2][r_own], x[3][r_own]));
+                    __stcg(a.xb + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(M));
+                }
+            }
+            if (st) TC_STAMP(i, 7);
+            if (act && !hf) sm.m_in[i % NSB][r_own] = m_in;
+            __syncwarp();
+            warp_arrive(&sm.m_full[i % NSB], lane);
+            if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
+                request_words(sm.tasks[(i + 1) % NTASK]);
+            } else {
+                w[0] = w[1] = w[2] = 0ull; // (no early request: the polls fetch the words themselves)
+            }
+        }
+    } else if (warp >= W_CTL) {
+    if constexpr (BATCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL_SPREAD ";");
+    if (warp == W_KPROD) {
+        if constexpr (BATCH) {
+            batch_producer(sm, a, lane);
+        } else {
+        if (lane == 0) { // the queries first
+            mbar_expect_tx(&sm.q_ready, Q_BYTES);
+            bulk_g2s(sm.q, reinterpret_cast<const uint8_t *>(J.Qp) + (size_t) g * Q_BYTES, Q_BYTES, &sm.q_ready);
+        }
+        const int side = (lane >> 2) & 1, tile = lane & 3;
+        const SideSrc src = make_src(kv, side, g, ws);
+        LastCopy last_copy;
+        for (int j = 0; j < G; j++) { // a group's task is computed here, once, and left for the other roles
+            const Task k = get_task(kk + j * tstep);
+            if (lane == 0) {
+                GroupRec & rec = sm.tasks[j % NTASK];
+                static_cast<AttnTask &>(rec) = k;
+                rec.flags = k.pos0 + GP > min(k.c1, n + 1) ? REC_MASK : 0; // (of a table's tasks, too: their c1 is their piece's end)
+            }
+            const TileSrc t = describe_tile(sm, j, src, side, tile, k.pos0 + tile * ATP, k.nt, k.c1, 0u, lane);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sm.rec_full[j % NTASK]);
+            if (!fetch_tile(sm, a, 0, j, k.nt, t, lane, last_copy)) break;
+        }
+        watch_end(sm, a, lane);
+        if (lane < GT) drain_copy(&sm.raw_full[0][lane], last_copy);
+        if (lane == 0) // (the query block too: the issuer may give up on it)
+            wait_landed(&sm.q_ready, 0u);
+        }
+    } else if (warp == W_VPROD) {
+        v_producer(sm, a, G, lane);
+    } else if (warp == W_SISSUE) {
+        // ---- S^T(j) = K Q^T, as K's operand slots fill ----
+        if (elect_one()) { // (with lane == 0 as the test an instruction took 50 % longer to issue: see elect_one)
+            if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc); // the queries are staged
+            // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S of the segment before is
+            // complete: they arrive while P V of an earlier group runs
+            bool q_next = batch, q_flight = false;
+            unsigned q_ph = 0;
+            const unsigned q_lo = desc_lo(smem_u32(sm.q), AR / 8 * 128), hi_128 = desc_hi(128); // (8-row groups 128 bytes apart)
+            unsigned ks = 0, kph = 0;
+            for (int j = 0; j < G && !sm.wc.dead; j++) {
+                const int sb = j % NSB;
+                if (batch && q_next) {
+                    tc_wait(&sm.rec_full[j % NTASK], (j / NTASK) & 1, &sm.wc);
+                    if (j > 0) tc_wait(&sm.s_full[(j - 1) % NSB], ((j - 1) / NSB) & 1, &sm.wc);
+                    if (sm.wc.dead) break;
+                    mbar_expect_tx(&sm.q_ready, Q_BYTES);
+                    bulk_g2s(sm.q, sm.tasks[j % NTASK].q, Q_BYTES, &sm.q_ready);
+                    q_flight = true, q_next = false;
+                }
+                if (j >= NSB) tc_wait(&sm.s_empty[sb], ((j / NSB) - 1) & 1, &sm.wc);
+                if (batch && q_flight) {
+                    tc_wait(&sm.q_ready, q_ph, &sm.wc);
+                    if (sm.wc.dead) break;
+                    q_ph ^= 1, q_flight = false;
+                }
+                const unsigned dcol = tb + S_COL + AR * sb;
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) {
+                    tc_wait(&sm.k_full[ks], kph, &sm.wc);
+                    tc_fence_after();
+                    const unsigned kcol = tb + K_COL + K_STRIDE * ks, qh_lo = q_lo + ((8 * h) * (2 * AR / 8 * 128) >> 4);
+#pragma unroll 2
+                    for (int x = 0; x < 8; x++)
+                        umma_ta(dcol, kcol + 8 * x, qh_lo + (x * (2 * AR / 8 * 128) >> 4), hi_128, IDESC_S, (unsigned) (h | x));
+                    umma_commit(&sm.k_empty[ks]);
+                    if (++ks == NKS) ks = 0, kph ^= 1;
+                }
+                umma_commit(&sm.s_full[sb]);
+                if (batch) { // (the record was written before the group's K was fetched)
+                    const int fl = sm.tasks[j % NTASK].flags;
+                    if (sm.wc.dead) break;
+                    if (fl & REC_END) G = j + 1;
+                    q_next = (fl & REC_LAST) != 0;
+                }
+            }
+            // every instruction issued above is complete before the tensor memory is freed and the CTA's shared memory released
+            // (bounded; in a normal run the softmax warps have already waited for the last one)
+            if (batch && q_flight) // (given up with the query block in flight: it lands before the CTA's shared memory is released)
+                wait_landed(&sm.q_ready, q_ph);
+            umma_commit(&sm.fin[0]);
+            wait_landed(&sm.fin[0], 0u);
+        }
+    } else if (warp == W_OISSUE) {
+        // ---- O^T += V^T P^T(j), P as its high and low parts ----
+        if (elect_one()) {
+            const unsigned p_lo = desc_lo(smem_u32(sm.p), 128), hi_2048 = desc_hi(2048); // (MN-major: 8-dim / 8-row groups 2048 bytes apart)
+            unsigned os = 0, oph = 0;
+            for (int j = 0; j < G && !sm.wc.dead; j++) {
+#if MKKV_TC_PROF == 1
+                TC_STAMP(j, 16);
+#endif
+                tc_wait(&sm.p_full, j & 1, &sm.wc);
+#if MKKV_TC_PROF == 1
+                TC_STAMP(j, 17);
+#endif
+                if (sm.wc.dead) break;
+                const int fl = batch ? sm.tasks[j % NTASK].flags : 0;
+                const bool fresh = batch ? (fl & REC_FIRST) != 0 : j == 0; // O^T starts from zero
+                if (fl & REC_END) G = j + 1;
+#pragma unroll 1
+                for (int h = 0; h < 2; h++) {
+                    tc_wait(&sm.op_full[os], oph, &sm.wc);
+#if MKKV_TC_PROF == 1
+                    if (h == 0) TC_STAMP(j, 18);
+#endif
+                    tc_fence_after();
+                    const unsigned v_lo = desc_lo(smem_u32(sm.op[os]), 128), dcol = tb + (h ? O_COL1 : O_COL0);
+#pragma unroll 2
+                    for (int x = 0; x < 8; x++)
+                        umma(dcol, v_lo + (x * 256 >> 4), hi_2048, p_lo + (x * 256 >> 4), hi_2048, IDESC_PV, (unsigned) (!fresh || x));
+                    umma_commit(&sm.op_empty[os]);
+                    if (++os == NOP) os = 0, oph ^= 1;
+                }
+                umma_commit(&sm.p_empty);
+#if MKKV_TC_PROF == 1
+                TC_STAMP(j, 19);
+#endif
+            }
+            umma_commit(&sm.fin[1]);
+            wait_landed(&sm.fin[1], 0u);
+        }
+    }
+    } else if (warp >= NSOFT) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_DQ ";");
+        // ---- unpack warps: packed rows of one side -> its operand slots, a tile's half to two warps. K and V have warps, raw slots and
+        // operand slots of their own: neither waits for the other. Everything besides the values' arithmetic is kept out of the loop: a
+        // side's body knows its format, a tile is one descriptor word, the bias constants stay in registers, and a warp reads its share of the
+        // whole row at once (8 bits: in two halves), which frees the raw slot for the next group's copy ----
+        const int w = warp - NSOFT, q = w & 3, c2 = w >> 3, side = (w >> 2) & 1;
+        const UnpackConst uc = unpack_const();
+        const bool st = w == 0 || w == 4;
+        (void) st;
+        uint64_t * const full = side ? sm.op_full : sm.k_full, * const empty = side ? sm.op_empty : sm.k_empty;
+        const unsigned slots = side ? NOP : NKS, raw = smem_u32(sm.raw[side][q]), prow = ATP * q + lane;
+        // K: the tile's lanes of tensor memory, the warp's 32 columns of a slot. V: the position's 16-byte unit inside a dim group
+        const unsigned k_dst = tb + ((unsigned) (ATP * q) << 16) + K_COL + 32 * c2, v_dst = smem_u32(sm.op[0]) + (prow >> 3) * 128 + (prow & 7) * 16;
+        unsigned os = 0, oph = 1; // operand slot / parity of its "empty" wait
+        auto slot_wait = [&]() {
+            tc_wait(&empty[os], oph, &sm.wc);
+            tc_fence_after();
+            __syncwarp();
+        };
+        auto slot_done = [&]() {
+            __syncwarp();
+            warp_arrive(&full[os], lane);
+            if (++os == slots) os = 0, oph ^= 1;
+        };
+        auto raw_read = [&]() {
+            __syncwarp();
+            warp_arrive(&sm.raw_empty[side][q], lane);
+        };
+        auto k_half = [&](auto bits_c, const auto & b0, const auto & b1) {
+            constexpr int B = decltype(bits_c)::value;
+            slot_wait();
+            block_to_tmem<B>(b0, uc, k_dst + K_STRIDE * os);
+            block_to_tmem<B>(b1, uc, k_dst + K_STRIDE * os + 16);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            slot_done();
+        };
+        auto v_half = [&](auto bits_c, const auto & b0, const auto & b1, int jr0, int jr1) {
+            constexpr int B = decltype(bits_c)::value;
+            slot_wait();
+            store_block<B>(b0, uc, v_dst + os * OP_SLOT + jr0 * 8192, lane);
+            store_block<B>(b1, uc, v_dst + os * OP_SLOT + jr1 * 8192, lane);
+            fence_async_smem();
+            slot_done();
+        };
+        auto scales = [&](bool valid) {
+            const uint4 sc = row_scales(raw, lane);
+            return valid ? sc : make_uint4(0u, 0u, 0u, 0u); // (a row past the chunk end holds stale bytes)
+        };
+        // (both halves' packed bytes are read at once, then the raw slot is free; the halves run through one body: see the instruction cache)
+        auto k_tile = [&](auto bits_c, bool valid) {
+            constexpr int B = decltype(bits_c)::value;
+            const uint4 sc = scales(valid);
+            PackedBlock<B> b[2][2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                load_pair<B>(b[h][0], b[h][1], raw, lane, c2, h);
+                b[h][0].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(2 * c2)), b[h][1].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(2 * c2 + 1));
+            }
+            raw_read();
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                k_half(bits_c, b[0][0], b[0][1]);
+                b[0][0] = b[1][0], b[0][1] = b[1][1];
+            }
+        };
+        auto v_tile = [&](auto bits_c, bool valid) {
+            constexpr int B = decltype(bits_c)::value;
+            const int jr0 = (2 * c2 + v_rotation<B>(lane)) & 3, jr1 = (jr0 + 1) & 3;
+            const uint4 sc = scales(valid);
+            PackedBlock<B> b[2][2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                load_block<B>(b[h][0], raw, lane, jr0 + 4 * h);
+                load_block<B>(b[h][1], raw, lane, jr1 + 4 * h);
+                b[h][0].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(jr0)), b[h][1].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(jr1));
+            }
+            raw_read();
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                v_half(bits_c, b[0][0], b[0][1], jr0, jr1);
+                b[0][0] = b[1][0], b[0][1] = b[1][1];
+            }
+        };
+        // 8 bits (twice the registers): half by half. Beside other formats one body serves both sides: contexts of a few window lengths have
+        // as many tiles of one kind as of the other, and four bodies do not fit the instruction cache
+        auto tile8 = [&](bool valid) {
+            const uint4 sc = scales(valid);
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                PackedBlock<8> b[2];
+                load_pair<8>(b[0], b[1], raw, lane, c2, h);
+                b[0].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(2 * c2)), b[1].d = __byte_perm(h ? sc.z : sc.x, h ? sc.w : sc.y, scale_pick(2 * c2 + 1));
+                __syncwarp();
+                if (h) warp_arrive(&sm.raw_empty[side][q], lane);
+                slot_wait();
+#pragma unroll
+                for (int x = 0; x < 2; x++) {
+                    unsigned r[16];
+                    block_units<8>(b[x], uc, [&](int u, unsigned p0, unsigned p1, unsigned p2, unsigned p3) { r[4 * u] = p0, r[4 * u + 1] = p1, r[4 * u + 2] = p2, r[4 * u + 3] = p3; });
+                    if (side) {
+#pragma unroll
+                        for (int u = 0; u < 4; u++) sts128(v_dst + os * OP_SLOT + (2 * c2 + x) * 8192 + u * 2048, r[4 * u], r[4 * u + 1], r[4 * u + 2], r[4 * u + 3]);
+                    } else {
+                        tmem_st16(k_dst + K_STRIDE * os + 16 * x, r);
+                    }
+                }
+                if (side) {
+                    fence_async_smem();
+                } else {
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    tc_fence_before();
+                }
+                slot_done();
+            }
+        };
+        for (int j = 0; j < G; j++) {
+            if (st) TC_STAMP(j, side ? 8 : 11);
+            if (!tc_wait_all(&sm.raw_full[side][q], j & 1, &sm.wc)) break;
+            if (st) TC_STAMP(j, side ? 9 : 12);
+            const unsigned ud = sm.udesc[j % NTASK][side][q];
+            const bool valid = lane < (int) (ud & UD_ROWS);
+            const int bits = (int) (ud >> 8);
+            if (bits == 8) tile8(valid);
+            else if (side) v_tile(IntC<VB>{}, valid);
+            else k_tile(IntC<KB>{}, valid);
+            if (st) TC_STAMP(j, side ? 10 : 13);
+            if (batch && (ud & UD_END)) break;
+        }
+    } else {
+        if constexpr (BATCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
+        else asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT_SPREAD ";");
+#if MKKV_TC_PROF
+        const unsigned long long t_loop = globaltimer_ns();
+#endif
+        // ---- softmax warps: warp 4 c + q holds tile q of a group and rows RS c .. of the query rows, a thread one position. What belongs to a row --
+        // the running max, the reference max -- is kept by thread lane = row - RS c of the four warps c alike, computed once per group from
+        // the four tiles' maxima, and handed to the threads of a warp through shared memory; a thread's sums of its positions' weights are registers,
+        // added up over the threads when a segment ends. In the accumulator's read-out and rescaling a warp's lanes are dims. The two sets of
+        // four warps share nothing but that each reads out one half of the accumulator. ----
+        const int q = warp & 3, half = warp >> 2, row0 = RS * half;
+        const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
+        const bool st = warp == 0;
+        auto & tab = sm.row[warp];
+        float m_acc = -CUDART_INF_F, carry = -CUDART_INF_F; // row row0 + lane: reference max, running max (batch mode)
+        F2 l_acc[RS / 2]; // rows row0 + (2 i, 2 i + 1)
+#pragma unroll
+        for (int i = 0; i < RS / 2; i++) l_acc[i] = 0ull;
+        // batch mode: the partial of a finished segment (O^T lanes are dims in the unpacked units' order, columns are query rows), read
+        // out when its last P V is complete and before the next P allows the MMA that overwrites O^T: between the two the tensor cores
+        // stand still, so the next group's exponentials are computed first
+        int flush_slot = -1, flush_rows = 0;
+        const int prow = ATP * q + lane, pdim = (prow & ~7) | unit_perm(prow & 7);
+        auto read_out = [&](int to_slot, int rows, bool any) { // (of all rows: either set of warps reads one half of the dims)
+#pragma unroll 1
+            for (int r0 = 0; r0 < rows; r0 += 8) {
+                unsigned v[8], w[8];
+                if (any) {
+                    const unsigned col = lane_addr + (half ? O_COL1 : O_COL0) + r0;
+                    tmem_ld8_two(col, col + AR, v, w);
+                }
+                float * dst = a.part + ((size_t) to_slot * AR + r0) * HD + 128 * half + pdim;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (r0 + j < rows) dst[j * HD] = any ? __uint_as_float(v[j]) + __uint_as_float(w[j]) : 0.f;
+            }
+        };
+        // the segment's row sums and maxima (the four warps of the rows)
+        auto close_rows = [&](int to_slot, int rows) {
+#pragma unroll
+            for (int b = 0; b < RS / 8; b++)
+                if (8 * b < rows) { // eight sums over 32 lanes: at each step half of them go to the partner
+                    float x[8];
+#pragma unroll
+                    for (int i = 0; i < 4; i++) f2_unpack(l_acc[4 * b + i], x[2 * i], x[2 * i + 1]);
+#pragma unroll
+                    for (int i = 0, m = 16; m >= 4; i++, m >>= 1)
+#pragma unroll
+                        for (int j = 0; j < (4 >> i); j++) {
+                            const float send = (lane & m) ? x[j] : x[j + (4 >> i)], keep = (lane & m) ? x[j + (4 >> i)] : x[j];
+                            x[j] = keep + __shfl_xor_sync(FULL_MASK, send, m);
+                        }
+                    x[0] += __shfl_xor_sync(FULL_MASK, x[0], 2);
+                    x[0] += __shfl_xor_sync(FULL_MASK, x[0], 1);
+                    if (!(lane & 3)) sm.lsum[q][row0 + 8 * b + (lane >> 2)] = x[0];
+                }
+            if (rows > 0) named_bar(1 + half, GT * 32);
+            if (q == 0 && lane < rows) {
+                const int r = row0 + lane;
+                a.ml[(size_t) to_slot * AR + r] = make_float2(m_acc, (sm.lsum[0][r] + sm.lsum[1][r]) + (sm.lsum[2][r] + sm.lsum[3][r]));
+            }
+        };
+        // P of group i (rows of the RS; none: the warp only keeps step) from the masked scores s and the maxima of its tiles, sm.tmax[i % NSB]. start: the
+        // running max before it of row row0 + lane; restart: bit t: tile t opens a chunk, the running max starts anew.
+        auto softmax = [&](int i, int rows, float start, unsigned restart, auto && scores) {
+            unsigned moved = 0u;
+            unsigned hi[RS / 2], lo[RS / 2]; // rows (2 c, 2 c + 1)
+            if (rows > 0) {
+                float factor = 1.f;
+                bool mv = false;
+                const float(&x)[GT][TROWS] = sm.tmax[i % NSB];
+                const int r = row0 + lane;
+                // running maxima after each tile; M: the largest of them
+                const float t0 = x[0][r], t1 = x[1][r], t2 = x[2][r], t3 = x[3][r];
+                const float r0 = (restart & 1u) ? t0 : fmaxf(start, t0), r1 = (restart & 2u) ? t1 : fmaxf(r0, t1);
+                const float r2 = (restart & 4u) ? t2 : fmaxf(r1, t2), r3 = (restart & 8u) ? t3 : fmaxf(r2, t3);
+                const float M = fmaxf(fmaxf(r0, r1), fmaxf(r2, r3));
+                carry = r3;
+                if (M != -CUDART_INF_F && lane < rows) {
+                    if (m_acc == -CUDART_INF_F) m_acc = M - REF_BELOW;
+                    else if (M > m_acc + REF_SLACK) { // the reference max moves: the row sums follow at once, the accumulator when it is at rest (below)
+                        factor = exp_any(m_acc - (M - REF_BELOW));
+                        m_acc = M - REF_BELOW;
+                        mv = true;
+                    }
+                }
+                const float mr = q == 0 ? r0 : q == 1 ? r1 : q == 2 ? r2 : r3;
+                const float beta = mr == -CUDART_INF_F ? 0.f : exp_any(mr - m_acc);
+                const __half bh = __float2half_rn(beta);
+                tab.nm[lane] = mr == -CUDART_INF_F ? mr : -mr; // (nothing visible yet: exp2 gives 0)
+                tab.beta[lane] = beta;
+                tab.bh[lane] = __half_as_ushort(bh);
+                tab.bl[lane] = __half_as_ushort(__float2half_rn(beta - __half2float(bh)));
+                moved = __ballot_sync(FULL_MASK, mv);
+                if (moved) tab.f[lane] = factor;
+                __syncwarp();
+                if (__builtin_expect(moved != 0u, 0)) {
+#pragma unroll
+                    for (int c = 0; c < RS / 2; c++) l_acc[c] = f2_mul(l_acc[c], f2_pack(tab.f[2 * c], tab.f[2 * c + 1]));
+                }
+                if (st) TC_STAMP(i, 4);
+                float s[RS];
+                scores(s);
+#pragma unroll
+                for (int b = 0; b < RS / 8; b++)
+                    if (8 * b < rows) {
+                        const float4 nm0 = *reinterpret_cast<const float4 *>(&tab.nm[8 * b]), nm1 = *reinterpret_cast<const float4 *>(&tab.nm[8 * b + 4]);
+                        const float4 be0 = *reinterpret_cast<const float4 *>(&tab.beta[8 * b]), be1 = *reinterpret_cast<const float4 *>(&tab.beta[8 * b + 4]);
+                        const uint4 bhv = *reinterpret_cast<const uint4 *>(&tab.bh[8 * b]), blv = *reinterpret_cast<const uint4 *>(&tab.bl[8 * b]);
+                        const F2 nm[4] = {f2_pack(nm0.x, nm0.y), f2_pack(nm0.z, nm0.w), f2_pack(nm1.x, nm1.y), f2_pack(nm1.z, nm1.w)};
+                        const F2 be[4] = {f2_pack(be0.x, be0.y), f2_pack(be0.z, be0.w), f2_pack(be1.x, be1.y), f2_pack(be1.z, be1.w)};
+                        const unsigned bhw[4] = {bhv.x, bhv.y, bhv.z, bhv.w}, blw[4] = {blv.x, blv.y, blv.z, blv.w};
+#pragma unroll
+                        for (int c = 0; c < 4; c++) {
+                            float p0, p1;
+                            f2_unpack(f2_mul(f2_add(f2_pack(s[8 * b + 2 * c], s[8 * b + 2 * c + 1]), nm[c]), f2_pack(LOG2E, LOG2E)), p0, p1);
+                            p0 = ex2(p0), p1 = ex2(p1);
+                            l_acc[4 * b + c] = f2_fma(be[c], f2_pack(p0, p1), l_acc[4 * b + c]);
+                            const __half2 bh = *reinterpret_cast<const __half2 *>(&bhw[c]), bl = *reinterpret_cast<const __half2 *>(&blw[c]);
+                            const __half2 ph = __floats2half2_rn(p0, p1); // the reference's fp16 P
+                            const __half2 hh = __hmul2(ph, bh);           // P beta = hh + ll up to 2^-22: the product's exact residual
+                            const __half2 ll = __hfma2(ph, bl, __hfma2(ph, bh, __hneg2(hh))); // plus the low part of beta
+                            hi[4 * b + c] = *reinterpret_cast<const unsigned *>(&hh);
+                            lo[4 * b + c] = *reinterpret_cast<const unsigned *>(&ll);
+                        }
+                    }
+            }
+            if (st && i < 15) TC_STAMP(i, 15);
+            tc_wait(&sm.p_empty, (i + 1) & 1, &sm.wc); // (the first: at once) P V of the previous group is complete: P is free, O^T at rest
+            if (st) TC_STAMP(i, 5);
+            tc_fence_after();
+#if MKKV_TC_PROF
+            if (moved && a.prof && st && lane == 0) a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 15] += 1ull;
+#endif
+            if (batch && __builtin_expect(flush_slot >= 0, 0)) { // (a segment's first group: no reference max moves at it)
+                read_out(flush_slot, flush_rows, true);
+                flush_slot = -1;
+            } else if (__builtin_expect(moved != 0u, 0)) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference: a row is one
+                         // column in each of the four blocks (two halves x high / low part); the four loads of a row are in flight together
+#pragma unroll 1
+                while (moved) {
+                    const int r = __ffs(moved) - 1;
+                    moved &= moved - 1;
+                    const float fr = tab.f[r];
+                    const unsigned ad = lane_addr + row0 + r;
+                    unsigned v0, v1, v2, v3;
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v0) : "r"(ad + O_COL0));
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v1) : "r"(ad + O_COL0 + AR));
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v2) : "r"(ad + O_COL1));
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v3) : "r"(ad + O_COL1 + AR));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(v0), "+r"(v1), "+r"(v2), "+r"(v3)::"memory");
+                    v0 = __float_as_uint(__uint_as_float(v0) * fr), v1 = __float_as_uint(__uint_as_float(v1) * fr);
+                    v2 = __float_as_uint(__uint_as_float(v2) * fr), v3 = __float_as_uint(__uint_as_float(v3) * fr);
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0), "r"(v0) : "memory");
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL0 + AR), "r"(v1) : "memory");
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1), "r"(v2) : "memory");
+                    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(ad + O_COL1 + AR), "r"(v3) : "memory");
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            }
+            uint8_t * const dst = sm.p[0] + (row0 / 8) * P_ROWGROUP + (prow >> 3) * 128 + (prow & 7) * 16;
+#pragma unroll
+            for (int b = 0; b < RS / 8; b++)
+                if (8 * b < rows) { // 8 rows of a position: one 16-byte unit of each part
+                    *reinterpret_cast<uint4 *>(dst + b * P_ROWGROUP) = make_uint4(hi[4 * b], hi[4 * b + 1], hi[4 * b + 2], hi[4 * b + 3]);
+                    *reinterpret_cast<uint4 *>(dst + P_PART + b * P_ROWGROUP) = make_uint4(lo[4 * b], lo[4 * b + 1], lo[4 * b + 2], lo[4 * b + 3]);
+                }
+            fence_async_smem();
+            tc_fence_before();
+            __syncwarp();
+            warp_arrive(&sm.p_full, lane);
+            if (st) TC_STAMP(i, 6);
+        };
+
+        if constexpr (BATCH) {
+            for (int i = 0; i < G; i++) {
+                if (st) TC_STAMP(i, 0);
+                // After a wait that gave up the group's record may not be written: the wait's result is voted on, and the barrier that hands the
+                // maxima out carries the flag, so that the four warps of a set of rows leave together.
+                const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc);
+                if (st) TC_STAMP(i, 1);
+                tc_fence_after();
+                const GroupRec & k = sm.tasks[i % NTASK];
+                const int4 hot = *reinterpret_cast<const int4 *>(&k.flags);
+                const int flags = hot.x, to = hot.y, rows = there ? min(hot.z - row0, RS) : 0;
+                float s[RS];
+                if (rows > 0) tmem_scores(lane_addr + S_COL + AR * (i % NSB) + row0, s);
+                tc_fence_before();
+                __syncwarp();
+                warp_arrive(&sm.s_empty[i % NSB], lane);
+                if (rows > 0) {
+                    if (__builtin_expect(flags & REC_MASK, 0)) mask_scores(k, k.n, k.T, q, row0, lane, s);
+                    tile_maxima(s, rows, lane, &sm.tmax[i % NSB][q][row0]);
+                }
+                if (st) TC_STAMP(i, 2);
+                if (named_bar_or(1 + half, GT * 32, !there || sm.wc.dead != 0)) break;
+                if (st) TC_STAMP(i, 3);
+                softmax(i, rows, carry, (unsigned) flags >> REC_RESTART, [&](float (&x)[RS]) {
+#pragma unroll
+                    for (int c = 0; c < RS; c++) x[c] = s[c];
+                });
+                if (flags & REC_END) G = i + 1;
+                if (!(flags & REC_LAST)) continue;
+                // the segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below)
+                close_rows(to, rows);
+#pragma unroll
+                for (int c = 0; c < RS / 2; c++) l_acc[c] = 0ull;
+                m_acc = -CUDART_INF_F;
+                flush_slot = to, flush_rows = hot.z;
+            }
+            if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
+                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
+                tc_fence_after();
+                read_out(flush_slot, flush_rows, true);
+            }
+        } else {
+        // tile maxima and incoming running max come from the maxima warps (above)
+        const int rows = min(R - row0, RS);
+        for (int i = 0; i < G; i++) {
+            tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc);
+            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc); // (long since: orders this warp's reads behind the MMA)
+            tc_fence_after();
+            __syncwarp();
+            const GroupRec & k = sm.tasks[i % NTASK];
+            if (st) TC_STAMP(i, 3);
+            if (rows <= 0) warp_arrive(&sm.s_empty[i % NSB], lane);
+            softmax(i, rows, sm.m_in[i % NSB][row0 + lane], 0u, [&](float (&x)[RS]) {
+                tmem_scores(lane_addr + S_COL + AR * (i % NSB) + row0, x);
+                tc_fence_before();
+                __syncwarp();
+                warp_arrive(&sm.s_empty[i % NSB], lane); // (the last read of this S buffer and of the group's maxima)
+                if (k.flags & REC_MASK) mask_scores(k, n, T, q, row0, lane, x);
+            });
+        }
+        if (G > 0) {
+            tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
+            tc_fence_after();
+            __syncwarp();
+        }
+#if MKKV_TC_PROF
+        if (warp == 0) { // the tail's stamps go to group slot 15 (stamps 8 .. 13, after the main loop's own use of them)
+            if (a.prof && lane == 0) {
+                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 8] = t_entry;
+                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 9] = t_loop;
+                unsigned smid;
+                asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
+                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 14] = smid; // (which SM ran this CTA)
+            }
+            TC_STAMP(15, 10);
+        }
+#endif
+        // (a CTA without groups: zeros, with a reference of minus infinity)
+        read_out(slot, R, G > 0);
+        close_rows(slot, rows);
+#if MKKV_TC_PROF
+        if (warp == 0) TC_STAMP(15, 11);
+#endif
+        if (a.done) tail_merge(sm, a, g, kk, T, warp, lane);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == W_SISSUE) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(TMEM_COLS) : "memory");
+}
+
+} // namespace ts
+
+TcKernel ts_kernel_for(int kb, int vb, bool batch) {
+    if (kb == 5 && vb == 6) return batch ? ts::attn_ts_kernel<5, 6, true> : ts::attn_ts_kernel<5, 6, false>;
+    if (kb == 5 && vb == 5) return batch ? ts::attn_ts_kernel<5, 5, true> : ts::attn_ts_kernel<5, 5, false>;
+    if (kb == 6 && vb == 5) return batch ? ts::attn_ts_kernel<6, 5, true> : ts::attn_ts_kernel<6, 5, false>;
+    return nullptr;
+}
+size_t ts_smem_bytes() { return sizeof(ts::Smem) + 128; }
+static_assert(sizeof(ts::Smem) + 128 <= 232448, "shared memory of one CTA");
+cudaError_t ts_for_each(cudaError_t (*f)(TcKernel, size_t)) {
+    static const int formats[][2] = {{5, 6}, {5, 5}, {6, 5}};
+    for (const int(&b)[2] : formats)
+        for (int batch = 0; batch < 2; batch++) {
+            const cudaError_t e = f(ts_kernel_for(b[0], b[1], batch != 0), ts_smem_bytes());
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+} // namespace tc
+} // namespace mkkv
