@@ -121,33 +121,6 @@ struct Smem {
     uint64_t m_full[NSB];
 };
 
-// Wait for a phase of an mbarrier. A try suspends the thread in hardware (it wakes when the phase completes, or after a time of the
-// hardware's choosing), so waiting warps take next to no issue slots. (try_wait with a time limit of its own becomes a loop that polls,
-// sleeps and reads the clock.) Bounded: after the limit the status word and the CTA's `dead` flag are set; from then on no wait of this
-// CTA blocks, and the kernel runs to its end. The limit, hint x rounds nanoseconds, is multiplied on the host: this code stands at every
-// wait, and with the product made here a one-layer call of 101,600 positions took 101.3 us instead of 99.9, of 100,000 in q8_0 91.8 instead
-// of 89.8.
-// Returns whether the phase is complete.
-__device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    if (mbar_test_wait(bar, parity)) return true; // (the common case: no limit loaded)
-    const unsigned long long limit = wc->limit;
-    if (limit && mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = globaltimer_ns();
-    do {
-        if (wc->dead) return false;
-        if (globaltimer_ns() - t0 >= limit) {
-            wc->dead = 1;
-            atomicExch(status, (int) KS_WAIT_TIMEOUT);
-            return false;
-        }
-    } while (!mbar_try_wait(bar, parity));
-    return true;
-}
-// The same for a warp whose lanes must agree on the result: whether every lane's wait succeeded. (Warp-wide instructions that stand behind a
-// wait whatever its result need no such vote; a __syncwarp before each of them cost 16 calls of 24,003 positions 1.3 %.)
-__device__ __forceinline__ bool tc_wait_all(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    return __all_sync(FULL_MASK, tc_wait(bar, parity, wc, status)) != 0;
-}
 // The last copies of a producer lane, newest first, as bytes (slot << 1 | phase parity; 0xff: nothing was copied for that slot's turn):
 // they must land before the CTA's shared memory is released, also when a consumer gives up after the producer has fetched everything
 // and left its loop. Only the last turn of each of the lane's slots can be in flight (the one before it was waited for before the slot
@@ -324,7 +297,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         const int rs = rseq % NRAW;
         const unsigned round = rseq / NRAW;
         if (waiting) wait_previous(), waiting = false;
-        if (lane < GT && round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
+        if (lane < GT && round > 0) watched_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
         if (gave_up(FULL_MASK, &sm.wc)) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
         if (lane < GT) {
             if (lane < nt) issue_copy(t.val, t.sc, t.rb, t.np, sm.raw[rs], &sm.raw_full[rs]);
@@ -336,6 +309,7 @@ __device__ __forceinline__ void batch_producer(Smem & sm, const Args & a, int la
         if (isK) nk++;
         else nv++;
     }
+    if (lane == 0) watched_wait(&sm.fin, 0u, &sm.wc, a.status); // (everything is fetched: the issuer's last commit stands behind every other wait)
     if (lane < GT) drain_copies(sm.raw_full, issued, NRAW / GT);
 }
 
@@ -461,7 +435,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // tile maxima of group j, its own maxima published
         auto maxima = [&](int j) {
             if (st) TC_STAMP(j, 0);
-            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc, a.status);
+            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc);
             const GroupRec & k = sm.tasks[j % NTASK];
             if (st) TC_STAMP(j, 1);
             tc_fence_after();
@@ -567,7 +541,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 const SideSrc & S = isK ? ksrc : vsrc;
                 const int rs = rseq % NRAW;
                 const unsigned round = rseq / NRAW;
-                if (round > 0) tc_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
+                if (round > 0) watched_wait(&sm.raw_empty[rs], (round - 1) & 1, &sm.wc, a.status);
                 if (gave_up(0xfu, &sm.wc)) break; // (nothing is fetched into a slot that may still be read, no barrier is over-subscribed)
                 if (lane < k.nt) issue_tile(S, k.pos0 + lane * ATP, k.c1, sm.raw[rs], &sm.raw_full[rs]);
                 else mbar_arrive(&sm.raw_full[rs]);
@@ -576,6 +550,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 if (isK) nk++;
                 else nv++;
             }
+            if (lane == 0) watched_wait(&sm.fin, 0u, &sm.wc, a.status); // (everything is fetched: see batch_producer)
             if (lane == 0) // (the query block too: the issuer may give up on it)
                 wait_landed(&sm.q_ready, 0u);
             drain_copies(sm.raw_full, issued, NRAW / GT);
@@ -585,14 +560,14 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // ---- issuer: S(0) .. S(NSB - 1), then PV(i), S(i + NSB) ----
         if (elect_one()) { // (with lane == 0 as the test an instruction took 50 % longer to issue: see elect_one)
             unsigned oseq = 0;
-            if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc, a.status); // the queries are staged
+            if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc); // the queries are staged
             // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S of the segment before is
             // complete: they arrive while P V of an earlier group runs
             bool q_flight = false;
             unsigned q_ph = 0;
             auto fetch_queries = [&](int k) {
-                tc_wait(&sm.rec_full[k % NTASK], (k / NTASK) & 1, &sm.wc, a.status);
-                if (k > 0) tc_wait(&sm.s_full[(k - 1) % NSB], ((k - 1) / NSB) & 1, &sm.wc, a.status);
+                tc_wait(&sm.rec_full[k % NTASK], (k / NTASK) & 1, &sm.wc);
+                if (k > 0) tc_wait(&sm.s_full[(k - 1) % NSB], ((k - 1) / NSB) & 1, &sm.wc);
                 if (sm.wc.dead) return;
                 mbar_expect_tx(&sm.q_ready, Q_BYTES);
                 bulk_g2s(sm.q, sm.tasks[k % NTASK].q, Q_BYTES, &sm.q_ready);
@@ -605,9 +580,9 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 const bool isK = nk < G && nk < nv + NSB;
                 if (isK) { // S(nk) = Q K^T
                     const int sb = nk % NSB;
-                    if (nk >= NSB) tc_wait(&sm.s_empty[sb], ((nk / NSB) - 1) & 1, &sm.wc, a.status);
+                    if (nk >= NSB) tc_wait(&sm.s_empty[sb], ((nk / NSB) - 1) & 1, &sm.wc);
                     if (batch && q_flight) {
-                        tc_wait(&sm.q_ready, q_ph, &sm.wc, a.status);
+                        tc_wait(&sm.q_ready, q_ph, &sm.wc);
                         if (sm.wc.dead) break;
                         q_ph ^= 1, q_flight = false;
                     }
@@ -615,7 +590,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 #pragma unroll 1
                     for (int h = 0; h < 2; h++, oseq++) {
                         const int os = oseq % NOP;
-                        tc_wait(&sm.op_full[os], (oseq / NOP) & 1, &sm.wc, a.status);
+                        tc_wait(&sm.op_full[os], (oseq / NOP) & 1, &sm.wc);
                         tc_fence_after();
                         const unsigned k_lo = desc_lo(smem_u32(sm.op[os]), 2048), qh_lo = q_lo + ((8 * h) * (2 * AR / 8 * 128) >> 4);
 #pragma unroll
@@ -635,7 +610,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 #if MKKV_TC_PROF == 1
                     TC_STAMP(nv, 16);
 #endif
-                    tc_wait(&sm.p_full, nv & 1, &sm.wc, a.status);
+                    tc_wait(&sm.p_full, nv & 1, &sm.wc);
 #if MKKV_TC_PROF == 1
                     TC_STAMP(nv, 17);
 #endif
@@ -643,7 +618,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 #pragma unroll 1
                     for (int h = 0; h < 2; h++, oseq++) {
                         const int os = oseq % NOP;
-                        tc_wait(&sm.op_full[os], (oseq / NOP) & 1, &sm.wc, a.status);
+                        tc_wait(&sm.op_full[os], (oseq / NOP) & 1, &sm.wc);
 #if MKKV_TC_PROF == 1
                         if (h == 0) TC_STAMP(nv, 18);
 #endif
@@ -697,19 +672,20 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             // slot as that slot frees up
             PackedBlock<B> b0, b1;
             dq_load<B>(b0, b1, rawa, lane, jr, valid);
-            tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            store_block<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
-            hand_over();
-            tc_wait(&sm.op_empty[os], oph, &sm.wc, a.status);
-            store_block<B>(b1, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
-            hand_over();
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) { // (one body for both halves: what bounds the hot loops is the instruction cache)
+                tc_wait(&sm.op_empty[os], oph, &sm.wc);
+                store_block<B>(b0, uc, op0 + os * OP_SLOT + 4 * jr * 2048, lane);
+                hand_over();
+                b0 = b1;
+            }
         };
         // one side of group j; false: the CTA has given up
         auto unpack_side = [&](auto side_c, int j, unsigned & ud) -> bool {
             constexpr int SIDE = decltype(side_c)::value, FIXED = SIDE ? VB : KB; // the side's compiled-in main format, or 0: any
             const unsigned rs = q + GT * (rseq & 1);
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 8 : 11);
-            if (!tc_wait_all(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc, a.status)) return false;
+            if (!tc_wait_all(&sm.raw_full[rs], (rseq >> 1) & 1, &sm.wc)) return false;
             if (st) TC_STAMP(SIDE ? j : j - NSB, SIDE ? 9 : 12);
             ud = sm.udesc[j % NTASK][SIDE][q];
             const bool valid = lane < (int) (ud & UD_ROWS);
@@ -844,7 +820,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 warp_arrive(&sm.s_empty[i % NSB], lane);
             }
             if (st && i < 15) TC_STAMP(i, 15);
-            if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc, a.status); // P V of the previous group is complete: P is free, O^T at rest
+            if (i > 0) tc_wait(&sm.p_empty, (i - 1) & 1, &sm.wc); // P V of the previous group is complete: P is free, O^T at rest
             if (st) TC_STAMP(i, 5);
             tc_fence_after();
 #if MKKV_TC_PROF
@@ -905,7 +881,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 // After a wait that gave up the group's record may not be written: the wait's result is voted on, so that the warp-wide
                 // instructions under `act` are executed by all lanes or none, and a warp without a record has nothing to do but the barriers
                 // that carry the flag (softmax).
-                const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
+                const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc);
                 const GroupRec & k = sm.tasks[i % NTASK];
                 if (st) TC_STAMP(i, 1);
                 tc_fence_after();
@@ -940,7 +916,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 flush_slot = k.slot, flush_rows = rows;
             }
             if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
-                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
                 tc_fence_after();
                 read_out(flush_slot, flush_rows, true);
             }
@@ -948,8 +924,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // tile maxima and incoming running max come from the maxima warps (above)
         const bool act = 16 * q < R;
         for (int i = 0; i < G; i++) {
-            tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status);
-            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc, a.status); // (long since: orders this warp's reads behind the MMA)
+            tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc);
+            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc); // (long since: orders this warp's reads behind the MMA)
             tc_fence_after();
             const GroupRec & k = sm.tasks[i % NTASK];
             if (st) TC_STAMP(i, 3);
@@ -967,7 +943,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             });
         }
         if (G > 0) {
-            tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc, a.status);
+            tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
             tc_fence_after();
         }
 #if MKKV_TC_PROF

@@ -99,34 +99,6 @@ struct Smem {
     uint64_t m_full[NSB];
 };
 
-// Waits for a phase of an mbarrier. A try suspends the thread in hardware (it wakes when the phase completes, or after a time of the hardware's
-// choosing), so waiting warps take next to no issue slots. Every wait is bounded: K's producer warp, which waits for someone as long as the
-// CTA has work (watched_wait), measures its waits, and after the limit (hint x rounds nanoseconds, multiplied on the host) sets the status word
-// and the CTA's `dead` flag; from then on no wait of this CTA blocks, and the kernel runs to its end. The other warps' waits only look at the
-// flag: this code stands at some twenty places of the hot loops, and what bounds these is the instruction cache.
-// Returns whether the phase is complete.
-__device__ __forceinline__ bool tc_wait(uint64_t * bar, unsigned parity, const volatile WaitCtl * wc) {
-    while (!mbar_try_wait(bar, parity))
-        if (wc->dead) return false;
-    return true;
-}
-// The same for a warp whose lanes must agree on the result: whether every lane's wait succeeded. (Warp-wide instructions that stand behind a
-// wait whatever its result need no such vote; a __syncwarp before each of them cost 16 calls of 24,003 positions 1.3 %.)
-__device__ __forceinline__ bool tc_wait_all(uint64_t * bar, unsigned parity, const volatile WaitCtl * wc) {
-    return __all_sync(FULL_MASK, tc_wait(bar, parity, wc)) != 0;
-}
-__device__ __forceinline__ void watched_wait(uint64_t * bar, unsigned parity, volatile WaitCtl * wc, int * status) {
-    if (mbar_test_wait(bar, parity)) return;
-    const unsigned long long limit = wc->limit, t0 = globaltimer_ns();
-    do {
-        if (wc->dead) return;
-        if (globaltimer_ns() - t0 >= limit) {
-            wc->dead = 1;
-            atomicExch(status, (int) KS_WAIT_TIMEOUT);
-            return;
-        }
-    } while (!mbar_try_wait(bar, parity));
-}
 // The last copy of a producer lane must land before the CTA's shared memory is released, also when a consumer gives up after the producer
 // has fetched everything and left its loop. Only the lane's last turn can be in flight (the one before it was waited for before the slot
 // was filled again). Bounded; in a normal run the producer has nothing else to do and every copy lands.
