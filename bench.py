@@ -52,8 +52,8 @@ NH, NKV, HD = 24, 4, 256
 # dram__bytes_read.sum + dram__bytes_write.sum at this workload's shapes per layer, from ncu captures of this benchmark with fewer layers; one
 # entry per attention kernel instance, since a launch of one layer and a launch of all layers of a step move different partials
 NCU_TRAFFIC = {
-    "one": (164.2e6, "ncu capture of `bench.py --layers 1 --steps 2 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, false>, one launch (partials and merge in it)"),
-    "batch": (166.6e6, "ncu capture of `bench.py --layers 8 --steps 1 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, true> and attn_merge_kernel of one step, divided by 8"),
+    "one": (163.2e6, "ncu capture of `bench.py --layers 1 --steps 2 --warmup 3 --no-cpu`, attn_tc_kernel<5, 6, false>, one launch (partials and merge in it)"),
+    "batch": (167.1e6, "ncu capture of `bench.py --layers 8 --steps 1 --warmup 3 --no-cpu`, attn_ts_kernel<5, 6> and attn_merge_kernel of one step, divided by 8"),
 }
 WORKLOAD = "config2: 16 attention layers, 101,600 positions, preset F layout K5r/V6 + q8_0 window 2048, 8 queries/step, streaming append+spill+attend"
 REPEATS = 5  # the timed K-step loop is run this many times; the line's value is the median run
@@ -663,7 +663,7 @@ def main():
         if us_layer < att_us:
             att_us, att_from = us_layer, "timed steps (time per layer: 1/%d of the step's append, attention and merge launches)" % layers
             if layers > 1:
-                kernel, inst = "attn_tc_kernel<5, 6, true> (the batch instance: all layers in one launch), attn_merge_kernel", "batch"
+                kernel, inst = "attn_ts_kernel<5, 6> (all layers in one launch), attn_merge_kernel", "batch"
         traffic, traffic_from = NCU_TRAFFIC[inst] if layers == LAYERS and ctx0 == CTX0 else (None, None)
         achieved = att_bytes / att_us / 1e3  # GB/s
         line = {

@@ -45,7 +45,6 @@
 #include <math_constants.h>
 
 #include "kv_attend_tc_parts.cuh"
-#include "kv_plan.h"
 #include "kv_attend_tc_unpack.cuh"
 #include "kv_unpack.h"
 
@@ -1080,17 +1079,6 @@ cudaError_t preload_attend_tc() {
     return e != cudaSuccess ? e : tc_prepare();
 }
 
-// Which kernel: attn_ts_kernel (kv_attend_ts.cu) has the compiled-in low-bit pairs and wins where a CTA has work for a while; it starts slower, and of
-// q8_0 alone (8 layers of 60,000 positions, 8 tokens: 357 us against 396) attn_tc_kernel stays the faster.
-// Spread over the SMs (groups a CTA, of the context's end rounded up to 640 positions, so that T does not matter; us, attn_tc_kernel / attn_ts_kernel, per
-// layer): 5 groups (20,000 positions, K5r / V5, 5 tokens) 36.2 / 36.3, 6 (24,003, 4 tokens) 37.2 / 36.9, 9 (38,000, K5r / V6, 8) 52.5 / 48.4.
-// Item by item (groups of a CTA's items): 2 (3,000, K6 / V5, 5 tokens, one layer) 20.6 / 22.6, up to 3 (6 sequences of 442 .. 4,469) 29.9 / 30.8, 8 (20,011, 2 tokens,
-// one layer) 37.4 / 35.5, 17 (16 layers of 3,000, 2 tokens) 82.6 / 80.2, 20 sequences of 900 .. 12,000 (4 layers) 277 / 267.
-// Contexts whose chunks are one group (up to 2,560 positions) stay: there the layers' outputs are the same bits one by one and together.
-constexpr int TS_GROUPS_SPREAD = 6, TS_GROUPS_BATCH = 5;
-static TcKernel ts_long(int kb, int vb, bool batch, int groups) {
-    return groups >= (batch ? TS_GROUPS_BATCH : TS_GROUPS_SPREAD) ? tc::ts_kernel_for(kb, vb, batch) : nullptr;
-}
 cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, float2 * ml, int part_slots, unsigned long long * xa,
                              unsigned long long * xb, int nbmax, int epoch, int * status, cudaStream_t stream, const AttnTask * tasks_dev,
                              int ntasks, int tasks_B, float * raw_part, float2 * raw_ml, unsigned long long * prof, unsigned * done,
@@ -1133,10 +1121,7 @@ cudaError_t launch_attend_tc(const AttnJob & job, int num_sms, float * part, flo
     a.done = fused ? done : nullptr;
     a.done_target = fused ? (*done_seq + 1u) * (unsigned) a.cph : 0u;
     void * args[] = {&a};
-    const int kb = job.kv.s[0].bits, vb = job.kv.s[1].bits, groups = (plan_end(job) - job.pos_lo + tc::GP - 1) / tc::GP;
-    const TcKernel ts = ts_long(kb, vb, false, (groups + a.cph - 1) / a.cph), kern = ts ? ts : tc_kernel_for(kb, vb, false);
-    e = cudaLaunchCooperativeKernel((const void *) kern, dim3(NKV * a.cph), dim3(ts ? tc::TS_THREADS_SPREAD : tc::NTHREADS_SPREAD), args,
-                                    ts ? tc::ts_smem_bytes() : attend_tc_smem_bytes(), stream);
+    e = cudaLaunchCooperativeKernel((const void *) tc_kernel_for(job.kv.s[0].bits, job.kv.s[1].bits, false), dim3(NKV * a.cph), dim3(tc::NTHREADS_SPREAD), args, attend_tc_smem_bytes(), stream);
     if (e != cudaSuccess) return e;
     if (fused) {
         *done_seq += 1u;
@@ -1189,9 +1174,14 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     // they gain as soon as CTAs have more than one item (an earlier build: 102 -> 111 us for 16 layers of 4,000 positions).
     const int grid = std::min(nitems, num_sms), per_cta = (nitems + grid - 1) / grid * std::max(first.cpi, 1) * ((first.cs / ATP + tc::GT - 1) / tc::GT);
     const int kb = first.kv.s[0].bits, vb = first.kv.s[1].bits;
-    const TcKernel ts = one_format && first.cs > tc::GP ? ts_long(kb, vb, true, per_cta) : nullptr;
+    // attn_ts_kernel (kv_attend_ts.cu; 5-bit K) where every item is a long run: it starts an item more slowly and runs a group faster. us, attn_tc_kernel /
+    // attn_ts_kernel: 16 layers of 2,700 positions (2 groups an item) 81.5 / 87.2, of 6,000 (3) 106.2 / 110.8, 8 layers of 9,000 (4) 76.0 / 77.4, of 20,011 (8 groups:
+    // the line) 143.9 / 141.1, 2 layers (two items a CTA) 61.8 / 56.4, one (one item a CTA) 36.8 / 36.9, 8 of 38,000 (15) 240.7 / 231.0, 16 of 101,600 (40) 1,017 / 962, 1 token 963 / 888,
+    // one of 8 GPUs' part of 262,136 (22) 389 / 367. Jobs of unequal length stay (32 sequences of 3,063 .. 83,693: 2,096 / 2,130), and so does 6-bit K (8 layers of
+    // 101,600, 8 tokens: 576 / 582).
+    const TcKernel ts = one_format && a.uniform && first.cs >= 8 * tc::GP && per_cta >= 16 ? tc::ts_kernel_for(kb, vb) : nullptr;
     const TcKernel kern = ts ? ts : one_format ? tc_kernel_for(kb, vb, true) : tc::attn_tc_kernel<0, 0, true>;
-    e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(ts ? tc::TS_THREADS_BATCH : tc::NTHREADS), ts ? tc::ts_smem_bytes() : attend_tc_smem_bytes(), stream, a);
+    e = launch_dependent(per_cta <= 20, kern, dim3(grid), dim3(ts ? tc::TS_THREADS : tc::NTHREADS), ts ? tc::ts_smem_bytes() : attend_tc_smem_bytes(), stream, a);
     if (e != cudaSuccess) return e;
     return launch_merge(jobs_dev, &first, njobs, max_T, part, ml, stream, raw_part, raw_ml, true, nitems <= num_sms);
 }

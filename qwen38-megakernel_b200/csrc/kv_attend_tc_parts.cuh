@@ -1,5 +1,4 @@
-// What the two kernels of the tensor-core decode attention share (kv_attend_tc.cu: scores with query rows on tensor-memory lanes; kv_attend_ts.cu:
-// K's operand in tensor memory): launch arguments, mbarrier and tcgen05 wrappers, exponentials, the exchange of running maxima between CTAs, the
+// What the two kernels of the tensor-core decode attention (kv_attend_tc.cu; kv_attend_ts.cu: long runs of 5-bit keys) are built from: launch arguments, mbarrier and tcgen05 wrappers, exponentials, the exchange of running maxima between CTAs, the
 // tasks of a job spread over the grid and the merge in the kernel's tail.
 #pragma once
 #include <cuda_fp16.h>
@@ -288,9 +287,8 @@ template <class Smem> __device__ __forceinline__ void tail_merge(Smem & sm, cons
 
 // ---- kv_attend_ts.cu ----
 typedef void (*TcKernel)(const Args);
-constexpr int TS_THREADS_BATCH = 28 * 32, TS_THREADS_SPREAD = 32 * 32;
-// the instance for a pair of main formats; null: there is none
-TcKernel ts_kernel_for(int kb, int vb, bool batch);
+constexpr int TS_THREADS = 28 * 32;
+TcKernel ts_kernel_for(int kb, int vb); // the instance for a pair of main formats; null: there is none
 size_t ts_smem_bytes();
 cudaError_t ts_for_each(cudaError_t (*f)(TcKernel, size_t smem)); // on every instance, until it fails
 

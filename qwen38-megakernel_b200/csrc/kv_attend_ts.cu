@@ -1,22 +1,23 @@
-// The tensor-core decode attention for long contexts in the low-bit formats: the arithmetic, the modes, the records and the merge are those of
-// attn_tc_kernel (kv_attend_tc.cu); what differs is where operands and scores lie and which warps wait for one another.
+// The tensor-core decode attention for long runs of 5-bit keys, item by item (the batch mode of attn_tc_kernel, kv_attend_tc.cu: the same
+// arithmetic, items, records and partials; attn_merge_kernel afterwards). What differs is where operands and scores lie and which warps wait for
+// one another:
 //   - K's operand lies in tensor memory: its 8 unpack warps write a position's fp16(d q) into the position's lane (tcgen05.st, 16 columns a
-//     block), and S^T[128 positions x 48 rows] = K Q^T takes it from there (Q, K-major, is the B operand). That is 128 KB less through shared
-//     memory a group, no proxy fence, and 26 cycles an instruction instead of the 68 of M = 64, N = 128.
+//     block), and S^T[128 positions x 48 rows] = K Q^T takes it from there (Q, K-major, is the B operand): 128 KB less through shared memory a
+//     group, no proxy fence for K, and 26 cycles an instruction instead of the 68 of M = 64, N = 128.
 //   - K and V have unpack warps, raw slots, operand slots, a producer and an issuer of their own; neither side waits for the other. A warp
 //     unpacks a quarter of a tile's side (2 blocks of either half) instead of an eighth of both sides: half the waits and hand-overs.
-//   - S^T has positions on lanes, so a softmax thread owns a position and 24 of the query rows (8 warps: tile q, half of the rows). A row's tile maximum is
-//     one redux.sync; what belongs to a row (running and reference max, factors) is computed by the thread lane = row from the four tiles' maxima
-//     and read back by all. P is the B operand of P V with rows contiguous.
-// What bounds it: the softmax warps (5,000 of a group's 5,400 cycles busy at 8 tokens, 4,400 at 1, in a chain of short steps), V's unpack warps
-// (4,300 .. 4,700) and behind both the instruction cache, 32 KB: straight code of 32 KB and more runs at a third of the rate (3.1 cycles an
-// instruction and warp against 1.07 below), and the first form of this kernel, with both halves of a side, all waits with their clocks and 48 rows
-// in a softmax warp unrolled, missed it in 44 % of its requests (1,050 lines a group) and took 1,643 us for the step below; with loops over the halves, waits of five
-// instructions and 24 rows a warp 6 % are missed. Hence what looks like thrift: one body for both halves, one for both sides of 8-bit tiles,
-// issue loops unrolled twice, one place for every wait.
-// Measured against attn_tc_kernel (us): 16 layers of 101,600 positions, K5r / V6, 8 tokens 1,076 -> 967, 1 token 1,045 -> 926; 8 layers K5r / V5, 8
-// tokens 593 -> 545, K6 / V5 600 -> 580; one layer of 38,000, 8 tokens, 52.5 -> 48.4. It starts slower (a side's tile has 8 warps, not 16): see
-// the rules at ts_long.
+//   - S^T has positions on lanes, so a softmax thread owns a position and 24 of the query rows (8 warps: tile q, half of the rows). A row's tile
+//     maximum is one redux.sync; what belongs to a row (running and reference max, factors) is computed by the thread lane = row from the four
+//     tiles' maxima and read back by all. P is the B operand of P V with rows contiguous.
+// What bounds it: the softmax warps (5,000 of a group's 5,400 cycles busy at 8 tokens, 4,400 at 1, in a chain of short steps through shared
+// memory), V's unpack warps (4,300 .. 4,700) and behind both the instruction cache, 32 KB: straight code that does not fit runs at a third of the
+// rate (3.1 cycles an instruction and warp, 1.07 where it fits). The first form, with both halves of a side, every wait's clock and 48 rows a
+// softmax warp in line, missed in 44 % of its requests and took 1,643 us for the 1,076 of attn_tc_kernel (16 layers of 101,600 positions, 8 tokens);
+// with loops over the halves, waits of five instructions and 24 rows a warp it misses 6 % and takes 963. Hence what looks like thrift: one body for both
+// halves, one for both sides of 8-bit tiles, issue loops unrolled twice. Tried and slower: the maxima in four warps of their own (1,111), four blocks of a
+// side through one body (1,158), two sets of softmax warps taking the groups in turn, a round without data to warm the cache, K's first
+// tile shared with V's warps, 64 registers for the unpack warps (1,027), shuffles instead of redux.sync (+1 .. 4 %).
+// Where it is used, and what both kernels take: launch_attend_tc_batch.
 #include <cuda_fp16.h>
 #include <math_constants.h>
 
@@ -34,19 +35,14 @@ constexpr int NDQ = 16;        // then the unpack warps: 8 c2 + 4 side + q: side
 constexpr int NSIDE = NDQ / 2; // unpack warps of a side
 // then the control warps: a producer and an issuer for either side of the pipeline, which share nothing but the groups' records
 constexpr int W_CTL = NSOFT + NDQ, W_KPROD = W_CTL, W_VPROD = W_CTL + 1, W_SISSUE = W_CTL + 2, W_OISSUE = W_CTL + 3;
-constexpr int W_MAX = W_CTL + 4;      // spread mode only: four warps that take the tile maxima and exchange the running maxima
-constexpr int NTHREADS = TS_THREADS_BATCH, NTHREADS_SPREAD = TS_THREADS_SPREAD;
-static_assert(NTHREADS == W_MAX * 32 && NTHREADS_SPREAD == (W_MAX + 4) * 32, "warps");
+constexpr int NTHREADS = TS_THREADS;
+static_assert(NTHREADS == (W_CTL + 4) * 32, "warps");
 // registers per thread after the reallocation (the launch gives 65536 / NTHREADS rounded down to 8; the three shares sum to at
 // most the CTA's launch allocation -- a larger sum faults)
 #define MKKV_TC_REGS_SOFT "112"
 #define MKKV_TC_REGS_DQ "56"
 #define MKKV_TC_REGS_CTL "56"
 static_assert(NTHREADS == 896 && 8 * 112 + 16 * 56 + 4 * 56 <= 28 * 72, "register shares");
-#define MKKV_TC_REGS_SOFT_SPREAD "88"
-#define MKKV_TC_REGS_CTL_SPREAD "56"
-#define MKKV_TC_REGS_MAX "56"
-static_assert(NTHREADS_SPREAD == 1024 && 8 * 88 + 16 * 56 + 4 * 56 + 4 * 56 <= 32 * 64, "register shares");
 constexpr int TROWS = RS + 32;              // (a warp's lanes reach beyond the last row)
 constexpr int RAW_SLOT = ATP * HD + ATP * SCALE_ROW; // one tile of the widest format and its scales: 8704 bytes
 constexpr int OP_SLOT = GP * 128 * 2;       // V's fp16 operand: 128 positions x 128 dims
@@ -61,8 +57,8 @@ constexpr int P_ROWGROUP = GP * 16;
 constexpr unsigned S_COL = 0, K_COL = S_COL + NSB * AR, K_STRIDE = 64, O_COL0 = K_COL + NKS * K_STRIDE, O_COL1 = O_COL0 + 2 * AR, TMEM_COLS = 512;
 static_assert(O_COL1 + 2 * AR <= TMEM_COLS, "tensor-memory columns");
 static_assert(Q_BYTES == QP_HEAD_BYTES, "the staged query block of a kv head");
-// A group's task record as K's producer leaves it for the other roles. The fields behind AttnTask serve the batch mode, where one CTA works for
-// several (job, kv head) pairs in turn: a segment is a run of chunks of one pair, with its own queries, partial and row sums.
+// A group's task record as K's producer leaves it for the other roles. A CTA works for several (job, kv head) pairs in turn: a segment is a run of chunks of
+// one pair, with its own queries, partial and row sums.
 struct alignas(16) GroupRec : AttnTask {
     const uint16_t * q;       // the segment's staged queries
     int n, T;                 // of the segment's job
@@ -79,12 +75,11 @@ struct Smem {
     uint8_t q[Q_BYTES];         // [dim group 32][row group 6][8 rows][8 dims]
     uint8_t p[2][P_PART];       // high part, low part: [row group 6][position group 16][8 positions][8 rows]
     unsigned tmem_base;
-    int merge_ok;               // the tail's merge: the head's CTAs have all arrived
     WaitCtl wc;                 // the launch's wait limits; dead: a wait of this CTA gave up, no later wait blocks
     GroupRec tasks[NTASK];      // the CTA's groups as K's producer reaches them, by group % NTASK (no role is that far from it: its group j + 1
                                 // is fetched when K(j) has been read, which is behind S(j - 3), which is behind the softmax of j - 3 - NSB)
     uint64_t raw_full[2][GT], raw_empty[2][GT], k_full[NKS], k_empty[NKS], op_full[NOP], op_empty[NOP], s_full[NSB], s_empty[NSB], p_full, p_empty, q_ready, fin[2];
-    AttnJob job;
+    AttnJob job;                // the producer's copy of the current segment's job
     unsigned udesc[NTASK][2][GT]; // K / V tiles of a group, by group % NTASK (see UD_ROWS)
     TileSrc vsrc[NTASK][GT];    // the V tiles of the groups whose K has been fetched
     uint64_t rec_full[NTASK];   // record (group % NTASK) is written
@@ -94,9 +89,6 @@ struct Smem {
         uint16_t bh[32], bl[32];       // and beta as two fp16 parts
     } row[NSOFT];
     float lsum[GT][AR];         // a finished segment's row sums over a warp's positions
-    // spread mode only
-    float m_in[NSB][TROWS];        // the running max before a group, by group % NSB
-    uint64_t m_full[NSB];
 };
 
 // The last copy of a producer lane must land before the CTA's shared memory is released, also when a consumer gives up after the producer
@@ -226,7 +218,7 @@ __device__ __forceinline__ void v_producer(Smem & sm, const Args & a, int G, int
     if (lane < GT) drain_copy(&sm.raw_full[1][lane], last_copy);
 }
 
-// ---- batch mode: K's producer warp ----
+// ---- K's producer warp ----
 // Walks the CTA's segments and their groups, fetches K and leaves every group's record before it; lanes 0 .. 3 fetch one tile of the group
 // each. V's producer follows the records. An item is a run of cpi chunks of one
 // kv head of one job and makes one segment and one partial (slot: the job's item0 + g nch + run). Items come in descending order of
@@ -350,30 +342,18 @@ __device__ __forceinline__ void tile_maxima(const float (&s)[RS], int rows, int 
         }
 }
 
-// KB / VB: the bits of the K / V main rows the instance is compiled for (0: any, decided per tile at run time). A compiled-in
-// format leaves two unpack bodies per side (the format and the q8_0 ring) instead of five: a smaller instruction footprint.
-// BATCH: the instance for several jobs (persistent CTAs over runs of chunks, no exchange between CTAs); the instance for one
-// job spread over the SMs carries none of that mode's code (with both modes in one body the spread mode's loops came out 1.7 %
-// slower).
-template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? NTHREADS : NTHREADS_SPREAD, 1) attn_ts_kernel(const __grid_constant__ Args a) {
+// KB / VB: the bits of the K / V main rows. Persistent CTAs over runs of chunks, one per SM; no CTA waits for another.
+template <int KB, int VB> __global__ void __launch_bounds__(NTHREADS, 1) attn_ts_kernel(const __grid_constant__ Args a) {
     // (the dynamic shared memory starts on a 128-byte boundary -- there is no static shared memory in this kernel --, which is all the
     // bulk copies, matrix descriptors and barriers need; no pointer arithmetic here, so every access below is a shared-space one)
     extern __shared__ __align__(128) uint8_t smem_raw[];
     Smem & sm = *reinterpret_cast<Smem *>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#if MKKV_TC_PROF
-    const unsigned long long t_entry = globaltimer_ns();
-#endif
-    if (!BATCH) {
-        const unsigned * src = reinterpret_cast<const unsigned *>(&a.one);
-        unsigned * dst = reinterpret_cast<unsigned *>(&sm.job);
-        for (int i = tid; i < (int) (sizeof(AttnJob) / 4); i += NTHREADS_SPREAD) dst[i] = src[i];
-    }
     if (tid == 0) {
         for (int s = 0; s < 2 * GT; s++) { mbar_init(&sm.raw_full[s / GT][s % GT], 1); mbar_init(&sm.raw_empty[s / GT][s % GT], NSIDE / GT); }
         for (int s = 0; s < NKS; s++) { mbar_init(&sm.k_full[s], NSIDE); mbar_init(&sm.k_empty[s], 1); }
         for (int s = 0; s < NOP; s++) { mbar_init(&sm.op_full[s], NSIDE); mbar_init(&sm.op_empty[s], 1); }
-        for (int s = 0; s < NSB; s++) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.s_empty[s], BATCH ? NSOFT : NSOFT + 4); mbar_init(&sm.m_full[s], 4); }
+        for (int s = 0; s < NSB; s++) { mbar_init(&sm.s_full[s], 1); mbar_init(&sm.s_empty[s], NSOFT); }
         mbar_init(&sm.p_full, NSOFT);
         mbar_init(&sm.p_empty, 1);
         for (int s = 0; s < 2; s++) mbar_init(&sm.fin[s], 1);
@@ -391,169 +371,35 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
     }
     __syncthreads();
     tc_fence_after();
-    if (BATCH) { // (the prologue above ran beside the launch before this one; every CTA of this launch is resident: at most one per SM)
-        release_next();
-        if (warp != W_KPROD) wait_previous(); // (K's producer warp: batch_producer)
-    }
+    // (the prologue above ran beside the launch before this one; every CTA of this launch is resident: at most one per SM)
+    release_next();
+    if (warp != W_KPROD) wait_previous(); // (K's producer warp: batch_producer)
     const unsigned tb = sm.tmem_base;
-    const AttnJob & J = sm.job;
-    const KvView & kv = J.kv;
-    // spread mode: CTA kk of kv head g runs tasks kk, kk + cph, .. of the head; batch mode: the producer walks the CTA's segments
-    // (runs of chunks of one (job, kv head), the groups of a chunk in order with the running max carried in registers) and leaves a
-    // record per group, from which the other roles take everything they need, the end of the CTA's work included
-    constexpr bool batch = BATCH;
-    const int g = batch ? 0 : (int) blockIdx.x / a.cph, kk = batch ? 0 : (int) blockIdx.x % a.cph;
-    const int slot = (int) blockIdx.x, tstep = batch ? 1 : a.cph;
-    const int T = J.T, n = J.n, R = GQ * T, ws = J.ws;
-    Geo4 geo4;
-    geo4.g = make_geo(J, GT);
-    geo4.mul_nch = geo4.g.nch > 1 ? 0xffffffffu / (unsigned) geo4.g.nch + 1u : 0u;
-    geo4.mul_nch1 = geo4.g.nch > 2 ? 0xffffffffu / (unsigned) (geo4.g.nch - 1) + 1u : 0u;
-    const AttnTask * const ttab = a.tasks;
-    const int t_end = ttab ? a.ntasks : geo4.g.ntasks_head;
-    auto get_task = [&](int t) -> Task { return ttab ? ttab[t] : make_task4(geo4, t); };
-    // this CTA's groups: tasks kk, kk + tstep, .. (batch mode: known to a role once it has read the record with REC_END)
-    int G = batch ? 0x7fffffff : kk < t_end ? (t_end - kk + tstep - 1) / tstep : 0;
+    // K's producer walks the CTA's segments (runs of chunks of one (job, kv head), the groups of a chunk in order with the running max carried in
+    // registers) and leaves a record per group, from which the other roles take everything they need, the end of the CTA's work included
+    int G = 0x7fffffff; // the CTA's groups, known to a role once it has read the record with REC_END
 
     // The kv head's query rows come staged (qprep: fp16 -> fp32 -> K's rotation -> x 1/16 -> fp16 in the K-major B operand's layout,
     // row = (head % 6) T + t): the producer fetches the block with one bulk copy, the issuer waits for it.
     // registers move from the unpack / control warps to the softmax warps
-    if (!BATCH && warp >= W_MAX) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_MAX ";");
-        // ---- spread mode, maxima warps: warp W_MAX + q takes the tile maxima of query rows 16 q .. + 15 (a thread: one row, two of the tiles),
-        // publishes each group's, collects the running max before it and leaves both for the softmax warp of the same rows. Tile maxima
-        // run ahead of P, so that a group's own maxima are published well before the CTAs that hold the chunk's next groups need them: the
-        // CTAs of a kv head may drift apart by a group without a poll having to wait. The lead grows from none (the first P needs only
-        // its own group's scores) to MAX_AHEAD groups. (In the softmax warps, between one P and the next, maxima and polls took 2,900 of a
-        // group's 7,800 cycles: one layer of 101,600 positions 111 us, 103 with warps of their own, 99.6 with the words polled together.) ----
-        const int q = warp & 3, hf = lane >> 4, r_own = 16 * q + (lane & 15);
-        const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
-        const bool st = q == 0, act = q < 3 && 16 * q < R, pub = act && !hf && r_own < R;
-        (void) st;
-        auto xbase = [&](const Task & k) -> size_t { return (((size_t) g * ATT_NCH + k.c) * a.nbmax) * AR + r_own; };
-        // the exchange arrays are only touched by a CTA that has not given up (after a give-up the task records of groups the
-        // producer never reached are not valid) and only inside their bounds
-        auto exch_ok = [&](const Task & k) -> bool { return !sm.wc.dead && (unsigned) k.c < (unsigned) ATT_NCH && (unsigned) k.b < (unsigned) a.nbmax; };
-        unsigned long long w[3] = {0ull, 0ull, 0ull};
-        // the words of the groups one and two before, and the cumulative one of the group three before
-        auto words = [&](const Task & k, const unsigned long long * (&src)[3]) {
-            const size_t xb0 = xbase(k);
-            src[0] = k.b >= 1 ? a.xa + xb0 + (size_t) (k.b - 1) * AR : nullptr;
-            src[1] = k.b >= 2 ? a.xa + xb0 + (size_t) (k.b - 2) * AR : nullptr;
-            src[2] = k.b >= 3 ? a.xb + xb0 + (size_t) (k.b - 3) * AR : nullptr;
-        };
-        // tile maxima of group j, its own maxima published
-        auto maxima = [&](int j) {
-            if (st) TC_STAMP(j, 0);
-            tc_wait(&sm.s_full[j % NSB], (j / NSB) & 1, &sm.wc);
-            const GroupRec & k = sm.tasks[j % NTASK];
-            if (st) TC_STAMP(j, 1);
-            tc_fence_after();
-#pragma unroll 1
-            for (int row0 = 0; row0 < R; row0 += RS) {
-                float s[RS];
-                tmem_scores(lane_addr + S_COL + AR * (j % NSB) + row0, s);
-                if (k.flags & REC_MASK) mask_scores(k, n, T, q, row0, lane, s);
-                tile_maxima(s, R - row0, lane, &sm.tmax[j % NSB][q][row0]);
-            }
-            tc_fence_before();
-            __syncwarp();
-            warp_arrive(&sm.s_empty[j % NSB], lane);
-            named_bar(3, 4 * 32); // (the four tiles' maxima are there)
-            const float(&x)[GT][TROWS] = sm.tmax[j % NSB];
-            const float group = pub ? fmaxf(fmaxf(x[0][r_own], x[1][r_own]), fmaxf(x[2][r_own], x[3][r_own])) : 0.f;
-            if (pub && k.nb > 1 && k.b + 1 < k.nb && exch_ok(k))
-                __stcg(a.xa + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(group));
-            if (st) TC_STAMP(j, 2);
-        };
-        // the words the running max of group k will need: requested one phase before they are used, when the CTAs that hold
-        // the chunk's previous groups have most likely published them
-        auto request_words = [&](const Task & k) {
-            if (pub && k.nb > 1 && exch_ok(k)) {
-                const unsigned long long * src[3];
-                words(k, src);
-#pragma unroll
-                for (int x = 0; x < 3; x++)
-                    if (src[x]) w[x] = __ldcv(src[x]);
-            }
-        };
-        constexpr int MAX_AHEAD = 2;
-        static_assert(MAX_AHEAD + 1 < NSB, "S of the groups ahead stays until their P");
-        int maxima_done = 0;
-        for (int i = 0; i < G; i++) {
-            const int want = min(G, i + 1 + min(i, MAX_AHEAD));
-            while (maxima_done < want) maxima(maxima_done++);
-            const GroupRec & k = sm.tasks[i % NTASK];
-            float m_in = -CUDART_INF_F;
-            if (pub && k.nb > 1 && exch_ok(k)) {
-                const unsigned long long * src[3];
-                words(k, src);
-                poll_words(src, w, a.epoch, &sm.wc, a.status);
-#pragma unroll
-                for (int x = 0; x < 3; x++)
-                    if (src[x]) m_in = fmaxf(m_in, __uint_as_float((unsigned) w[x]));
-                if (k.b + 3 < k.nb) {
-                    const float(&x)[GT][TROWS] = sm.tmax[i % NSB];
-                    const float M = fmaxf(fmaxf(m_in, fmaxf(x[0][r_own], x[1][r_own])), fmaxf(x[2][r_own], x[3][r_own]));
-                    __stcg(a.xb + xbase(k) + (size_t) k.b * AR, ((unsigned long long) (unsigned) a.epoch << 32) | __float_as_uint(M));
-                }
-            }
-            if (st) TC_STAMP(i, 7);
-            if (act && !hf) sm.m_in[i % NSB][r_own] = m_in;
-            __syncwarp();
-            warp_arrive(&sm.m_full[i % NSB], lane);
-            if (i + 1 < maxima_done) { // (the next group's task record is known to be written: its scores have been waited for)
-                request_words(sm.tasks[(i + 1) % NTASK]);
-            } else {
-                w[0] = w[1] = w[2] = 0ull; // (no early request: the polls fetch the words themselves)
-            }
-        }
-    } else if (warp >= W_CTL) {
-    if constexpr (BATCH) asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
-    else asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL_SPREAD ";");
+    if (warp >= W_CTL) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 " MKKV_TC_REGS_CTL ";");
     if (warp == W_KPROD) {
-        if constexpr (BATCH) {
-            batch_producer(sm, a, lane);
-        } else {
-        if (lane == 0) { // the queries first
-            mbar_expect_tx(&sm.q_ready, Q_BYTES);
-            bulk_g2s(sm.q, reinterpret_cast<const uint8_t *>(J.Qp) + (size_t) g * Q_BYTES, Q_BYTES, &sm.q_ready);
-        }
-        const int side = (lane >> 2) & 1, tile = lane & 3;
-        const SideSrc src = make_src(kv, side, g, ws);
-        LastCopy last_copy;
-        for (int j = 0; j < G; j++) { // a group's task is computed here, once, and left for the other roles
-            const Task k = get_task(kk + j * tstep);
-            if (lane == 0) {
-                GroupRec & rec = sm.tasks[j % NTASK];
-                static_cast<AttnTask &>(rec) = k;
-                rec.flags = k.pos0 + GP > min(k.c1, n + 1) ? REC_MASK : 0; // (of a table's tasks, too: their c1 is their piece's end)
-            }
-            const TileSrc t = describe_tile(sm, j, src, side, tile, k.pos0 + tile * ATP, k.nt, k.c1, 0u, lane);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.rec_full[j % NTASK]);
-            if (!fetch_tile(sm, a, 0, j, k.nt, t, lane, last_copy)) break;
-        }
-        watch_end(sm, a, lane);
-        if (lane < GT) drain_copy(&sm.raw_full[0][lane], last_copy);
-        if (lane == 0) // (the query block too: the issuer may give up on it)
-            wait_landed(&sm.q_ready, 0u);
-        }
+        batch_producer(sm, a, lane);
     } else if (warp == W_VPROD) {
         v_producer(sm, a, G, lane);
     } else if (warp == W_SISSUE) {
         // ---- S^T(j) = K Q^T, as K's operand slots fill ----
         if (elect_one()) { // (with lane == 0 as the test an instruction took 50 % longer to issue: see elect_one)
-            if (!batch) tc_wait(&sm.q_ready, 0u, &sm.wc); // the queries are staged
-            // batch mode: the queries of the segment that opens with group k, fetched as soon as the last S of the segment before is
+            // The queries of the segment that opens with group k, fetched as soon as the last S of the segment before is
             // complete: they arrive while P V of an earlier group runs
-            bool q_next = batch, q_flight = false;
+            bool q_next = true, q_flight = false;
             unsigned q_ph = 0;
             const unsigned q_lo = desc_lo(smem_u32(sm.q), AR / 8 * 128), hi_128 = desc_hi(128); // (8-row groups 128 bytes apart)
             unsigned ks = 0, kph = 0;
             for (int j = 0; j < G && !sm.wc.dead; j++) {
                 const int sb = j % NSB;
-                if (batch && q_next) {
+                if (q_next) {
                     tc_wait(&sm.rec_full[j % NTASK], (j / NTASK) & 1, &sm.wc);
                     if (j > 0) tc_wait(&sm.s_full[(j - 1) % NSB], ((j - 1) / NSB) & 1, &sm.wc);
                     if (sm.wc.dead) break;
@@ -562,7 +408,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                     q_flight = true, q_next = false;
                 }
                 if (j >= NSB) tc_wait(&sm.s_empty[sb], ((j / NSB) - 1) & 1, &sm.wc);
-                if (batch && q_flight) {
+                if (q_flight) {
                     tc_wait(&sm.q_ready, q_ph, &sm.wc);
                     if (sm.wc.dead) break;
                     q_ph ^= 1, q_flight = false;
@@ -580,16 +426,14 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                     if (++ks == NKS) ks = 0, kph ^= 1;
                 }
                 umma_commit(&sm.s_full[sb]);
-                if (batch) { // (the record was written before the group's K was fetched)
-                    const int fl = sm.tasks[j % NTASK].flags;
-                    if (sm.wc.dead) break;
-                    if (fl & REC_END) G = j + 1;
-                    q_next = (fl & REC_LAST) != 0;
-                }
+                const int fl = sm.tasks[j % NTASK].flags; // (the record was written before the group's K was fetched)
+                if (sm.wc.dead) break;
+                if (fl & REC_END) G = j + 1;
+                q_next = (fl & REC_LAST) != 0;
             }
             // every instruction issued above is complete before the tensor memory is freed and the CTA's shared memory released
             // (bounded; in a normal run the softmax warps have already waited for the last one)
-            if (batch && q_flight) // (given up with the query block in flight: it lands before the CTA's shared memory is released)
+            if (q_flight) // (given up with the query block in flight: it lands before the CTA's shared memory is released)
                 wait_landed(&sm.q_ready, q_ph);
             umma_commit(&sm.fin[0]);
             wait_landed(&sm.fin[0], 0u);
@@ -608,8 +452,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
                 TC_STAMP(j, 17);
 #endif
                 if (sm.wc.dead) break;
-                const int fl = batch ? sm.tasks[j % NTASK].flags : 0;
-                const bool fresh = batch ? (fl & REC_FIRST) != 0 : j == 0; // O^T starts from zero
+                const int fl = sm.tasks[j % NTASK].flags;
+                const bool fresh = (fl & REC_FIRST) != 0; // O^T starts from zero
                 if (fl & REC_END) G = j + 1;
 #pragma unroll 1
                 for (int h = 0; h < 2; h++) {
@@ -762,14 +606,10 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             else if (side) v_tile(IntC<VB>{}, valid);
             else k_tile(IntC<KB>{}, valid);
             if (st) TC_STAMP(j, side ? 10 : 13);
-            if (batch && (ud & UD_END)) break;
+            if (ud & UD_END) break;
         }
     } else {
-        if constexpr (BATCH) asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT_SPREAD ";");
-#if MKKV_TC_PROF
-        const unsigned long long t_loop = globaltimer_ns();
-#endif
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 " MKKV_TC_REGS_SOFT ";");
         // ---- softmax warps: warp 4 c + q holds tile q of a group and rows RS c .. of the query rows, a thread one position. What belongs to a row --
         // the running max, the reference max -- is kept by thread lane = row - RS c of the four warps c alike, computed once per group from
         // the four tiles' maxima, and handed to the threads of a warp through shared memory; a thread's sums of its positions' weights are registers,
@@ -779,27 +619,25 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
         const bool st = warp == 0;
         auto & tab = sm.row[warp];
-        float m_acc = -CUDART_INF_F, carry = -CUDART_INF_F; // row row0 + lane: reference max, running max (batch mode)
+        float m_acc = -CUDART_INF_F, carry = -CUDART_INF_F; // row row0 + lane: reference max, running max
         F2 l_acc[RS / 2]; // rows row0 + (2 i, 2 i + 1)
 #pragma unroll
         for (int i = 0; i < RS / 2; i++) l_acc[i] = 0ull;
-        // batch mode: the partial of a finished segment (O^T lanes are dims in the unpacked units' order, columns are query rows), read
+        // the partial of a finished segment (O^T lanes are dims in the unpacked units' order, columns are query rows), read
         // out when its last P V is complete and before the next P allows the MMA that overwrites O^T: between the two the tensor cores
         // stand still, so the next group's exponentials are computed first
         int flush_slot = -1, flush_rows = 0;
         const int prow = ATP * q + lane, pdim = (prow & ~7) | unit_perm(prow & 7);
-        auto read_out = [&](int to_slot, int rows, bool any) { // (of all rows: either set of warps reads one half of the dims)
+        auto read_out = [&](int to_slot, int rows) { // (of all rows: either set of warps reads one half of the dims)
 #pragma unroll 1
             for (int r0 = 0; r0 < rows; r0 += 8) {
                 unsigned v[8], w[8];
-                if (any) {
-                    const unsigned col = lane_addr + (half ? O_COL1 : O_COL0) + r0;
-                    tmem_ld8_two(col, col + AR, v, w);
-                }
+                const unsigned col = lane_addr + (half ? O_COL1 : O_COL0) + r0;
+                tmem_ld8_two(col, col + AR, v, w);
                 float * dst = a.part + ((size_t) to_slot * AR + r0) * HD + 128 * half + pdim;
 #pragma unroll
                 for (int j = 0; j < 8; j++)
-                    if (r0 + j < rows) dst[j * HD] = any ? __uint_as_float(v[j]) + __uint_as_float(w[j]) : 0.f;
+                    if (r0 + j < rows) dst[j * HD] = __uint_as_float(v[j]) + __uint_as_float(w[j]);
             }
         };
         // the segment's row sums and maxima (the four warps of the rows)
@@ -899,8 +737,8 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 #if MKKV_TC_PROF
             if (moved && a.prof && st && lane == 0) a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 15] += 1ull;
 #endif
-            if (batch && __builtin_expect(flush_slot >= 0, 0)) { // (a segment's first group: no reference max moves at it)
-                read_out(flush_slot, flush_rows, true);
+            if (__builtin_expect(flush_slot >= 0, 0)) { // (a segment's first group: no reference max moves at it)
+                read_out(flush_slot, flush_rows);
                 flush_slot = -1;
             } else if (__builtin_expect(moved != 0u, 0)) { // bring the accumulator columns of the rows whose reference max moved (one, as a rule) to the new reference: a row is one
                          // column in each of the four blocks (two halves x high / low part); the four loads of a row are in flight together
@@ -939,90 +777,45 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
             if (st) TC_STAMP(i, 6);
         };
 
-        if constexpr (BATCH) {
-            for (int i = 0; i < G; i++) {
-                if (st) TC_STAMP(i, 0);
-                // After a wait that gave up the group's record may not be written: the wait's result is voted on, and the barrier that hands the
-                // maxima out carries the flag, so that the four warps of a set of rows leave together.
-                const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc);
-                if (st) TC_STAMP(i, 1);
-                tc_fence_after();
-                const GroupRec & k = sm.tasks[i % NTASK];
-                const int4 hot = *reinterpret_cast<const int4 *>(&k.flags);
-                const int flags = hot.x, to = hot.y, rows = there ? min(hot.z - row0, RS) : 0;
-                float s[RS];
-                if (rows > 0) tmem_scores(lane_addr + S_COL + AR * (i % NSB) + row0, s);
-                tc_fence_before();
-                __syncwarp();
-                warp_arrive(&sm.s_empty[i % NSB], lane);
-                if (rows > 0) {
-                    if (__builtin_expect(flags & REC_MASK, 0)) mask_scores(k, k.n, k.T, q, row0, lane, s);
-                    tile_maxima(s, rows, lane, &sm.tmax[i % NSB][q][row0]);
-                }
-                if (st) TC_STAMP(i, 2);
-                if (named_bar_or(1 + half, GT * 32, !there || sm.wc.dead != 0)) break;
-                if (st) TC_STAMP(i, 3);
-                softmax(i, rows, carry, (unsigned) flags >> REC_RESTART, [&](float (&x)[RS]) {
-#pragma unroll
-                    for (int c = 0; c < RS; c++) x[c] = s[c];
-                });
-                if (flags & REC_END) G = i + 1;
-                if (!(flags & REC_LAST)) continue;
-                // the segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below)
-                close_rows(to, rows);
-#pragma unroll
-                for (int c = 0; c < RS / 2; c++) l_acc[c] = 0ull;
-                m_acc = -CUDART_INF_F;
-                flush_slot = to, flush_rows = hot.z;
-            }
-            if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
-                tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
-                tc_fence_after();
-                read_out(flush_slot, flush_rows, true);
-            }
-        } else {
-        // tile maxima and incoming running max come from the maxima warps (above)
-        const int rows = min(R - row0, RS);
         for (int i = 0; i < G; i++) {
-            tc_wait(&sm.m_full[i % NSB], (i / NSB) & 1, &sm.wc);
-            tc_wait(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc); // (long since: orders this warp's reads behind the MMA)
+            if (st) TC_STAMP(i, 0);
+            // After a wait that gave up the group's record may not be written: the wait's result is voted on, and the barrier that hands the
+            // maxima out carries the flag, so that the four warps of a set of rows leave together.
+            const bool there = tc_wait_all(&sm.s_full[i % NSB], (i / NSB) & 1, &sm.wc);
+            if (st) TC_STAMP(i, 1);
             tc_fence_after();
-            __syncwarp();
             const GroupRec & k = sm.tasks[i % NTASK];
+            const int4 hot = *reinterpret_cast<const int4 *>(&k.flags);
+            const int flags = hot.x, to = hot.y, rows = there ? min(hot.z - row0, RS) : 0;
+            float s[RS];
+            if (rows > 0) tmem_scores(lane_addr + S_COL + AR * (i % NSB) + row0, s);
+            tc_fence_before();
+            __syncwarp();
+            warp_arrive(&sm.s_empty[i % NSB], lane);
+            if (rows > 0) {
+                if (__builtin_expect(flags & REC_MASK, 0)) mask_scores(k, k.n, k.T, q, row0, lane, s);
+                tile_maxima(s, rows, lane, &sm.tmax[i % NSB][q][row0]);
+            }
+            if (st) TC_STAMP(i, 2);
+            if (named_bar_or(1 + half, GT * 32, !there || sm.wc.dead != 0)) break;
             if (st) TC_STAMP(i, 3);
-            if (rows <= 0) warp_arrive(&sm.s_empty[i % NSB], lane);
-            softmax(i, rows, sm.m_in[i % NSB][row0 + lane], 0u, [&](float (&x)[RS]) {
-                tmem_scores(lane_addr + S_COL + AR * (i % NSB) + row0, x);
-                tc_fence_before();
-                __syncwarp();
-                warp_arrive(&sm.s_empty[i % NSB], lane); // (the last read of this S buffer and of the group's maxima)
-                if (k.flags & REC_MASK) mask_scores(k, n, T, q, row0, lane, x);
+            softmax(i, rows, carry, (unsigned) flags >> REC_RESTART, [&](float (&x)[RS]) {
+#pragma unroll
+                for (int c = 0; c < RS; c++) x[c] = s[c];
             });
+            if (flags & REC_END) G = i + 1;
+            if (!(flags & REC_LAST)) continue;
+            // the segment's row sums and maxima are complete (its accumulator follows with the next group's P, or below)
+            close_rows(to, rows);
+#pragma unroll
+            for (int c = 0; c < RS / 2; c++) l_acc[c] = 0ull;
+            m_acc = -CUDART_INF_F;
+            flush_slot = to, flush_rows = hot.z;
         }
-        if (G > 0) {
+        if (flush_slot >= 0) { // (every P of the CTA is out: the last P V)
             tc_wait(&sm.p_empty, (G - 1) & 1, &sm.wc);
             tc_fence_after();
-            __syncwarp();
-        }
-#if MKKV_TC_PROF
-        if (warp == 0) { // the tail's stamps go to group slot 15 (stamps 8 .. 13, after the main loop's own use of them)
-            if (a.prof && lane == 0) {
-                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 8] = t_entry;
-                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 9] = t_loop;
-                unsigned smid;
-                asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-                a.prof[((size_t) blockIdx.x * 16 + 15) * 20 + 14] = smid; // (which SM ran this CTA)
-            }
-            TC_STAMP(15, 10);
-        }
-#endif
-        // (a CTA without groups: zeros, with a reference of minus infinity)
-        read_out(slot, R, G > 0);
-        close_rows(slot, rows);
-#if MKKV_TC_PROF
-        if (warp == 0) TC_STAMP(15, 11);
-#endif
-        if (a.done) tail_merge(sm, a, g, kk, T, warp, lane);
+            read_out(flush_slot, flush_rows);
         }
     }
     tc_fence_before();
@@ -1032,21 +825,14 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
 
 } // namespace ts
 
-TcKernel ts_kernel_for(int kb, int vb, bool batch) {
-    if (kb == 5 && vb == 6) return batch ? ts::attn_ts_kernel<5, 6, true> : ts::attn_ts_kernel<5, 6, false>;
-    if (kb == 5 && vb == 5) return batch ? ts::attn_ts_kernel<5, 5, true> : ts::attn_ts_kernel<5, 5, false>;
-    if (kb == 6 && vb == 5) return batch ? ts::attn_ts_kernel<6, 5, true> : ts::attn_ts_kernel<6, 5, false>;
-    return nullptr;
-}
+TcKernel ts_kernel_for(int kb, int vb) { return kb != 5 ? nullptr : vb == 6 ? ts::attn_ts_kernel<5, 6> : vb == 5 ? ts::attn_ts_kernel<5, 5> : nullptr; }
 size_t ts_smem_bytes() { return sizeof(ts::Smem) + 128; }
 static_assert(sizeof(ts::Smem) + 128 <= 232448, "shared memory of one CTA");
 cudaError_t ts_for_each(cudaError_t (*f)(TcKernel, size_t)) {
-    static const int formats[][2] = {{5, 6}, {5, 5}, {6, 5}};
-    for (const int(&b)[2] : formats)
-        for (int batch = 0; batch < 2; batch++) {
-            const cudaError_t e = f(ts_kernel_for(b[0], b[1], batch != 0), ts_smem_bytes());
-            if (e != cudaSuccess) return e;
-        }
+    for (int vb : {5, 6}) {
+        const cudaError_t e = f(ts_kernel_for(5, vb), ts_smem_bytes());
+        if (e != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
