@@ -33,10 +33,12 @@
 //     order with the running max carried in registers and started anew at a chunk's first tile (a group may hold tiles of several
 //     chunks: with groups that ended with their chunk, half of each was padding at 1,187 positions and 16 layers took 47.5 us instead
 //     of 37.3), no exchange; attn_merge_kernel afterwards. The copies, the unpacking and S of the next item run on while the softmax
-//     warps finish the one before. What bounds it: a group costs 3.0 us of CTA time at any length, most of it the unpack warps'
-//     instructions, an item about 2 us more.
+//     warps finish the one before. What bounds it: a group costs 2.9 us of CTA time at any length, most of it the unpack warps'
+//     instructions, an item about 2 us more. (Long runs of 5-bit keys: kv_attend_ts.cu.)
 //     Per layer of a 16-layer step (K5r / V6), one launch against 16 spread launches: 1,187 positions, 1 token 2.2 us against 18.8;
-//     101,600, 8 tokens 69 (the same cache in every step) .. 74 (another cache each step) against 100.
+//     101,600, 8 tokens 64 against 88.
+// The hot code has to be small: it misses the 32 KB instruction cache in 14 % of its requests (10 % of the spread instance's since every wait lost its clock and
+// the two halves of a tile share one body: one layer of 101,600 positions 99.6 -> 87.8 us, 60,000 in q8_0 61.9 -> 55.8).
 // Every wait is bounded (about two seconds by default; the limits are launch arguments), then the status word and a CTA-wide
 // flag are set, no later wait of the CTA blocks, the producer waits (bounded) for its copies still in flight, and the kernel
 // runs to its end and frees its tensor memory.
@@ -414,7 +416,7 @@ template <int KB, int VB, bool BATCH> __global__ void __launch_bounds__(BATCH ? 
         // run ahead of P, so that a group's own maxima are published well before the CTAs that hold the chunk's next groups need them: the
         // CTAs of a kv head may drift apart by a group without a poll having to wait. The lead grows from none (the first P needs only
         // its own group's scores) to MAX_AHEAD groups. (In the softmax warps, between one P and the next, maxima and polls took 2,900 of a
-        // group's 7,800 cycles: one layer of 101,600 positions 111 us, 103 with warps of their own, 99.6 with the words polled together.) ----
+        // group's 7,800 cycles: one layer of 101,600 positions 111 us, 103 with warps of their own, 99.6 with the words polled together, each measured then.) ----
         const int q = warp & 3, hf = lane >> 4, r_own = 16 * q + (lane & 15);
         const unsigned lane_addr = tb + ((unsigned) (ATP * q) << 16);
         const bool st = q == 0, act = 16 * q < R, pub = act && !hf && r_own < R;
@@ -1176,7 +1178,7 @@ cudaError_t launch_attend_tc_batch(const AttnJob * jobs_dev, const AttnJob & fir
     const int kb = first.kv.s[0].bits, vb = first.kv.s[1].bits;
     // attn_ts_kernel (kv_attend_ts.cu; 5-bit K) where every item is a long run: it starts an item more slowly and runs a group faster. us, attn_tc_kernel /
     // attn_ts_kernel: 16 layers of 2,700 positions (2 groups an item) 81.5 / 87.2, of 6,000 (3) 106.2 / 110.8, 8 layers of 9,000 (4) 76.0 / 77.4, of 20,011 (8 groups:
-    // the line) 143.9 / 141.1, 2 layers (two items a CTA) 61.8 / 56.4, one (one item a CTA) 36.8 / 36.9, 8 of 38,000 (15) 240.7 / 231.0, 16 of 101,600 (40) 1,017 / 962, 1 token 963 / 888,
+    // the line) 143.9 / 141.1, 2 layers (two items a CTA) 61.8 / 56.4, one (one item a CTA) 34.9 / 36.9, 8 of 38,000 (15) 240.7 / 231.0, 16 of 101,600 (40) 1,017 / 962, 1 token 963 / 888,
     // one of 8 GPUs' part of 262,136 (22) 389 / 367. Jobs of unequal length stay (32 sequences of 3,063 .. 83,693: 2,096 / 2,130), and so does 6-bit K (8 layers of
     // 101,600, 8 tokens: 576 / 582).
     const TcKernel ts = one_format && a.uniform && first.cs >= 8 * tc::GP && per_cta >= 16 ? tc::ts_kernel_for(kb, vb) : nullptr;

@@ -39,14 +39,14 @@ inline int busiest_cta(int nlayers, const AttnJob & j, int ctas) {
 }
 
 // Whether nlayers layers of one step (job j's shape, each) go out as one launch of the tensor-core kernel's batch mode, or one by one
-// in its spread mode. In tenths of a 128-position group's time on one CTA of the batch launch (3.0 us): it takes the busiest CTA's and 43
+// in its spread mode. In tenths of a 128-position group's time on one CTA of the batch launch (3.0 us; 2.8 in attn_ts_kernel): it takes the busiest CTA's and 43
 // for itself, its append and its merge; a spread launch deals a layer's groups over all CTAs, a group there takes 12 (exchange of maxima)
-// and the launch 54 (slowest CTA, merge). Measured (us, batch against spread, K5r / V6, 8 tokens unless said otherwise):
-//   1 layer: 2,900 positions 22.0 / 22.6, 3,700 20.6 / 24.6, 4,096 (q8_0, 1 token) 20.5 / 20.5, 4,097 22.4 / 22.6, 4,900 20.5 / 24.6, 5,111
-//     20.6 / 24.6; from 5,121 on the rule takes the spread mode: 5,130 24.6 / 24.6, 6,390 23.3 / 24.6, 7,600 23.3 / 24.6, 9,003 28.8 / 26.9,
-//     24,003 45.2 / 39.0, 101,600 134 / 103 (two or three groups a chunk: the batch launch is never slower, by up to 1.4 us faster beyond the line)
-//   (9,003 and longer and several layers: measured when the rule was made, two builds earlier.)
-//   2 layers: 13,003 55.5 / 58.5, 38,000 112 / 99, 101,600 258 / 201; 4 layers: 38,000 156 / 193, 101,600 368 / 396; 8 layers: 101,600 598 / 785.
+// and the launch 54 (slowest CTA, merge). Measured (us with the append, batch against spread, K5r / V6, 8 tokens unless said otherwise):
+//   1 layer: 2,900 positions 22.6 / 22.3, 3,700 20.6 / 24.7, 4,096 (q8_0, 1 token) 20.5 / 20.5, 4,900 20.6 / 25.8; from 5,121 on the rule takes the spread
+//     mode: 5,130 24.6 / 26.7, 6,390 24.6 / 26.7, 7,600 24.6 / 26.7, 9,003 28.7 / 29.1, 24,003 44.8 / 39.0, 101,600 129 / 88.5 (two or three groups a chunk: the
+//     batch launch is up to 2.1 us faster from the line to 9,000; the line stays where a call's launches and bits have changed before).
+//   2 layers: 13,003 53.7 / 57.9, 38,000 104 / 90, 101,600 240 / 173; 4 layers: 13,003 73 / 113, 38,000 148 / 172, 101,600 346 / 336; 8 layers: 101,600 552 / 660.
+//   (The constants are fits of an earlier build, whose spread group took 12 instead of today's 10.3: 4 layers beyond 97,280 positions are 1 .. 3 % on the wrong side.)
 // Contexts whose chunks are one group (up to 2,560 positions) always take the batch mode: there the layers' outputs are the same bits one
 // by one and together. Beyond, the two modes' outputs differ by rounding (about 1e-7, relative 2-norm).
 inline bool items_mode(int nlayers, AttnJob j, int sms) {
